@@ -109,6 +109,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// What is left of two numbers when their bfloat16 roundings (`packed`) are taken off, as bfloat16.
+__device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
+    return pack_bf16(lo - __uint_as_float(packed << 16), hi - __uint_as_float(packed & 0xffff0000u));
+}
+
 // Keys j0 .. j0+63 of one request and key/value head into shared memory, asynchronously: rows
 // [KB][DP+PAD] and [KB][DVP+PAD].  Rows outside lo..hi and the kept first keys become zeros (they may hold
 // anything in the pages, or have none).  The caller commits the group and waits for it.
@@ -174,7 +179,7 @@ __device__ __forceinline__ void load_q(uint32_t (&qf)[DP / 16][4], const bf16* q
 // One warp, its 16 rows, NT * 8 keys of the block in shared memory starting at key `k_first`:
 // scores, masks, the running maximum and sum, and O += P V.  pos/lo: the two rows' own last and first
 // visible key (pos < 0: a row without a token); keys below `keep` are visible too.
-template <int DP, int DVP, int NT>
+template <int DP, int DVP, int NT, bool FULL_P>
 __device__ __forceinline__ void attend(const uint32_t (&qf)[DP / 16][4], const bf16* ks, const bf16* vs, int k_first,
                                        int j_first, const int (&pos)[2], const int (&lo)[2], bool all_visible,
                                        float scale_log2, float (&m)[2], float (&l)[2], float (&o)[DVP / 8][4], int lane,
@@ -265,12 +270,23 @@ __device__ __forceinline__ void attend(const uint32_t (&qf)[DP / 16][4], const b
         a[1] = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
         a[2] = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]);
         a[3] = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+        uint32_t rest[4];                                  // what rounding took off the weights
+        if (FULL_P) {
+            rest[0] = pack_rest(s[2 * kk][0], s[2 * kk][1], a[0]);
+            rest[1] = pack_rest(s[2 * kk][2], s[2 * kk][3], a[1]);
+            rest[2] = pack_rest(s[2 * kk + 1][0], s[2 * kk + 1][1], a[2]);
+            rest[3] = pack_rest(s[2 * kk + 1][2], s[2 * kk + 1][3], a[3]);
+        }
 #pragma unroll
         for (int n = 0; n < DVP / 8; n += 2) {
             uint32_t b[4];
             ldsm4_t(b, vs + (k_first + kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * (DVP + PAD) + n * 8 + (lane >> 4) * 8);
             mma16816(o[n], a, b[0], b[1]);
             mma16816(o[n + 1], a, b[2], b[3]);
+            if (FULL_P) {
+                mma16816(o[n], rest, b[0], b[1]);
+                mma16816(o[n + 1], rest, b[2], b[3]);
+            }
         }
     }
 }
@@ -278,7 +294,7 @@ __device__ __forceinline__ void attend(const uint32_t (&qf)[DP / 16][4], const b
 __device__ __forceinline__ float logistic(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // ---- portions of prompts ---------------------------------------------------------------------------
-template <int DP, int DVP>
+template <int DP, int DVP, bool FULL_P>
 __global__ void __launch_bounds__(128, (DP + DVP <= 160) ? 3 : ((DP + DVP <= 192) ? 2 : 1))
 attention_tiles_kernel(const AttnParams p) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -355,7 +371,7 @@ attention_tiles_kernel(const AttnParams p) {
         }
         __syncthreads();
         if (j0 <= warp_hi)
-            attend<DP, DVP, 8>(qf, ks + buf * STAGE, vs + buf * STAGE, 0, j0, pos, lo,
+            attend<DP, DVP, 8, FULL_P>(qf, ks + buf * STAGE, vs + buf * STAGE, 0, j0, pos, lo,
                                j0 + KB - 1 <= warp_first_pos && (j0 >= warp_max_lo || j0 + KB <= p.keep_first), p.scale_log2, m, l,
                                o, lane, slope_log2, biased, p.cap_log2, p.keep_first);
         __syncthreads();                                    // the buffer is free for the block after the next
@@ -383,7 +399,7 @@ attention_tiles_kernel(const AttnParams p) {
 }
 
 // ---- single tokens, the keys cut into ranges ---------------------------------------------------------
-template <int DP, int DVP>
+template <int DP, int DVP, bool FULL_P>
 __global__ void __launch_bounds__(128)
 attention_split_kernel(const AttnParams p) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -452,7 +468,7 @@ attention_split_kernel(const AttnParams p) {
             }
             __syncthreads();
             if (j0 + warp * 16 <= position)
-                attend<DP, DVP, 2>(qf, ks + buf * STAGE, vs + buf * STAGE, warp * 16, j0 + warp * 16, pos, lo, false,
+                attend<DP, DVP, 2, FULL_P>(qf, ks + buf * STAGE, vs + buf * STAGE, warp * 16, j0 + warp * 16, pos, lo, false,
                                    p.scale_log2, m, l, o, lane, slope_log2, biased, p.cap_log2, p.keep_first);
             __syncthreads();
         }
@@ -846,22 +862,22 @@ int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, size_t s
     return MG_OK;
 }
 
-template <int DP, int DVP>
+template <int DP, int DVP, bool FULL_P>
 int launch(const AttnParams& p, int single_tokens, int n_tiles, cudaStream_t s) {
     size_t smem = (size_t)2 * KB * (DP + PAD + DVP + PAD) * sizeof(bf16);      // two buffers
     cudaError_t e;
     if (single_tokens) {
         const size_t meet = (size_t)(4 * 16 * 2 + 4 * 16 * DVP) * sizeof(float);
         if (meet > smem) smem = meet;
-        e = cudaFuncSetAttribute(attention_split_kernel<DP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(attention_split_kernel<DP, DVP, FULL_P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            e = mg_launch(attention_split_kernel<DP, DVP>, dim3(p.n_tokens, p.n_kv_head, p.splits), dim3(128), smem, s, true, p);
+            e = mg_launch(attention_split_kernel<DP, DVP, FULL_P>, dim3(p.n_tokens, p.n_kv_head, p.splits), dim3(128), smem, s, true, p);
         if (e == cudaSuccess && p.counters == nullptr)
             e = mg_launch(attention_merge_kernel, dim3(p.n_tokens, p.n_head), dim3(p.dv >= 128 ? 128 : 64), 0, s, true, p);
     } else {
-        e = cudaFuncSetAttribute(attention_tiles_kernel<DP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(attention_tiles_kernel<DP, DVP, FULL_P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            e = mg_launch(attention_tiles_kernel<DP, DVP>, dim3(n_tiles, p.n_kv_head), dim3(128), smem, s, true, p);
+            e = mg_launch(attention_tiles_kernel<DP, DVP, FULL_P>, dim3(n_tiles, p.n_kv_head), dim3(128), smem, s, true, p);
     }
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention (mma): %s", cudaGetErrorString(e));
     return MG_OK;
@@ -890,15 +906,15 @@ MG_API long long mg_attention_mma_scratch_floats(int n_tokens, int n_head, int d
 // as zeros, or null to merge the ranges in a second kernel); 0: n_tiles tiles of tile_tokens tokens, found
 // from req_q_start / req_q_len.  slopes: [n_head] 32-bit or null; key_block <= 0: no block mask; softcap <= 0: none;
 // sinks: [n_head] 32-bit or null; v_stride: elements between value rows (0: dv); keep_first: keys at the sequence's
-// start that stay in sight beside a window.  Returns MG_ERR_UNSUPPORTED for sizes
-// it does not take.
+// start that stay in sight beside a window; full_weights: the softmax weights as two bfloat16 numbers.  Returns
+// MG_ERR_UNSUPPORTED for sizes it does not take.
 MG_API int mg_attention_mma(const void* q, int q_stride, const void* k_pages, const void* v_pages, const int* block_table,
                             const int* token_request, const int* positions, const int* req_q_start,
                             const int* req_q_len, const void* gate, int gate_stride, void* out, float* scratch,
                             int* counters, int n_tokens, int n_requests, int n_head, int n_kv_head, int d, int dv, int page_tokens,
                             int max_pages, int window, float scale, int num_pages, int single_tokens, int n_tiles,
                             int tile_tokens, int splits, int split_keys, const float* slopes, int key_block, float softcap,
-                            const float* sinks, int v_stride, int keep_first, void* stream) {
+                            const float* sinks, int v_stride, int keep_first, int full_weights, void* stream) {
     if (n_tokens == 0) return MG_OK;
     MG_REQUIRE(keep_first >= 0, "attention: a negative number of kept keys");
     MG_REQUIRE(n_tokens > 0 && n_head > 0 && n_kv_head > 0 && n_head % n_kv_head == 0 && page_tokens > 0 && max_pages > 0,
@@ -931,12 +947,18 @@ MG_API int mg_attention_mma(const void* q, int q_stride, const void* k_pages, co
     }
     cudaStream_t s = (cudaStream_t)stream;
     const int dp = d <= 64 ? 64 : d <= 96 ? 96 : 128, dvp = dv <= 64 ? 64 : 128;
-    if (dp == 64 && dvp == 64) return launch<64, 64>(p, single_tokens, n_tiles, s);
-    if (dp == 64) return launch<64, 128>(p, single_tokens, n_tiles, s);
-    if (dp == 96 && dvp == 64) return launch<96, 64>(p, single_tokens, n_tiles, s);
-    if (dp == 96) return launch<96, 128>(p, single_tokens, n_tiles, s);
-    if (dvp == 64) return launch<128, 64>(p, single_tokens, n_tiles, s);
-    return launch<128, 128>(p, single_tokens, n_tiles, s);
+#define MG_LAUNCH_SIZES(FULL_P)                                                                   \
+    if (dp == 64 && dvp == 64) return launch<64, 64, FULL_P>(p, single_tokens, n_tiles, s);       \
+    if (dp == 64) return launch<64, 128, FULL_P>(p, single_tokens, n_tiles, s);                   \
+    if (dp == 96 && dvp == 64) return launch<96, 64, FULL_P>(p, single_tokens, n_tiles, s);       \
+    if (dp == 96) return launch<96, 128, FULL_P>(p, single_tokens, n_tiles, s);                   \
+    if (dvp == 64) return launch<128, 64, FULL_P>(p, single_tokens, n_tiles, s);                  \
+    return launch<128, 128, FULL_P>(p, single_tokens, n_tiles, s)
+    if (!full_weights) {
+        MG_LAUNCH_SIZES(false);
+    }
+    MG_LAUNCH_SIZES(true);
+#undef MG_LAUNCH_SIZES
 }
 
 // Rows of 32 (token, head) pairs that the wide-row kernel takes for a prompt portion of `tokens` tokens.

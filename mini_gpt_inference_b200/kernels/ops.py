@@ -878,6 +878,22 @@ class CudaOps:
             if code != library.UNSUPPORTED:
                 self._run(code, "paged_attention (prefill, tensor cores)")
                 return out
+        if qkv.dtype == torch.bfloat16 and self.use_tensor_cores and self.use_mma_attention:
+            # heads that neither of the two kernels above takes (up to 128 features, a multiple of 8): tiles of the
+            # warp-level tensor cores, their softmax weights as two bfloat16 numbers each.  A prompt of 2,048 tokens,
+            # 16 heads of 128: 0.28 ms a layer; the kernel of a warp per token and head, 18 ms.
+            args = self._mma_plan(n, n_head, n_kv_head, head_dim, window, 0, 0, ctx)
+            if args is not None:
+                code = self.lib.mg_attention_mma(
+                    _ptr(qkv), qkv.shape[1], _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table), _ptr(ctx.token_request),
+                    _ptr(ctx.positions), _ptr(getattr(ctx, "req_q_start", None)), _ptr(getattr(ctx, "req_q_len", None)),
+                    None, 0, _ptr(out), _ptr(args[0]), None, n, table.shape[0], n_head, n_kv_head, head_dim, head_dim,
+                    cache.page_tokens, table.shape[1], window, float(scale), cache.k_pages.shape[0], *args[1:], None, 0, 0.0,
+                    None, 0, 0, 1, self._stream())
+                if code != library.UNSUPPORTED:
+                    self._run(code, "paged_attention (tensor cores, full weights)")
+                    self.launches += args[1]                     # single tokens: the merge of the ranges
+                    return out
         self._run(self.lib.mg_paged_attention_generic(
             _ptr(qkv), _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table),
             _ptr(ctx.token_request), _ptr(ctx.positions), _ptr(out), n, n_head, n_kv_head, head_dim,
@@ -980,32 +996,21 @@ class CudaOps:
         if q.dtype == torch.bfloat16 and self.use_tensor_cores and self.use_mma_attention:
             # bfloat16: tiles of (token, head) rows on the warp-level tensor cores; single tokens
             # with their keys cut into ranges that a second kernel merges
-            single = bool(getattr(ctx, "decode_only", False))
-            q_len = getattr(ctx, "host_q_len", None)
-            group = n_head // n_kv_head
-            args = None
-            if single:
-                keys, splits = self._key_ranges(int(ctx.max_ctx_after), int(cache.window or 0), block, keep_first)
-                floats = self.lib.mg_attention_mma_scratch_floats(n, n_head, v_dim, splits)
-                scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
+            args = self._mma_plan(n, n_head, n_kv_head, v_dim, int(cache.window or 0), block, keep_first, ctx)
+            if args is not None:
                 # (measured at batch 8, context 2,048: the ranges merged by a second kernel, 0.273 ms a
                 # step; by the last CTA of each token and key/value head, 0.283 ms)
-                counters = self._counters(n * n_kv_head) if self.merge_ranges_in_last_cta else None
-                args = [_ptr(scratch), _ptr(counters), 1, 0, 1, splits, keys]
-            elif q_len and group <= 64 and getattr(ctx, "req_q_start", None) is not None:
-                tile = max(1, 64 // group)
-                args = [None, None, 0, sum(-(-int(t) // tile) for t in q_len), tile, 0, 0]
-            if args is not None:
+                counters = self._counters(n * n_kv_head) if self.merge_ranges_in_last_cta and args[1] else None
                 code = self.lib.mg_attention_mma(
                     _ptr(q), q.shape[1], _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table), _ptr(ctx.token_request),
                     _ptr(ctx.positions), _ptr(getattr(ctx, "req_q_start", None)), _ptr(getattr(ctx, "req_q_len", None)),
-                    _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(out), args[0], args[1], n, table.shape[0],
-                    n_head, n_kv_head, head_dim, v_dim, cache.page_tokens, table.shape[1], int(cache.window or 0),
-                    float(scale), cache.k_pages.shape[0], *args[2:], _ptr(slopes), block, softcap, _ptr(sinks),
-                    head_dim if in_keys else 0, keep_first, self._stream())
+                    _ptr(gate), gate.stride(0) if gate is not None else 0, _ptr(out), _ptr(args[0]), _ptr(counters), n,
+                    table.shape[0], n_head, n_kv_head, head_dim, v_dim, cache.page_tokens, table.shape[1],
+                    int(cache.window or 0), float(scale), cache.k_pages.shape[0], *args[1:], _ptr(slopes), block, softcap, _ptr(sinks),
+                    head_dim if in_keys else 0, keep_first, 0, self._stream())
                 if code != library.UNSUPPORTED:
                     self._run(code, "paged_attention (tensor cores, general)")
-                    if single and args[1] is None:
+                    if args[1] and counters is None:
                         self.launches += 1                       # the merge of the ranges as a kernel of its own
                     return out
         if q.dtype == torch.bfloat16 and self.use_tensor_cores and self.use_mma_attention and in_keys and not biased and keep_first == 0:
@@ -1041,6 +1046,19 @@ class CudaOps:
             float(scale), cache.k_pages.shape[0], table.shape[0], self._is_bf16(q), _ptr(slopes), block,
             softcap, _ptr(sinks), head_dim if in_keys else 0, keep_first, self._stream()), "paged_attention (general)")
         return out
+
+    def _mma_plan(self, n, n_head, n_kv_head, v_dim, window, block, keep_first, ctx):
+        """How the warp-level tensor-core attention cuts a step: ``[scratch, single tokens, tiles, tokens a tile, ranges,
+        keys a range]``; None where it takes no such step."""
+        if getattr(ctx, "decode_only", False):
+            keys, splits = self._key_ranges(int(ctx.max_ctx_after), window, block, keep_first)
+            floats = self.lib.mg_attention_mma_scratch_floats(n, n_head, v_dim, splits)
+            return [torch.empty((floats,), dtype=torch.float32, device=self.device), 1, 0, 1, splits, keys]
+        q_len, group = getattr(ctx, "host_q_len", None), n_head // n_kv_head
+        if q_len and group <= 64 and getattr(ctx, "req_q_start", None) is not None:
+            tile = max(1, 64 // group)
+            return [None, 0, sum(-(-int(t) // tile) for t in q_len), tile, 0, 0]
+        return None
 
     def _key_ranges(self, max_context, window, block, keep_first=0):
         """Keys per range and ranges per token for single tokens with contexts of up to ``max_context`` keys.  With a

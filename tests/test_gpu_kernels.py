@@ -559,7 +559,7 @@ def test_qkv_projection_writes_keys_and_values_to_their_pages(ops, m, heads):
 
 
 def _attention_case(ops, dtype, n_head, n_kv_head, head_dim, page_tokens, window, lengths, q_lens,
-                    seed=0, spike=None):
+                    seed=0, spike=None, portions=False):
     """Requests with `lengths[i]` tokens in total, of which the last `q_lens[i]` are new.
     spike = (request, key position, gain): that key is `gain` in every feature and the request's
     queries of head 0 are all ones, so that its score stands far above every other."""
@@ -618,6 +618,12 @@ def _attention_case(ops, dtype, n_head, n_kv_head, head_dim, page_tokens, window
                           positions=torch.tensor(positions, dtype=torch.int32).cuda(),
                           decode_only=all(q == 1 for q in q_lens), max_ctx_after=max(lengths),
                           extra={k: torch.from_numpy(v).cuda() for k, v in plan.arrays.items()})
+    if portions:                                   # what a step of the runner has besides: each request's rows
+        ctx.host_q_len, starts = list(q_lens), [sum(q_lens[:i]) for i in range(R)]
+        ctx.req_q_start = torch.tensor(starts, dtype=torch.int32).cuda()
+        ctx.req_q_len = torch.tensor(q_lens, dtype=torch.int32).cuda()
+        ctx.host_ctx_before = [n - ql for n, ql in zip(lengths, q_lens)]
+        ctx.req_ctx_before = torch.tensor(ctx.host_ctx_before, dtype=torch.int32).cuda()
     qkv = torch.stack(qkv_rows).to(dtype).cuda()
     before = ops.launches
     got = ops.paged_attention(qkv, n_head, n_kv_head, head_dim, scale, cache, ctx)
@@ -636,6 +642,31 @@ def test_paged_attention_general(ops, dtype, n_head, n_kv_head, head_dim, page_t
     got, want = _attention_case(ops, dtype, n_head, n_kv_head, head_dim, pt, window, lengths, q_lens)
     assert not torch.isnan(got).any(), "attention read a cache row beyond a request's length"
     assert (got - want).abs().max() <= _tol(dtype, 1.0)
+
+
+@pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
+@pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window", [
+    (4, 4, 128, 64, 0), (6, 2, 104, 16, 0), (5, 1, 48, 4, 0), (4, 4, 80, 24, 70), (2, 2, 96, 16, 0), (64, 1, 8, 8, 0),
+    (2, 1, 128, 16, 64)])
+def test_heads_of_other_sizes_on_the_warp_level_tensor_cores(ops, n_head, n_kv_head, head_dim, page_tokens, window, single):
+    """bfloat16 heads that the tcgen05 and the single-token kernels do not take: no further from the 64-bit result than the
+    kernel of a warp per token and head, whose softmax weights are 32-bit numbers."""
+    lengths = [1, 63, 64, 65, 127, 128, 129, 300, 17]
+    q_lens = [1] * len(lengths) if single else [1, 63, 1, 65, 64, 63, 2, 257, 17]
+    args = (ops, torch.bfloat16, n_head, n_kv_head, head_dim, page_tokens, window, lengths, q_lens)
+    ops.use_split_attention = False
+    try:
+        got, want = _attention_case(*args, seed=8, portions=True)
+        ops.use_mma_attention = False
+        general, _ = _attention_case(*args, seed=8, portions=True)
+    finally:
+        ops.use_split_attention = ops.use_mma_attention = True
+    ops.check_status()
+    assert not torch.isnan(got).any()
+    assert (got - want).abs().max() <= _tol(torch.bfloat16, 1.0)
+    # both round their outputs to bfloat16, which is nearly all of either error; one rounding that falls the other way may
+    # move the sum of squares of some thousand outputs by a few per cent
+    assert (got - want).norm() <= 1.03 * (general - want).norm()
 
 
 @pytest.mark.parametrize("gain", [4.0, 9.0, 24.0])
