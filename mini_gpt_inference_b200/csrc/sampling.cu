@@ -1,4 +1,5 @@
 // Sampling from 32-bit logits: greedy (argmax) here; the stochastic sampler follows below.
+#include <cooperative_groups.h>
 #include <float.h>
 #include <math.h>
 
@@ -265,6 +266,22 @@ __device__ float block_reduce_sum(float v, float* scratch) {
     return scratch[0];
 }
 
+// The lowest index among a row's largest values, by one CTA.
+__device__ __forceinline__ void greedy_row(const float* lr, int limit, int* out, float* scratch, int* found) {
+    float v = -INFINITY;
+    int idx = 0x7fffffff;
+    for (int i = threadIdx.x; i < limit; i += SAMPLE_THREADS) {
+        const float x = lr[i];
+        if (x > v || (x == v && i < idx)) { v = x; idx = i; }
+    }
+    const float best = block_reduce_max(v, scratch);
+    if (threadIdx.x == 0) *found = 0x7fffffff;
+    __syncthreads();
+    if (v == best && idx != 0x7fffffff) atomicMin(found, idx);
+    __syncthreads();
+    if (threadIdx.x == 0) *out = *found == 0x7fffffff ? 0 : *found;
+}
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
@@ -281,18 +298,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     const float temp = temperature[row];
 
     if (temp <= 0.f) {   // greedy row: lowest index among the largest
-        float v = -INFINITY;
-        int idx = 0x7fffffff;
-        for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-            const float x = lr[i];
-            if (x > v || (x == v && i < idx)) { v = x; idx = i; }
-        }
-        const float best = block_reduce_max(v, scratch);
-        if (tid == 0) sh_found = 0x7fffffff;
-        __syncthreads();
-        if (v == best && idx != 0x7fffffff) atomicMin(&sh_found, idx);
-        __syncthreads();
-        if (tid == 0) out[row] = sh_found == 0x7fffffff ? 0 : sh_found;
+        greedy_row(lr, limit, out + row, scratch, &sh_found);
         return;
     }
 
@@ -444,6 +450,235 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 #undef ROW
 }
 
+// ---- the same with a cluster of CTAs per row ------------------------------------------------------
+// What bounds a row is a chain of passes over it: eight counting passes and three sums.  One CTA holds a row in shared
+// memory and reads it anew in every pass (98 values a thread at 50,304 ids), one thread looks through a pass's 256 bins,
+// and its 64-bit sums of probability mass meet in a few bins, lane after lane.  Here a row's values stay in the registers
+// of a cluster's CTAs (16 a thread), lanes that meet in one bin of mass add up among themselves first, a warp picks the
+// digit, and a pass ends in one cluster barrier behind which every CTA sums all histograms itself.
+// 50,304 ids, before and now: 24 rows with top-k 50 and top-p 0.8, 572 -> 45 us; with top-p 0.9 alone, 526 -> 69; plain
+// draws, 70 -> 17; 256 rows with both, 1,133 -> 336, plain draws, 123 -> 96.  1,000 ids, 24 rows with both: 60 -> 25.
+
+// Descending over 256 bins: the digit and the sum in front of it.  `by_count`: the first bin whose inclusive sum reaches
+// `goal`; otherwise the last non-empty bin in front of which at most `goal` lies (the first non-empty one if none is).
+// One warp, 8 bins a lane.
+__device__ __forceinline__ void pick_digit(const unsigned long long* total, unsigned long long start, unsigned long long goal,
+                                           bool by_count, uint32_t* digit, unsigned long long* before) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long bin[8], sum = 0ull;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        bin[j] = total[255 - 8 * lane - j];
+        sum += bin[j];
+    }
+    unsigned long long incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    unsigned long long run = start + incl - sum, first_run = run, hit_run = run;
+    int first = -1, hit = -1;                                   // bins of this lane, counted from 255 down
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (bin[j] != 0ull && first < 0) { first = j; first_run = run; }
+        if (by_count ? (hit < 0 && bin[j] != 0ull && run + bin[j] >= goal) : (bin[j] != 0ull && run <= goal)) { hit = j; hit_run = run; }
+        run += bin[j];
+    }
+    const uint32_t hits = __ballot_sync(0xffffffffu, hit >= 0), any = __ballot_sync(0xffffffffu, first >= 0);
+    const int chosen = hits ? (by_count ? __ffs(hits) - 1 : 31 - __clz(hits)) : any ? __ffs(any) - 1 : 0;
+    if (lane == chosen) {
+        const int j = hits ? hit : first;
+        *digit = j < 0 ? 0u : (uint32_t)(255 - 8 * lane - j);
+        *before = hits ? hit_run : first_run;
+    }
+}
+
+template <int ROW_CTAS, int NV>
+__global__ void __cluster_dims__(ROW_CTAS, 1, 1) __launch_bounds__(SAMPLE_THREADS, NV > 16 ? 1 : 2)
+sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
+                      const int* __restrict__ top_k, const float* __restrict__ top_p,
+                      const uint32_t* __restrict__ seed_lo, const uint32_t* __restrict__ seed_hi,
+                      const uint32_t* __restrict__ counter, int* __restrict__ out, int vocab, int limit, int chunk) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ float scratch[SAMPLE_THREADS / 32];
+    __shared__ unsigned long long hist[2][256];                 // two in turn: a pass clears the other one
+    __shared__ unsigned long long total[256];
+    __shared__ float sh_max, sh_kept, sh_mass;                  // this CTA's share of a cluster-wide reduction, one each
+    __shared__ int sh_index, sh_last;
+    __shared__ uint32_t sh_digit;
+    __shared__ unsigned long long sh_before;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = blockIdx.x / ROW_CTAS, rank = (int)cluster.block_rank();
+    const float* lr = logits + (size_t)row * vocab;
+    const int begin = rank * chunk, end = min(limit, begin + chunk);      // this CTA's ids; thread t has begin + t, + 512, ...
+    const float temp = temperature[row];
+    if (temp <= 0.f) {   // greedy row: one CTA, lowest index among the largest
+        if (rank == 0) greedy_row(lr, limit, out + row, scratch, &sh_index);
+        return;
+    }
+    const float safe_t = fmaxf(temp, 1e-6f);
+
+    float x[NV];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const int i = begin + v * SAMPLE_THREADS + tid;
+        x[v] = i < end ? lr[i] / safe_t : -INFINITY;
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) mx = fmaxf(mx, x[v]);
+    const float block_max = block_reduce_max(mx, scratch);
+    if (tid == 0) { sh_max = block_max; sh_index = 0x7fffffff; sh_last = -1; }
+    if (tid < 256) hist[0][tid] = 0ull;
+    cluster.sync();
+    mx = -INFINITY;
+    for (int r = 0; r < ROW_CTAS; ++r) mx = fmaxf(mx, *cluster.map_shared_rank(&sh_max, r));
+
+    uint32_t thr_key = 0u;
+    int turn = 0;
+    // One pass: the CTAs' histograms of 8 bits meet, and the digit is picked from their sum.
+    auto next_digit = [&](unsigned long long start, unsigned long long goal, bool by_count) {
+        cluster.sync();
+        if (tid < 256) {
+            unsigned long long sum = 0ull;
+#pragma unroll
+            for (int r = 0; r < ROW_CTAS; ++r) sum += *cluster.map_shared_rank(&hist[turn][tid], r);
+            total[tid] = sum;
+            hist[turn ^ 1][tid] = 0ull;                         // read by the others before this barrier, written after it
+        }
+        __syncthreads();
+        if (warp == 0) pick_digit(total, start, goal, by_count, &sh_digit, &sh_before);
+        __syncthreads();
+        turn ^= 1;
+    };
+
+    // top-k: key of the k-th largest scaled logit
+    const int k = top_k ? top_k[row] : 0;
+    if (k > 0 && k < limit) {
+        uint32_t prefix = 0u, mask = 0u;
+        unsigned long long remaining = (unsigned long long)k;
+        for (int shift = 24; shift >= 0; shift -= 8) {
+            uint32_t* counts = reinterpret_cast<uint32_t*>(hist[turn]);       // the low words of the bins
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const uint32_t key = order_key(x[v]);
+                if (begin + v * SAMPLE_THREADS + tid < end && (key & mask) == prefix) atomicAdd(counts + 2 * ((key >> shift) & 255u), 1u);
+            }
+            next_digit(0ull, remaining, true);
+            prefix |= sh_digit << shift;
+            remaining -= sh_before;
+            mask |= 255u << shift;
+        }
+        thr_key = prefix;
+    }
+
+    // top-p: lowest key whose mass of strictly larger keys is <= p * (mass kept by top-k)
+    const float p = top_p ? top_p[row] : 1.f;
+    if (p < 1.f) {
+        float part = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            if (begin + v * SAMPLE_THREADS + tid < end && order_key(x[v]) >= thr_key) part += expf(x[v] - mx);
+        part = block_reduce_sum(part, scratch);
+        if (tid == 0) sh_kept = part;
+        cluster.sync();
+        float z_k = 0.f;
+        for (int r = 0; r < ROW_CTAS; ++r) z_k += *cluster.map_shared_rank(&sh_kept, r);
+        const unsigned long long target = (unsigned long long)((double)p * (double)z_k * (double)FIXED_ONE);
+        uint32_t prefix = 0u, mask = 0u;
+        unsigned long long acc = 0ull;
+        for (int shift = 24; shift >= 0; shift -= 8) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const uint32_t key = order_key(x[v]);
+                const bool in = begin + v * SAMPLE_THREADS + tid < end && key >= thr_key && (key & mask) == prefix;
+                if (!in) continue;
+                // + 1 so that a token whose probability underflows still marks its bin
+                const unsigned long long e = (unsigned long long)(expf(x[v] - mx) * FIXED_ONE) + 1ull;
+                const uint32_t bin = (key >> shift) & 255u;
+                if (e >> 56) {                                  // not a number
+                    atomicAdd(&hist[turn][bin], e);
+                    continue;
+                }
+                const uint32_t peers = __match_any_sync(__activemask(), bin);
+                // 32 numbers of up to 2^40 + 1: their low 24 and high bits add up in 32 bits each
+                const uint32_t low = __reduce_add_sync(peers, (uint32_t)e & 0xffffffu);
+                const uint32_t high = __reduce_add_sync(peers, (uint32_t)(e >> 24));
+                if (lane == __ffs(peers) - 1) atomicAdd(&hist[turn][bin], ((unsigned long long)high << 24) + low);
+            }
+            next_digit(acc, target, false);
+            prefix |= sh_digit << shift;
+            acc = sh_before;
+            mask |= 255u << shift;
+        }
+        if (prefix > thr_key) thr_key = prefix;
+    }
+
+    // normaliser of what is kept, CTA by CTA in index order
+    float part = 0.f;
+    int last_kept = -1;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const int i = begin + v * SAMPLE_THREADS + tid;
+        x[v] = i < end && order_key(x[v]) >= thr_key ? expf(x[v] - mx) : 0.f;       // from here on: the weights
+        part += x[v];
+        if (x[v] > 0.f) last_kept = i;
+    }
+    part = block_reduce_sum(part, scratch);
+    if (last_kept >= 0) atomicMax(&sh_last, last_kept);
+    if (tid == 0) sh_mass = part;
+    cluster.sync();
+    float mass[ROW_CTAS], z = 0.f;
+    int last = -1;
+    for (int r = 0; r < ROW_CTAS; ++r) {
+        mass[r] = *cluster.map_shared_rank(&sh_mass, r);
+        z += mass[r];
+        last = max(last, *cluster.map_shared_rank(&sh_last, r));
+    }
+    cluster.sync();                                             // the others' shared memory is not read from here on
+    const uint32_t rnd = philox_first(seed_lo[row], seed_hi[row], counter[row], 0u);
+    const float u = (float)(rnd >> 8) * (1.0f / 16777216.0f);      // [0, 1)
+    const float target = u * z;
+    float base = 0.f;
+    int owner = -1;                                             // the CTA in whose ids the sum passes the target
+    for (int r = 0; r < ROW_CTAS; ++r) {
+        if (base + mass[r] > target) { owner = r; break; }
+        base += mass[r];
+    }
+    if (owner < 0) {                                            // rounding left the target just above the sum
+        if (rank == 0 && tid == 0) out[row] = last < 0 ? 0 : last;
+        return;
+    }
+    if (owner != rank) return;
+    // the inverse-CDF walk in index order through this CTA's weights
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        if (v * SAMPLE_THREADS >= chunk) break;
+        float incl = x[v];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float n = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += n;
+        }
+        __syncthreads();
+        if (lane == 31) scratch[warp] = incl;
+        __syncthreads();
+        float before = 0.f, sum = 0.f;
+        for (int w = 0; w < SAMPLE_THREADS / 32; ++w) {
+            const float s = scratch[w];
+            if (w < warp) before += s;
+            sum += s;
+        }
+        if (x[v] > 0.f && base + before + incl > target) atomicMin(&sh_index, begin + v * SAMPLE_THREADS + tid);
+        __syncthreads();
+        if (sh_index != 0x7fffffff) break;
+        base += sum;
+    }
+    if (tid == 0) out[row] = sh_index != 0x7fffffff ? sh_index : max(0, sh_last);
+}
+
 }  // namespace
 
 // temperature: [rows]; top_k: [rows] int (<= 0: off) or null; top_p: [rows] (>= 1: off) or null;
@@ -455,6 +690,18 @@ MG_API int mg_sample(const float* logits, const float* temperature, const int* t
     MG_REQUIRE(rows > 0 && vocab > 0, "sample: bad sizes");
     MG_REQUIRE(temperature && seed_lo && seed_hi && counter, "sample: missing per-row parameters");
     if (limit <= 0 || limit > vocab) limit = vocab;
+    // As many CTAs a row as hold it with 16 values a thread (two such CTAs share an SM), with 32 beyond 65,536 ids (24 rows
+    // of 131,072 with both cuts: 1,802 -> 91 us); wider rows, which eight CTAs do not hold, keep to the kernel of one CTA.
+    if (limit <= 32 * 8 * SAMPLE_THREADS) {
+        const int held = 16 * SAMPLE_THREADS, ctas = limit <= held ? 1 : limit <= 2 * held ? 2 : limit <= 4 * held ? 4 : 8;
+        auto kernel = ctas == 1 ? sample_cluster_kernel<1, 16> : ctas == 2 ? sample_cluster_kernel<2, 16> :
+                      ctas == 4 ? sample_cluster_kernel<4, 16> : limit <= 8 * held ? sample_cluster_kernel<8, 16> :
+                                                                                     sample_cluster_kernel<8, 32>;
+        kernel<<<rows * ctas, SAMPLE_THREADS, 0, (cudaStream_t)stream>>>(logits, temperature, top_k, top_p, seed_lo, seed_hi,
+                                                                         counter, out, vocab, limit, ceil_div(limit, ctas));
+        MG_CHECK_LAUNCH("sample (cluster)");
+        return MG_OK;
+    }
     const size_t row_bytes = (size_t)limit * sizeof(float);
     const int cached = row_bytes <= 220 * 1024;
     static bool configured = false;

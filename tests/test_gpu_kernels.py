@@ -875,6 +875,30 @@ def test_sampler_draws_from_the_reference_distribution(ops, vocab, temperature, 
     assert ((freq - want[top]).abs() <= 5 * sigma + 2e-3).all(), (freq, want[top])
 
 
+@pytest.mark.parametrize("vocab", [1, 7, 512, 8192, 8193, 16385, 32769, 65536, 65537, 131072, 131073])
+def test_sampler_at_the_edges_of_its_cuts(ops, vocab):
+    """One CTA a row up to 8,192 ids, clusters of 2, 4 and 8 beyond, twice the values a thread beyond 65,536, one CTA again
+    beyond 131,072: drawn ids lie in the support the oracle gives them, also where it is one id at an end of the row, on a
+    limit in front of the row's largest value, in a row with infinities and in a greedy row between drawn ones."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(6, vocab, generator=g) * 3.0
+    logits[1, vocab - 1], logits[2, 0] = 60.0, 60.0
+    limit = max(1, vocab - 1)
+    if vocab > 2:
+        logits[3, 1: vocab // 2] = float("-inf")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()              # noqa: E731
+    temperature, k, p = [0.9, 0.7, 0.7, 1.1, 0.0, 1.0], [9, 0, 0, 5, 3, 0], [0.8, 0.5, 1.0, 1.0, 0.5, 0.6]
+    for n in range(4):
+        got = ops.sample(logits.cuda(), torch.tensor(temperature).cuda(), i32(k), torch.tensor(p).cuda(), i32([n] * 6),
+                         i32(list(range(6))), i32([5 + n] * 6), limit).tolist()
+        assert got[4] == int(logits[4, :limit].argmax())
+        for r in (0, 1, 2, 3, 5):
+            # (a mass within 32-bit rounding of top-p may fall either way)
+            want = plain_gpt.sampling_distribution(logits[r, :limit], temperature[r], k[r] or None,
+                                                   min(1.0, p[r] + 1e-5) if p[r] < 1 else None)
+            assert 0 <= got[r] < limit and want[got[r]] > 0, (r, got[r])
+
+
 def test_sampler_is_greedy_at_zero_and_repeatable_by_seed(ops):
     g = torch.Generator().manual_seed(4)
     logits = torch.randn(6, 1000, generator=g).cuda()
