@@ -66,6 +66,18 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
 }
 
+// True in one lane of the (converged) warp.  The compiler knows then that a single thread runs the branch: what takes
+// uniform registers there (TMA, tcgen05) needs no loop over the lanes around it.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one != 0;
+}
+
 // One 2-D tile by TMA into shared memory, counted on an mbarrier.  x (the innermost coordinate)
 // times the element size must be a multiple of 16 bytes.  No multicast.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
@@ -108,6 +120,97 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+
+// ---- the same for a pair of CTAs (a cluster of two) that share one product ------------------------------
+// Each CTA of the pair holds its half of the rows of A, of the rows of B and of the accumulator's rows; the CTA of rank 0
+// issues the products, and both CTAs' loads count on its barriers.  CG is 1 (one CTA by itself) or 2.
+
+// A shared-memory address with the bit that tells the pair's CTAs apart cleared: the same place in the CTA of rank 0.
+constexpr uint32_t PAIR_LEADER_MASK = 0xFEFFFFFFu;
+
+template <int CG>
+__device__ __forceinline__ void tma_load_2d_group(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+    if (CG == 1) { tma_load_2d(dst, map, bar, x, y); return; }
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"((uint64_t)map), "r"(bar & PAIR_LEADER_MASK), "r"(x), "r"(y)
+        : "memory");
+}
+
+template <int CG>
+__device__ __forceinline__ void tmem_alloc_group(uint32_t holder, uint32_t cols) {
+    if (CG == 1) { tmem_alloc(holder, cols); return; }
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(holder), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+template <int CG>
+__device__ __forceinline__ void tmem_dealloc_group(uint32_t taddr, uint32_t cols) {
+    if (CG == 1) { tmem_dealloc(taddr, cols); return; }
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+
+template <int CG>
+__device__ __forceinline__ void umma_bf16_group(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    if (CG == 1) { umma_bf16(tmem_d, desc_a, desc_b, idesc, accumulate); return; }
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// Arrive on the barrier (in both CTAs of a pair) once all products issued so far by this thread have completed.
+template <int CG>
+__device__ __forceinline__ void umma_commit_group(uint32_t bar) {
+    if (CG == 1) { umma_commit(bar); return; }
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+// Arrive on the barrier at the same place in the CTA of rank 0 of the cluster.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
+        ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// All threads of all CTAs of the cluster.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ---- stores of tiles by TMA: from shared memory, written or added to what is there -----------------------
+// The writes to the tile in shared memory have to be made visible to the copy engine first (async_proxy_fence by every
+// writer, then a barrier); the tile may be written again after tma_store_wait_read.
+__device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"((uint64_t)map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"((uint64_t)map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // 32 lanes x 32 columns of 32-bit: thread t of the warp gets lane (base lane + t), 32 columns.
 __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&r)[32]) {

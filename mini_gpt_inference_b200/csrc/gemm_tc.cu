@@ -1,29 +1,31 @@
-// bfloat16 matrix product on the 5th-generation tensor cores: TMA -> shared memory ->
-// tcgen05.mma -> TMEM -> epilogue.
+// bfloat16 matrix product on the 5th-generation tensor cores: TMA -> shared memory -> tcgen05.mma -> TMEM ->
+// shared memory -> TMA.
 //
-//   D[p, q] = sum_k P[p, k] * Q[q, k]        P: [rows_p, K], Q: [rows_q, K], both K-major bf16
+//   D[m, n] = sum_k A[m, k] * B[n, k]        A: [M, K] activations, B: [N, K] weights, both K-major bf16
 //
-// One CTA computes a 128 x BN tile of D.  Thread 0 is the producer: it arms a "full"
-// mbarrier with the bytes to come and issues two TMA tile loads (128 x 64 of P, BN x 64 of
-// Q, 128-byte swizzle) per k block into a ring of stages.  Thread 32 is the issuer: it waits
-// for a stage, issues four tcgen05.mma (K = 16 each) whose 32-bit accumulator lives in TMEM,
-// and commits them to the stage's "empty" mbarrier, which frees the stage when the tensor
-// core has read it.  After the last k block a commit to a third barrier tells all four warps
-// that the accumulator is complete; each warp reads its 32 TMEM lanes with tcgen05.ld and
-// applies the epilogue: bias, tanh-GELU, conversion, or an add into the 32-bit residual
-// stream.  Edges need no special case on the load side: TMA fills what lies outside the
-// matrices with zeros (also a K that is no multiple of 64); stores are predicated.
+// A CTA, or a pair of CTAs (CG = 2, a cluster of two on neighbouring SMs whose tensor cores work on one product), computes
+// tiles of 128 * CG x BN of D, one after the other.  Six warps: four for the epilogue, one whose first thread loads (64
+// columns of K at a time into a ring of stages, 128-byte swizzle), one whose first thread issues the products.  In a pair
+// each CTA loads its own 128 rows of A and its half of the BN rows of B; the CTA of rank 0 issues for both.  The accumulator
+// lies in TMEM, twice if a CTA has more than one tile: the epilogue of a tile then runs beside the products of the next.
 //
-// Two orientations share the kernel.  For many tokens, P is the activations and Q the weights
-// (a thread ends up with one token's row of features).  For a few tokens (decoding), P is
-// the weights and Q the activations: the 128 rows of the tensor-core tile are filled with
-// weight rows and the batch sits on the narrow side (BN = 16, 32 or 64), so no tensor-core
-// work is wasted on padding and a CTA streams 128 x K weights.
+// Epilogue: a warp reads its 32 TMEM lanes (rows) 32 columns at a time, applies bias and activation, and lays the values
+// into its own 4 KB of shared memory in the swizzled order that the copy engine wants; one thread stores the box, or adds it
+// to the 32-bit residual stream (every element has one summand, so the sum is that of a load, an add and a store).  Keys and
+// values of the QKV projection are copied from the same 4 KB to their cache rows, eight lanes to 128 bytes.  Rows of D that
+// are no multiple of 16 bytes are written from there with plain stores, 32 neighbouring columns at a time.
 //
-// Every wait on an mbarrier is bounded.  If one runs out, the kernel records a code in
-// `status`, skips the rest of its work, waits a moment for copies in flight, frees its TMEM
-// and returns; the host reads `status` later.  No thread-block clusters and no multicast
-// are used: each CTA loads its own tiles.
+// What bounds it: reading the tiles from L2.  A tile of 128 x 128 asks 32 KB for every 64 columns of K, 256 clocks of
+// tensor-core work; an SM takes in some 50 to 60 bytes a clock, so such a tile cannot run above half the tensor cores'
+// rate.  A pair with BN = 256 asks 32 KB a CTA for 512 clocks.  (The earlier epilogue, a thread to a row, stored and read
+// 16 bytes from each of 32 lines an instruction: 4 to 8 us of the 13 that a product of 2,048 x 512 x 512 took.)
+//
+// Edges need no special case on the load side: TMA fills what lies outside the matrices with zeros (also a K that is no
+// multiple of 64), and its stores leave out what lies outside.
+//
+// Every wait on an mbarrier is bounded.  If one runs out, the kernel records a code in `status`, skips the rest of its
+// work, waits a moment for copies in flight, frees its TMEM and returns; the host reads `status` later.  No multicast
+// loads: each CTA loads its own tiles.
 #include <cuda.h>
 
 #include <mutex>
@@ -42,16 +44,23 @@ MG_GUARD_DECLARE(linear_tc)
 
 namespace {
 
-constexpr int TILE_P = 128;         // rows of P per CTA = UMMA M
+constexpr int TILE_M = 128;         // rows of A per CTA
 constexpr int BLOCK_K = 64;         // bf16 elements per k block = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
 constexpr int MAX_STAGES = 8;
-constexpr int P_TILE_BYTES = TILE_P * BLOCK_K * 2;
+constexpr int MAX_BN = 256;
+constexpr int A_TILE_BYTES = TILE_M * BLOCK_K * 2;
+constexpr int EPI_WARPS = 8;                                 // two to each 32 lanes of TMEM
+constexpr int BOX_BYTES = 32 * 128;                          // 32 rows of 128 bytes: what a warp stores at a time
+constexpr int BOXES = 2;                                     // ... of which it has two that take turns
+constexpr int THREADS = 32 * (EPI_WARPS + 2);
+constexpr int SMS = 148;
 
-struct __align__(8) Barriers {
+struct __align__(16) Control {
     uint64_t full[MAX_STAGES];
     uint64_t empty[MAX_STAGES];
-    uint64_t accumulator;
+    uint64_t acc_full[2];
+    uint64_t acc_empty[2];
     uint32_t tmem_base;
     uint32_t failed;
 };
@@ -66,345 +75,382 @@ struct KvSink {
     int num_pages;                   // pages of the pool (what a cache row is held against in guarded builds)
 };
 
-// First element of feature n (>= q_width) of the token in cache row `slot`; *is_value says which array.
-__device__ __forceinline__ size_t kv_sink_index(const KvSink& k, int slot, int n, bool* is_value) {
-    const int kv_width = k.n_kv_head * k.head_dim;
-    const int f = n - k.q_width;
-    const int which = f / kv_width, fi = f - which * kv_width;
-    const int h = fi / k.head_dim, d = fi - h * k.head_dim;
-    const int page = slot / k.page_tokens, off = slot - page * k.page_tokens;
-    *is_value = which != 0;
-    return (((size_t)page * k.n_kv_head + h) * k.page_tokens + off) * k.head_dim + d;
-}
+struct GemmArgs {
+    const float* bias;
+    void* out;                       // [M, N] bf16 or 32-bit; the residual stream for EPI_RESIDUAL
+    int M, N, K, bn, stages;
+    int epilogue, out_bf16;
+    int boxes;                       // rows of the output are multiples of 16 bytes: stored by TMA
+    KvSink sink;
+    int* status;
+};
 
-template <int BN, bool SWAP>
-__global__ void __launch_bounds__(128)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
-               const float* __restrict__ bias, void* __restrict__ out_ptr, float* __restrict__ residual,
-               int rows_p, int rows_q, int K, int ld_out, int epilogue, int out_bf16, int stages,
-               const KvSink sink, int* __restrict__ status) {
-    constexpr int Q_TILE_BYTES = BN * BLOCK_K * 2;
-    constexpr int STAGE_BYTES = P_TILE_BYTES + Q_TILE_BYTES;
-    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+template <int CG, int SUB>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+               const __grid_constant__ CUtensorMap map_out, const GemmArgs g) {
     extern __shared__ uint8_t smem_raw[];
     // 128-byte swizzle wants tiles aligned to 1024 bytes
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    Barriers* bars = (Barriers*)(smem + (size_t)stages * STAGE_BYTES);
+    const int bn = g.bn, stages = g.stages;
+    const int b_rows = bn / CG;
+    constexpr uint32_t B_OFFSET = SUB * A_TILE_BYTES;        // a stage: SUB tiles of A, then as many of B
+    const uint32_t b_tile_bytes = b_rows * BLOCK_K * 2, stage_bytes = B_OFFSET + SUB * b_tile_bytes;
+    uint8_t* boxes = smem + (size_t)stages * stage_bytes;
+    Control* ctl = (Control*)(boxes + EPI_WARPS * BOXES * BOX_BYTES);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int p0 = blockIdx.x * TILE_P, q0 = blockIdx.y * BN;
-    const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
-    // The epilogue's operands are asked for while the main loop runs: the tile's slice of the
-    // bias goes to shared memory, the thread's row of the residual stream is pulled towards L2.
-    __shared__ __align__(16) float bias_tile[BN];
-    int cache_row = -1;                                   // of this thread's token (not SWAP)
-    if (!SWAP) {
-        if (sink.k_pages != nullptr && p0 + tid < rows_p) cache_row = sink.slots[p0 + tid];
-        // (guarded builds: a row beyond the pool is recorded and its keys and values are not copied)
-        if (cache_row >= 0 && !MG_GUARDED(linear_tc, MG_GUARD_CACHE_ROW, cache_row, (long long)sink.num_pages * sink.page_tokens))
-            cache_row = -1;
-        for (int j = tid; j < BN; j += 128) bias_tile[j] = (bias && q0 + j < rows_q) ? bias[q0 + j] : 0.f;
-        if (epilogue == EPI_RESIDUAL && p0 + tid < rows_p) {
-            const float* rrow = residual + (size_t)(p0 + tid) * ld_out + q0;
-            for (int j = 0; j < BN && q0 + j < rows_q; j += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(rrow + j));
-        }
-    }
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (the same register value in all lanes)
+    const int rank = CG == 2 ? (int)cluster_rank() : 0;
+    const int m_tiles = (g.M + CG * TILE_M - 1) / (CG * TILE_M), n_tiles = (g.N + bn - 1) / bn;
+    const int tiles = m_tiles * n_tiles, first_tile = (int)blockIdx.x / CG, tile_step = (int)gridDim.x / CG;
+    const int num_kb = (g.K + SUB * BLOCK_K - 1) / (SUB * BLOCK_K);     // stages' worth of K
+    const bool twice = tiles > tile_step;                    // some CTA has several tiles: two accumulators
+    uint32_t tmem_cols = 32;
+    while (tmem_cols < (uint32_t)(twice ? 2 * bn : bn)) tmem_cols *= 2;
 
     MG_STAMP(gemm, 0);
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
-            mbar_init(smem_u32(&bars->full[s]), 1);
-            mbar_init(smem_u32(&bars->empty[s]), 1);
+            mbar_init(smem_u32(&ctl->full[s]), 1);
+            mbar_init(smem_u32(&ctl->empty[s]), 1);
         }
-        mbar_init(smem_u32(&bars->accumulator), 1);
-        bars->failed = 0;
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(smem_u32(&ctl->acc_full[a]), 1);
+            mbar_init(smem_u32(&ctl->acc_empty[a]), CG * EPI_WARPS);
+        }
+        ctl->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(smem_u32(&bars->tmem_base), TMEM_COLS);
+    if (warp == EPI_WARPS + 1) tmem_alloc_group<CG>(smem_u32(&ctl->tmem_base), tmem_cols);
     tc_fence_before();
     __syncthreads();
+    if (CG == 2) cluster_barrier();                          // the pair's barriers and both halves of TMEM are there
     tc_fence_after();
-    const uint32_t tmem_base = bars->tmem_base;
-    // Barriers, tensor memory and the bias are set up while the kernel in front drains; its
-    // results (the activations, the residual stream) are touched only from here on.
+    const uint32_t tmem_base = ctl->tmem_base;
+    // Barriers and tensor memory are set up while the kernel in front drains; its results (the activations, the residual
+    // stream) are touched only behind the wait.  The weights do not come from the kernel in front: their tiles of the
+    // first round of stages are asked for before it.
     MG_STAMP(gemm, 2);
     pdl_trigger();
-    // The weights do not come from the kernel in front: their tiles of the first round of stages are
-    // asked for before the wait (tokens x weights: the q operand; weights x tokens: the p operand).
     const int early = num_kb < stages ? num_kb : stages;
-    if (tid == 0) {
+    const bool loads = warp == EPI_WARPS, issues = warp == EPI_WARPS + 1;
+    if (loads && elect_one()) {
+        const int n0 = (first_tile / m_tiles) * bn + rank * b_rows;
         for (int kb = 0; kb < early; ++kb) {
-            const uint32_t full = smem_u32(&bars->full[kb]);
-            mbar_expect_tx(full, STAGE_BYTES);
-            uint8_t* stage = smem + (size_t)kb * STAGE_BYTES;
-            if (SWAP) tma_load_2d(smem_u32(stage), &map_p, full, kb * BLOCK_K, p0);
-            else tma_load_2d(smem_u32(stage + P_TILE_BYTES), &map_q, full, kb * BLOCK_K, q0);
+            const uint32_t full = smem_u32(&ctl->full[kb]), tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
+            if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
+#pragma unroll
+            for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
         }
     }
     pdl_wait();
     MG_STAMP(gemm, 3);
 
-    if (tid == 0) {
-        // ---- producer: TMA loads into the ring of stages ----
-        for (int kb = 0; kb < num_kb; ++kb) {
-            const int s = kb % stages;
-            const uint32_t full = smem_u32(&bars->full[s]);
-            uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
-            if (kb < early) {                             // the weights' tile is on its way already
-                if (SWAP) tma_load_2d(smem_u32(stage + P_TILE_BYTES), &map_q, full, kb * BLOCK_K, q0);
-                else tma_load_2d(smem_u32(stage), &map_p, full, kb * BLOCK_K, p0);
-                continue;
+    // A single thread runs each of the next two loops, and the chain of its instructions is what bounds small tiles: some
+    // 300 clocks a stage, whatever its size.  So the ring's place and parity are carried along (the two divisions that found
+    // them took as long as the rest), the thread is chosen by elect.sync (behind a comparison with threadIdx the compiler
+    // wraps each load and product in a loop over the lanes: 560 clocks a stage), and small tiles take two k blocks a stage.
+    if (loads) {
+        // ---- loads into the ring of stages ----
+        if (elect_one()) {
+            int s = 0, ahead = early;                        // stages whose weights are on their way already
+            uint32_t parity = 1;
+            bool ok = true;
+            for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+                const int m0 = (tile % m_tiles) * CG * TILE_M + rank * TILE_M, n0 = (tile / m_tiles) * bn + rank * b_rows;
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    const uint32_t full = smem_u32(&ctl->full[s]), stage = smem_u32(smem) + s * stage_bytes;
+                    if (ahead > 0) {
+                        --ahead;
+#pragma unroll
+                        for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, (kb * SUB + i) * BLOCK_K, m0);
+                    } else {
+                        if (!mbar_wait(smem_u32(&ctl->empty[s]), parity)) {
+                            atomicExch(g.status, 1);
+                            ctl->failed = 1;
+                            ok = false;
+                            break;
+                        }
+                        if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
+#pragma unroll
+                        for (int i = 0; i < SUB; ++i) {
+                            tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, (kb * SUB + i) * BLOCK_K, m0);
+                            tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
+                        }
+                    }
+                    if (++s == stages) { s = 0; parity ^= 1; }
+                }
             }
-            if (!mbar_wait(smem_u32(&bars->empty[s]), ((kb / stages) & 1) ^ 1)) {
-                atomicExch(status, 1);
-                bars->failed = 1;
-                break;
-            }
-            mbar_expect_tx(full, STAGE_BYTES);
-            tma_load_2d(smem_u32(stage), &map_p, full, kb * BLOCK_K, p0);
-            tma_load_2d(smem_u32(stage + P_TILE_BYTES), &map_q, full, kb * BLOCK_K, q0);
         }
-        MG_STAMP(gemm, 4);
-    } else if (tid == 32) {
-        // ---- issuer: tcgen05.mma over the stages, accumulator in TMEM ----
-        constexpr uint32_t idesc = instr_desc_bf16(TILE_P, BN);
-        bool ok = true;
-        for (int kb = 0; kb < num_kb && ok; ++kb) {
-            const int s = kb % stages;
-            if (!mbar_wait(smem_u32(&bars->full[s]), (kb / stages) & 1)) {
-                atomicExch(status, 2);
-                bars->failed = 1;
-                ok = false;
-                break;
+    } else if (issues) {
+        // ---- products of the stages as they arrive ----
+        if (rank == 0 && elect_one()) {
+            const uint32_t idesc = instr_desc_bf16(CG * TILE_M, bn);
+            const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+            int s = 0, round = 0;
+            uint32_t parity = 0;
+            bool ok = true;
+            for (int tile = first_tile; tile < tiles && ok; tile += tile_step, ++round) {
+                const int a = twice ? round & 1 : 0;
+                const uint32_t acc = tmem_base + a * bn;
+                // (the first use of an accumulator waits for nobody)
+                ok = mbar_wait(smem_u32(&ctl->acc_empty[a]), ((round >> 1) & 1) ^ 1);
+                tc_fence_after();
+                for (int kb = 0; kb < num_kb && ok; ++kb) {
+                    if (!(ok = mbar_wait(smem_u32(&ctl->full[s]), parity))) break;
+                    tc_fence_after();
+                    // (shared memory ends below 2^18 bytes: the 14 bits of the address field hold address / 16 without a carry)
+                    const uint64_t desc_a = desc0 + (uint64_t)((s * stage_bytes) >> 4), desc_b = desc_a + (B_OFFSET >> 4);
+#pragma unroll
+                    for (int i = 0; i < SUB; ++i)
+#pragma unroll
+                        for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                            // 16 elements further along K: 32 bytes inside the swizzled row
+                            const uint64_t step = (uint64_t)((k * UMMA_K * 2) >> 4);
+                            umma_bf16_group<CG>(acc, desc_a + (uint64_t)(i * (A_TILE_BYTES >> 4)) + step,
+                                                desc_b + (uint64_t)(i * (b_tile_bytes >> 4)) + step, idesc,
+                                                (i | k) != 0 || kb != 0 ? 1u : 0u);
+                        }
+                    umma_commit_group<CG>(smem_u32(&ctl->empty[s]));
+                    if (++s == stages) { s = 0; parity ^= 1; }
+                }
+                umma_commit_group<CG>(smem_u32(&ctl->acc_full[a]));
             }
+            if (!ok) {
+                atomicExch(g.status, 2);
+                ctl->failed = 1;
+            }
+        }
+    } else if (warp < EPI_WARPS) {
+        // ---- epilogue: four warps, each on its own 32 lanes of TMEM ----
+        const int per_box = g.out_bf16 ? 64 : 32;            // columns of a 128-byte row
+        const int quarter = warp & 3, first_box = (warp >> 2) * per_box;       // this warp's lanes, and its first columns
+        const bool bias_wide = ((uintptr_t)g.bias & 15) == 0;
+        int used = 0, round = 0;                             // boxes filled so far, tiles done so far
+        for (int tile = first_tile; tile < tiles; tile += tile_step, ++round) {
+            const int a = twice ? round & 1 : 0;
+            const int row0 = (tile % m_tiles) * CG * TILE_M + rank * TILE_M + quarter * 32, n0 = (tile / m_tiles) * bn;
+            // asked for while the products run: the cache row of this lane's token
+            long long kv_row = -1;                           // the cache row's first element for kv head 0, in head rows
+            if (g.sink.k_pages != nullptr && n0 + bn > g.sink.q_width && row0 + lane < g.M) {
+                const int slot = g.sink.slots[row0 + lane];
+                // (guarded builds: a row beyond the pool is recorded and its keys and values are not copied)
+                if (slot >= 0 && MG_GUARDED(linear_tc, MG_GUARD_CACHE_ROW, slot, (long long)g.sink.num_pages * g.sink.page_tokens)) {
+                    const int page = slot / g.sink.page_tokens;
+                    kv_row = (long long)page * g.sink.n_kv_head * g.sink.page_tokens + (slot - page * g.sink.page_tokens);
+                }
+            }
+            bool good = mbar_wait(smem_u32(&ctl->acc_full[a]), twice ? (round >> 1) & 1 : 0);
+            if (!good) atomicExch(g.status, 3);
+            good = good && (*(volatile uint32_t*)&ctl->failed == 0);
+            if (!__all_sync(0xffffffffu, good)) break;       // tcgen05.ld needs the whole warp
             tc_fence_after();
-            uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
-            const uint64_t desc_p = smem_desc_sw128(smem_u32(stage));
-            const uint64_t desc_q = smem_desc_sw128(smem_u32(stage + P_TILE_BYTES));
+            MG_STAMP(gemm, 5);
+            const uint32_t lane_addr = tmem_base + a * bn + ((uint32_t)(quarter * 32) << 16);
+            const int columns = min(bn, g.N - n0);
+            // all of the accumulator's columns that are this warp's are in registers: the next tile's products may overwrite them
+            auto release = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2) mbar_arrive_leader(smem_u32(&ctl->acc_empty[a]));
+                    else mbar_arrive(smem_u32(&ctl->acc_empty[a]));
+                }
+            };
+            if (first_box >= columns) release();
+            for (int c0 = first_box; c0 < columns; c0 += 2 * per_box, ++used) {
+                uint8_t* box = boxes + (warp * BOXES + used % BOXES) * BOX_BYTES;
+                // the copy engine has read what this box held before
+                if (g.boxes && lane == 0) tma_store_wait_read<BOXES - 1>();
+                __syncwarp();
+                for (int half = 0; half < per_box; half += 32) {
+                    uint32_t r[32];
+                    tmem_load_32(lane_addr + (uint32_t)(c0 + half), r);
+                    float v[32];                             // the bias first: all lanes read the same 16 bytes
+                    const int n = n0 + c0 + half;
+                    if (g.bias != nullptr && bias_wide && n + 32 <= g.N) {
 #pragma unroll
-            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                // 16 elements further along K: 32 bytes inside the swizzled row
-                const uint64_t step = (uint64_t)((k * UMMA_K * 2) >> 4);
-                umma_bf16(tmem_base, desc_p + step, desc_q + step, idesc, (kb | k) != 0 ? 1u : 0u);
-            }
-            umma_commit(smem_u32(&bars->empty[s]));
-        }
-        umma_commit(smem_u32(&bars->accumulator));
-    }
-    __syncwarp();
-
-    // ---- epilogue: all four warps, each on its own 32 lanes of TMEM ----
-    bool good = mbar_wait(smem_u32(&bars->accumulator), 0);
-    if (!good) atomicExch(status, 3);
-    good = good && (*(volatile uint32_t*)&bars->failed == 0);
-    good = __all_sync(0xffffffffu, good);               // tcgen05.ld needs the whole warp
-    tc_fence_after();
-    MG_STAMP(gemm, 5);
-    if (good) {
-        const int p = p0 + warp * 32 + lane;             // this thread's row of D
-        // first element of the token's cache row for kv head 0: [page][kv head][offset in page][feature]
-        long long kv_row_base = 0;
-        if (cache_row >= 0) {
-            const int page = cache_row / sink.page_tokens;
-            kv_row_base = (long long)page * sink.n_kv_head * sink.page_tokens + (cache_row - page * sink.page_tokens);
-        }
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-        constexpr int CHUNK = BN < 32 ? BN : 32;
-        // one chunk of the accumulator (this thread's row, CHUNK columns from c0) through the epilogue
-        auto finish_chunk = [&](const uint32_t (&r)[32], const int c0) {
-            if (p < rows_p) {
-                if (!SWAP) {
-                    // p is a token, q runs over features: contiguous in the output row
-                    const size_t row = (size_t)p * ld_out;
-                    const int qc = q0 + c0;
-                    const bool full = (CHUNK == 32) && (qc + CHUNK <= rows_q) && (ld_out % 8 == 0);
-                    if (full) {
-                        // whole chunk inside the matrix and 16-byte aligned: vector loads and stores
-                        float v[32];
+                        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(v + j) = *reinterpret_cast<const float4*>(g.bias + n + j);
+                    } else {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            const float4 b4 = *reinterpret_cast<const float4*>(bias_tile + c0 + j);
-                            v[j] = __uint_as_float(r[j]) + b4.x;
-                            v[j + 1] = __uint_as_float(r[j + 1]) + b4.y;
-                            v[j + 2] = __uint_as_float(r[j + 2]) + b4.z;
-                            v[j + 3] = __uint_as_float(r[j + 3]) + b4.w;
-                        }
-                        if (epilogue == EPI_GELU) {
-                            // results that become bfloat16 take the hardware tanh; 32-bit results the exact one
-                            if (out_bf16) {
+                        for (int j = 0; j < 32; ++j) v[j] = g.bias != nullptr && n + j < g.N ? g.bias[n + j] : 0.f;
+                    }
+                    tmem_wait_ld();
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) v[j] = gelu_tanh_fast(v[j]);
-                            } else {
+                    for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r[j]);
+                    if (g.epilogue == EPI_GELU) {
+                        // results that become bfloat16 take the hardware tanh; 32-bit results the exact one
+                        if (g.out_bf16) {
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
-                            }
-                        }
-                        if (epilogue == EPI_RELU_SQ) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = relu_sq(v[j]);
-                        }
-                        if (epilogue == EPI_RESIDUAL) {
-                            // all loads first, then the adds and stores: a load after a store to the
-                            // same array cannot be moved up by the compiler, and eight dependent
-                            // round trips to memory would follow one another
-                            float4* dst = reinterpret_cast<float4*>(residual + row + qc);
-                            float4 old[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) old[j] = dst[j];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                float4 o = old[j];
-                                o.x += v[4 * j]; o.y += v[4 * j + 1]; o.z += v[4 * j + 2]; o.w += v[4 * j + 3];
-                                dst[j] = o;
-                            }
-                        } else if (out_bf16) {
-                            uint4* dst = reinterpret_cast<uint4*>((bf16*)out_ptr + row + qc);
-                            int kv_which = 0, kv_h = 0, kv_d = -1;        // -1: not worked out for this chunk yet
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                __nv_bfloat162 h0 = __floats2bfloat162_rn(v[8 * j], v[8 * j + 1]);
-                                __nv_bfloat162 h1 = __floats2bfloat162_rn(v[8 * j + 2], v[8 * j + 3]);
-                                __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * j + 4], v[8 * j + 5]);
-                                __nv_bfloat162 h3 = __floats2bfloat162_rn(v[8 * j + 6], v[8 * j + 7]);
-                                uint4 o;
-                                o.x = *reinterpret_cast<uint32_t*>(&h0); o.y = *reinterpret_cast<uint32_t*>(&h1);
-                                o.z = *reinterpret_cast<uint32_t*>(&h2); o.w = *reinterpret_cast<uint32_t*>(&h3);
-                                dst[j] = o;
-                                if (cache_row >= 0 && qc + 8 * j >= sink.q_width) {
-                                    // eight features of one head (head sizes are multiples of 8 here); the
-                                    // place of the chunk's first such group is worked out once, the groups
-                                    // after it step through the head, the heads and from keys to values
-                                    if (kv_d < 0) {
-                                        const int f = qc + 8 * j - sink.q_width, kv_width = sink.n_kv_head * sink.head_dim;
-                                        kv_which = f >= kv_width ? 1 : 0;
-                                        const int fi = f - kv_which * kv_width;
-                                        kv_h = fi / sink.head_dim;
-                                        kv_d = fi - kv_h * sink.head_dim;
-                                    } else {
-                                        kv_d += 8;
-                                        if (kv_d >= sink.head_dim) {
-                                            kv_d = 0;
-                                            if (++kv_h == sink.n_kv_head) { kv_h = 0; kv_which = 1; }
-                                        }
-                                    }
-                                    const size_t at = ((size_t)kv_row_base + (size_t)kv_h * sink.page_tokens) * sink.head_dim + kv_d;
-                                    *reinterpret_cast<uint4*>((kv_which ? sink.v_pages : sink.k_pages) + at) = o;
-                                }
-                            }
+                            for (int j = 0; j < 32; ++j) v[j] = gelu_tanh_fast(v[j]);
                         } else {
-                            float4* dst = reinterpret_cast<float4*>((float*)out_ptr + row + qc);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                            for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
+                        }
+                    } else if (g.epilogue == EPI_RELU_SQ) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = relu_sq(v[j]);
+                    }
+                    // 16-byte pieces of this lane's row, in the 128-byte swizzle's places
+                    if (g.out_bf16) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint4 o;
+                            __nv_bfloat162 h[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
+                            o = *reinterpret_cast<uint4*>(h);
+                            *reinterpret_cast<uint4*>(box + lane * 128 + (((half / 8 + j) ^ (lane & 7)) << 4)) = o;
                         }
                     } else {
 #pragma unroll
-                        for (int j = 0; j < CHUNK; ++j) {
-                            const int q = qc + j;
-                            if (q < rows_q) {
-                                float v = __uint_as_float(r[j]) + bias_tile[c0 + j];
-                                if (epilogue == EPI_GELU) v = gelu_tanh(v);
-                                if (epilogue == EPI_RELU_SQ) v = relu_sq(v);
-                                if (epilogue == EPI_RESIDUAL) residual[row + q] += v;
-                                else if (out_bf16) {
-                                    const bf16 hv = __float2bfloat16_rn(v);
-                                    ((bf16*)out_ptr)[row + q] = hv;
-                                    if (cache_row >= 0 && q >= sink.q_width) {
-                                        bool is_value;
-                                        const size_t at = kv_sink_index(sink, cache_row, q, &is_value);
-                                        (is_value ? sink.v_pages : sink.k_pages)[at] = hv;
-                                    }
-                                } else ((float*)out_ptr)[row + q] = v;
-                            }
+                        for (int j = 0; j < 8; ++j)
+                            *reinterpret_cast<float4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                                make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                }
+                if (c0 + 2 * per_box >= columns) release();
+                if (g.boxes) async_proxy_fence();
+                __syncwarp();
+                if (g.boxes) {
+                    if (lane == 0) {
+                        if (row0 < g.M) {
+                            if (g.epilogue == EPI_RESIDUAL) tma_add_2d(&map_out, smem_u32(box), n0 + c0, row0);
+                            else tma_store_2d(&map_out, smem_u32(box), n0 + c0, row0);
                         }
+                        tma_store_commit();
                     }
                 } else {
-                    // p is a feature, q runs over tokens: a warp writes 32 neighbouring features
-                    const float b = bias ? bias[p] : 0.f;
-                    float old[32];
-                    if (epilogue == EPI_RESIDUAL) {
-                        // the residual values of the whole chunk are fetched before any is written back
-#pragma unroll
-                        for (int j = 0; j < CHUNK; ++j) {
-                            const int q = q0 + c0 + j;
-                            old[j] = q < rows_q ? residual[(size_t)q * ld_out + p] : 0.f;
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < CHUNK; ++j) {
-                        const int q = q0 + c0 + j;
-                        if (q < rows_q) {
-                            float v = __uint_as_float(r[j]) + b;
-                            if (epilogue == EPI_GELU) v = gelu_tanh(v);
-                                if (epilogue == EPI_RELU_SQ) v = relu_sq(v);
-                            const size_t idx = (size_t)q * ld_out + p;
-                            if (epilogue == EPI_RESIDUAL) residual[idx] = old[j] + v;
-                            else if (out_bf16) ((bf16*)out_ptr)[idx] = __float2bfloat16_rn(v);
-                            else ((float*)out_ptr)[idx] = v;
+                    // rows that TMA cannot address: a row's columns from neighbouring lanes
+                    const int wide = min(per_box, columns - c0), high = min(32, g.M - row0);
+                    for (int j = lane; j < wide; j += 32) {
+                        const int byte = g.out_bf16 ? 2 * j : 4 * j;
+#pragma unroll 8
+                        for (int i = 0; i < high; ++i) {
+                            const uint8_t* from = box + i * 128 + (((byte >> 4) ^ (i & 7)) << 4) + (byte & 15);
+                            const size_t to = (size_t)(row0 + i) * g.N + n0 + c0 + j;
+                            if (g.out_bf16) ((bf16*)g.out)[to] = *reinterpret_cast<const bf16*>(from);
+                            else if (g.epilogue == EPI_RESIDUAL) atomicAdd((float*)g.out + to, *reinterpret_cast<const float*>(from));
+                            else ((float*)g.out)[to] = *reinterpret_cast<const float*>(from);
                         }
                     }
                 }
-            }
-        };
-        // Two register buffers take turns: while one chunk goes through the epilogue the next one is
-        // on its way from tensor memory.
-        uint32_t ra[32], rb[32];
-        auto fetch = [&](uint32_t (&r)[32], const int c0) {
-            if (CHUNK == 32) tmem_load_32(lane_addr + (uint32_t)c0, r);
-            else tmem_load_16(lane_addr + (uint32_t)c0, r);
-        };
-        fetch(ra, 0);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 2 * CHUNK) {
-            if (q0 + c0 >= rows_q) break;                 // uniform over the CTA
-            tmem_wait_ld();
-            const bool second = c0 + CHUNK < BN && q0 + c0 + CHUNK < rows_q;
-            if (second) fetch(rb, c0 + CHUNK);
-            finish_chunk(ra, c0);
-            if (second) {
-                tmem_wait_ld();
-                if (c0 + 2 * CHUNK < BN && q0 + c0 + 2 * CHUNK < rows_q) fetch(ra, c0 + 2 * CHUNK);
-                finish_chunk(rb, c0 + CHUNK);
+                if (g.sink.k_pages != nullptr && n0 + c0 + per_box > g.sink.q_width) {
+                    // eight lanes to a row of 64 features, eight features (of one head: head sizes are multiples of 8) each
+                    const int n = n0 + c0 + 8 * (lane & 7);
+                    const bool mine = n >= g.sink.q_width && n < g.N;
+                    const int kv_width = g.sink.n_kv_head * g.sink.head_dim;
+                    const int f = n - g.sink.q_width, which = f >= kv_width ? 1 : 0, fi = f - which * kv_width;
+                    const int h = fi / g.sink.head_dim, d = fi - h * g.sink.head_dim;
+                    bf16* pages = which ? g.sink.v_pages : g.sink.k_pages;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = 4 * i + (lane >> 3);
+                        const long long base = __shfl_sync(0xffffffffu, kv_row, r);
+                        if (mine && base >= 0)
+                            *reinterpret_cast<uint4*>(pages + (base + (long long)h * g.sink.page_tokens) * g.sink.head_dim + d) =
+                                *reinterpret_cast<const uint4*>(box + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                    }
+                }
+                __syncwarp();
             }
         }
-    } else if (tid == 0) {
-        // something timed out: give copies that may still be in flight a moment to land
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+        if (g.boxes && lane == 0) tma_store_wait_all();
+        MG_STAMP(gemm, 6);
     }
-    MG_STAMP(gemm, 6);
+    __syncwarp();
+    // something timed out: give copies that may still be in flight a moment to land
+    if (*(volatile uint32_t*)&ctl->failed != 0 && lane == 0)
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     tc_fence_before();
     __syncthreads();
+    if (CG == 2) cluster_barrier();                          // nobody's products, barriers or TMEM are in use any more
+    tc_fence_after();
     MG_STAMP(gemm, 7);
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+    if (warp == EPI_WARPS + 1) tmem_dealloc_group<CG>(tmem_base, tmem_cols);
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-template <int BN, bool SWAP>
-int launch(const void* p, const void* q, int rows_p, int rows_q, int K, const float* bias, void* out,
-           float* residual, int ld_out, int epilogue, int out_bf16, const KvSink& sink, int* status,
-           cudaStream_t s) {
-    CUtensorMap map_p, map_q;
-    int rc = tensor_map(p, rows_p, K, TILE_P, &map_p);
-    if (rc != MG_OK) return rc;
-    rc = tensor_map(q, rows_q, K, BN, &map_q);
-    if (rc != MG_OK) return rc;
-    constexpr int stage_bytes = P_TILE_BYTES + BN * BLOCK_K * 2;
-    const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
-    // Many tiles: a ring short enough for two CTAs per SM, so that one CTA's epilogue overlaps
-    // another's main loop.  Few tiles (decoding): one CTA per SM with everything in flight.
-    const long long tiles = (long long)ceil_div(rows_p, TILE_P) * ceil_div(rows_q, BN);
-    int stages = ((tiles > 148 ? 100 : 200) * 1024) / stage_bytes;
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    if (stages > num_kb) stages = num_kb;
-    const size_t smem = (size_t)stages * stage_bytes + sizeof(Barriers) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear: cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
+// How a product is cut: CTAs per tile, columns of a tile, k blocks per stage.
+struct Cut {
+    int cg, bn, sub;
+};
+
+// The cut with the least time by a count of what bounds a tile, in microseconds (each figure from products of 64 to 2,048
+// rows by 512 to 50,304 columns at K of 512 to 8,192):
+//   a k block takes 0.175 of issue (0.125 where a stage holds two), or 0.0017 (in a pair, which reads half of B per CTA,
+//   0.0014) for each column of products, or its bytes at the 18.5 MB/us that all SMs together read from L2, whichever is most;
+//   a tile's epilogue takes 0.005 a column, beside the next tile's products if there is one, and a next tile 0.5 besides;
+//   a launch takes 2.8, that of pairs 4.5 (they wait for each other at both ends).
+// So pairs win where rounds of large tiles bound the time (2,048 x 6,144 x 2,048: 37.0 us, single CTAs 42.8), and single CTAs
+// below (2,048 x 1,536 x 512: 6.9 us, pairs 8.0).
+inline Cut choose_cut(int M, int N, int K, bool out_bf16) {
+    Cut best = {1, 64, 1};
+    double least = 1e30;
+    const int num_kb = ceil_div(K, BLOCK_K), grain = out_bf16 ? 64 : 32;
+    for (int cg = 1; cg <= (M > TILE_M ? 2 : 1); ++cg) {
+        for (int bn = grain; bn <= MAX_BN; bn = bn < 64 ? 64 : bn + 64) {
+            if (bn > grain && bn >= 2 * N) break;
+            const long long tiles = (long long)ceil_div(M, cg * TILE_M) * ceil_div(N, bn);
+            const long long places = SMS / cg, rounds = (tiles + places - 1) / places;
+            const int block_bytes = A_TILE_BYTES + bn / cg * BLOCK_K * 2, sub = block_bytes <= 24 * 1024 && num_kb > 1 ? 2 : 1;
+            double block = sub == 2 ? 0.125 : 0.175;
+            const double products = (cg == 2 ? 0.0014 : 0.0017) * bn, reads = (double)(tiles < places ? tiles : places) * cg * block_bytes / 18.5e6;
+            if (products > block) block = products;
+            if (reads > block) block = reads;
+            const double tile = num_kb * block, epilogue = 0.005 * bn;
+            const double t = (cg == 2 ? 4.5 : 2.8) + (double)(rounds - 1) * (0.5 + (tile > epilogue ? tile : epilogue)) + tile + epilogue;
+            if (t < least) { least = t; best = Cut{cg, bn, sub}; }
+        }
     }
-    dim3 grid(ceil_div(rows_p, TILE_P), ceil_div(rows_q, BN));
-    const cudaError_t le = mg_launch(gemm_tc_kernel<BN, SWAP>, grid, dim3(128), smem, s, true, map_p, map_q, bias, out,
-                                     residual, rows_p, rows_q, K, ld_out, epilogue, out_bf16, stages, sink, status);
+    return best;
+}
+
+template <int CG, int SUB>
+int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s) {
+    CUtensorMap map_a, map_b, map_out = {};
+    int rc = tensor_map(a, g.M, g.K, TILE_M, &map_a);
+    if (rc != MG_OK) return rc;
+    rc = tensor_map(b, g.N, g.K, g.bn / CG, &map_b);
+    if (rc != MG_OK) return rc;
+    if (g.boxes && (rc = tensor_map_store(g.out, g.M, g.N, 32, !g.out_bf16, &map_out)) != MG_OK) return rc;
+    const int stage_bytes = SUB * (A_TILE_BYTES + g.bn / CG * BLOCK_K * 2);
+    const int num_kb = ceil_div(g.K, SUB * BLOCK_K);
+    const long long tiles = (long long)ceil_div(g.M, CG * TILE_M) * ceil_div(g.N, g.bn);
+    const size_t fixed = EPI_WARPS * BOXES * BOX_BYTES + sizeof(Control) + 1024;
+    constexpr size_t most = 227 * 1024;
+    if (g.stages == 0) g.stages = (int)((most - fixed) / stage_bytes);
+    if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
+    if (tiles <= SMS / CG && g.stages > num_kb) g.stages = num_kb;
+    const size_t smem = (size_t)g.stages * stage_bytes + fixed;
+    static std::once_flag configured;
+    static cudaError_t e = cudaSuccess;
+    std::call_once(configured, [] {
+        e = cudaFuncSetAttribute(gemm_tc_kernel<CG, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    });
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear: cannot raise shared memory: %s", cudaGetErrorString(e));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CG * (tiles < SMS / CG ? tiles : SMS / CG)));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (CG > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = CG;
+        attr[n_attr].val.clusterDim.y = attr[n_attr].val.clusterDim.z = 1;
+        ++n_attr;
+    }
+    if (mg_dependent_launch_enabled()) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<CG, SUB>, map_a, map_b, map_out, g);
     if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "gemm_tc: %s", cudaGetErrorString(le));
     MG_CHECK_LAUNCH("gemm_tc");
     return MG_OK;
@@ -426,30 +472,25 @@ MG_API int mg_linear_tc(const void* x, const void* w, const float* bias, void* o
     MG_REQUIRE(status != nullptr, "linear: missing status word");
     if (K % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))
         return mg_set_error(MG_ERR_UNSUPPORTED, "linear: tensor-core path needs K %% 8 == 0 and 16-byte aligned operands");
-    cudaStream_t s = (cudaStream_t)stream;
-    KvSink sink = {};
+    GemmArgs g = {};
     if (k_pages != nullptr) {
         MG_REQUIRE(v_pages && slots && out_bf16 && epilogue == EPI_STORE, "linear: the key/value copy wants a bfloat16 store");
         MG_REQUIRE(head_dim > 0 && head_dim % 8 == 0 && q_width % 8 == 0 && n_kv_head > 0 && page_tokens > 0 &&
                        q_width + 2 * n_kv_head * head_dim == N,
                    "linear: key/value copy with q_width=%d n_kv_head=%d head_dim=%d N=%d", q_width, n_kv_head, head_dim, N);
-        sink = KvSink{(bf16*)k_pages, (bf16*)v_pages, slots, q_width, n_kv_head, head_dim, page_tokens, num_pages};
+        g.sink = KvSink{(bf16*)k_pages, (bf16*)v_pages, slots, q_width, n_kv_head, head_dim, page_tokens, num_pages};
     }
-    if (M <= 64 && k_pages == nullptr) {
-        // few tokens: weight rows fill the 128-row side of the tile, the batch sits on the narrow side
-        if (ceil_div(N, TILE_P) > 2147483647) return mg_set_error(MG_ERR_ARG, "linear: N too large");
-        if (M <= 16) return launch<16, true>(w, x, N, M, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
-        if (M <= 32) return launch<32, true>(w, x, N, M, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
-        return launch<64, true>(w, x, N, M, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
-    }
-    MG_REQUIRE(ceil_div(N, 64) <= 65535, "linear: N too large for one launch (%d)", N);
-    if (N <= 64 || (long long)ceil_div(M, TILE_P) * ceil_div(N, 128) < 120)
-        return launch<64, false>(x, w, M, N, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
-    // Very many tokens on a large matrix: tiles of 128 x 256 (two CTAs of two stages per SM hold all 512
-    // TMEM columns) ask L2 for a quarter fewer bytes per flop, which is what bounds these products
-    // (measured at 1600 x 4800 / 6400: +12 to 18 % from 4,096 tokens on; nothing below, where the tiles
-    // do not fill two rounds of the 296 places).
-    if ((long long)ceil_div(M, TILE_P) * ceil_div(N, 256) >= 2 * 296)
-        return launch<256, false>(x, w, M, N, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
-    return launch<128, false>(x, w, M, N, K, bias, out, residual, N, epilogue, out_bf16, sink, status, s);
+    g.bias = bias;
+    g.epilogue = epilogue;
+    g.out_bf16 = epilogue == EPI_RESIDUAL ? 0 : out_bf16;
+    g.out = epilogue == EPI_RESIDUAL ? (void*)residual : out;
+    g.M = M; g.N = N; g.K = K;
+    g.boxes = N % (g.out_bf16 ? 8 : 4) == 0 && ((uintptr_t)g.out & 15) == 0;
+    g.status = status;
+    const Cut cut = choose_cut(M, N, K, g.out_bf16 != 0);
+    MG_REQUIRE((long long)ceil_div(M, cut.cg * TILE_M) * ceil_div(N, cut.bn) < (1ll << 30), "linear: too many tiles");
+    g.bn = cut.bn;
+        cudaStream_t s = (cudaStream_t)stream;
+    if (cut.cg == 2) return cut.sub == 2 ? launch<2, 2>(x, w, g, s) : launch<2, 1>(x, w, g, s);
+    return cut.sub == 2 ? launch<1, 2>(x, w, g, s) : launch<1, 1>(x, w, g, s);
 }

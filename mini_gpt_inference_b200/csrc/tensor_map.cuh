@@ -71,6 +71,31 @@ inline int tensor_map(const void* ptr, int rows, int k, int box_rows, CUtensorMa
 }
 
 
+// Tensor map for stores to a row-major [rows, cols] matrix of bfloat16 (boxes of box_rows x 64) or 32-bit numbers
+// (box_rows x 32), 128-byte swizzle.  The caller has checked that a row's bytes are a multiple of 16 and ptr is
+// 16-byte aligned.
+inline int tensor_map_store(const void* ptr, int rows, int cols, int box_rows, bool f32, CUtensorMap* out) {
+    static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    MapKey key{ptr, rows, cols, box_rows, f32 ? 1 : 0};
+    auto it = cache.find(key);
+    if (it != cache.end()) { *out = it->second; return MG_OK; }
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return mg_set_error(MG_ERR_CUDA, "linear: cuTensorMapEncodeTiled is not available from this driver");
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * (f32 ? 4 : 2)};
+    cuuint32_t box[2] = {f32 ? 32u : 64u, (cuuint32_t)box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
+                    dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return mg_set_error(MG_ERR_CUDA, "linear: cuTensorMapEncodeTiled failed (%d)", (int)r);
+    if (cache.size() > 8192) cache.clear();
+    cache.emplace(key, *out);
+    return MG_OK;
+}
+
 // Tensor map of a row-major [rows, k] bfloat16 matrix, k a multiple of 64, seen as
 // [rows][k / 64 blocks][64 columns]: a box holds box_blocks consecutive blocks of box_rows rows, so
 // a row's bytes are asked of memory as one run.  In shared memory the box is [row][block][128

@@ -152,6 +152,29 @@ def test_tensor_core_tiles_of_256_columns_with_every_epilogue(ops):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 8200, 64), (2049, 4804, 200), (1100, 8192, 1032), (700, 8203, 72), (5000, 2056, 136),
+                                   (257, 9, 8), (130, 519, 200)])
+def test_tensor_core_tiles_by_one_cta_and_by_pairs(ops, m, n, k):
+    """Sizes on both sides of the rule that cuts a product into tiles: single CTAs and pairs, one tile a CTA and several
+    (two accumulators in turn), a last tile of few columns, rows that TMA cannot store (n no multiple of 4 or 8)."""
+    x = randn(m, k, dtype=torch.bfloat16, seed=21)
+    w = randn(n, k, dtype=torch.bfloat16, seed=22, scale=1 / math.sqrt(k))
+    b = randn(n, seed=23)
+    ref = x.double() @ w.double().T + b.double()
+    for act, fn in (("none", lambda t: t), ("gelu_tanh", plain_gpt.gelu_tanh), ("relu_sq", lambda t: t.clamp_min(0) ** 2)):
+        # bfloat16 results: half a unit in the last place (2^-9), the hardware tanh's 2^-11 and 32-bit sums of k products
+        want = fn(ref)
+        got = ops.linear(x, w, b, act, torch.bfloat16).double()
+        assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all(), act
+        got = ops.linear(x, w, b, act, torch.float32).double()
+        assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all(), act
+    res = randn(m, n, seed=24)
+    got = res.clone()
+    ops.linear_residual(x, w, b, got)
+    assert ((got.double() - res.double() - ref).abs() <= 3e-5).all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 11, 16])
 @pytest.mark.parametrize("n,k", [(1536, 512), (512, 2048), (509, 96), (50304, 512), (200, 200), (77, 40)])
 def test_small_batch_projection_with_fused_norm(ops, m, n, k):
