@@ -86,6 +86,12 @@ _SIGNATURES = {
     "mg_linear_cluster": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "mg_linear_tc": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "mg_paged_attention_generic": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P],
+    "mg_attention_fp32": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I,
+                          _I, _P, _P],
+    "mg_attention_fp32_blocks": [_I, _I],
+    "mg_attention_fp32_pass_blocks": [_I, _I, _I, _I],
+    "mg_attention_fp32_tiles": [_I],
+    "mg_attention_fp32_takes": [_I, _I, _I],
     "mg_paged_attention_split": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I,
                                  _F, _I, _I, _P, _P],
     "mg_attention_prefill_tc": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I,
@@ -103,7 +109,7 @@ _SIGNATURES = {
 
 # exported readers of the kernel files' index guards: mg_<name>_index_fault(long long[4])
 GUARDED_FILES = ("elementwise", "linear_skinny", "linear_stream", "linear_wide", "linear_cluster", "linear_tc",
-                 "attention_generic", "attention_split", "attention_prefill", "head_prepare", "moe", "attention_mma", "matrix_memory", "matrix_memory_chunked",
+                 "attention_generic", "attention_fp32", "attention_split", "attention_prefill", "head_prepare", "moe", "attention_mma", "matrix_memory", "matrix_memory_chunked",
                  "rotary_prepare", "short_conv", "recurrent_gate", "residual_norm")
 for _name in GUARDED_FILES:
     _SIGNATURES[f"mg_{_name}_index_fault"] = [_P]

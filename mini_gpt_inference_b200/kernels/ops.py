@@ -124,6 +124,7 @@ class CudaOps:
         self.use_dependent_launch = True
         self.use_prefill_tc = True
         self.use_mma_attention = True
+        self.use_fp32_attention = True
         self.use_chunked_memory = True     # prompt portions of the matrix-memory mixers chunk by chunk (bfloat16)
         self.use_recurrence_ranges = True  # long prompt portions of the gated recurrence with the warps sharing the tokens
         self.merge_ranges_in_last_cta = False
@@ -894,6 +895,8 @@ class CudaOps:
                     self._run(code, "paged_attention (tensor cores, full weights)")
                     self.launches += args[1]                     # single tokens: the merge of the ranges
                     return out
+        if self._attention_fp32(qkv, n_head, n_kv_head, head_dim, scale, cache, ctx, table, out, None, None):
+            return out
         self._run(self.lib.mg_paged_attention_generic(
             _ptr(qkv), _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table),
             _ptr(ctx.token_request), _ptr(ctx.positions), _ptr(out), n, n_head, n_kv_head, head_dim,
@@ -1039,6 +1042,9 @@ class CudaOps:
                     if single:
                         self.launches += 1                       # the merge of the ranges
                     return out
+        if (head_dim == v_dim and not biased and softcap == 0.0 and not in_keys and keep_first == 0
+                and self._attention_fp32(q, n_head, n_kv_head, head_dim, scale, cache, ctx, table, out, gate, sinks)):
+            return out
         self._run(self.lib.mg_paged_attention_general(
             _ptr(q), q.shape[1], _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table), _ptr(ctx.token_request),
             _ptr(ctx.positions), _ptr(out), n, n_head, n_kv_head, head_dim, v_dim, _ptr(gate),
@@ -1046,6 +1052,36 @@ class CudaOps:
             float(scale), cache.k_pages.shape[0], table.shape[0], self._is_bf16(q), _ptr(slopes), block,
             softcap, _ptr(sinks), head_dim if in_keys else 0, keep_first, self._stream()), "paged_attention (general)")
         return out
+
+    def _attention_fp32(self, q, n_head, n_kv_head, head_dim, scale, cache, ctx, table, out, gate, sinks) -> bool:
+        """The 32-bit attention in blocks of 64 keys, where the kernels have the sizes (which hang on the model alone: all
+        steps of a model take them, or none does, so that cuttings agree bit for bit).  True if it ran."""
+        if (q.dtype != torch.float32 or not self.use_fp32_attention
+                or not self.lib.mg_attention_fp32_takes(n_head, n_kv_head, head_dim)):
+            return False
+        n, window, single = q.shape[0], int(cache.window or 0), bool(getattr(ctx, "decode_only", False))
+        scratch, tiles, blocks, part = None, 0, 0, 0
+        if single:
+            blocks = self.lib.mg_attention_fp32_blocks(int(ctx.max_ctx_after), window)
+            part = self.lib.mg_attention_fp32_pass_blocks(n, n_head, head_dim, blocks)
+            scratch = torch.empty((n * n_head * (part + 1) * (head_dim + 2),), dtype=torch.float32, device=self.device)
+        else:
+            q_len = getattr(ctx, "host_q_len", None)
+            if not q_len or getattr(ctx, "req_q_start", None) is None:
+                return False
+            tiles = sum(self.lib.mg_attention_fp32_tiles(int(t)) for t in q_len)
+        code = self.lib.mg_attention_fp32(
+            _ptr(q), q.shape[1], _ptr(cache.k_pages), _ptr(cache.v_pages), _ptr(table), _ptr(ctx.token_request),
+            _ptr(ctx.positions), _ptr(getattr(ctx, "req_q_start", None)), _ptr(getattr(ctx, "req_q_len", None)), _ptr(gate),
+            gate.stride(0) if gate is not None else 0, _ptr(out), _ptr(scratch), n, table.shape[0], n_head, n_kv_head, head_dim,
+            cache.page_tokens, table.shape[1], window, float(scale), cache.k_pages.shape[0], tiles, blocks, part, _ptr(sinks),
+            self._stream())
+        if code == library.UNSUPPORTED:
+            return False
+        self._run(code, "paged_attention (32-bit)")
+        if single:
+            self.launches += 2 * -(-blocks // part) - 1          # per pass the blocks and their merge
+        return True
 
     def _mma_plan(self, n, n_head, n_kv_head, v_dim, window, block, keep_first, ctx):
         """How the warp-level tensor-core attention cuts a step: ``[scratch, single tokens, tiles, tokens a tile, ranges,

@@ -667,6 +667,72 @@ def test_paged_attention_general(ops, dtype, n_head, n_kv_head, head_dim, page_t
     assert (got - want).abs().max() <= _tol(dtype, 1.0)
 
 
+@pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window,sinks,gated,copies", [
+    (4, 4, 64, 16, 0, False, False, 1), (8, 2, 64, 24, 70, True, True, 1), (3, 3, 32, 8, 1, False, False, 1),
+    (4, 1, 128, 64, 129, True, False, 1), (16, 16, 32, 16, 0, False, True, 20)])
+def test_32_bit_attention_of_portions_and_single_tokens_agrees_bit_for_bit(ops, n_head, n_kv_head, head_dim, page_tokens,
+                                                                         window, sinks, gated, copies):
+    """330 tokens of one request as a whole, as portions, and one by one (with ``copies``: so often that the key blocks are
+    done in several passes): the same numbers, and those of the general kernel within rounding."""
+    n, g = 330, torch.Generator().manual_seed(5)
+    pages = -(-n // page_tokens)
+    order = torch.randperm(pages, generator=g)
+    kv = [torch.randn(pages, n_kv_head, page_tokens, head_dim, generator=g) for _ in range(2)]
+    for t in kv:                                     # behind the request's last token: no numbers
+        t[order[-1], :, (n - 1) % page_tokens + 1:] = float("nan")
+    cache = SimpleNamespace(k_pages=kv[0].cuda(), v_pages=kv[1].cuda(), group=0, page_tokens=page_tokens,
+                            window=window or None, writes=False)
+    q = torch.randn(n, n_head * head_dim, generator=g).cuda() * 2.0
+    gate = torch.randn(n, n_head * head_dim, generator=g).cuda() if gated else None
+    sink = torch.randn(n_head, generator=g).cuda() if sinks else None
+
+    def step(rows, lens, single=False):
+        rows, requests = torch.as_tensor(rows), len(lens)
+        i32 = lambda v: torch.as_tensor(v, dtype=torch.int32).cuda()
+        ctx = SimpleNamespace(block_tables=[i32(order).repeat(requests, 1)], positions=i32(rows),
+                              token_request=i32([r for r, m in enumerate(lens) for _ in range(m)]), decode_only=single,
+                              max_ctx_after=int(rows.max()) + 1, host_q_len=lens, req_q_len=i32(lens),
+                              req_q_start=i32([sum(lens[:r]) for r in range(requests)]))
+        return ops.paged_attention_general(q[rows.cuda()], n_head, n_kv_head, head_dim, head_dim, head_dim ** -0.5, cache, ctx,
+                                           gate=None if gate is None else gate[rows.cuda()], sinks=sink)
+
+    whole = step(list(range(n)), [n])
+    assert not torch.isnan(whole).any()
+    assert torch.equal(step(list(range(100, n)), [1, 63, 66, 100]), whole[100:])
+    before = ops.launches
+    ones = step(list(range(n)) * copies, [1] * n * copies, single=True)
+    assert (ops.launches - before > 2) == (copies > 1)
+    assert torch.equal(ones, whole.repeat(copies, 1))
+    ops.use_fp32_attention = False
+    try:
+        general = step(list(range(n)), [n])
+    finally:
+        ops.use_fp32_attention = True
+    # sums of up to 330 numbers of size 1, in another order
+    assert (whole - general).abs().max() <= 2e-5
+
+
+@pytest.mark.parametrize("n,k", [(512, 2048), (2048, 512), (50304, 64), (130, 100), (65, 129), (9, 4)])
+def test_32_bit_products_do_not_hang_on_the_rows_beside_them(ops, n, k):
+    """Tiles of every size and the kernel of a few rows: bit for bit the same, with every epilogue."""
+    m = 2304 if n <= 2048 else 300
+    x, w, b = randn(m, k, seed=31), randn(n, k, seed=32, scale=1 / math.sqrt(k)), randn(n, seed=33)
+    ref = x.double() @ w.double().T + b.double()
+    for act in ("none", "gelu_tanh", "relu_sq"):
+        whole = ops.linear(x, w, b, act, torch.float32)
+        for rows in (1, 8, 9, 16, 17, 64, 65, 129, 257):
+            assert torch.equal(ops.linear(x[:rows], w, b, act, torch.float32), whole[:rows]), (act, rows)
+        if act == "none":
+            assert (whole.double() - ref).abs().max() <= 2e-5
+    res = randn(m, n, seed=34)
+    whole = res.clone()
+    ops.linear_residual(x, w, b, whole)
+    assert (whole.double() - res.double() - ref).abs().max() <= 3e-5
+    few = res[:5].clone()
+    ops.linear_residual(x[:5], w, b, few)
+    assert torch.equal(few, whole[:5])
+
+
 @pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
 @pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window", [
     (4, 4, 128, 64, 0), (6, 2, 104, 16, 0), (5, 1, 48, 4, 0), (4, 4, 80, 24, 70), (2, 2, 96, 16, 0), (64, 1, 8, 8, 0),
