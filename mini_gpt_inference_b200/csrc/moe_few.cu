@@ -1,0 +1,160 @@
+// The experts' two matrix products for steps of up to 16 tokens (decoding), bfloat16.
+//
+// Such a step reads every chosen expert's matrices once and does next to nothing with them, so what counts is how many of
+// their bytes are asked for at once.  A CTA takes 16 outputs of one expert (16 matrix rows, 32 for a gated unit); its eight
+// warps share K, 128 columns at a time, and load their share of the rows straight into the registers of mma.sync's A
+// operand: a lane's 16 bytes of a row are eight neighbouring k, which serve as the k of two m16n8k16 products in an order of
+// their own (a sum over k does not mind, as long as the tokens' operand is read the same way).  No shared memory, no ring:
+// a whole CTA's 32 KB are in flight together.  The tokens are the product's 8 (or 16) columns; the warps' sums meet in
+// shared memory and are added in warp order.
+//
+// The entries (token, k) of an expert are found by each warp from the ids themselves, so no grouping kernel runs in front:
+// results lie by entry, and entry_slot is the identity (-1 for padding rows).
+//
+// 4 tokens, 8 experts of 1,024 x 1,024 and one that every token uses (19 MB a product): 12.7 and 14.0 us, and 3.4 for the
+// grouping, with the tiles of moe.cu.
+#include "common.cuh"
+#include "moe_units.cuh"
+
+MG_GUARD_DECLARE(moe_few)
+
+namespace {
+
+constexpr int WARPS = 8;
+constexpr int ROWS = 16;                 // outputs per CTA
+constexpr int MAX_TOKENS = 16;
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Forms as mg_moe_gemm: 1 gated, 2 plain, 0 out.
+template <int FORM>
+__global__ void __launch_bounds__(32 * WARPS)
+moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, long long w_expert_stride,
+               const int* __restrict__ ids, int n_entries, int top, const float* __restrict__ scale, void* __restrict__ out,
+               int* __restrict__ entry_slot, int n_experts, int N, int K, int x_rows, int act, float limit) {
+    constexpr int MI = FORM == 1 ? 2 : 1;                  // m16 tiles: a gated unit's gate rows, then its up rows
+    __shared__ int lists[WARPS][MAX_TOKENS];
+    __shared__ float sums[WARPS][MI * ROWS][MAX_TOKENS + 1];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int e = blockIdx.y, n0 = blockIdx.x * ROWS;
+    pdl_trigger();
+    pdl_wait();
+    // the expert's entries, in order; every warp finds them for itself
+    int count = 0;
+    for (int i0 = 0; i0 < n_entries; i0 += 32) {
+        const int i = i0 + lane, id = i < n_entries ? ids[i] : -1;
+        const unsigned mine = __ballot_sync(0xffffffffu, id == e);
+        const int rank = count + __popc(mine & ((1u << lane) - 1u));
+        if (id == e && rank < MAX_TOKENS) lists[warp][rank] = i;
+        count += __popc(mine);
+        if (FORM == 0 && e == 0 && blockIdx.x == 0 && warp == 0 && i < n_entries) entry_slot[i] = id >= 0 && id < n_experts ? i : -1;
+    }
+    if (count == 0) return;
+    count = min(count, MAX_TOKENS);
+    __syncwarp();
+    const bf16* we = w + (size_t)e * w_expert_stride;
+    const bf16* w_row[MI][2];                              // this lane's two rows of each tile
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int n = n0 + g + 8 * h;
+            w_row[i][h] = n < N ? we + (size_t)(i * N + n) * K + 8 * t : nullptr;
+        }
+    const bf16* x_row[2] = {nullptr, nullptr};             // its tokens (columns g and g + 8)
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+        if (g + 8 * c < count) {
+            const int entry = lists[warp][g + 8 * c], row = FORM != 0 ? entry / top : entry;
+            if (MG_GUARDED(moe_few, MG_GUARD_ROW, row, x_rows)) x_row[c] = x + (size_t)row * ldx + 8 * t;
+        }
+    float acc[MI][2][4];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) acc[i][c][0] = acc[i][c][1] = acc[i][c][2] = acc[i][c][3] = 0.f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const bool second = count > 8;                         // the same in all lanes
+    for (int k0 = warp * 128; k0 < K; k0 += WARPS * 128) {
+        uint4 a[MI][2][4], b[2][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {                      // 32 columns each: four lanes' 64 bytes of a row
+            const int k = k0 + 32 * q;
+            const bool in = k + 8 * t < K;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    a[i][h][q] = w_row[i][h] != nullptr && in ? __ldcs(reinterpret_cast<const uint4*>(w_row[i][h] + k)) : zero;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = k0 + 32 * q;
+            const bool in = k + 8 * t < K;
+            b[0][q] = x_row[0] != nullptr && in ? *reinterpret_cast<const uint4*>(x_row[0] + k) : zero;
+            b[1][q] = second && x_row[1] != nullptr && in ? *reinterpret_cast<const uint4*>(x_row[1] + k) : zero;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                const uint4 lo = a[i][0][q], hi = a[i][1][q];
+                mma_16816(acc[i][0], lo.x, hi.x, lo.y, hi.y, b[0][q].x, b[0][q].y);
+                mma_16816(acc[i][0], lo.z, hi.z, lo.w, hi.w, b[0][q].z, b[0][q].w);
+                if (second) {
+                    mma_16816(acc[i][1], lo.x, hi.x, lo.y, hi.y, b[1][q].x, b[1][q].y);
+                    mma_16816(acc[i][1], lo.z, hi.z, lo.w, hi.w, b[1][q].z, b[1][q].w);
+                }
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) sums[warp][i * ROWS + g + 8 * (r >> 1)][8 * c + 2 * t + (r & 1)] = acc[i][c][r];
+    __syncthreads();
+    for (int o = tid; o < ROWS * count; o += 32 * WARPS) {
+        const int row = o % ROWS, c = o / ROWS, n = n0 + row;
+        if (n >= N) continue;
+        float v[MI];
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            v[i] = 0.f;
+#pragma unroll
+            for (int k = 0; k < WARPS; ++k) v[i] += sums[k][i * ROWS + row][c];
+        }
+        const int entry = lists[warp][c];
+        const float s = scale ? scale[entry] : 1.f;
+        const size_t to = (size_t)entry * N + n;
+        if constexpr (FORM == 1) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(gated_value(act, limit, v[0] * s, v[MI - 1] * s));
+        else if constexpr (FORM == 2) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(plain_value(act, v[0] * s));
+        else reinterpret_cast<float*>(out)[to] = v[0] * s;
+    }
+}
+
+}  // namespace
+
+// One of the two products for every entry of a step of up to 16 tokens.  ids: [n_tokens * top] chosen experts (-1: none), an
+// expert at most once per token; scale: [entries] or null; x: [x_rows, ldx], rows by token (forms 1 and 2) or by entry (form 0);
+// out: [entries, N], bfloat16 (forms 1 and 2) or 32-bit; entry_slot: [entries], written by form 0: the entry itself, or -1.
+// Returns MG_ERR_UNSUPPORTED (and launches nothing) for sizes and alignments it does not take.
+MG_API int mg_moe_few(const void* x, int ldx, const void* w, const int* ids, int n_tokens, int top, const float* scale, void* out,
+                      int* entry_slot, int n_experts, int N, int K, int x_rows, int form, int act, float limit, void* stream) {
+    if (n_tokens == 0) return MG_OK;
+    MG_REQUIRE(n_tokens > 0 && n_experts > 0 && N > 0 && K > 0 && ldx >= K && top > 0 && form >= 0 && form <= 2, "moe (few tokens): bad sizes");
+    if (n_tokens > MAX_TOKENS || K % 8 != 0 || ldx % 8 != 0 || n_experts > 65535 || (uintptr_t)x % 16 != 0 || (uintptr_t)w % 16 != 0)
+        return mg_set_error(MG_ERR_UNSUPPORTED, "moe (few tokens): %d tokens, K=%d", n_tokens, K);
+    MG_REQUIRE(form != 0 || entry_slot != nullptr, "moe (few tokens): no room for the entries' places");
+    const long long stride = (long long)(form == 1 ? 2 : 1) * N * K;
+    auto kernel = form == 1 ? moe_few_kernel<1> : form == 2 ? moe_few_kernel<2> : moe_few_kernel<0>;
+    const cudaError_t e = mg_launch(kernel, dim3(ceil_div(N, ROWS), n_experts), dim3(32 * WARPS), 0, (cudaStream_t)stream, true,
+                                    (const bf16*)x, ldx, (const bf16*)w, stride, ids, n_tokens * top, top, scale, out, entry_slot,
+                                    n_experts, N, K, x_rows, act, limit);
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "moe (few tokens): %s", cudaGetErrorString(e));
+    return MG_OK;
+}

@@ -66,6 +66,7 @@ _SIGNATURES = {
     "mg_moe_route": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "mg_moe_group": [_P, _I, _I, _P, _P, _P, _P],
     "mg_moe_gemm": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P],
+    "mg_moe_few": [_P, _I, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "mg_moe_combine": [_P, _P, _I, _P, _I, _I, _I, _P],
     "mg_glu": [_P, _P, _P, _I, _I, _I, _I, _F, _P],
     "mg_layernorm": [_P, _P, _P, _P, _I, _I, _F, _I, _P],
@@ -109,7 +110,7 @@ _SIGNATURES = {
 
 # exported readers of the kernel files' index guards: mg_<name>_index_fault(long long[4])
 GUARDED_FILES = ("elementwise", "linear_skinny", "linear_stream", "linear_wide", "linear_cluster", "linear_tc",
-                 "attention_generic", "attention_fp32", "attention_split", "attention_prefill", "head_prepare", "moe", "attention_mma", "matrix_memory", "matrix_memory_chunked",
+                 "attention_generic", "attention_fp32", "attention_split", "attention_prefill", "head_prepare", "moe", "moe_few", "attention_mma", "matrix_memory", "matrix_memory_chunked",
                  "rotary_prepare", "short_conv", "recurrent_gate", "residual_norm")
 for _name in GUARDED_FILES:
     _SIGNATURES[f"mg_{_name}_index_fault"] = [_P]

@@ -20,6 +20,7 @@ from .library import KernelLibraryError, check
 EPILOGUES = {"none": 0, "gelu_tanh": 1, "residual": 2, "relu_sq": 3}
 PLAIN_ACTIVATIONS = {"relu_sq": 0, "gelu_tanh": 1, "silu": 2}           # ... and the activation of a unit without a gate
 GATED_ACTIVATIONS = {"silu": 0, "clamped_swish": 1, "gelu_tanh": 2}     # the gated product of a unit's two halves
+MOE_FEW_TOKENS = 16      # most tokens the experts' kernels for few tokens take
 SKINNY_ROWS = 16         # most tokens the small-batch projection kernel takes
 CLUSTER_ROWS = 128       # most tokens the mid-batch (K split over a cluster) projection kernel takes
 CLUSTER_WIDE_MAX_BYTES = 3 << 20   # ... and the largest matrix it is given for more than 64 tokens
@@ -125,6 +126,7 @@ class CudaOps:
         self.use_prefill_tc = True
         self.use_mma_attention = True
         self.use_fp32_attention = True
+        self.use_moe_few = True
         self.use_chunked_memory = True     # prompt portions of the matrix-memory mixers chunk by chunk (bfloat16)
         self.use_recurrence_ranges = True  # long prompt portions of the gated recurrence with the warps sharing the tokens
         self.merge_ranges_in_last_cta = False
@@ -1584,6 +1586,19 @@ class CudaOps:
         entries = n * top
         is_bf16 = self._is_bf16(y)
         act = (GATED_ACTIVATIONS if gated else PLAIN_ACTIVATIONS)[activation]
+        if (self.use_moe_few and is_bf16 and 0 < n <= MOE_FEW_TOKENS and width % 8 == 0 and inner % 8 == 0
+                and experts <= 65535 and not (_ptr(y) | _ptr(w_in) | _ptr(w_out)) % 16):
+            # few tokens: two kernels that find their entries themselves and read the matrices with all loads in flight
+            entry_slot = torch.empty((n, top), dtype=torch.int32, device=self.device)
+            hidden = torch.empty((entries, inner), dtype=y.dtype, device=self.device)
+            out = torch.empty((entries, width), dtype=torch.float32, device=self.device)
+            self._run(self.lib.mg_moe_few(_ptr(y), width, _ptr(w_in), _ptr(ids), n, top, _ptr(weights) if weigh_input else None,
+                                          _ptr(hidden), None, experts, inner, width, n, 1 if gated else 2, act, float(limit),
+                                          self._stream()), "moe experts (in, few tokens)")
+            self._run(self.lib.mg_moe_few(_ptr(hidden), inner, _ptr(w_out), _ptr(ids), n, top,
+                                          None if weigh_input else _ptr(weights), _ptr(out), _ptr(entry_slot), experts, width,
+                                          inner, entries, 0, 0, 0.0, self._stream()), "moe experts (out, few tokens)")
+            return EntrySum(out, entry_slot)
         offsets = torch.empty((experts + 1,), dtype=torch.int32, device=self.device)
         slot_entry = torch.empty((entries,), dtype=torch.int32, device=self.device)
         entry_slot = torch.empty((n, top), dtype=torch.int32, device=self.device)

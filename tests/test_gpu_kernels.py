@@ -581,6 +581,58 @@ def test_qkv_projection_writes_keys_and_values_to_their_pages(ops, m, heads):
     assert (qkv.double() - ref).abs().max() <= 5e-2
 
 
+@pytest.mark.parametrize("gated,activation,weigh_input", [(True, "silu", False), (True, "clamped_swish", False),
+                                                          (False, "relu_sq", True), (False, "gelu_tanh", False)])
+@pytest.mark.parametrize("n,width,inner,experts,top", [(1, 1024, 1024, 9, 3), (8, 136, 200, 5, 2), (9, 264, 72, 3, 3), (16, 1160, 24, 4, 4),
+                                                       (16, 8, 8, 70, 5)])
+def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input):
+    """Steps of up to 16 tokens: no further from the 64-bit result than the kernels of larger steps, at widths that end inside
+    a warp's share of K and inside a CTA's rows, with up to 16 tokens an expert and padding rows."""
+    g = torch.Generator().manual_seed(n * 31 + inner)
+    y = randn(n, width, dtype=torch.bfloat16, seed=41)
+    w_in = randn(experts, (2 if gated else 1) * inner, width, dtype=torch.bfloat16, seed=42, scale=1 / math.sqrt(width))
+    w_out = randn(experts, width, inner, dtype=torch.bfloat16, seed=43, scale=1 / math.sqrt(inner))
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(n)]).to(torch.int32)
+    if n > 8:
+        ids[5] = -1                                  # a padding row
+    weights = torch.rand(n, top, generator=g).cuda()
+    ids = ids.cuda()
+
+    def run():
+        residual = torch.zeros(n, width, device="cuda")
+        ops.moe_experts_residual(y, ids, weights, w_in, w_out, residual, activation, 7.0, gated, weigh_input)
+        return residual.double()
+
+    want = torch.zeros(n, width, dtype=torch.float64, device="cuda")
+    for t in range(n):
+        for k in range(top):
+            e = int(ids[t, k])
+            if e < 0:
+                continue
+            w = weights[t, k].double()
+            z = w_in[e].double() @ y[t].double() * (w if weigh_input else 1.0)
+            a, u = (z[:inner], z[inner:]) if gated else (z, None)
+            if activation == "silu":
+                h = a * torch.sigmoid(a) * u
+            elif activation == "clamped_swish":
+                a, u = a.clamp(max=7.0), u.clamp(-7.0, 7.0)
+                h = a * torch.sigmoid(1.702 * a) * (u + 1.0)
+            else:
+                h = a.clamp_min(0) ** 2 if activation == "relu_sq" else plain_gpt.gelu_tanh(a)
+            want[t] += w_out[e].double() @ h.to(torch.bfloat16).double() * (1.0 if weigh_input else w)
+    before = ops.launches
+    few = run()
+    assert ops.launches == before + 3
+    ops.use_moe_few = False
+    try:
+        tiles = run()
+    finally:
+        ops.use_moe_few = True
+    # the hidden features are rounded to bfloat16 on both sides, here and there to the other neighbour
+    assert (few - want).norm() <= 1.05 * (tiles - want).norm() + 1e-6 * want.norm()
+    assert (few - want).abs().max() <= 2e-2
+
+
 def _attention_case(ops, dtype, n_head, n_kv_head, head_dim, page_tokens, window, lengths, q_lens,
                     seed=0, spike=None, portions=False):
     """Requests with `lengths[i]` tokens in total, of which the last `q_lens[i]` are new.
