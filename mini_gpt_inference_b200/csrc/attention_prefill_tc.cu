@@ -174,7 +174,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 tma_load_2d(smem_u32(v_tiles + off), &map_v, bar, 0, y);
             }
         };
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(smem_u32(&sync->q_full), Q_BYTES);
             tma_load_2d(smem_u32(q_tile), &map_q, smem_u32(&sync->q_full), head * D, row0);
         }
@@ -192,7 +192,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             good = false;
         }
     } else if (warp == ISSUE_WARP) {
-        // ---- issuing warp: lane 0 issues tcgen05.mma / commit; all lanes walk the same path, so
+        // ---- issuing warp: one lane (elect.sync) issues tcgen05.mma / commit; all lanes walk the same path, so
         // the warp stays converged.  Scores of block j go to S buffer j % 2, its P lies in P tile j % 2.
         auto issue_scores = [&](int j) {                // S(j) = Q K(j)^T
             const int stage = j % KV_STAGES;
@@ -200,7 +200,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (j == 0) ok = warp_wait(smem_u32(&sync->q_full), 0);
             ok = ok && warp_wait(smem_u32(&sync->kv_full[stage]), (j / KV_STAGES) & 1);
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 constexpr uint32_t idesc_s = instr_desc_bf16(BQ, BK, false);
                 const uint64_t dq = smem_desc_sw128(smem_u32(q_tile));
                 const uint64_t dk = smem_desc_sw128(smem_u32(k_tiles + stage * KV_BYTES));
@@ -222,7 +222,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // landed together with its keys, for which S(it) waited
             if (!warp_wait(smem_u32(&sync->block_done[it & 1]), (it >> 1) & 1)) { code = 29; break; }
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 constexpr uint32_t idesc_pv = instr_desc_bf16(BQ, D, true);
                 const uint32_t p_addr = smem_u32(p_tiles + (it & 1) * P_BYTES);
                 const uint32_t v_addr = smem_u32(v_tiles + (it % KV_STAGES) * KV_BYTES);

@@ -247,14 +247,21 @@ __global__ void __launch_bounds__(THREADS, 1) linear_wide_kernel(const __grid_co
             for (int l = lane - 1; l < per_cta && line0 + l < a.next_lines; l += 31)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(a.next_w + (size_t)(line0 + l) * 128));
         }
-        if (lane == 0) {
+        // (elect.sync, not lane == 0: the compiler then wraps no loop over the lanes around the copy; and the ring's place is
+        // carried along, the divisions that would find it take longer than the rest)
+        if (elect_one()) {
             MG_STAMP_HERE(wide, 9);                                             // the ring is full
-            for (int n = stages; n < my_boxes; ++n) {
-                if (!mbar_poll(smem_u32(&bars->empty[n % stages]), ((n / stages) & 1) ^ 1)) {
+            int s = 0, row = (first_box + stages * a.groups) * ROWS;
+            uint32_t parity = 0;
+            for (int n = stages; n < my_boxes; ++n, row += a.groups * ROWS) {
+                if (!mbar_poll(smem_u32(&bars->empty[s]), parity)) {
                     atomicExch(a.status, 51);                                   // a stage never came free
                     break;                                                      // (the consumers' own waits run out then)
                 }
-                issue(n);
+                const uint32_t full = smem_u32(&bars->full[s]);
+                mbar_expect_tx(full, stage_bytes);
+                tma_load_3d(smem_u32(ring) + (uint32_t)s * stage_bytes, &map_w, full, 0, k0 / KB, row);
+                if (++s == stages) { s = 0; parity ^= 1; }
             }
         }
         if (lane == 0) MG_STAMP_HERE(wide, 10);                                  // the last copy is issued
