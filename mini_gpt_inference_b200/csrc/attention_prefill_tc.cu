@@ -1,5 +1,5 @@
 // Causal attention of prompt portions over the paged cache on the 5th-generation tensor cores
-// (bfloat16, head_dim 64).
+// (bfloat16, heads of 64 or 128 features).
 //
 // A work item is up to 128 consecutive query tokens of one request, one head, and one chunk of
 // the key positions those queries may see (the host cuts long contexts into chunks, see
@@ -45,30 +45,41 @@ MG_GUARD_DECLARE(attention_prefill)
 
 namespace {
 
-constexpr int D = 64;                 // head_dim of this kernel
 constexpr int BQ = 128;               // query rows per CTA = UMMA M
 constexpr int BK = 64;                // keys per block
-constexpr int KV_STAGES = 4;          // blocks of keys and values in flight
 constexpr int SOFTMAX_THREADS = 128;   // one per query row: warps 0..3, each on its 32 lanes of TMEM
 constexpr int ISSUE_WARP = 4;          // issues the tensor-core instructions
 constexpr int LOAD_WARP = 5;           // issues the TMA loads
 constexpr int THREADS = SOFTMAX_THREADS + 64;
-constexpr int Q_BYTES = BQ * D * 2;           // 16 KB
-constexpr int KV_BYTES = BK * D * 2;          // 8 KB per tensor and stage
-constexpr int P_BYTES = BQ * BK * 2;          // 16 KB, two of them
-constexpr uint32_t TMEM_COLS = 256;           // S: two buffers of 64 columns, O: 64 columns
+constexpr int MAX_KV_STAGES = 4;
+constexpr uint32_t TMEM_COLS = 256;           // S: two buffers of 64 columns, O: 64 or 128 columns
 constexpr uint32_t O_COL = 128;
 constexpr float REF_LIMIT = 1.152921504606846976e18f;   // 2^60: a block's sum of P above it moves the row's reference
 constexpr uint32_t ALIGN_SLACK = 768;         // bytes the tiles may have to move up to reach a 1024-byte boundary
 
+// Sizes by head: queries, keys and values lie in atoms of 64 features (a swizzled row of 128 bytes each), one after the
+// other; P of a head of 128 is two bfloat16 numbers per weight, its rounding and what that took off (two tiles, multiplied
+// one after the other), because this path's weights were 32-bit numbers before.
+template <int D>
+struct Sizes {
+    static constexpr int ATOMS = D / 64;
+    static constexpr int P_PARTS = D == 64 ? 1 : 2;
+    static constexpr int KV_STAGES = D == 64 ? 4 : 3;     // blocks of keys and values in flight
+    static constexpr int Q_ATOM = BQ * 128, KV_ATOM = BK * 128, P_TILE = BQ * BK * 2;
+    static constexpr int Q_BYTES = ATOMS * Q_ATOM;         // 16 or 32 KB
+    static constexpr int KV_BYTES = ATOMS * KV_ATOM;       // 8 or 16 KB per tensor and stage
+    static constexpr int P_BYTES = P_PARTS * P_TILE;       // 16 or 32 KB, two of them
+};
+
 struct __align__(8) Sync {
-    uint64_t q_full, kv_full[KV_STAGES], kv_free[KV_STAGES], s_done[2], pv_done[2], block_done[2];
+    uint64_t q_full, kv_full[MAX_KV_STAGES], kv_free[MAX_KV_STAGES], s_done[2], pv_done[2], block_done[2];
     uint32_t tmem_base;
     uint32_t failed;
     uint32_t last;            // this work item is the last of its tile to finish
 };
 
-__global__ void __launch_bounds__(THREADS, 2)
+template <int D>
+__global__ void __launch_bounds__(THREADS, D == 64 ? 2 : 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ work,
                             const int* __restrict__ block_table, const int* __restrict__ positions,
@@ -76,6 +87,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int n_head, int n_kv_head, int page_tokens, int box_rows, int max_pages, int window,
                             float scale_log2e, int* __restrict__ status, int n_tokens, int num_pages, int n_requests,
                             const bf16* __restrict__ gate, int gate_stride) {
+    using Z = Sizes<D>;
+    constexpr int KV_STAGES = Z::KV_STAGES, ATOMS = Z::ATOMS, Q_BYTES = Z::Q_BYTES, KV_BYTES = Z::KV_BYTES, P_BYTES = Z::P_BYTES;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
     if (pad > ALIGN_SLACK) {                           // uniform over the CTA; nothing is held yet
@@ -169,14 +182,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (lane == 0) mbar_expect_tx(bar, 2 * KV_BYTES);
             __syncwarp();
             if (lane * box_rows < BK) {
-                const uint32_t off = stage * KV_BYTES + lane * box_rows * (D * 2);
-                tma_load_2d(smem_u32(k_tiles + off), &map_k, bar, 0, y);
-                tma_load_2d(smem_u32(v_tiles + off), &map_v, bar, 0, y);
+#pragma unroll
+                for (int a = 0; a < ATOMS; ++a) {
+                    const uint32_t off = stage * KV_BYTES + a * Z::KV_ATOM + lane * box_rows * 128;
+                    tma_load_2d(smem_u32(k_tiles + off), &map_k, bar, a * 64, y);
+                    tma_load_2d(smem_u32(v_tiles + off), &map_v, bar, a * 64, y);
+                }
             }
         };
         if (elect_one()) {
             mbar_expect_tx(smem_u32(&sync->q_full), Q_BYTES);
-            tma_load_2d(smem_u32(q_tile), &map_q, smem_u32(&sync->q_full), head * D, row0);
+#pragma unroll
+            for (int a = 0; a < ATOMS; ++a)
+                tma_load_2d(smem_u32(q_tile + a * Z::Q_ATOM), &map_q, smem_u32(&sync->q_full), head * D + a * 64, row0);
         }
 #pragma unroll
         for (int j = 0; j < KV_STAGES; ++j)
@@ -205,8 +223,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const uint64_t dq = smem_desc_sw128(smem_u32(q_tile));
                 const uint64_t dk = smem_desc_sw128(smem_u32(k_tiles + stage * KV_BYTES));
 #pragma unroll
-                for (int k = 0; k < D / 16; ++k)
-                    umma_bf16(tmem_base + (uint32_t)((j & 1) * BK), dq + (uint64_t)(k * 2), dk + (uint64_t)(k * 2), idesc_s, k ? 1u : 0u);
+                for (int k = 0; k < D / 16; ++k)             // (four steps of 16 features an atom, 32 bytes apart)
+                    umma_bf16(tmem_base + (uint32_t)((j & 1) * BK), dq + (uint64_t)((k / 4 * Z::Q_ATOM + k % 4 * 32) >> 4),
+                              dk + (uint64_t)((k / 4 * Z::KV_ATOM + k % 4 * 32) >> 4), idesc_s, k ? 1u : 0u);
                 umma_commit(smem_u32(&sync->s_done[j & 1]));
             }
             __syncwarp();
@@ -223,15 +242,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (!warp_wait(smem_u32(&sync->block_done[it & 1]), (it >> 1) & 1)) { code = 29; break; }
             tc_fence_after();
             if (elect_one()) {
-                constexpr uint32_t idesc_pv = instr_desc_bf16(BQ, D, true);
+                constexpr uint32_t idesc_pv = instr_desc_bf16(BQ, 64, true);
                 const uint32_t p_addr = smem_u32(p_tiles + (it & 1) * P_BYTES);
                 const uint32_t v_addr = smem_u32(v_tiles + (it % KV_STAGES) * KV_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) {
-                    const uint64_t dp = smem_desc_sw128(p_addr + k * 32);
-                    const uint64_t dv = smem_desc_sw128(v_addr + k * (16 * D * 2));
-                    umma_bf16(tmem_base + O_COL, dp, dv, idesc_pv, (it | k) ? 1u : 0u);
-                }
+                for (int a = 0; a < ATOMS; ++a)              // 64 output features at a time
+#pragma unroll
+                    for (int part = 0; part < Z::P_PARTS; ++part)
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k) {
+                            const uint64_t dp = smem_desc_sw128(p_addr + part * Z::P_TILE + k * 32);
+                            const uint64_t dv = smem_desc_sw128(v_addr + a * Z::KV_ATOM + k * (16 * 128));
+                            umma_bf16(tmem_base + O_COL + a * 64, dp, dv, idesc_pv, (it | part | k) ? 1u : 0u);
+                        }
                 umma_commit(smem_u32(&sync->pv_done[it & 1]));
                 umma_commit(smem_u32(&sync->kv_free[it % KV_STAGES]));
             }
@@ -291,7 +314,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 float part_sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int cc = 0; cc < BK / 8; ++cc) {
-                    uint32_t packed[4];
+                    uint32_t packed[4], rest[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int c0 = cc * 8 + 2 * j;
@@ -300,8 +323,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         part_sum[j] += p0 + p1;
                         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
                         packed[j] = *reinterpret_cast<const uint32_t*>(&h);
+                        if (Z::P_PARTS == 2) {
+                            const __nv_bfloat162 r = __floats2bfloat162_rn(p0 - __bfloat162float(h.x), p1 - __bfloat162float(h.y));
+                            rest[j] = *reinterpret_cast<const uint32_t*>(&r);
+                        }
                     }
                     *reinterpret_cast<uint4*>(p_row + ((cc ^ (tid & 7)) * 16)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    if (Z::P_PARTS == 2)
+                        *reinterpret_cast<uint4*>(p_row + Z::P_TILE + ((cc ^ (tid & 7)) * 16)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
                 }
                 return (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
             };
@@ -352,9 +381,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (blk == last_key / BK && last_key - key0 + 1 < BK) {
                 if (!warp_wait(smem_u32(&sync->kv_full[it % KV_STAGES]), (it / KV_STAGES) & 1)) { good = false; atomicExch(status, 25); break; }
                 if (tid < BK && tid > last_key - key0) {
-                    uint4* vrow = reinterpret_cast<uint4*>(v_tiles + (it % KV_STAGES) * KV_BYTES + tid * (D * 2));
 #pragma unroll
-                    for (int c = 0; c < D * 2 / 16; ++c) vrow[c] = make_uint4(0u, 0u, 0u, 0u);
+                    for (int a = 0; a < ATOMS; ++a) {
+                        uint4* vrow = reinterpret_cast<uint4*>(v_tiles + (it % KV_STAGES) * KV_BYTES + a * Z::KV_ATOM + tid * 128);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) vrow[c] = make_uint4(0u, 0u, 0u, 0u);
+                    }
                 }
             }
             // S(it) is in registers no more, P(it) is written (and the accumulator rescaled where it had
@@ -504,11 +536,45 @@ int make_map(const void* ptr, long long rows, long long cols, int box_rows, CUte
     return MG_OK;
 }
 
+struct Prepared {
+    CUtensorMap map_q, map_k, map_v;
+    const int* work;
+    const int* block_table;
+    const int* positions;
+    bf16* out;
+    float* partial;
+    int* counters;
+    int n_items, n_head, n_kv_head, page_tokens, box_rows, max_pages, window;
+    float scale_log2e;
+    int* status;
+    int n_tokens, num_pages, n_requests;
+    const bf16* gate;
+    int gate_stride;
+};
+
+template <int D>
+int launch(const Prepared& a, cudaStream_t s) {
+    using Z = Sizes<D>;
+    // heads of 64: 113 KB, two CTAs per SM; of 128: 193 KB, one
+    constexpr size_t smem = Z::Q_BYTES + 2 * Z::KV_STAGES * Z::KV_BYTES + 2 * Z::P_BYTES + sizeof(Sync) + ALIGN_SLACK;
+    static const cudaError_t configured =
+        cudaFuncSetAttribute(attention_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (configured != cudaSuccess)
+        return mg_set_error(MG_ERR_CUDA, "attention (prefill): cannot raise shared memory: %s", cudaGetErrorString(configured));
+    const cudaError_t le =
+        mg_launch(attention_prefill_tc_kernel<D>, dim3(a.n_items, a.n_head), dim3(THREADS), smem, s, true, a.map_q, a.map_k, a.map_v, a.work,
+                  a.block_table, a.positions, a.out, a.partial, a.counters, a.n_head, a.n_kv_head, a.page_tokens, a.box_rows, a.max_pages,
+                  a.window, a.scale_log2e, a.status, a.n_tokens, a.num_pages, a.n_requests, a.gate, a.gate_stride);
+    if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention_prefill_tc: %s", cudaGetErrorString(le));
+    MG_CHECK_LAUNCH("attention_prefill_tc");
+    return MG_OK;
+}
+
 }  // namespace
 
 // Floats of scratch for the partial results of n_items work items.
-MG_API long long mg_attention_prefill_scratch_floats(int n_items, int n_head) {
-    return (long long)n_items * n_head * BQ * (D + 2);
+MG_API long long mg_attention_prefill_scratch_floats(int n_items, int n_head, int head_dim) {
+    return (long long)n_items * n_head * BQ * (head_dim + 2);
 }
 
 // Attention of prompt portions.  work: [n_items, 5] ints on the device = (request index, first row
@@ -517,12 +583,12 @@ MG_API long long mg_attention_prefill_scratch_floats(int n_items, int n_head) {
 // part `chunk`; the items of one tile are consecutive, chunk 0 first.  If any tile is cut
 // (merge != 0), `partial` holds mg_attention_prefill_scratch_floats() floats and `counters`
 // n_items * n_head ints that are zero before the call and zero again after it.
-// q_stride: elements per row of qkv if the rows are wider than q, k, v of 64 features each (0: exactly
-// that); gate: rows of gate_stride elements whose first n_head * 64 are gate values (the output is
+// q_stride: elements per row of qkv if the rows are wider than q, k, v of head_dim features each (0: exactly
+// that); gate: rows of gate_stride elements whose first n_head * head_dim are gate values (the output is
 // multiplied by their logistic function), or null.
-// qkv: [n_tokens, (n_head + 2 n_kv_head) * 64] bf16; pages: [num_pages, n_kv_head, page_tokens, 64];
-// out: [n_tokens, n_head * 64]; n_requests: rows of the block table (guarded builds hold the work
-// items' request numbers against it).  Returns MG_ERR_UNSUPPORTED unless head_dim is 64 and page_tokens
+// qkv: [n_tokens, (n_head + 2 n_kv_head) * head_dim] bf16; pages: [num_pages, n_kv_head, page_tokens, head_dim];
+// out: [n_tokens, n_head * head_dim]; n_requests: rows of the block table (guarded builds hold the work
+// items' request numbers against it).  Returns MG_ERR_UNSUPPORTED unless head_dim is 64 or 128 and page_tokens
 // is 8, 16, 32, 64, 128 or a multiple of 128.
 MG_API int mg_attention_prefill_tc(const void* qkv, const void* k_pages, const void* v_pages, const int* work,
                                    const int* block_table, const int* positions, void* out, float* partial,
@@ -537,34 +603,25 @@ MG_API int mg_attention_prefill_tc(const void* qkv, const void* k_pages, const v
                "attention (prefill): tiles are cut along the keys but no scratch or no counters were given");
     MG_REQUIRE(n_head % n_kv_head == 0, "attention: n_head %d is not a multiple of n_kv_head %d", n_head, n_kv_head);
     const bool pages_ok = (page_tokens % 8 == 0) && ((page_tokens <= 128 && 128 % page_tokens == 0) || page_tokens % 128 == 0);
-    if (head_dim != D || !pages_ok || n_head > 65535 || (((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15))
-        return mg_set_error(MG_ERR_UNSUPPORTED, "attention (prefill, tensor cores): needs head_dim 64 and a page size of 8..128 dividing 128 or a multiple of 128");
+    const int D = head_dim;
+    if ((D != 64 && D != 128) || !pages_ok || n_head > 65535 || (((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15))
+        return mg_set_error(MG_ERR_UNSUPPORTED, "attention (prefill, tensor cores): needs head_dim 64 or 128 and a page size of 8..128 dividing 128 or a multiple of 128");
     const int box_rows = page_tokens < BK ? page_tokens : BK;
     const int qkv_width = q_stride > 0 ? q_stride : (n_head + 2 * n_kv_head) * D;
     if (qkv_width < n_head * D || qkv_width % 8 != 0 ||
         (gate != nullptr && (gate_stride % 8 != 0 || gate_stride < n_head * D || ((uintptr_t)gate & 15))))
         return mg_set_error(MG_ERR_UNSUPPORTED, "attention (prefill, tensor cores): rows and gate must be 16-byte aligned");
-    CUtensorMap map_q, map_k, map_v;
-    int rc = make_map(qkv, n_tokens, qkv_width, BQ, &map_q);
+    Prepared a;
+    int rc = make_map(qkv, n_tokens, qkv_width, BQ, &a.map_q);
     if (rc != MG_OK) return rc;
     const long long kv_rows = num_pages * n_kv_head * page_tokens;
-    rc = make_map(k_pages, kv_rows, D, box_rows, &map_k);
+    rc = make_map(k_pages, kv_rows, D, box_rows, &a.map_k);
     if (rc != MG_OK) return rc;
-    rc = make_map(v_pages, kv_rows, D, box_rows, &map_v);
+    rc = make_map(v_pages, kv_rows, D, box_rows, &a.map_v);
     if (rc != MG_OK) return rc;
-    const size_t smem = Q_BYTES + 2 * KV_STAGES * KV_BYTES + 2 * P_BYTES + sizeof(Sync) + ALIGN_SLACK;   // 113 KB: two CTAs per SM
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention (prefill): cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
-    dim3 grid(n_items, n_head);
-    cudaError_t le = mg_launch(attention_prefill_tc_kernel, grid, dim3(THREADS), smem, (cudaStream_t)stream, true, map_q,
-                               map_k, map_v, work, block_table, positions, (bf16*)out, partial, counters, n_head, n_kv_head,
-                               page_tokens, box_rows, max_pages, window, scale * 1.4426950408889634f, status, n_tokens,
-                               (int)num_pages, n_requests, (const bf16*)gate, gate_stride);
-    if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention_prefill_tc: %s", cudaGetErrorString(le));
-    MG_CHECK_LAUNCH("attention_prefill_tc");
-    return MG_OK;
+    a.work = work; a.block_table = block_table; a.positions = positions; a.out = (bf16*)out; a.partial = partial; a.counters = counters;
+    a.n_items = n_items; a.n_head = n_head; a.n_kv_head = n_kv_head; a.page_tokens = page_tokens; a.box_rows = box_rows;
+    a.max_pages = max_pages; a.window = window; a.scale_log2e = scale * 1.4426950408889634f; a.status = status;
+    a.n_tokens = n_tokens; a.num_pages = (int)num_pages; a.n_requests = n_requests; a.gate = (const bf16*)gate; a.gate_stride = gate_stride;
+    return D == 64 ? launch<64>(a, (cudaStream_t)stream) : launch<128>(a, (cudaStream_t)stream);
 }

@@ -8,7 +8,10 @@ the cut); the attention mixer asks for it through ``CudaOps.plan_prompt_attentio
 from __future__ import annotations
 
 QUERY_TILE = 128       # most consecutive tokens of one request in a tile
-KEY_CHUNK = 512        # most key positions one work item walks over
+KEY_CHUNK = 512        # key positions one work item walks over, where all items run at once
+KEY_BLOCK = 64         # keys the kernel takes at a time
+ITEM_BLOCKS = 4        # what a work item costs besides its key blocks, in key blocks
+MERGE_BLOCKS = 3       # ... and what leaving its results to be merged adds
 
 
 def query_tiles(q_lens, ctx_befores, slots=None):
@@ -21,9 +24,11 @@ def query_tiles(q_lens, ctx_befores, slots=None):
     runs come longest item first, so that when the grid does not fit the GPU at once, the CTAs
     that start last are the short ones.
 
-    ``slots``: how many work items the GPU runs at once (per head).  If the items exceed it by
-    less than half, longer parts (up to twice KEY_CHUNK) are tried, so that a second round of a
-    few CTAs is not added to the first."""
+    ``slots``: how many work items the GPU runs at once (per head).  Where parts of KEY_CHUNK do not all fit at once, longer
+    parts (up to twice KEY_CHUNK) and whole runs are weighed against them: by the longest item, and the sum of all items
+    over the slots where there are several rounds, with ITEM_BLOCKS for what an item costs besides its key blocks and
+    MERGE_BLOCKS more where its results have to be merged.  (16 heads, 2,048 tokens, one CTA an SM: 9 slots a head; whole
+    runs, 16 items of up to 32 blocks, take 0.6 of the time of 40 parts.)"""
 
     runs = []                                     # (request, first row, rows, keys it may see)
     row = 0
@@ -33,16 +38,20 @@ def query_tiles(q_lens, ctx_befores, slots=None):
             runs.append((r, row + b, rows, before + b + rows))
         row += n
 
-    def count(limit):
-        return sum(max(1, -(-keys // limit)) for _, _, _, keys in runs)
-
     limit = KEY_CHUNK
-    items = count(limit)
-    if slots and slots < items <= slots + slots // 2:
-        for longer in range(KEY_CHUNK + QUERY_TILE, 2 * KEY_CHUNK + 1, QUERY_TILE):
-            if count(longer) <= slots:
-                limit = longer
-                break
+    if slots and sum(max(1, -(-keys // limit)) for _, _, _, keys in runs) > slots:
+        best = None
+        for longer in (*range(KEY_CHUNK, 2 * KEY_CHUNK + 1, QUERY_TILE), 1 << 30):
+            items, total, longest = 0, 0, 0
+            for _, _, _, keys in runs:
+                chunks, blocks = max(1, -(-keys // longer)), -(-keys // KEY_BLOCK)
+                besides = ITEM_BLOCKS + (MERGE_BLOCKS if chunks > 1 else 0)
+                items += chunks
+                total += blocks + chunks * besides
+                longest = max(longest, -(-blocks // chunks) + besides)
+            cost = longest if items <= slots else max(longest, total / slots) + 0.3 * longest
+            if best is None or cost < best:
+                best, limit = cost, longer
     cut = []
     for i, (r, row0, rows, keys) in enumerate(runs):
         chunks = max(1, -(-keys // limit))

@@ -145,7 +145,7 @@ def load(verbose: bool = True):
             raise KernelLibraryError(f"the kernel library lacks {name}; rebuild it") from None
         fn.argtypes = argtypes
         fn.restype = c_int
-    lib.mg_attention_prefill_scratch_floats.argtypes = [c_int, c_int]
+    lib.mg_attention_prefill_scratch_floats.argtypes = [c_int, c_int, c_int]
     lib.mg_attention_prefill_scratch_floats.restype = ctypes.c_longlong
     lib.mg_argmax_parts.argtypes = [c_int]
     lib.mg_argmax_parts.restype = c_int

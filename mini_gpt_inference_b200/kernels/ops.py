@@ -806,13 +806,13 @@ class CudaOps:
 
     SPLIT_HEAD_DIMS = (16, 32, 64, 128, 256)
 
-    PREFILL_TC_HEAD_DIMS = (64,)
+    PREFILL_TC_HEAD_DIMS = (64, 128)
 
-    def _attention_tiles_name(self, n_head: int) -> str:
+    def _attention_tiles_name(self, n_head: int, head_dim: int) -> str:
         if self._sm_count is None:
             self._sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
-        # work items of the tiled kernel that run at once, per head (two CTAs per SM)
-        return f"attention_tiles/{max(1, 2 * self._sm_count // n_head)}"
+        # work items of the tiled kernel that run at once, per head (two CTAs per SM for heads of 64, one for 128)
+        return f"attention_tiles/{max(1, (2 if head_dim == 64 else 1) * self._sm_count // n_head)}"
 
     def plan_prompt_attention(self, batch, plan, n_head, n_kv_head, head_dim) -> None:
         """Host half of the tiled prompt attention: the work list of a step (``attention_plan``),
@@ -821,7 +821,7 @@ class CudaOps:
         if (batch.decode_only or batch.act_dtype != torch.bfloat16 or not self.use_tensor_cores
                 or not self.use_prefill_tc or head_dim not in self.PREFILL_TC_HEAD_DIMS):
             return
-        name = self._attention_tiles_name(n_head)
+        name = self._attention_tiles_name(n_head, head_dim)
         if name not in plan.arrays:
             import numpy as np
 
@@ -859,17 +859,17 @@ class CudaOps:
             # a grid of several waves merges in a kernel of its own
             self.launches += self.lib.mg_attention_split_launches(n, n_head, n_kv_head, splits) - 1
             return out
-        work = getattr(ctx, "extra", {}).get(self._attention_tiles_name(n_head))
+        work = getattr(ctx, "extra", {}).get(self._attention_tiles_name(n_head, head_dim))
         if (qkv.dtype == torch.bfloat16 and work is not None and work.shape[0] > 0
                 and self.use_tensor_cores and self.use_prefill_tc
                 and head_dim in self.PREFILL_TC_HEAD_DIMS):
-            # portions of prompts: query tiles of 128 on the tensor cores
+            # portions of prompts: query tiles of 128 on the tensor cores (heads of 64 and 128)
             self._want(work, torch.int32, "attention tiles", 2)
             # tiles cut along the keys leave partial rows in scratch; the part that finishes last merges them
             merge = int(ctx.max_ctx_after > KEY_CHUNK)
             partial = counters = None
             if merge:
-                floats = self.lib.mg_attention_prefill_scratch_floats(work.shape[0], n_head)
+                floats = self.lib.mg_attention_prefill_scratch_floats(work.shape[0], n_head, head_dim)
                 partial = torch.empty((floats,), dtype=torch.float32, device=self.device)
                 counters = self._counters(work.shape[0] * n_head)
             code = self.lib.mg_attention_prefill_tc(
@@ -883,8 +883,7 @@ class CudaOps:
                 return out
         if qkv.dtype == torch.bfloat16 and self.use_tensor_cores and self.use_mma_attention:
             # heads that neither of the two kernels above takes (up to 128 features, a multiple of 8): tiles of the
-            # warp-level tensor cores, their softmax weights as two bfloat16 numbers each.  A prompt of 2,048 tokens,
-            # 16 heads of 128: 0.28 ms a layer; the kernel of a warp per token and head, 18 ms.
+            # warp-level tensor cores, their softmax weights as two bfloat16 numbers each.
             args = self._mma_plan(n, n_head, n_kv_head, head_dim, window, 0, 0, ctx)
             if args is not None:
                 code = self.lib.mg_attention_mma(
@@ -977,7 +976,7 @@ class CudaOps:
                                  or gate.shape != (n, n_head * v_dim)):
             raise KernelLibraryError("attention: the gate does not fit the heads")
         out = torch.empty((n, n_head * v_dim), dtype=q.dtype, device=self.device)
-        work = getattr(ctx, "extra", {}).get(self._attention_tiles_name(n_head)) if hasattr(ctx, "extra") else None
+        work = getattr(ctx, "extra", {}).get(self._attention_tiles_name(n_head, head_dim)) if hasattr(ctx, "extra") else None
         if (q.dtype == torch.bfloat16 and work is not None and work.shape[0] > 0 and head_dim == v_dim and not biased
                 and plain and head_dim in self.PREFILL_TC_HEAD_DIMS and self.use_tensor_cores and self.use_prefill_tc
                 and not getattr(ctx, "decode_only", False)):
@@ -986,7 +985,7 @@ class CudaOps:
             merge = int(ctx.max_ctx_after > KEY_CHUNK)
             partial = counters = None
             if merge:
-                floats = self.lib.mg_attention_prefill_scratch_floats(work.shape[0], n_head)
+                floats = self.lib.mg_attention_prefill_scratch_floats(work.shape[0], n_head, head_dim)
                 partial = torch.empty((floats,), dtype=torch.float32, device=self.device)
                 counters = self._counters(work.shape[0] * n_head)
             code = self.lib.mg_attention_prefill_tc(

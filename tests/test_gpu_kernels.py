@@ -810,6 +810,28 @@ def test_heads_of_other_sizes_on_the_warp_level_tensor_cores(ops, n_head, n_kv_h
     assert (got - want).norm() <= 1.03 * (general - want).norm()
 
 
+@pytest.mark.parametrize("n_head,n_kv_head,page_tokens,window", [(4, 4, 64, 0), (6, 2, 16, 0), (3, 1, 128, 200), (2, 2, 8, 33)])
+def test_prompt_portions_of_heads_of_128_on_the_tensor_cores(ops, n_head, n_kv_head, page_tokens, window):
+    """Whole prompts, later portions, single tokens among them, tiles cut along the keys: no further from the 64-bit result
+    than the kernel of a warp per token and head, whose softmax weights are 32-bit numbers."""
+    lengths = [1, 64, 129, 300, 1100, 700]
+    q_lens = [1, 64, 129, 150, 130, 1]
+    args = (ops, torch.bfloat16, n_head, n_kv_head, 128, page_tokens, window, lengths, q_lens)
+    ops.use_mma_attention = False
+    try:
+        got, want = _attention_case(*args, seed=9)
+        ops.use_prefill_tc = False
+        general, _ = _attention_case(*args, seed=9)
+    finally:
+        ops.use_mma_attention = ops.use_prefill_tc = True
+    ops.check_status()
+    assert not torch.equal(got, general), "the two kernels were expected to differ in rounding"
+    assert not torch.isnan(got).any()
+    assert (got - want).abs().max() <= _tol(torch.bfloat16, 1.0)
+    # (nearly all of either error is the outputs' rounding to bfloat16, see above)
+    assert (got - want).norm() <= 1.03 * (general - want).norm()
+
+
 @pytest.mark.parametrize("gain", [4.0, 9.0, 24.0])
 def test_prompt_attention_with_a_key_far_above_the_others(ops, gain):
     """One key, hundreds of positions into the prompt, scores 8 * gain above the rest (head 0; other
