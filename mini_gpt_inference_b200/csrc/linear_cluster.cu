@@ -1,4 +1,4 @@
-// Projection of a few dozen tokens (decoding at batch 17 to 128): out[m, n] = x[m, :] . w[n, :].
+// Projection of a few dozen tokens (decoding at batch 17 to 64): out[m, n] = x[m, :] . w[n, :].
 //
 // At this size a projection is still a stream over the weights, but the activations are no
 // longer small: 64 tokens of width 2048 are 256 KB, too much for every CTA to stage whole, and a
@@ -22,7 +22,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int MAX_M = 128;
+constexpr int MAX_M = 64;
 constexpr int TILE_N = 8;            // weight rows per warp
 constexpr int WARPS = 8;             // tiles per cluster
 constexpr int THREADS = WARPS * 32;
@@ -37,16 +37,15 @@ struct ClusterArgs {
     int xstride;                     // bytes between staged activation rows
 };
 
-// MG: groups of 16 tokens held: 2, 4, 6 or 8.  NTW: tiles of 8 weight rows per warp (2 for matrices of
+// MG: groups of 16 tokens held: 2 or 4.  NTW: tiles of 8 weight rows per warp (2 for matrices of
 // so many rows that one tile per warp would need several rounds of CTAs: half the CTAs, and a
 // fragment of the activations feeds two tiles).
 template <int MG, int NTW>
 __global__ void __launch_bounds__(THREADS, 2) linear_cluster_kernel(const ClusterArgs a) {
     constexpr int MT = MG * 16;
     constexpr int CTILES = WARPS * NTW;                                            // tiles per cluster
-    // k blocks (of 32) whose weights a lane holds at once: fewer where the sums take more registers,
-    // so that two CTAs still share an SM
-    constexpr int PRE = (MG <= 4 ? 8 : 4) / NTW;
+    // k blocks (of 32) whose weights a lane holds at once (two CTAs share an SM)
+    constexpr int PRE = 8 / NTW;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int ranks = a.ranks;
@@ -202,7 +201,7 @@ MG_API int mg_linear_cluster_max_rows() { return MAX_M; }
 MG_GUARD_EXPORT(linear_cluster, linear_index_fault)
 
 // x: [M, K] bf16; w: [N, K] bf16; epilogues and the key/value sink as mg_linear_skinny.
-// Returns MG_ERR_UNSUPPORTED (nothing launched) for M > 128, K % 8 != 0, operands that are not
+// Returns MG_ERR_UNSUPPORTED (nothing launched) for M > 64, K % 8 != 0, operands that are not
 // 16-byte aligned or a slice of activations beyond the shared memory.
 MG_API int mg_linear_cluster(const void* x, const void* w, const float* bias, void* out, float* residual, int M, int N,
                              int K, int epilogue, int out_bf16, void* k_pages, void* v_pages, const int* slots,
@@ -219,14 +218,13 @@ MG_API int mg_linear_cluster(const void* x, const void* w, const float* bias, vo
     const int per_rank = (kblocks + ranks - 1) / ranks;
     const int slice_bytes = per_rank * 64;
     const int xstride = slice_bytes + (slice_bytes % 128 == 0 ? 64 : 0);               // rows 64 bytes apart mod 128
-    const int mg = M <= 32 ? 2 : M <= 64 ? 4 : M <= 96 ? 6 : 8;
+    const int mg = M <= 32 ? 2 : 4;
     const int tiles = (N + TILE_N - 1) / TILE_N;
-    // two tiles per warp where one would make more CTAs than two rounds of them hold (up to 64 tokens:
-    // beyond, the sums of two tiles do not fit the registers beside two CTAs per SM)
-    const int ntw = (mg <= 4 && (long long)((tiles + WARPS - 1) / WARPS) * ranks > 2 * 296) ? 2 : 1;
+    // two tiles per warp where one would make more CTAs than two rounds of them hold
+    const int ntw = ((long long)((tiles + WARPS - 1) / WARPS) * ranks > 2 * 296) ? 2 : 1;
     const size_t smem = (size_t)mg * 16 * xstride + (size_t)WARPS * ntw * mg * 16 * TILE_N * sizeof(float);
     if (M > MAX_M || K % 8 != 0 || smem > 200 * 1024 || ((uintptr_t)w & 15) || ((uintptr_t)x & 15))
-        return mg_set_error(MG_ERR_UNSUPPORTED, "linear (cluster): needs M <= 128, K %% 8 == 0, aligned operands");
+        return mg_set_error(MG_ERR_UNSUPPORTED, "linear (cluster): needs M <= 64, K %% 8 == 0, aligned operands");
     ClusterArgs a;
     a.x = (const bf16*)x; a.w = (const bf16*)w; a.K = K; a.ranks = ranks; a.per_rank = per_rank; a.xstride = xstride;
     a.ep.bias = bias; a.ep.out = out; a.ep.residual = residual; a.ep.M = M; a.ep.N = N;
@@ -235,8 +233,7 @@ MG_API int mg_linear_cluster(const void* x, const void* w, const float* bias, vo
     a.ep.q_width = q_width; a.ep.n_kv_head = n_kv_head; a.ep.head_dim = head_dim; a.ep.page_tokens = page_tokens; a.ep.num_pages = num_pages;
     void (*kernel)(const ClusterArgs) = nullptr;
     if (ntw == 2) kernel = mg == 2 ? linear_cluster_kernel<2, 2> : linear_cluster_kernel<4, 2>;
-    else kernel = mg == 2 ? linear_cluster_kernel<2, 1> : mg == 4 ? linear_cluster_kernel<4, 1>
-                  : mg == 6 ? linear_cluster_kernel<6, 1> : linear_cluster_kernel<8, 1>;
+    else kernel = mg == 2 ? linear_cluster_kernel<2, 1> : linear_cluster_kernel<4, 1>;
     {
         // (once per variant: the attribute is cheap to set again)
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);

@@ -22,8 +22,7 @@ PLAIN_ACTIVATIONS = {"relu_sq": 0, "gelu_tanh": 1, "silu": 2}           # ... an
 GATED_ACTIVATIONS = {"silu": 0, "clamped_swish": 1, "gelu_tanh": 2}     # the gated product of a unit's two halves
 MOE_FEW_TOKENS = 16      # most tokens the experts' kernels for few tokens take
 SKINNY_ROWS = 16         # most tokens the small-batch projection kernel takes
-CLUSTER_ROWS = 128       # most tokens the mid-batch (K split over a cluster) projection kernel takes
-CLUSTER_WIDE_MAX_BYTES = 3 << 20   # ... and the largest matrix it is given for more than 64 tokens
+CLUSTER_ROWS = 64        # most tokens the mid-batch (K split over a cluster) projection kernel takes
 PREFETCH_MAX_BYTES = 32 << 20   # most of a following matrix that a streaming projection asks into L2
 STREAM_MIN_ROWS = 8192   # a matrix this tall (the head) goes through the streaming kernel ...
 STREAM_ROWS = 16         # ... for up to this many tokens (it takes 64; beyond 16 the tensor-core GEMM measured faster)
@@ -521,6 +520,17 @@ class CudaOps:
                 and SKINNY_ROWS * (2 * k + 64) + 8 * SKINNY_ROWS * 8 * 4 + 8 * k <= 200 * 1024)
 
     @staticmethod
+    def _cluster_pays(m, n, k) -> bool:
+        """Whether a bfloat16 product of 17 to 64 tokens is left to the kernel that cuts K over a cluster: its time grows with
+        the tokens and the matrix, that of the tensor-core GEMM with K alone.  Microseconds, cluster / GEMM, at 32 tokens:
+        512 x 128 4.2 / 3.2, 512 x 256 3.3 / 3.4, 2,048 x 512 3.8 / 4.3, 512 x 2,048 3.6 / 6.1, 1,600 x 6,400 11.3 / 16.2, but
+        2,304 x 768 6.4 / 4.9; at 64: 512 x 512 4.3 / 3.7, 2,048 x 512 5.7 / 4.2, 256 x 1,024 4.4 / 4.4, 512 x 2,048 5.6 / 6.1,
+        1,600 x 6,400 26 / 16.  Matrices of one tile (128 rows) stay here, 2.7 / 3.4 and 3.8 / 3.5 at K = 512."""
+        if n <= 128:
+            return True
+        return (n <= 2048 and k >= 256) if m <= 32 else (n <= 512 and k >= 1024)
+
+    @staticmethod
     def _sink_args(kv_sink):
         """The key/value sink of a QKV projection as the C functions take it."""
         if kv_sink is None:
@@ -638,12 +648,7 @@ class CudaOps:
         if deferred is not None:
             x = deferred.materialize()
         self._want(x, weight.dtype, "linear input", 2)
-        # (a matrix of thousands of 8-row tiles, the head, is left to the tensor-core GEMM: every one
-        # of its clusters would stage the activations and meet at a barrier for a few KB of weights)
-        # (and beyond 64 tokens it keeps only matrices of up to 3 MB: measured with 96 and 128 tokens, it
-        # is faster than the tensor-core GEMM at 512 x 2048, slower from 3 x 768 x 768 elements on)
-        if (x.dtype == torch.bfloat16 and self.use_cluster and 0 < m <= CLUSTER_ROWS and k % 8 == 0
-                and n <= 8192 and (m <= 64 or 2 * n * k <= CLUSTER_WIDE_MAX_BYTES)):
+        if x.dtype == torch.bfloat16 and self.use_cluster and 0 < m <= CLUSTER_ROWS and k % 8 == 0 and self._cluster_pays(m, n, k):
             sink = self._sink_args(kv_sink)
             code = self.lib.mg_linear_cluster(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(residual),
                                               m, n, k, epilogue, out_bf16, *sink, self._stream())
