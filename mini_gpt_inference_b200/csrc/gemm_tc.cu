@@ -32,6 +32,7 @@
 #include <unordered_map>
 
 #include "blackwell.cuh"
+#include "moe_units.cuh"
 #include "tensor_map.cuh"
 
 MG_STAMP_DECLARE(gemm)
@@ -75,6 +76,12 @@ struct KvSink {
     int num_pages;                   // pages of the pool (what a cache row is held against in guarded builds)
 };
 
+// What the products are of.
+constexpr int PLAIN = 0;             // one matrix
+constexpr int HEADS = 1;             // a small matrix per head: columns a_off + h * a_head .. of A give columns o_off + h * o_head .. of D
+constexpr int EXPERTS = 2;           // a matrix per expert: rows offsets[e] .. offsets[e + 1] of A (and D) belong to expert e
+constexpr int MAX_EXPERTS = 256;
+
 struct GemmArgs {
     const float* bias;
     void* out;                       // [M, N] bf16 or 32-bit; the residual stream for EPI_RESIDUAL
@@ -83,9 +90,24 @@ struct GemmArgs {
     int boxes;                       // rows of the output are multiples of 16 bytes: stored by TMA
     KvSink sink;
     int* status;
+    int ld_out;                      // elements between rows of D
+    int heads, a_off, a_head, o_off, o_head;               // HEADS; N and K are a head's
+    // EXPERTS: form 0 (32-bit results), 1 (gated: a matrix has N gate rows, then N up rows), 2 (activation), as in moe.cu;
+    // scale: factor on the sums of row r's entry, slot_entry[r] (null: none)
+    const int* offsets;
+    const int* slot_entry;
+    const float* scale;
+    int n_experts, form, act;
+    float limit;
 };
 
-template <int CG, int SUB>
+// A tile's place: first row of this CTA's part of A (and D), columns of A, rows of B, columns of a head's or matrix's results
+// and of D, and the row of D behind its last.
+struct Place {
+    int row, a_col, b_row, n0, out_col, rows_end;
+};
+
+template <int CG, int SUB, int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_out, const GemmArgs g) {
@@ -102,12 +124,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (the same register value in all lanes)
     const int rank = CG == 2 ? (int)cluster_rank() : 0;
-    const int m_tiles = (g.M + CG * TILE_M - 1) / (CG * TILE_M), n_tiles = (g.N + bn - 1) / bn;
-    const int tiles = m_tiles * n_tiles, first_tile = (int)blockIdx.x / CG, tile_step = (int)gridDim.x / CG;
+    const bool glu = MODE == EXPERTS && g.form == 1;         // bn / 2 gate columns, then the up columns of the same results
+    const int bn_out = glu ? bn / 2 : bn;                    // results a tile has
+    int m_tiles = (g.M + CG * TILE_M - 1) / (CG * TILE_M);
+    const int n_tiles = (g.N + bn_out - 1) / bn_out;
+    int tiles = m_tiles * n_tiles * (MODE == HEADS ? g.heads : 1);
+    const int first_tile = (int)blockIdx.x / CG, tile_step = (int)gridDim.x / CG;
+    __shared__ int expert_row[MODE == EXPERTS ? MAX_EXPERTS + 1 : 1], expert_tile[MODE == EXPERTS ? MAX_EXPERTS + 1 : 1];
     const int num_kb = (g.K + SUB * BLOCK_K - 1) / (SUB * BLOCK_K);     // stages' worth of K
-    const bool twice = tiles > tile_step;                    // some CTA has several tiles: two accumulators
+    const bool twice = MODE == EXPERTS || tiles > tile_step;                    // some CTA has several tiles: two accumulators
     uint32_t tmem_cols = 32;
     while (tmem_cols < (uint32_t)(twice ? 2 * bn : bn)) tmem_cols *= 2;
+
+    auto place_of = [&](int tile) {
+        Place p;
+        if (MODE == EXPERTS) {
+            const int mt = tile % m_tiles, nt = tile / m_tiles;
+            int e = 0;
+            for (int half = MAX_EXPERTS; half > 0; half >>= 1)             // the last expert whose tiles begin at or before mt
+                if (e + half < g.n_experts && expert_tile[e + half] <= mt) e += half;
+            p.row = expert_row[e] + (mt - expert_tile[e]) * TILE_M;
+            p.rows_end = expert_row[e + 1];
+            p.a_col = 0;
+            p.n0 = p.out_col = nt * bn_out;
+            p.b_row = e * (glu ? 2 : 1) * g.N + p.n0;
+            return p;
+        }
+        int nt = tile / m_tiles;
+        const int h = MODE == HEADS ? nt / n_tiles : 0;
+        nt -= h * n_tiles;
+        p.row = (tile % m_tiles) * CG * TILE_M + rank * TILE_M;
+        p.rows_end = g.M;
+        p.n0 = nt * bn;
+        p.a_col = MODE == HEADS ? g.a_off + h * g.a_head : 0;
+        p.b_row = (MODE == HEADS ? h * g.N : 0) + p.n0 + rank * b_rows;
+        p.out_col = (MODE == HEADS ? g.o_off + h * g.o_head : 0) + p.n0;
+        return p;
+    };
 
     MG_STAMP(gemm, 0);
     if (tid == 0) {
@@ -133,10 +186,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // first round of stages are asked for before it.
     MG_STAMP(gemm, 2);
     pdl_trigger();
-    const int early = num_kb < stages ? num_kb : stages;
+    // (Which experts have rows is the kernel in front's to say: nothing of theirs is asked for before it.)
+    const int early = MODE == EXPERTS ? 0 : num_kb < stages ? num_kb : stages;
     const bool loads = warp == EPI_WARPS, issues = warp == EPI_WARPS + 1;
-    if (loads && elect_one()) {
-        const int n0 = (first_tile / m_tiles) * bn + rank * b_rows;
+    if (MODE != EXPERTS && loads && elect_one()) {
+        const int n0 = place_of(first_tile).b_row;
         for (int kb = 0; kb < early; ++kb) {
             const uint32_t full = smem_u32(&ctl->full[kb]), tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
             if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
@@ -146,6 +200,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     pdl_wait();
     MG_STAMP(gemm, 3);
+    if (MODE == EXPERTS) {
+        for (int e = tid; e <= g.n_experts; e += THREADS) expert_row[e] = g.offsets[e];
+        __syncthreads();
+        for (int e = tid; e <= g.n_experts; e += THREADS) {
+            int before = 0;
+            for (int i = 0; i < e; ++i) before += (expert_row[i + 1] - expert_row[i] + TILE_M - 1) / TILE_M;
+            expert_tile[e] = before;
+        }
+        __syncthreads();
+        m_tiles = expert_tile[g.n_experts];
+        tiles = m_tiles * n_tiles;
+    }
 
     // A single thread runs each of the next two loops, and the chain of its instructions is what bounds small tiles: some
     // 300 clocks a stage, whatever its size.  So the ring's place and parity are carried along (the two divisions that found
@@ -158,13 +224,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             uint32_t parity = 1;
             bool ok = true;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
-                const int m0 = (tile % m_tiles) * CG * TILE_M + rank * TILE_M, n0 = (tile / m_tiles) * bn + rank * b_rows;
+                const Place p = place_of(tile);
+                const int m0 = p.row, n0 = p.b_row, k0 = p.a_col;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     const uint32_t full = smem_u32(&ctl->full[s]), stage = smem_u32(smem) + s * stage_bytes;
                     if (ahead > 0) {
                         --ahead;
 #pragma unroll
-                        for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, (kb * SUB + i) * BLOCK_K, m0);
+                        for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
                     } else {
                         if (!mbar_wait(smem_u32(&ctl->empty[s]), parity)) {
                             atomicExch(g.status, 1);
@@ -175,8 +242,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
 #pragma unroll
                         for (int i = 0; i < SUB; ++i) {
-                            tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, (kb * SUB + i) * BLOCK_K, m0);
+                            tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
                             tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
+                            if (glu)                         // (the map's boxes are bn / 2 rows high)
+                                tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes + b_tile_bytes / 2, &map_b, full,
+                                                      (kb * SUB + i) * BLOCK_K, n0 + g.N);
                         }
                     }
                     if (++s == stages) { s = 0; parity ^= 1; }
@@ -230,7 +300,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int used = 0, round = 0;                             // boxes filled so far, tiles done so far
         for (int tile = first_tile; tile < tiles; tile += tile_step, ++round) {
             const int a = twice ? round & 1 : 0;
-            const int row0 = (tile % m_tiles) * CG * TILE_M + rank * TILE_M + quarter * 32, n0 = (tile / m_tiles) * bn;
+            const Place p = place_of(tile);
+            const int row0 = p.row + quarter * 32, n0 = p.n0, out_col = p.out_col;
+            float row_scale = 1.f;
+            if (MODE == EXPERTS && g.scale != nullptr && row0 + lane < p.rows_end) row_scale = g.scale[g.slot_entry[row0 + lane]];
             // asked for while the products run: the cache row of this lane's token
             long long kv_row = -1;                           // the cache row's first element for kv head 0, in head rows
             if (g.sink.k_pages != nullptr && n0 + bn > g.sink.q_width && row0 + lane < g.M) {
@@ -248,7 +321,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tc_fence_after();
             MG_STAMP(gemm, 5);
             const uint32_t lane_addr = tmem_base + a * bn + ((uint32_t)(quarter * 32) << 16);
-            const int columns = min(bn, g.N - n0);
+            const int columns = min(bn_out, g.N - n0);
             // all of the accumulator's columns that are this warp's are in registers: the next tile's products may overwrite them
             auto release = [&] {
                 tc_fence_before();
@@ -279,7 +352,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tmem_wait_ld();
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r[j]);
-                    if (g.epilogue == EPI_GELU) {
+                    if (MODE == EXPERTS) {
+                        if (glu) {
+                            tmem_load_32(lane_addr + (uint32_t)(bn_out + c0 + half), r);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = gated_value(g.act, g.limit, v[j] * row_scale, __uint_as_float(r[j]) * row_scale);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = g.form == 2 ? plain_value(g.act, v[j] * row_scale) : v[j] * row_scale;
+                        }
+                    } else if (g.epilogue == EPI_GELU) {
                         // results that become bfloat16 take the hardware tanh; 32-bit results the exact one
                         if (g.out_bf16) {
 #pragma unroll
@@ -311,25 +394,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
                 if (c0 + 2 * per_box >= columns) release();
-                if (g.boxes) async_proxy_fence();
+                // (the rows behind an expert's last are the next expert's: such a box is not stored as one)
+                const bool as_box = g.boxes && (MODE != EXPERTS || row0 + 32 <= p.rows_end);
+                if (as_box) async_proxy_fence();
                 __syncwarp();
-                if (g.boxes) {
+                if (as_box) {
                     if (lane == 0) {
                         if (row0 < g.M) {
-                            if (g.epilogue == EPI_RESIDUAL) tma_add_2d(&map_out, smem_u32(box), n0 + c0, row0);
-                            else tma_store_2d(&map_out, smem_u32(box), n0 + c0, row0);
+                            if (g.epilogue == EPI_RESIDUAL) tma_add_2d(&map_out, smem_u32(box), out_col + c0, row0);
+                            else tma_store_2d(&map_out, smem_u32(box), out_col + c0, row0);
                         }
                         tma_store_commit();
                     }
                 } else {
+                    if (g.boxes && lane == 0) tma_store_commit();            // (an empty group keeps the count of boxes in use)
                     // rows that TMA cannot address: a row's columns from neighbouring lanes
-                    const int wide = min(per_box, columns - c0), high = min(32, g.M - row0);
+                    const int wide = min(per_box, columns - c0), high = min(32, p.rows_end - row0);
                     for (int j = lane; j < wide; j += 32) {
                         const int byte = g.out_bf16 ? 2 * j : 4 * j;
 #pragma unroll 8
                         for (int i = 0; i < high; ++i) {
                             const uint8_t* from = box + i * 128 + (((byte >> 4) ^ (i & 7)) << 4) + (byte & 15);
-                            const size_t to = (size_t)(row0 + i) * g.N + n0 + c0 + j;
+                            const size_t to = (size_t)(row0 + i) * g.ld_out + out_col + c0 + j;
                             if (g.out_bf16) ((bf16*)g.out)[to] = *reinterpret_cast<const bf16*>(from);
                             else if (g.epilogue == EPI_RESIDUAL) atomicAdd((float*)g.out + to, *reinterpret_cast<const float*>(from));
                             else ((float*)g.out)[to] = *reinterpret_cast<const float*>(from);
@@ -407,27 +493,36 @@ inline Cut choose_cut(int M, int N, int K, bool out_bf16) {
     return best;
 }
 
-template <int CG, int SUB>
-int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s) {
+// Rows and columns of A, rows of B and columns of D in memory, where they are not those of one product.
+struct Extent {
+    int a_rows, a_cols, b_rows;
+    long long tiles;                 // the most there can be
+};
+
+template <int CG, int SUB, int MODE>
+int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s, const Extent* extent = nullptr) {
+    const bool glu = MODE == EXPERTS && g.form == 1;
+    if (MODE == PLAIN) g.ld_out = g.N;
     CUtensorMap map_a, map_b, map_out = {};
-    int rc = tensor_map(a, g.M, g.K, TILE_M, &map_a);
+    int rc = tensor_map(a, MODE == PLAIN ? g.M : extent->a_rows, MODE == PLAIN ? g.K : extent->a_cols, TILE_M, &map_a);
     if (rc != MG_OK) return rc;
-    rc = tensor_map(b, g.N, g.K, g.bn / CG, &map_b);
+    rc = tensor_map(b, MODE == PLAIN ? g.N : extent->b_rows, g.K, glu ? g.bn / 2 : g.bn / CG, &map_b);
     if (rc != MG_OK) return rc;
-    if (g.boxes && (rc = tensor_map_store(g.out, g.M, g.N, 32, !g.out_bf16, &map_out)) != MG_OK) return rc;
+    if (g.boxes && (rc = tensor_map_store(g.out, g.M, g.ld_out, 32, !g.out_bf16, &map_out)) != MG_OK) return rc;
     const int stage_bytes = SUB * (A_TILE_BYTES + g.bn / CG * BLOCK_K * 2);
     const int num_kb = ceil_div(g.K, SUB * BLOCK_K);
-    const long long tiles = (long long)ceil_div(g.M, CG * TILE_M) * ceil_div(g.N, g.bn);
-    const size_t fixed = EPI_WARPS * BOXES * BOX_BYTES + sizeof(Control) + 1024;
+    const long long tiles = MODE == PLAIN ? (long long)ceil_div(g.M, CG * TILE_M) * ceil_div(g.N, g.bn) : extent->tiles;
+    const size_t fixed = EPI_WARPS * BOXES * BOX_BYTES + sizeof(Control) + 1024 + (MODE == EXPERTS ? 2 * 4 * (MAX_EXPERTS + 1) + 64 : 64);
     constexpr size_t most = 227 * 1024;
     if (g.stages == 0) g.stages = (int)((most - fixed) / stage_bytes);
     if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
     if (tiles <= SMS / CG && g.stages > num_kb) g.stages = num_kb;
-    const size_t smem = (size_t)g.stages * stage_bytes + fixed;
+    const size_t smem = (size_t)g.stages * stage_bytes + EPI_WARPS * BOXES * BOX_BYTES + sizeof(Control) + 1024;
+    constexpr size_t most_dynamic = most - (MODE == EXPERTS ? 2 * 4 * (MAX_EXPERTS + 1) + 64 : 64);
     static std::once_flag configured;
     static cudaError_t e = cudaSuccess;
     std::call_once(configured, [] {
-        e = cudaFuncSetAttribute(gemm_tc_kernel<CG, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        e = cudaFuncSetAttribute(gemm_tc_kernel<CG, SUB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_dynamic);
     });
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear: cannot raise shared memory: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
@@ -450,7 +545,7 @@ int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<CG, SUB>, map_a, map_b, map_out, g);
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<CG, SUB, MODE>, map_a, map_b, map_out, g);
     if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "gemm_tc: %s", cudaGetErrorString(le));
     MG_CHECK_LAUNCH("gemm_tc");
     return MG_OK;
@@ -491,6 +586,52 @@ MG_API int mg_linear_tc(const void* x, const void* w, const float* bias, void* o
     MG_REQUIRE((long long)ceil_div(M, cut.cg * TILE_M) * ceil_div(N, cut.bn) < (1ll << 30), "linear: too many tiles");
     g.bn = cut.bn;
         cudaStream_t s = (cudaStream_t)stream;
-    if (cut.cg == 2) return cut.sub == 2 ? launch<2, 2>(x, w, g, s) : launch<2, 1>(x, w, g, s);
-    return cut.sub == 2 ? launch<1, 2>(x, w, g, s) : launch<1, 1>(x, w, g, s);
+    if (cut.cg == 2) return cut.sub == 2 ? launch<2, 2, PLAIN>(x, w, g, s) : launch<2, 1, PLAIN>(x, w, g, s);
+    return cut.sub == 2 ? launch<1, 2, PLAIN>(x, w, g, s) : launch<1, 1, PLAIN>(x, w, g, s);
+}
+
+// One small product per head, bfloat16: out[m, o_off + h * o_head + n] = sum_k x[m, x_off + h * x_head + k] * w[h * N + n, k] for
+// n < N, k < K.  x: rows of x_ld elements, out: rows of out_ld.  Returns MG_ERR_UNSUPPORTED (and launches nothing) unless K and N
+// are multiples of 64 and the rows' parts lie on 16-byte boundaries (TMA).
+MG_API int mg_head_linear_tc(const void* x, int x_ld, int x_off, int x_head, const void* w, void* out, int out_ld, int out_off,
+                             int out_head, int M, int heads, int K, int N, int* status, void* stream) {
+    if (M == 0) return MG_OK;
+    MG_REQUIRE(M > 0 && heads > 0 && K > 0 && N > 0 && status != nullptr, "head_linear: bad sizes");
+    MG_REQUIRE(x_off >= 0 && x_head >= K && x_off + (long long)(heads - 1) * x_head + K <= x_ld && out_off >= 0 && out_head >= N &&
+                   out_off + (long long)(heads - 1) * out_head + N <= out_ld,
+               "head_linear: heads outside the rows");
+    if (K % 64 != 0 || N % 64 != 0 || x_ld % 8 != 0 || x_off % 8 != 0 || x_head % 8 != 0 || out_ld % 8 != 0 || out_off % 8 != 0 ||
+        out_head % 8 != 0 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) || (long long)heads * N > (1 << 30))
+        return mg_set_error(MG_ERR_UNSUPPORTED, "head_linear: no tensor-core tiles for %d x %d", K, N);
+    GemmArgs g = {};
+    g.out = out; g.out_bf16 = 1; g.boxes = 1; g.epilogue = EPI_STORE;
+    g.M = M; g.N = N; g.K = K; g.ld_out = out_ld; g.status = status;
+    g.heads = heads; g.a_off = x_off; g.a_head = x_head; g.o_off = out_off; g.o_head = out_head;
+    g.bn = N % 128 == 0 ? 128 : 64;
+    const Extent extent = {M, x_ld, heads * N, (long long)ceil_div(M, TILE_M) * heads * (N / g.bn)};
+    MG_REQUIRE(extent.tiles < (1ll << 30), "head_linear: too many tiles");
+    return launch<1, 1, HEADS>(x, w, g, (cudaStream_t)stream, &extent);
+}
+
+// The products of mg_moe_gemm on the tensor cores, rows by slot: x [n_entries, K] bfloat16 (a token's row for each of its
+// entries, gathered: mg_moe_gather), w [n_experts, N (2 N for form 1), K], out [n_entries, N] bfloat16 (forms 1 and 2) or 32-bit
+// (form 0).  Returns MG_ERR_UNSUPPORTED (and launches nothing) for sizes or alignments that TMA or the kernel do not take.
+MG_API int mg_moe_gemm_tc(const void* x, const void* w, const int* offsets, const int* slot_entry, const float* scale, void* out,
+                          int n_entries, int n_experts, int N, int K, int form, int act, float limit, int* status, void* stream) {
+    if (n_entries == 0) return MG_OK;
+    MG_REQUIRE(n_entries > 0 && n_experts > 0 && N > 0 && K > 0 && form >= 0 && form <= 2 && status != nullptr, "moe gemm: bad sizes");
+    const long long b_rows = (long long)n_experts * (form == 1 ? 2 : 1) * N;
+    if (K % 8 != 0 || n_experts > MAX_EXPERTS || b_rows > (1 << 30) || (((uintptr_t)x | (uintptr_t)w) & 15))
+        return mg_set_error(MG_ERR_UNSUPPORTED, "moe gemm: no tensor-core tiles for %d experts of %d x %d", n_experts, N, K);
+    GemmArgs g = {};
+    g.out = out; g.out_bf16 = form != 0; g.epilogue = EPI_STORE;
+    g.M = n_entries; g.N = N; g.K = K; g.ld_out = N; g.status = status;
+    g.boxes = N % (g.out_bf16 ? 8 : 4) == 0 && ((uintptr_t)out & 15) == 0;
+    g.offsets = offsets; g.slot_entry = slot_entry; g.scale = scale; g.n_experts = n_experts; g.form = form; g.act = act; g.limit = limit;
+    // 128 results a tile: at 6,144 slots x 1,024 x 1,024 448 tiles, three rounds
+    g.bn = form == 1 ? 256 : 128;
+    const int bn_out = form == 1 ? g.bn / 2 : g.bn;
+    const Extent extent = {n_entries, K, (int)b_rows, ((long long)n_entries / TILE_M + n_experts) * ceil_div(N, bn_out)};
+    MG_REQUIRE(extent.tiles < (1ll << 30), "moe gemm: too many tiles");
+    return launch<1, 1, EXPERTS>(x, w, g, (cudaStream_t)stream, &extent);
 }

@@ -598,6 +598,20 @@ moe_gemm_mma_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict_
         }
 }
 
+// ---- out[slot] = x[token of slot]: rows of 16-byte words, a warp per slot ---------------------------
+__global__ void __launch_bounds__(256)
+moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ offsets, int n_experts, const int* __restrict__ slot_entry,
+                  int top, uint4* __restrict__ out, int words, int x_rows) {
+    pdl_trigger();
+    pdl_wait();
+    const int slot = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (slot >= offsets[n_experts]) return;                // (padding rows have no slots)
+    const int row = slot_entry[slot] / top;
+    if (!MG_GUARDED(moe, MG_GUARD_ROW, row, x_rows)) return;
+#pragma unroll 4
+    for (int c = lane; c < words; c += 32) out[(size_t)slot * words + c] = x[(size_t)row * words + c];
+}
+
 // ---- x[token] += sum over the token's entries, in entry order ----------------------------------
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ entry_slot, int top,
                                    float* __restrict__ residual, int width, int n_slots) {
@@ -757,6 +771,18 @@ MG_API int mg_moe_gemm(const void* x, int ldx, const void* w, const int* offsets
                       scale, out, N, K, x_rows, act, limit);
     }
     MG_LAUNCHED(e, "moe gemm");
+    return MG_OK;
+}
+
+// x: [x_rows, width] bfloat16, width a multiple of 8 and both 16-byte aligned; out: [n_entries, width], rows by slot.
+MG_API int mg_moe_gather(const void* x, const int* offsets, int n_experts, const int* slot_entry, int top, void* out, int n_entries,
+                         int width, int x_rows, void* stream) {
+    if (n_entries == 0) return MG_OK;
+    MG_REQUIRE(n_entries > 0 && n_experts > 0 && top > 0 && width > 0 && width % 8 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0,
+               "moe gather: bad sizes");
+    const cudaError_t e = mg_launch(moe_gather_kernel, dim3(ceil_div(n_entries, 8)), dim3(256), 0, (cudaStream_t)stream, true,
+                                    (const uint4*)x, offsets, n_experts, slot_entry, top, (uint4*)out, width / 8, x_rows);
+    MG_LAUNCHED(e, "moe gather");
     return MG_OK;
 }
 

@@ -20,6 +20,9 @@ from .library import KernelLibraryError, check
 EPILOGUES = {"none": 0, "gelu_tanh": 1, "residual": 2, "relu_sq": 3}
 PLAIN_ACTIVATIONS = {"relu_sq": 0, "gelu_tanh": 1, "silu": 2}           # ... and the activation of a unit without a gate
 GATED_ACTIVATIONS = {"silu": 0, "clamped_swish": 1, "gelu_tanh": 2}     # the gated product of a unit's two halves
+MOE_TC_TOKENS = 64       # more tokens than this take the experts' tensor-core tiles ...
+MOE_TC_EXPERTS = 256     # ... for up to this many experts
+HEAD_TC_TOKENS = 64      # more tokens than this take the heads' small products on the tensor-core GEMM
 MOE_FEW_TOKENS = 16      # most tokens the experts' kernels for few tokens take
 SKINNY_ROWS = 16         # most tokens the small-batch projection kernel takes
 CLUSTER_ROWS = 64        # most tokens the mid-batch (K split over a cluster) projection kernel takes
@@ -1437,6 +1440,16 @@ class CudaOps:
             self._is_bf16(proj), self._stream()), "latent_pair_prepare")
         return out
 
+    def _head_rows(self, weight, n_head, n_in, n_out):
+        """The heads' matrices ``[n_head * n_in, n_out]``, whose rows are inputs, copied once with a row per output: a layout
+        change made when a matrix is first seen, not a computation of the step."""
+        key = ("head rows", weight.data_ptr())
+        hit = self._packed.get(key)
+        if hit is None or hit[0] is not weight:
+            hit = (weight, weight.view(n_head, n_in, n_out).transpose(1, 2).contiguous())
+            self._packed[key] = hit
+        return hit[1]
+
     def head_linear(self, x, x_off, x_head, weight, rows_are_inputs, n_head, n_in, n_out, gate=None, out=None, out_off=0,
                     out_head=None):
         """One small matrix per head: ``out[n, h, j] = sum_i x[n, h, i] * W_h[j, i]`` with ``weight``
@@ -1461,6 +1474,14 @@ class CudaOps:
             out_head = n_out if out_head is None else out_head
             if out.shape[0] != n:
                 raise KernelLibraryError("head_linear: one output row per token")
+        if (self.use_tensor_cores and gate is None and x.dtype == torch.bfloat16 and n > HEAD_TC_TOKENS and n_in % 64 == 0
+                and n_out % 64 == 0):
+            code = self.lib.mg_head_linear_tc(
+                _ptr(x), x.shape[1], x_off, x_head, _ptr(self._head_rows(weight, n_head, n_in, n_out) if rows_are_inputs else weight),
+                _ptr(out), out.shape[1], out_off, out_head, n, n_head, n_in, n_out, _ptr(self.status), self._stream())
+            if code != library.UNSUPPORTED:
+                self._run(code, "head_linear (tensor cores)")
+                return out
         self._run(self.lib.mg_head_linear(
             _ptr(x), x.shape[1], x_off, x_head, _ptr(weight), 1 if rows_are_inputs else 0, _ptr(gate),
             gate.stride(0) if gate is not None else 0, 1 if gate is not None and gate.shape[1] == n_head else 0, _ptr(out),
@@ -1609,6 +1630,21 @@ class CudaOps:
         self._run(self.lib.mg_moe_group(_ptr(ids), entries, experts, _ptr(offsets), _ptr(slot_entry), _ptr(entry_slot),
                                         self._stream()), "moe group")
         hidden = torch.empty((entries, inner), dtype=y.dtype, device=self.device)
+        if (self.use_tensor_cores and is_bf16 and n > MOE_TC_TOKENS and width % 8 == 0 and inner % 8 == 0
+                and experts <= MOE_TC_EXPERTS and not (_ptr(y) | _ptr(w_in) | _ptr(w_out)) % 16):
+            # many tokens: their rows gathered by slot, then the GEMM's tiles over each expert's rows
+            rows = torch.empty((entries, width), dtype=y.dtype, device=self.device)
+            self._run(self.lib.mg_moe_gather(_ptr(y), _ptr(offsets), experts, _ptr(slot_entry), top, _ptr(rows), entries, width, n,
+                                             self._stream()), "moe gather")
+            self._run(self.lib.mg_moe_gemm_tc(_ptr(rows), _ptr(w_in), _ptr(offsets), _ptr(slot_entry),
+                                              _ptr(weights) if weigh_input else None, _ptr(hidden), entries, experts, inner, width,
+                                              1 if gated else 2, act, float(limit), _ptr(self.status), self._stream()),
+                      "moe experts (in, tensor cores)")
+            out = torch.empty((entries, width), dtype=torch.float32, device=self.device)
+            self._run(self.lib.mg_moe_gemm_tc(_ptr(hidden), _ptr(w_out), _ptr(offsets), _ptr(slot_entry),
+                                              None if weigh_input else _ptr(weights), _ptr(out), entries, experts, width, inner, 0,
+                                              0, 0.0, _ptr(self.status), self._stream()), "moe experts (out, tensor cores)")
+            return EntrySum(out, entry_slot)
         self._run(self.lib.mg_moe_gemm(_ptr(y), width, _ptr(w_in), _ptr(offsets), _ptr(slot_entry), top,
                                        _ptr(weights) if weigh_input else None, _ptr(hidden), experts, n, inner, width, n, 1 if gated else 2, is_bf16, act, float(limit),
                                        self._stream()),

@@ -581,6 +581,59 @@ def test_qkv_projection_writes_keys_and_values_to_their_pages(ops, m, heads):
     assert (qkv.double() - ref).abs().max() <= 5e-2
 
 
+@pytest.mark.parametrize("rows_are_inputs", [True, False])
+@pytest.mark.parametrize("n,heads,n_in,n_out,gap", [(65, 3, 128, 512, 64), (300, 2, 64, 192, 8), (129, 16, 512, 128, 0)])
+def test_heads_small_products_of_many_tokens(ops, n, heads, n_in, n_out, gap, rows_are_inputs):
+    """Inputs and outputs of a head among other columns, which stay as they are; against 64 bits."""
+    x = randn(n, heads * (n_in + gap) + 8, dtype=torch.bfloat16, seed=51)
+    w = randn(heads * (n_in if rows_are_inputs else n_out), n_out if rows_are_inputs else n_in, dtype=torch.bfloat16, seed=52,
+              scale=1 / math.sqrt(n_in))
+    out = randn(n, heads * (n_out + gap) + 8, dtype=torch.bfloat16, seed=53)
+    before, kept = ops.launches, out.clone()
+    ops.head_linear(x, 8, n_in + gap, w, rows_are_inputs, heads, n_in, n_out, out=out, out_off=8, out_head=n_out + gap)
+    assert ops.launches == before + 1
+    mats = w.double().view(heads, n_in, n_out) if rows_are_inputs else w.double().view(heads, n_out, n_in).transpose(1, 2)
+    ins = x[:, 8:].double().reshape(n, heads, n_in + gap)[..., :n_in]
+    want = torch.einsum("nhi,hij->nhj", ins, mats)
+    got = out[:, 8:].reshape(n, heads, n_out + gap)
+    # half a unit in the last place of bfloat16, and 32-bit sums of up to 512 products
+    assert ((got[..., :n_out].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+    rest = kept[:, 8:].reshape(n, heads, n_out + gap)[..., n_out:]
+    assert torch.equal(got[..., n_out:], rest) and torch.equal(out[:, :8], kept[:, :8])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("gated,activation,weigh_input", [(True, "silu", False), (False, "relu_sq", True)])
+@pytest.mark.parametrize("n,width,inner,experts,top", [(65, 136, 200, 5, 2), (300, 264, 68 * 4, 3, 3), (700, 512, 384, 17, 2), (130, 72, 520, 200, 1)])
+def test_experts_of_many_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input):
+    """Tiles over each expert's rows: experts without rows, rows that end inside a tile and inside a box of 32, widths that end
+    inside a tile; against the products in 64 bits, hidden features rounded to bfloat16."""
+    g = torch.Generator().manual_seed(n)
+    y = randn(n, width, dtype=torch.bfloat16, seed=44)
+    w_in = randn(experts, (2 if gated else 1) * inner, width, dtype=torch.bfloat16, seed=45, scale=1 / math.sqrt(width))
+    w_out = randn(experts, width, inner, dtype=torch.bfloat16, seed=46, scale=1 / math.sqrt(inner))
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(n)]).to(torch.int32)
+    if experts > 3:
+        ids[ids == 2] = 1                            # an expert without rows (a token may then have one expert twice)
+    ids[7] = -1                                      # a padding row
+    weights = torch.rand(n, top, generator=g).cuda()
+    residual = randn(n, width, seed=47)
+    want = residual.double()
+    for e in range(experts):
+        for t, k in (ids == e).nonzero().tolist():
+            w = weights[t, k].double()
+            z = w_in[e].double() @ y[t].double() * (w if weigh_input else 1.0)
+            h = z[:inner] * torch.sigmoid(z[:inner]) * z[inner:] if gated else z.clamp_min(0) ** 2
+            want[t] += w_out[e].double() @ h.to(torch.bfloat16).double() * (1.0 if weigh_input else w)
+    before = ops.launches
+    ops.moe_experts_residual(y, ids.cuda(), weights, w_in, w_out, residual, activation, 0.0, gated, weigh_input)
+    assert ops.launches == before + 5
+    # here and there a hidden feature is rounded to the other neighbour: 2^-8 of it, times a weight of 1 / sqrt(inner)
+    assert (residual.double() - want).abs().max() <= 2e-2
+    assert (residual.double() - want).norm() <= 1e-3 * want.norm()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("gated,activation,weigh_input", [(True, "silu", False), (True, "clamped_swish", False),
                                                           (False, "relu_sq", True), (False, "gelu_tanh", False)])
 @pytest.mark.parametrize("n,width,inner,experts,top", [(1, 1024, 1024, 9, 3), (8, 136, 200, 5, 2), (9, 264, 72, 3, 3), (16, 1160, 24, 4, 4),
