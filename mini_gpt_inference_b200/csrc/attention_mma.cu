@@ -547,12 +547,13 @@ attention_split_kernel(const AttnParams p) {
 }
 
 // out[token, head] = (sum over ranges of 2^(m_s - M) O_s) / (sum of 2^(m_s - M) l_s), times the gate.
-// The ranges' maxima and sums come to shared memory in one trip, their weights are worked out there
-// once, and every thread then sums its column over the ranges with independent loads.
+// The ranges' maxima and sums come to shared memory, and the first ranges' results to registers, in one trip; the weights
+// are worked out once, and every thread sums its column over the ranges.
+constexpr int MERGE_AHEAD = 32;   // ranges whose results are asked for before the weights are known
 constexpr int MERGE_MAX = 1024;   // most ranges (mg_attention_mma_split_keys keeps to it)
 
 __global__ void attention_merge_kernel(const AttnParams p) {
-    __shared__ float weight[MERGE_MAX];
+    __shared__ float weight[MERGE_MAX], sums[MERGE_MAX];
     __shared__ float norm;
     pdl_trigger();
     pdl_wait();
@@ -566,7 +567,16 @@ __global__ void attention_merge_kernel(const AttnParams p) {
     }
     const int live = min(min(p.splits, MERGE_MAX),
                          KeyWalk(p, first_visible(p, position)).last(position) / p.split_keys + 1);   // ranges that hold keys
-    for (int s = threadIdx.x; s < live; s += blockDim.x) weight[s] = p.part_ml[(base + s) * 2];
+    // everything is asked for at once: the ranges' maxima, and this thread's first column of the first MERGE_AHEAD ranges
+    float ahead[MERGE_AHEAD];
+#pragma unroll
+    for (int s = 0; s < MERGE_AHEAD; ++s)
+        ahead[s] = s < live && threadIdx.x < p.dv ? p.part_o[(base + s) * p.dv + threadIdx.x] : 0.f;
+    for (int s = threadIdx.x; s < live; s += blockDim.x) {
+        const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + (base + s) * 2);
+        weight[s] = ml.x;
+        sums[s] = ml.y;
+    }
     __syncthreads();
     if (threadIdx.x < 32) {
         float mm = -INFINITY;
@@ -577,7 +587,7 @@ __global__ void attention_merge_kernel(const AttnParams p) {
             const float ms = weight[s];
             const float w = ms == -INFINITY ? 0.f : exp2f(ms - mm);
             weight[s] = w;
-            sum += w * p.part_ml[(base + s) * 2 + 1];
+            sum += w * sums[s];
         }
         sum = warp_sum(sum) + sink_term(p, head, mm);
         if (threadIdx.x == 0) norm = sum > 0.f ? 1.0f / sum : 0.f;
@@ -586,8 +596,13 @@ __global__ void attention_merge_kernel(const AttnParams p) {
     const bf16* grow = p.gate ? p.gate + (size_t)token * p.gate_stride + (size_t)head * p.dv : nullptr;
     for (int c = threadIdx.x; c < p.dv; c += blockDim.x) {
         float acc = 0.f;
+        if (c == threadIdx.x) {
+#pragma unroll
+            for (int s = 0; s < MERGE_AHEAD; ++s)
+                if (s < live) acc = fmaf(weight[s], ahead[s], acc);
+        }
 #pragma unroll 8
-        for (int s = 0; s < live; ++s) acc = fmaf(weight[s], p.part_o[(base + s) * p.dv + c], acc);
+        for (int s = c == threadIdx.x ? MERGE_AHEAD : 0; s < live; ++s) acc = fmaf(weight[s], p.part_o[(base + s) * p.dv + c], acc);
         acc *= norm;
         if (grow) acc *= logistic(__bfloat162float(grow[c]));
         orow[c] = __float2bfloat16_rn(acc);
@@ -885,12 +900,12 @@ int launch(const AttnParams& p, int single_tokens, int n_tiles, cudaStream_t s) 
 
 }  // namespace
 
-// Ranges of keys per token for contexts of up to max_context keys, and the keys per range.
-MG_API int mg_attention_mma_split_keys(int max_context) {
-    // short ranges: many CTAs with two blocks each (a CTA's blocks follow one another at a memory
-    // round trip apiece); ranges beyond a token's own context leave at once, so the count only sizes
-    // the grid and the scratch
-    int keys = 128;
+// Ranges of keys per token for contexts of up to max_context keys, and the keys per range; rows: tokens times key/value heads.
+MG_API int mg_attention_mma_split_keys(int max_context, int rows) {
+    // short ranges: many CTAs with two blocks each (a CTA's blocks follow one another), or one where there are few rows and
+    // the SMs would not all have a CTA (3 tokens, 4 heads, 1,300 keys: 132 CTAs or 252); ranges beyond a token's own context
+    // leave at once, so the count only sizes the grid and the scratch
+    int keys = rows <= 16 ? 64 : 128;
     while ((max_context + keys - 1) / keys > 1024) keys *= 2;
     return keys;
 }

@@ -160,7 +160,7 @@ def load(verbose: bool = True):
     lib.mg_attention_split_launches.restype = c_int
     lib.mg_mlp_pack_elements.argtypes = [c_int, c_int]
     lib.mg_mlp_pack_elements.restype = ctypes.c_longlong
-    lib.mg_attention_mma_split_keys.argtypes = [c_int]
+    lib.mg_attention_mma_split_keys.argtypes = [c_int, c_int]
     lib.mg_attention_mma_split_keys.restype = c_int
     lib.mg_attention_mma_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
     lib.mg_attention_mma_scratch_floats.restype = ctypes.c_longlong

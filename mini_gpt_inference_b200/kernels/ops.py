@@ -1033,7 +1033,7 @@ class CudaOps:
             group = n_head // n_kv_head
             args = None
             if single:
-                keys, splits = self._key_ranges(int(ctx.max_ctx_after), int(cache.window or 0), 0)
+                keys, splits = self._key_ranges(n * n_kv_head, int(ctx.max_ctx_after), int(cache.window or 0), 0)
                 floats = self.lib.mg_attention_mma_scratch_floats(n, n_head, v_dim, splits)
                 scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
                 args = [_ptr(scratch), 1, 0, splits, keys]
@@ -1096,7 +1096,7 @@ class CudaOps:
         """How the warp-level tensor-core attention cuts a step: ``[scratch, single tokens, tiles, tokens a tile, ranges,
         keys a range]``; None where it takes no such step."""
         if getattr(ctx, "decode_only", False):
-            keys, splits = self._key_ranges(int(ctx.max_ctx_after), window, block, keep_first)
+            keys, splits = self._key_ranges(n * n_kv_head, int(ctx.max_ctx_after), window, block, keep_first)
             floats = self.lib.mg_attention_mma_scratch_floats(n, n_head, v_dim, splits)
             return [torch.empty((floats,), dtype=torch.float32, device=self.device), 1, 0, 1, splits, keys]
         q_len, group = getattr(ctx, "host_q_len", None), n_head // n_kv_head
@@ -1105,8 +1105,8 @@ class CudaOps:
             return [None, 0, sum(-(-int(t) // tile) for t in q_len), tile, 0, 0]
         return None
 
-    def _key_ranges(self, max_context, window, block, keep_first=0):
-        """Keys per range and ranges per token for single tokens with contexts of up to ``max_context`` keys.  With a
+    def _key_ranges(self, rows, max_context, window, block, keep_first=0):
+        """Keys per range and ranges per token for single tokens (``rows``: tokens times key/value heads) with contexts of up to ``max_context`` keys.  With a
         window or a block mask a token's keys begin at its own first position: ranges are counted from the key block of
         64 that holds it, so they cover at most the window's (the block's) length and 63 keys in front of it, behind the blocks that hold first tokens
         which stay in sight."""
@@ -1114,7 +1114,7 @@ class CudaOps:
         for reach in (window, block):
             if reach > 0:
                 span = min(span, reach + 64 + -(-keep_first // 64) * 64)
-        keys = self.lib.mg_attention_mma_split_keys(span)
+        keys = self.lib.mg_attention_mma_split_keys(span, rows)
         return keys, max(1, -(-span // keys))
 
     # ---- several residual streams ------------------------------------------------------------------
