@@ -619,22 +619,29 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 // keys' weights (the sums meet after the last block), the weights go to shared memory as bfloat16, and the warp
 // then adds the block's 64 keys into columns CW cg .. CW cg + CW - 1 of its rows' results.  `single`: the rows are one
 // token's heads and the CTA takes one range of its keys; results go to scratch as the merge kernel reads them.
-constexpr int WIDE_ROWS = 32;
+//
+// RT: tiles of 16 rows a warp takes, one or two.  With two (64 rows a CTA; steps of many rows) a key fragment from shared memory
+// serves twice the products and a block of keys twice the rows.  Rows in shared memory are multiples of 128 bytes, their 16-byte
+// chunks in the order (chunk ^ row % 8), so that eight rows' chunks meet no bank twice without padding: 64 rows and two blocks
+// of 576 features just fit.  Prompts of 4 requests of 1,021 tokens, 16 heads, 576 / 512 features, a window of 512, in three layers:
+// six launches of 279 us with one, 57 us less each with two.
+__device__ __forceinline__ int swizzled(int row, int chunk, int row_elements) { return row * row_elements + ((chunk ^ (row & 7)) << 3); }
 
-template <int CW>
+template <int CW, int RT>
 __global__ void __launch_bounds__(256, 1)
 attention_wide_kernel(const AttnParams p, const int single, const int dpad, const int row_tiles) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int stride = dpad + PAD;
-    bf16* qs = reinterpret_cast<bf16*>(smem_raw);                     // [32][stride]
-    bf16* kbuf = qs + WIDE_ROWS * stride;                              // [2][KB][stride]
-    bf16* ps = kbuf + 2 * KB * stride;                                 // [32][KB + PAD]
-    float* mx = reinterpret_cast<float*>(ps + WIDE_ROWS * (KB + PAD)); // [4][32]
+    constexpr int WIDE_ROWS = 32 * RT;
+    bf16* qs = reinterpret_cast<bf16*>(smem_raw);                     // [32 RT][dpad]
+    bf16* kbuf = qs + WIDE_ROWS * dpad;                                // [2][KB][dpad]
+    bf16* ps = kbuf + 2 * KB * dpad;                                   // [32 RT][KB]
+    float* mx = reinterpret_cast<float*>(ps + WIDE_ROWS * KB);         // [4][32 RT]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 1, cg = warp >> 1;
     // columns d .. dpad of the key rows are never loaded: zeros, once
     if (p.d < dpad) {
-        const int extra = dpad - p.d;
-        for (int i = tid; i < 2 * KB * extra; i += 256) kbuf[(i / extra) * stride + p.d + i % extra] = __float2bfloat16_rn(0.f);
+        const int extra = (dpad - p.d) >> 3;
+        for (int i = tid; i < 2 * KB * extra; i += 256)
+            *reinterpret_cast<uint4*>(kbuf + swizzled(i / extra, (p.d >> 3) + i % extra, dpad)) = make_uint4(0u, 0u, 0u, 0u);
     }
     pdl_trigger();
     pdl_wait();
@@ -686,24 +693,27 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
                 const int t = single ? 0 : row / group, h = single ? row : row - t * group;
                 v = *reinterpret_cast<const uint4*>(p.q + (size_t)(first_token + t) * p.q_stride + (size_t)(kv_head * group + h) * p.d + c);
             }
-            *reinterpret_cast<uint4*>(qs + r * stride + c) = v;
+            *reinterpret_cast<uint4*>(qs + swizzled(r, c >> 3, dpad)) = v;
         }
     }
-    // this lane's two rows
-    int pos[2], lo[2], token[2], head[2];
+    // this lane's two rows of each tile
+    int pos[RT][2], lo[RT][2];
+    float m[RT][2], l[RT][2], o[RT][CW / 8][4];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int row = row_base + rg * 16 + (lane >> 2) + 8 * r;
-        const bool live = row < rows_total;
-        const int t = (single || !live) ? 0 : row / group;
-        token[r] = first_token + t;
-        head[r] = kv_head * group + (live ? row - t * group : 0);
-        pos[r] = live ? p.positions[token[r]] : -1;
-        lo[r] = pos[r] >= 0 ? first_visible(p, pos[r]) : 0;
+    for (int i = 0; i < RT; ++i) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int row = row_base + (rg * RT + i) * 16 + (lane >> 2) + 8 * r;
+            const bool live = row < rows_total;
+            const int t = (single || !live) ? 0 : row / group;
+            pos[i][r] = live ? p.positions[first_token + t] : -1;
+            lo[i][r] = pos[i][r] >= 0 ? first_visible(p, pos[i][r]) : 0;
+            m[i][r] = -INFINITY;
+            l[i][r] = 0.f;
+        }
+#pragma unroll
+        for (int n = 0; n < CW / 8; ++n) o[i][n][0] = o[i][n][1] = o[i][n][2] = o[i][n][3] = 0.f;
     }
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[CW / 8][4];
-#pragma unroll
-    for (int n = 0; n < CW / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
     const int page_shift = (p.page_tokens & (p.page_tokens - 1)) == 0 ? __ffs(p.page_tokens) - 1 : -1;
     const int chunks = p.d >> 3;
@@ -720,161 +730,194 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
                 if (!MG_GUARDED(attention_mma, MG_GUARD_PAGE, page, p.num_pages)) page = 0;
                 row = ((size_t)page * p.n_kv_head + kv_head) * p.page_tokens + within;
             }
-            for (int c = lane; c < chunks; c += 32) cp_async16(dst + key * stride + c * 8, p.k_pages + row * p.d + c * 8, real);
+            for (int c = lane; c < chunks; c += 32) cp_async16(dst + swizzled(key, c, dpad), p.k_pages + row * p.d + c * 8, real);
         }
     };
     load_keys(j_first, kbuf);
     cp_async_commit();
-    if (j_first + KB <= j_last) load_keys(j_first + KB, kbuf + KB * stride);
+    if (j_first + KB <= j_last) load_keys(j_first + KB, kbuf + KB * dpad);
     cp_async_commit();
     int buf = 0;
     for (int j0 = j_first; j0 <= j_last; j0 += KB, buf ^= 1) {
         cp_async_wait<1>();                                // (one group a block, empty ones behind the last)
         __syncthreads();                                   // the block is here, for everyone
-        const bf16* kb = kbuf + buf * KB * stride;
-        float s[2][4];
+        const bf16* kb = kbuf + buf * KB * dpad;
+        float s[RT][2][4];
 #pragma unroll
-        for (int n = 0; n < 2; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-        const bf16* a_ptr = qs + (rg * 16 + (lane & 15)) * stride + (lane >> 4) * 8;
-        const bf16* b_ptr = kb + (cg * 16 + (lane >> 4) * 8 + (lane & 7)) * stride + ((lane >> 3) & 1) * 8;
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) s[i][n][0] = s[i][n][1] = s[i][n][2] = s[i][n][3] = 0.f;
+        const int a_row = rg * RT * 16 + (lane & 15), b_row = cg * 16 + (lane >> 4) * 8 + (lane & 7);
 #pragma unroll 4
         for (int kk = 0; kk < dpad; kk += 16) {
-            uint32_t a[4], b[4];
-            ldsm4(a, a_ptr + kk);
-            ldsm4(b, b_ptr + kk);
-            mma16816(s[0], a, b[0], b[1]);
-            mma16816(s[1], a, b[2], b[3]);
-        }
-        float bm[2] = {-INFINITY, -INFINITY};
+            uint32_t b[4];
+            ldsm4(b, kb + swizzled(b_row, (kk >> 3) + ((lane >> 3) & 1), dpad));
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = j0 + cg * 16 + n * 8 + 2 * (lane & 3) + (e & 1), r = e >> 1;
-                float sc = s[n][e] * p.scale_log2;
-                if (p.cap_log2 > 0.f) sc = p.cap_log2 * tanhf(sc / p.cap_log2);
-                const float v = (j <= pos[r] && j >= lo[r]) ? sc : -INFINITY;
-                s[n][e] = v;
-                bm[r] = fmaxf(bm[r], v);
+            for (int i = 0; i < RT; ++i) {
+                uint32_t a[4];
+                ldsm4(a, qs + swizzled(a_row + 16 * i, (kk >> 3) + (lane >> 4), dpad));
+                mma16816(s[i][0], a, b[0], b[1]);
+                mma16816(s[i][1], a, b[2], b[3]);
             }
+        }
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 1));
-            bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 2));
-            if ((lane & 3) == 0) mx[cg * WIDE_ROWS + rg * 16 + (lane >> 2) + 8 * r] = bm[r];
+        for (int i = 0; i < RT; ++i) {
+            float bm[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = j0 + cg * 16 + n * 8 + 2 * (lane & 3) + (e & 1), r = e >> 1;
+                    float sc = s[i][n][e] * p.scale_log2;
+                    if (p.cap_log2 > 0.f) sc = p.cap_log2 * tanhf(sc / p.cap_log2);
+                    const float v = (j <= pos[i][r] && j >= lo[i][r]) ? sc : -INFINITY;
+                    s[i][n][e] = v;
+                    bm[r] = fmaxf(bm[r], v);
+                }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 1));
+                bm[r] = fmaxf(bm[r], __shfl_xor_sync(0xffffffffu, bm[r], 2));
+                if ((lane & 3) == 0) mx[cg * WIDE_ROWS + (rg * RT + i) * 16 + (lane >> 2) + 8 * r] = bm[r];
+            }
         }
         __syncthreads();
-        float corr[2], base[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int row = rg * 16 + (lane >> 2) + 8 * r;
-            const float all = fmaxf(fmaxf(mx[row], mx[WIDE_ROWS + row]), fmaxf(mx[2 * WIDE_ROWS + row], mx[3 * WIDE_ROWS + row]));
-            const float nm = fmaxf(m[r], all);
-            corr[r] = (m[r] == -INFINITY) ? 0.f : exp2_approx(m[r] - nm);
-            base[r] = (nm == -INFINITY) ? 0.f : nm;
-            m[r] = nm;
-        }
-        float bs[2] = {0.f, 0.f};
+        for (int i = 0; i < RT; ++i) {
+            float corr[2], base[2];
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
+            for (int r = 0; r < 2; ++r) {
+                const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r;
+                const float all = fmaxf(fmaxf(mx[row], mx[WIDE_ROWS + row]), fmaxf(mx[2 * WIDE_ROWS + row], mx[3 * WIDE_ROWS + row]));
+                const float nm = fmaxf(m[i][r], all);
+                corr[r] = (m[i][r] == -INFINITY) ? 0.f : exp2_approx(m[i][r] - nm);
+                base[r] = (nm == -INFINITY) ? 0.f : nm;
+                m[i][r] = nm;
+            }
+            float bs[2] = {0.f, 0.f};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float pr = exp2_approx(s[n][e] - base[e >> 1]);
-                s[n][e] = pr;
-                bs[e >> 1] += pr;
+            for (int n = 0; n < 2; ++n) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float pr = exp2_approx(s[i][n][e] - base[e >> 1]);
+                    s[i][n][e] = pr;
+                    bs[e >> 1] += pr;
+                }
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    *reinterpret_cast<uint32_t*>(ps + swizzled((rg * RT + i) * 16 + (lane >> 2) + 8 * r, cg * 2 + n, KB) + 2 * (lane & 3)) =
+                        pack_bf16(s[i][n][2 * r], s[i][n][2 * r + 1]);
             }
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-                *reinterpret_cast<uint32_t*>(ps + (rg * 16 + (lane >> 2) + 8 * r) * (KB + PAD) + cg * 16 + n * 8 + 2 * (lane & 3)) =
-                    pack_bf16(s[n][2 * r], s[n][2 * r + 1]);
-        }
+            for (int r = 0; r < 2; ++r) {
+                bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 1);
+                bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 2);
+                l[i][r] = l[i][r] * corr[r] + bs[r];
+            }
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 1);
-            bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 2);
-            l[r] = l[r] * corr[r] + bs[r];
-        }
-#pragma unroll
-        for (int n = 0; n < CW / 8; ++n) {
-            o[n][0] *= corr[0];
-            o[n][1] *= corr[0];
-            o[n][2] *= corr[1];
-            o[n][3] *= corr[1];
+            for (int n = 0; n < CW / 8; ++n) {
+                o[i][n][0] *= corr[0];
+                o[i][n][1] *= corr[0];
+                o[i][n][2] *= corr[1];
+                o[i][n][3] *= corr[1];
+            }
         }
         __syncthreads();                                   // all 64 keys' weights of the warp's rows are there
 #pragma unroll
         for (int kk = 0; kk < KB / 16; ++kk) {
-            uint32_t a[4];
-            ldsm4(a, ps + (rg * 16 + (lane & 15)) * (KB + PAD) + kk * 16 + (lane >> 4) * 8);
-            const bf16* v_ptr = kb + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * stride + cg * CW + (lane >> 4) * 8;
+            uint32_t a[RT][4];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) ldsm4(a[i], ps + swizzled((rg * RT + i) * 16 + (lane & 15), kk * 2 + (lane >> 4), KB));
+            const int v_row = kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
 #pragma unroll
             for (int n = 0; n < CW / 8; n += 2) {
                 uint32_t b[4];
-                ldsm4_t(b, v_ptr + n * 8);
-                mma16816(o[n], a, b[0], b[1]);
-                mma16816(o[n + 1], a, b[2], b[3]);
+                ldsm4_t(b, kb + swizzled(v_row, cg * (CW / 8) + n + (lane >> 4), dpad));
+#pragma unroll
+                for (int i = 0; i < RT; ++i) {
+                    mma16816(o[i][n], a[i], b[0], b[1]);
+                    mma16816(o[i][n + 1], a[i], b[2], b[3]);
+                }
             }
         }
         __syncthreads();                                   // everyone has left the buffer: it takes the block after the next
-        if (j0 + 2 * KB <= j_last) load_keys(j0 + 2 * KB, kbuf + buf * KB * stride);
+        if (j0 + 2 * KB <= j_last) load_keys(j0 + 2 * KB, kbuf + buf * KB * dpad);
         cp_async_commit();
     }
     // the four warps of a row group kept the sums of their own keys: they meet here
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-        if ((lane & 3) == 0) mx[cg * WIDE_ROWS + rg * 16 + (lane >> 2) + 8 * r] = l[r];
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            if ((lane & 3) == 0) mx[cg * WIDE_ROWS + (rg * RT + i) * 16 + (lane >> 2) + 8 * r] = l[i][r];
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        if (pos[r] < 0) continue;
-        const int row = rg * 16 + (lane >> 2) + 8 * r;
-        float sum = mx[row] + mx[WIDE_ROWS + row] + mx[2 * WIDE_ROWS + row] + mx[3 * WIDE_ROWS + row];
-        if (single) {
-            const size_t slot = ((size_t)token[r] * p.n_head + head[r]) * p.splits + blockIdx.z;
-            if (cg == 0 && (lane & 3) == 0) {
-                p.part_ml[slot * 2] = m[r];
-                p.part_ml[slot * 2 + 1] = sum;
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (pos[i][r] < 0) continue;
+            const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r, t = single ? 0 : (row_base + row) / group;
+            const int token = first_token + t, head = kv_head * group + row_base + row - t * group;
+            float sum = mx[row] + mx[WIDE_ROWS + row] + mx[2 * WIDE_ROWS + row] + mx[3 * WIDE_ROWS + row];
+            if (single) {
+                const size_t slot = ((size_t)token * p.n_head + head) * p.splits + blockIdx.z;
+                if (cg == 0 && (lane & 3) == 0) {
+                    p.part_ml[slot * 2] = m[i][r];
+                    p.part_ml[slot * 2 + 1] = sum;
+                }
+#pragma unroll
+                for (int n = 0; n < CW / 8; ++n) {
+                    const int c = cg * CW + n * 8 + 2 * (lane & 3);
+                    if (c >= p.dv) continue;
+                    *reinterpret_cast<float2*>(p.part_o + slot * p.dv + c) = make_float2(o[i][n][2 * r], o[i][n][2 * r + 1]);
+                }
+                continue;
             }
+            sum += sink_term(p, head, m[i][r]);
+            const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+            bf16* orow = p.out + (size_t)token * p.n_head * p.dv + (size_t)head * p.dv;
+            const bf16* grow = p.gate ? p.gate + (size_t)token * p.gate_stride + (size_t)head * p.dv : nullptr;
 #pragma unroll
             for (int n = 0; n < CW / 8; ++n) {
                 const int c = cg * CW + n * 8 + 2 * (lane & 3);
                 if (c >= p.dv) continue;
-                *reinterpret_cast<float2*>(p.part_o + slot * p.dv + c) = make_float2(o[n][2 * r], o[n][2 * r + 1]);
+                float a = o[i][n][2 * r] * inv, b = o[i][n][2 * r + 1] * inv;
+                if (grow) {
+                    const __nv_bfloat162 g = *reinterpret_cast<const __nv_bfloat162*>(grow + c);
+                    a *= logistic(__bfloat162float(g.x));
+                    b *= logistic(__bfloat162float(g.y));
+                }
+                *reinterpret_cast<uint32_t*>(orow + c) = pack_bf16(a, b);
             }
-            continue;
         }
-        sum += sink_term(p, head[r], m[r]);
-        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
-        bf16* orow = p.out + (size_t)token[r] * p.n_head * p.dv + (size_t)head[r] * p.dv;
-        const bf16* grow = p.gate ? p.gate + (size_t)token[r] * p.gate_stride + (size_t)head[r] * p.dv : nullptr;
-#pragma unroll
-        for (int n = 0; n < CW / 8; ++n) {
-            const int c = cg * CW + n * 8 + 2 * (lane & 3);
-            if (c >= p.dv) continue;
-            float a = o[n][2 * r] * inv, b = o[n][2 * r + 1] * inv;
-            if (grow) {
-                const __nv_bfloat162 g = *reinterpret_cast<const __nv_bfloat162*>(grow + c);
-                a *= logistic(__bfloat162float(g.x));
-                b *= logistic(__bfloat162float(g.y));
-            }
-            *reinterpret_cast<uint32_t*>(orow + c) = pack_bf16(a, b);
-        }
-    }
 }
 
-template <int CW>
-int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, size_t smem, cudaStream_t s) {
-    const int group = p.n_head / p.n_kv_head, row_tiles = (group + WIDE_ROWS - 1) / WIDE_ROWS;
-    cudaError_t e = cudaFuncSetAttribute(attention_wide_kernel<CW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Bytes of shared memory of a CTA of `rows` rows of dpad features.
+constexpr size_t wide_smem(int rows, int dpad) { return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) + (size_t)4 * rows * sizeof(float); }
+constexpr size_t WIDE_MOST = 227 * 1024;
+
+template <int CW, int RT>
+int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, cudaStream_t s) {
+    const int group = p.n_head / p.n_kv_head, row_tiles = (group + 32 * RT - 1) / (32 * RT);
+    const size_t smem = wide_smem(32 * RT, dpad);
+    cudaError_t e = cudaFuncSetAttribute(attention_wide_kernel<CW, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) {
         const dim3 grid = single ? dim3(p.n_tokens * row_tiles, p.n_kv_head, p.splits) : dim3(n_tiles, p.n_kv_head);
-        e = mg_launch(attention_wide_kernel<CW>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
+        e = mg_launch(attention_wide_kernel<CW, RT>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
     }
     if (e == cudaSuccess && single)
         e = mg_launch(attention_merge_kernel, dim3(p.n_tokens, p.n_head), dim3(p.dv > 256 ? 512 : p.dv > 128 ? 256 : 128), 0, s, true, p);
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention (wide rows): %s", cudaGetErrorString(e));
     return MG_OK;
+}
+
+// The columns of a CTA's rows: the values', in four equal parts of whole pairs of 8-column tiles, and the keys', padded (with
+// zeros) to whole 128-byte lines that hold them all.
+inline int wide_values(int dv) { return dv <= 64 ? 64 : dv <= 128 ? 128 : dv <= 256 ? 256 : 512; }
+inline int wide_columns(int d, int dv) {
+    const int lines = (d + 63) / 64 * 64;
+    return lines > wide_values(dv) ? lines : wide_values(dv);
 }
 
 template <int DP, int DVP, bool FULL_P>
@@ -976,18 +1019,21 @@ MG_API int mg_attention_mma(const void* q, int q_stride, const void* k_pages, co
 #undef MG_LAUNCH_SIZES
 }
 
-// Rows of 32 (token, head) pairs that the wide-row kernel takes for a prompt portion of `tokens` tokens.
-MG_API int mg_attention_wide_tiles(int tokens, int group) { return (tokens * group + WIDE_ROWS - 1) / WIDE_ROWS; }
+// Rows, (token, head) pairs, of a CTA of the wide-row kernel for a prompt step of `rows` rows in all: 64 where they are enough for
+// two CTAs an SM and fit (2,048 tokens of 16 heads: 512 CTAs), else 32.
+MG_API int mg_attention_wide_rows(int rows, int d, int dv) {
+    return rows >= 2 * 148 * 64 && dv <= 512 && wide_smem(64, wide_columns(d, dv)) <= WIDE_MOST ? 64 : 32;
+}
 
 // Attention over key rows of d features whose first dv features are the values (one row per token and key/value
 // head, k_pages [page, G, page_tokens, d]); the other arguments as mg_attention_mma.  single_tokens = 1: splits ranges
 // of split_keys keys, scratch of mg_attention_mma_scratch_floats floats, merged by a second kernel; 0: n_tiles is the
-// sum of mg_attention_wide_tiles over the requests.  Returns MG_ERR_UNSUPPORTED for sizes it does not take.
+// sum over the requests of their rows (tokens times heads of a group) over tile_rows (mg_attention_wide_rows), rounded up.  Returns MG_ERR_UNSUPPORTED for sizes it does not take.
 MG_API int mg_attention_wide(const void* q, int q_stride, const void* k_pages, const int* block_table, const int* token_request,
                              const int* positions, const int* req_q_start, const int* req_q_len, const void* gate,
                              int gate_stride, void* out, float* scratch, int n_tokens, int n_requests, int n_head, int n_kv_head,
                              int d, int dv, int page_tokens, int max_pages, int window, float scale, int num_pages,
-                             int single_tokens, int n_tiles, int splits, int split_keys, float softcap, const float* sinks,
+                             int single_tokens, int n_tiles, int tile_rows, int splits, int split_keys, float softcap, const float* sinks,
                              void* stream) {
     if (n_tokens == 0) return MG_OK;
     MG_REQUIRE(n_tokens > 0 && n_head > 0 && n_kv_head > 0 && n_head % n_kv_head == 0 && page_tokens > 0 && max_pages > 0 &&
@@ -995,12 +1041,9 @@ MG_API int mg_attention_wide(const void* q, int q_stride, const void* k_pages, c
     const bool aligned = d % 8 == 0 && dv % 8 == 0 && q_stride % 8 == 0 && (gate == nullptr || gate_stride % 2 == 0) &&
                          ((uintptr_t)q % 16 == 0) && ((uintptr_t)k_pages % 16 == 0) && ((uintptr_t)out % 4 == 0) &&
                          ((uintptr_t)gate % 4 == 0);
-    // the values' columns, padded, in four equal parts of whole pairs of 8-column tiles; the key rows in shared memory are
-    // padded (with zeros) to hold them all
-    const int dv_pad = dv <= 64 ? 64 : dv <= 128 ? 128 : dv <= 256 ? 256 : 512;
-    const int dpad = (d + 15) / 16 * 16 > dv_pad ? (d + 15) / 16 * 16 : dv_pad;
-    const size_t smem = ((size_t)(WIDE_ROWS + 2 * KB) * (dpad + PAD) + WIDE_ROWS * (KB + PAD)) * sizeof(bf16) + 4 * WIDE_ROWS * sizeof(float);
-    if (!aligned || dv > 512 || smem > 227 * 1024 || n_kv_head > 65535) return MG_ERR_UNSUPPORTED;
+    const int dv_pad = wide_values(dv), dpad = wide_columns(d, dv), rows = single_tokens ? 32 : tile_rows;
+    if (!aligned || dv > 512 || wide_smem(32, dpad) > WIDE_MOST || n_kv_head > 65535) return MG_ERR_UNSUPPORTED;
+    MG_REQUIRE((rows == 32 || rows == 64) && wide_smem(rows, dpad) <= WIDE_MOST, "attention (wide rows): no tiles of %d rows", rows);
     AttnParams p;
     p.q = (const bf16*)q; p.q_stride = q_stride; p.k_pages = (const bf16*)k_pages; p.v_pages = (const bf16*)k_pages;
     p.block_table = block_table; p.token_request = token_request; p.positions = positions;
@@ -1020,8 +1063,10 @@ MG_API int mg_attention_wide(const void* q, int q_stride, const void* k_pages, c
         MG_REQUIRE(req_q_start && req_q_len && n_tiles > 0, "attention (wide rows): no tiles");
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (dv_pad == 64) return launch_wide<16>(p, single_tokens, n_tiles, dpad, smem, s);
-    if (dv_pad == 128) return launch_wide<32>(p, single_tokens, n_tiles, dpad, smem, s);
-    if (dv_pad == 256) return launch_wide<64>(p, single_tokens, n_tiles, dpad, smem, s);
-    return launch_wide<128>(p, single_tokens, n_tiles, dpad, smem, s);
+#define MG_LAUNCH_WIDE(CW) return rows == 64 ? launch_wide<CW, 2>(p, single_tokens, n_tiles, dpad, s) : launch_wide<CW, 1>(p, single_tokens, n_tiles, dpad, s)
+    if (dv_pad == 64) MG_LAUNCH_WIDE(16);
+    if (dv_pad == 128) MG_LAUNCH_WIDE(32);
+    if (dv_pad == 256) MG_LAUNCH_WIDE(64);
+    MG_LAUNCH_WIDE(128);
+#undef MG_LAUNCH_WIDE
 }

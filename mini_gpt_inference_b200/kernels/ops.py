@@ -1026,7 +1026,7 @@ class CudaOps:
                         self.launches += 1                       # the merge of the ranges as a kernel of its own
                     return out
         if q.dtype == torch.bfloat16 and self.use_tensor_cores and self.use_mma_attention and in_keys and not biased and keep_first == 0:
-            # rows too wide for that kernel's registers (cached latents of several hundred features): tiles of 32
+            # rows too wide for that kernel's registers (cached latents of several hundred features): tiles of 32 or 64
             # (token, head) rows whose queries wait in shared memory
             single = bool(getattr(ctx, "decode_only", False))
             q_len = getattr(ctx, "host_q_len", None)
@@ -1036,9 +1036,10 @@ class CudaOps:
                 keys, splits = self._key_ranges(n * n_kv_head, int(ctx.max_ctx_after), int(cache.window or 0), 0)
                 floats = self.lib.mg_attention_mma_scratch_floats(n, n_head, v_dim, splits)
                 scratch = torch.empty((floats,), dtype=torch.float32, device=self.device)
-                args = [_ptr(scratch), 1, 0, splits, keys]
+                args = [_ptr(scratch), 1, 0, 32, splits, keys]
             elif q_len and getattr(ctx, "req_q_start", None) is not None:
-                args = [None, 0, sum(self.lib.mg_attention_wide_tiles(int(t), group) for t in q_len), 0, 0]
+                rows = self.lib.mg_attention_wide_rows(sum(q_len) * group, head_dim, v_dim)
+                args = [None, 0, sum(-(-int(t) * group // rows) for t in q_len), rows, 0, 0]
             if args is not None:
                 code = self.lib.mg_attention_wide(
                     _ptr(q), q.shape[1], _ptr(cache.k_pages), _ptr(table), _ptr(ctx.token_request), _ptr(ctx.positions),
@@ -1106,8 +1107,8 @@ class CudaOps:
         return None
 
     def _key_ranges(self, rows, max_context, window, block, keep_first=0):
-        """Keys per range and ranges per token for single tokens (``rows``: tokens times key/value heads) with contexts of up to ``max_context`` keys.  With a
-        window or a block mask a token's keys begin at its own first position: ranges are counted from the key block of
+        """Keys per range and ranges per token for single tokens (``rows``: tokens times key/value heads) with
+        contexts of up to ``max_context`` keys.  With a window or a block mask a token's keys begin at its own first position: ranges are counted from the key block of
         64 that holds it, so they cover at most the window's (the block's) length and 63 keys in front of it, behind the blocks that hold first tokens
         which stay in sight."""
         span = max_context

@@ -581,6 +581,43 @@ def test_qkv_projection_writes_keys_and_values_to_their_pages(ops, m, heads):
     assert (qkv.double() - ref).abs().max() <= 5e-2
 
 
+@pytest.mark.parametrize("n_head,d,dv,window,softcap", [(16, 576, 512, 200, 0.0), (24, 328, 264, 0, 20.0), (16, 704, 512, 0, 0.0)])
+def test_wide_rows_of_long_prompts(ops, n_head, d, dv, window, softcap):
+    """Key rows that hold their values, steps of so many rows that a CTA takes 64 (32 where 64 do not fit): as the general
+    kernel has it, within the rounding of weights and outputs to bfloat16."""
+    g = torch.Generator().manual_seed(d)
+    lens, befores, pt = [901, 330], [0, 77], 16
+    ends = [b + n for b, n in zip(befores, lens)]
+    pages = sum(-(-e // pt) for e in ends) + 1
+    order, tables = torch.randperm(pages, generator=g).tolist(), torch.full((2, 64), -1, dtype=torch.int32)
+    rows = torch.full((pages, 1, pt, d), float("nan"))
+    for r, e in enumerate(ends):
+        for i in range(-(-e // pt)):
+            tables[r, i] = page = order.pop()
+            have = min(e - i * pt, pt)                # behind a request's last token: no numbers
+            rows[page, 0, :have] = torch.randn(have, d, generator=g)
+    pages_cuda = rows.to(torch.bfloat16).cuda()
+    cache = SimpleNamespace(k_pages=pages_cuda, v_pages=pages_cuda, group=0, page_tokens=pt, window=window or None, writes=False,
+                            values_in_keys=True)
+    i32 = lambda v: torch.as_tensor(v, dtype=torch.int32).cuda()
+    ctx = SimpleNamespace(block_tables=[tables.cuda()], positions=i32([b + i for b, n in zip(befores, lens) for i in range(n)]),
+                          token_request=i32([r for r, n in enumerate(lens) for _ in range(n)]), decode_only=False,
+                          max_ctx_after=max(ends), host_q_len=lens, req_q_len=i32(lens), req_q_start=i32([0, lens[0]]))
+    q = (torch.randn(sum(lens), n_head * d, generator=g) * 1.5).to(torch.bfloat16).cuda()
+    sink = torch.randn(n_head, generator=g).cuda()
+    run = lambda: ops.paged_attention_general(q, n_head, 1, d, dv, d ** -0.5, cache, ctx, softcap=softcap, sinks=sink).float()
+    before = ops.launches
+    got = run()
+    assert ops.launches == before + 1 and not torch.isnan(got).any()
+    ops.use_mma_attention = False
+    try:
+        want = run()
+    finally:
+        ops.use_mma_attention = True
+    assert (got - want).abs().max() <= _tol(torch.bfloat16, 1.5)
+    assert (got - want).norm() <= 6e-3 * want.norm()      # two roundings of 2^-9 and one of the weights
+
+
 @pytest.mark.parametrize("rows_are_inputs", [True, False])
 @pytest.mark.parametrize("n,heads,n_in,n_out,gap", [(65, 3, 128, 512, 64), (300, 2, 64, 192, 8), (129, 16, 512, 128, 0)])
 def test_heads_small_products_of_many_tokens(ops, n, heads, n_in, n_out, gap, rows_are_inputs):
