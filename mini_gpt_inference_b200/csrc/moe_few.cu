@@ -30,9 +30,19 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// What becomes of an entry's finished sums (u: the up feature of a gated unit).
+template <int FORM>
+__device__ __forceinline__ void finish(float v, float u, int entry, int n, int N, const float* scale, int act, float limit, void* out) {
+    const float s = scale ? scale[entry] : 1.f;
+    const size_t to = (size_t)entry * N + n;
+    if constexpr (FORM == 1) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(gated_value(act, limit, v * s, u * s));
+    else if constexpr (FORM == 2) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(plain_value(act, v * s));
+    else reinterpret_cast<float*>(out)[to] = v * s;
+}
+
 // Forms as mg_moe_gemm: 1 gated, 2 plain, 0 out.
 template <int FORM>
-__global__ void __launch_bounds__(32 * WARPS)
+__global__ void __launch_bounds__(32 * WARPS, FORM == 1 ? 0 : 5)
 moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, long long w_expert_stride,
                const int* __restrict__ ids, int n_entries, int top, const float* __restrict__ scale, void* __restrict__ out,
                int* __restrict__ entry_slot, int n_experts, int N, int K, int x_rows, int act, float limit) {
@@ -54,6 +64,7 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
         if (FORM == 0 && e == 0 && blockIdx.x == 0 && warp == 0 && i < n_entries) entry_slot[i] = id >= 0 && id < n_experts ? i : -1;
     }
     if (count == 0) return;
+    const int entries = count;
     count = min(count, MAX_TOKENS);
     __syncwarp();
     const bf16* we = w + (size_t)e * w_expert_stride;
@@ -128,19 +139,34 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
 #pragma unroll
             for (int k = 0; k < WARPS; ++k) v[i] += sums[k][i * ROWS + row][c];
         }
-        const int entry = lists[warp][c];
-        const float s = scale ? scale[entry] : 1.f;
-        const size_t to = (size_t)entry * N + n;
-        if constexpr (FORM == 1) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(gated_value(act, limit, v[0] * s, v[MI - 1] * s));
-        else if constexpr (FORM == 2) reinterpret_cast<bf16*>(out)[to] = __float2bfloat16_rn(plain_value(act, v[0] * s));
-        else reinterpret_cast<float*>(out)[to] = v[0] * s;
+        finish<FORM>(v[0], v[MI - 1], lists[warp][c], n, N, scale, act, limit, out);
+    }
+    if (entries <= MAX_TOKENS) return;
+    // More than 16 entries: tokens named the expert several times (a router does so for a row whose scores are not numbers).
+    // The rest one after the other, a warp to an output: rare, and the columns above keep their registers.
+    for (int i0 = 0, before = 0; i0 < n_entries; i0 += 32) {
+        unsigned mine = __ballot_sync(0xffffffffu, i0 + lane < n_entries && ids[i0 + lane] == e);
+        for (; mine != 0; mine &= mine - 1, ++before) {
+            if (before < MAX_TOKENS) continue;
+            const int entry = i0 + __ffs(mine) - 1, row = FORM != 0 ? entry / top : entry;
+            const bool there = MG_GUARDED(moe_few, MG_GUARD_ROW, row, x_rows);
+            for (int n = n0 + warp; n < min(n0 + ROWS, N); n += WARPS) {
+                float v[2] = {0.f, 0.f};
+                for (int k = lane; there && k < K; k += 32)
+#pragma unroll
+                    for (int i = 0; i < MI; ++i) v[i] = fmaf(to_float(x[(size_t)row * ldx + k]), to_float(we[(size_t)(i * N + n) * K + k]), v[i]);
+#pragma unroll
+                for (int i = 0; i < MI; ++i) v[i] = warp_sum(v[i]);
+                if (lane == 0) finish<FORM>(v[0], v[MI - 1], entry, n, N, scale, act, limit, out);
+            }
+        }
     }
 }
 
 }  // namespace
 
-// One of the two products for every entry of a step of up to 16 tokens.  ids: [n_tokens * top] chosen experts (-1: none), an
-// expert at most once per token; scale: [entries] or null; x: [x_rows, ldx], rows by token (forms 1 and 2) or by entry (form 0);
+// One of the two products for every entry of a step of up to 16 tokens.  ids: [n_tokens * top] chosen experts (-1: none; a token
+// may name an expert several times); scale: [entries] or null; x: [x_rows, ldx], rows by token (forms 1 and 2) or by entry (form 0);
 // out: [entries, N], bfloat16 (forms 1 and 2) or 32-bit; entry_slot: [entries], written by form 0: the entry itself, or -1.
 // Returns MG_ERR_UNSUPPORTED (and launches nothing) for sizes and alignments it does not take.
 MG_API int mg_moe_few(const void* x, int ldx, const void* w, const int* ids, int n_tokens, int top, const float* scale, void* out,

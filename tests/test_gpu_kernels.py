@@ -675,9 +675,11 @@ def test_experts_of_many_tokens(ops, n, width, inner, experts, top, gated, activ
                                                           (False, "relu_sq", True), (False, "gelu_tanh", False)])
 @pytest.mark.parametrize("n,width,inner,experts,top", [(1, 1024, 1024, 9, 3), (8, 136, 200, 5, 2), (9, 264, 72, 3, 3), (16, 1160, 24, 4, 4),
                                                        (16, 8, 8, 70, 5)])
-def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input):
+@pytest.mark.parametrize("repeats", [False, True])
+def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input, repeats):
     """Steps of up to 16 tokens: no further from the 64-bit result than the kernels of larger steps, at widths that end inside
-    a warp's share of K and inside a CTA's rows, with up to 16 tokens an expert and padding rows."""
+    a warp's share of K and inside a CTA's rows, with up to 16 tokens an expert and padding rows; with tokens that name one
+    expert several times (as a router's choice for a row of scores that are not numbers), up to 64 entries an expert."""
     g = torch.Generator().manual_seed(n * 31 + inner)
     y = randn(n, width, dtype=torch.bfloat16, seed=41)
     w_in = randn(experts, (2 if gated else 1) * inner, width, dtype=torch.bfloat16, seed=42, scale=1 / math.sqrt(width))
@@ -685,6 +687,9 @@ def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activa
     ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(n)]).to(torch.int32)
     if n > 8:
         ids[5] = -1                                  # a padding row
+    if repeats:
+        ids[::2] = 0                                 # expert 0 alone, `top` times
+        ids[1:4, 0] = 0
     weights = torch.rand(n, top, generator=g).cuda()
     ids = ids.cuda()
 
