@@ -7,19 +7,22 @@ the cut); the attention mixer asks for it through ``CudaOps.plan_prompt_attentio
 
 from __future__ import annotations
 
+import numpy as np
+
 QUERY_TILE = 128       # most consecutive tokens of one request in a tile
 KEY_CHUNK = 512        # key positions one work item walks over, where all items run at once
 KEY_BLOCK = 64         # keys the kernel takes at a time
 ITEM_BLOCKS = 4        # what a work item costs besides its key blocks, in key blocks
 MERGE_BLOCKS = 3       # ... and what leaving its results to be merged adds
+_LIMITS = np.array([*range(KEY_CHUNK, 2 * KEY_CHUNK + 1, QUERY_TILE), 1 << 30])   # most keys of an item: what is weighed
 
 
 def query_tiles(q_lens, ctx_befores, slots=None):
     """Cut a ragged batch into work items ``(request, first row, rows, chunk, chunks)``.
 
     The tokens of each request are cut into runs of at most QUERY_TILE rows.  The keys a run
-    may see (positions 0 .. its last token) are cut into ``chunks`` parts of at most KEY_CHUNK
-    positions, one work item each, so that a long context is spread over several CTAs; their
+    may see (positions 0 .. its last token) are cut into ``chunks`` equal parts, of at most KEY_CHUNK
+    positions where all items run at once, one work item each, so that a long context is spread over several CTAs; their
     partial results are merged afterwards.  Items of one run are consecutive, chunk 0 first; the
     runs come longest item first, so that when the grid does not fit the GPU at once, the CTAs
     that start last are the short ones.
@@ -39,19 +42,17 @@ def query_tiles(q_lens, ctx_befores, slots=None):
         row += n
 
     limit = KEY_CHUNK
-    if slots and sum(max(1, -(-keys // limit)) for _, _, _, keys in runs) > slots:
-        best = None
-        for longer in (*range(KEY_CHUNK, 2 * KEY_CHUNK + 1, QUERY_TILE), 1 << 30):
-            items, total, longest = 0, 0, 0
-            for _, _, _, keys in runs:
-                chunks, blocks = max(1, -(-keys // longer)), -(-keys // KEY_BLOCK)
-                besides = ITEM_BLOCKS + (MERGE_BLOCKS if chunks > 1 else 0)
-                items += chunks
-                total += blocks + chunks * besides
-                longest = max(longest, -(-blocks // chunks) + besides)
-            cost = longest if items <= slots else max(longest, total / slots) + 0.3 * longest
-            if best is None or cost < best:
-                best, limit = cost, longer
+    # (where no run sees more than KEY_CHUNK keys there is nothing to weigh)
+    if (slots and max((keys for _, _, _, keys in runs), default=0) > KEY_CHUNK
+            and sum(-(-keys // limit) for _, _, _, keys in runs) > slots):
+        keys = np.array([keys for _, _, _, keys in runs])
+        blocks, limits = -(-keys // KEY_BLOCK), _LIMITS
+        chunks = -(-keys // limits[:, None])                  # [limit, run], as the three below
+        besides = ITEM_BLOCKS + MERGE_BLOCKS * (chunks > 1)
+        items, total = chunks.sum(1), blocks.sum() + (chunks * besides).sum(1)
+        longest = (-(-blocks // chunks) + besides).max(1)
+        cost = np.where(items <= slots, longest, np.maximum(longest, total / slots) + 0.3 * longest)
+        limit = int(limits[cost.argmin()])                    # (the shortest of equals)
     cut = []
     for i, (r, row0, rows, keys) in enumerate(runs):
         chunks = max(1, -(-keys // limit))

@@ -5,6 +5,7 @@ come first."""
 from __future__ import annotations
 
 import random
+import time
 
 import pytest
 
@@ -71,3 +72,38 @@ def test_random_batches(seed):
     ctx = [rng.choice([0, 0, 1, 63, 511, 512, 513, 1500, 4000]) for _ in range(n)]
     _check(q_lens, ctx)
     _check(q_lens, ctx, slots=rng.choice([1, 8, 37, 296]))
+
+
+def test_weighing_of_longer_parts_is_the_plain_sum_over_runs():
+    """The limit on an item's keys is the cheapest of a few, each weighed run by run; the shortest of equals."""
+    rng = random.Random(5)
+    for _ in range(200):
+        requests, slots = rng.randint(1, 70), rng.choice([1, 9, 37, 74])
+        q_lens = [rng.choice([1, 1, rng.randint(1, 700)]) for _ in range(requests)]
+        before = [rng.randint(0, 4000) for _ in range(requests)]
+        keys = [b + min(n, at + QUERY_TILE) for n, b in zip(q_lens, before) for at in range(0, n, QUERY_TILE)]
+        limit, best = KEY_CHUNK, None
+        if sum(-(-k // KEY_CHUNK) for k in keys) > slots:
+            for longer in (*range(KEY_CHUNK, 2 * KEY_CHUNK + 1, QUERY_TILE), max(keys)):
+                costs = []
+                for k in keys:
+                    chunks = -(-k // longer)
+                    costs.append((chunks, -(-k // 64), 4 + 3 * (chunks > 1)))
+                longest = max(-(-blocks // chunks) + besides for chunks, blocks, besides in costs)
+                share = sum(blocks + chunks * besides for chunks, blocks, besides in costs) / slots
+                cost = longest if sum(c for c, _, _ in costs) <= slots else max(longest, share) + 0.3 * longest
+                if best is None or cost < best:
+                    best, limit = cost, longer
+        got = {(r, row): chunks for r, row, _, _, chunks in query_tiles(q_lens, before, slots)}
+        assert sorted(got.values()) == sorted(-(-k // limit) for k in keys)
+
+
+def test_weighing_costs_less_than_cutting():
+    """It is done on the host in every step with prompt portions: all of it within three times the plain cut's time."""
+    def least(slots):
+        def once():
+            begin = time.perf_counter()
+            query_tiles([8] * 255, [1000] * 255, slots)
+            return time.perf_counter() - begin
+        return min(once() for _ in range(30))
+    assert least(18) <= 3 * least(None)
