@@ -175,6 +175,25 @@ def test_tensor_core_tiles_by_one_cta_and_by_pairs(ops, m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m", [8, 17, 64, 65, 128, 129, 700])
+@pytest.mark.parametrize("n", [520, 2048, 2052])
+def test_gelu_of_bfloat16_results_is_right_to_its_last_place(ops, m, n):
+    """Also where it is nearly zero: the products are exact here (one term each), so a result is the rounding of GELU(u).
+    Only the whole columns of prompts take the hardware's tanh."""
+    x, w = torch.zeros(m, 64), torch.zeros(n, 64)
+    x[:, 0], w[:, 0] = 1.0 + torch.arange(m) / 128.0, torch.linspace(-4.0, 4.0, n)
+    x, w = x.to(torch.bfloat16).cuda(), w.to(torch.bfloat16).cuda()
+    u = x.double() @ w.double().T
+    # 2^-8 from rounding (and 2^-15 before it); the kernels of few tokens use tanhf, which is off by up to two units in the last
+    # place: below one 2^-24 each, halved by the formula, so |u| 2^-24, and as much again for what its argument (2^-22 of it)
+    # and 1 + tanh are off; the hardware's tanh is off by up to 2^-10.98 of one
+    want = 0.5 * u * (1.0 + torch.tanh(math.sqrt(2.0 / math.pi) * (u + 0.044715 * u ** 3)))
+    tanh_off = 2.0 ** -10.9 if m > 128 and n % 8 == 0 else 2.0 ** -22
+    got = ops.linear(x, w, None, "gelu_tanh", torch.bfloat16).double()
+    assert ((got - want).abs() <= 2.0 ** -7.99 * want.abs() + 0.5 * tanh_off * u.abs()).all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 11, 16])
 @pytest.mark.parametrize("n,k", [(1536, 512), (512, 2048), (509, 96), (50304, 512), (200, 200), (77, 40)])
 def test_small_batch_projection_with_fused_norm(ops, m, n, k):
