@@ -47,10 +47,11 @@ struct Args {
     float scale;
 };
 
-// One block's (m, l, acc) into what has been merged so far.
+// One block's (m, l, acc) into what has been merged so far.  (A block in which a token sees no key has l = 0; one whose scores are
+// all no numbers has m = -inf too, maxima pass them over, but l is no number, and neither is the token's result.)
 template <int N>
 __device__ __forceinline__ void merge_block(float& M, float& L, float (&A)[N], float m, float l, const float (&acc)[N]) {
-    if (m == -INFINITY) return;
+    if (m == -INFINITY && l == 0.f) return;
     const float top = fmaxf(M, m);
     const float ca = M == -INFINITY ? 0.f : expf(M - top), cb = expf(m - top);
     L = fmaf(l, cb, __fmul_rn(L, ca));
@@ -68,7 +69,7 @@ __device__ __forceinline__ float finish_row(float M, float L, const float* sinks
         *corr = expf(M - top);
         L = __fadd_rn(__fmul_rn(L, *corr), expf(sinks[head] - top));
     }
-    return L > 0.f || L != L ? 1.0f / L : 0.f;
+    return 1.0f / L;                                         // (a token sees itself: only scores of -inf alone leave 0, and 0 / 0)
 }
 
 __device__ __forceinline__ float gated(float o, const float* gate) {

@@ -878,6 +878,45 @@ def test_32_bit_attention_of_portions_and_single_tokens_agrees_bit_for_bit(ops, 
     assert (whole - general).abs().max() <= 2e-5
 
 
+@pytest.mark.parametrize("what", ["query", "key", "block", "low query"])
+@pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
+def test_32_bit_attention_keeps_what_is_no_number(ops, what, single):
+    """Results are no numbers exactly where the general kernel's are: a token whose query is none, tokens that see a key (or a
+    whole block of 64) that is none, a token all of whose scores are -inf."""
+    n, n_head, head_dim, page_tokens, g = 150, 2, 64, 16, torch.Generator().manual_seed(9)
+    pages = -(-n // page_tokens)
+    kv = [torch.randn(pages, n_head, page_tokens, head_dim, generator=g) for _ in range(2)]
+    q = torch.randn(n, n_head * head_dim, generator=g)
+    if what == "query":
+        q[140, 3] = float("nan")
+    elif what == "key":
+        kv[0][90 // page_tokens, 1, 90 % page_tokens, 5] = float("nan")
+    elif what == "block":
+        kv[0][:4, 0, :, 7] = float("nan")                    # keys 0 to 63 of one head
+    else:
+        q[140, 0] = -float("inf")
+        kv[0][:, 0, :, 0].abs_().add_(1.0)
+    i32 = lambda v: torch.as_tensor(v, dtype=torch.int32).cuda()
+    lens = [1] * n if single else [n]
+    cache = SimpleNamespace(k_pages=kv[0].cuda(), v_pages=kv[1].cuda(), group=0, page_tokens=page_tokens, window=None, writes=False)
+    ctx = SimpleNamespace(block_tables=[torch.arange(pages, dtype=torch.int32).repeat(len(lens), 1).cuda()], positions=i32(range(n)),
+                          token_request=i32([r for r, m in enumerate(lens) for _ in range(m)]), decode_only=single,
+                          max_ctx_after=n, host_q_len=lens, req_q_len=i32(lens), req_q_start=i32(range(len(lens))))
+
+    def run():
+        return ops.paged_attention_general(q.cuda(), n_head, n_head, head_dim, head_dim, 0.125, cache, ctx)
+
+    got = run()
+    ops.use_fp32_attention = False
+    try:
+        general = run()
+    finally:
+        ops.use_fp32_attention = True
+    assert torch.isnan(general).any() and not torch.isnan(general).all()
+    assert torch.equal(torch.isnan(got), torch.isnan(general))
+    assert torch.allclose(got, general, rtol=0, atol=2e-5, equal_nan=True)
+
+
 @pytest.mark.parametrize("n,k", [(512, 2048), (2048, 512), (50304, 64), (130, 100), (65, 129), (9, 4)])
 def test_32_bit_products_do_not_hang_on_the_rows_beside_them(ops, n, k):
     """Tiles of every size and the kernel of a few rows: bit for bit the same, with every epilogue."""
