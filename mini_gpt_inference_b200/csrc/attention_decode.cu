@@ -547,14 +547,10 @@ int launch(const void* qkv, const void* k_pages, const void* v_pages, const int*
     const size_t rest = (size_t)WARPS * nh_max * (D + 8) * sizeof(bf16) + (size_t)split_keys(D) * sizeof(int) +
                         (size_t)WARPS * nh_max * (D + 2) * sizeof(float);
     const size_t tile = (size_t)split_keys(D) * D * sizeof(bf16);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaSuccess;
-        for (auto fn : {attention_split_kernel<D, 1, false>, attention_split_kernel<D, 2, false>,
-                        attention_split_kernel<D, 1, true>, attention_split_kernel<D, 2, true>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    for (auto fn : {attention_split_kernel<D, 1, false>, attention_split_kernel<D, 2, false>,
+                    attention_split_kernel<D, 1, true>, attention_split_kernel<D, 2, true>}) {
+        const cudaError_t e = mg_raise_shared(fn, 160 * 1024);
         if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention (split): cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
     }
     dim3 grid(n_tokens, n_kv_head * head_tiles, max_splits);
     const long long ctas = (long long)n_tokens * n_kv_head * head_tiles * max_splits;

@@ -388,12 +388,12 @@ cudaError_t launch(const Args& a, int tiles, int all_blocks, cudaStream_t s) {
     const int group = a.n_head / a.n_kv_head;
     if (tiles > 0) {
         constexpr int smem = (2 * D * (TQ + 4) + TK * D + TK * (TQ + 4)) * (int)sizeof(float);
-        static const cudaError_t configured = cudaFuncSetAttribute(attention_fp32_tiles<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t configured = mg_raise_shared(attention_fp32_tiles<D>, smem);
         if (configured != cudaSuccess) return configured;
         return mg_launch(attention_fp32_tiles<D>, dim3(tiles, a.n_head), dim3(256), smem, s, true, a);
     }
     constexpr int most = (2 * TK * (D + 4) + MAX_GROUP * (D + TK + 1)) * (int)sizeof(float);
-    static const cudaError_t configured = cudaFuncSetAttribute(attention_fp32_split<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const cudaError_t configured = mg_raise_shared(attention_fp32_split<D>, most);
     if (configured != cudaSuccess) return configured;
     const int smem = (2 * TK * (D + 4) + group * (D + TK + 1)) * (int)sizeof(float);
     Args pass = a;

@@ -901,7 +901,7 @@ template <int CW, int RT>
 int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, cudaStream_t s) {
     const int group = p.n_head / p.n_kv_head, row_tiles = (group + 32 * RT - 1) / (32 * RT);
     const size_t smem = wide_smem(32 * RT, dpad);
-    cudaError_t e = cudaFuncSetAttribute(attention_wide_kernel<CW, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = mg_raise_shared(attention_wide_kernel<CW, RT>, smem);
     if (e == cudaSuccess) {
         const dim3 grid = single ? dim3(p.n_tokens * row_tiles, p.n_kv_head, p.splits) : dim3(n_tiles, p.n_kv_head);
         e = mg_launch(attention_wide_kernel<CW, RT>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
@@ -927,13 +927,13 @@ int launch(const AttnParams& p, int single_tokens, int n_tiles, cudaStream_t s) 
     if (single_tokens) {
         const size_t meet = (size_t)(4 * 16 * 2 + 4 * 16 * DVP) * sizeof(float);
         if (meet > smem) smem = meet;
-        e = cudaFuncSetAttribute(attention_split_kernel<DP, DVP, FULL_P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = mg_raise_shared(attention_split_kernel<DP, DVP, FULL_P>, smem);
         if (e == cudaSuccess)
             e = mg_launch(attention_split_kernel<DP, DVP, FULL_P>, dim3(p.n_tokens, p.n_kv_head, p.splits), dim3(128), smem, s, true, p);
         if (e == cudaSuccess && p.counters == nullptr)
             e = mg_launch(attention_merge_kernel, dim3(p.n_tokens, p.n_head), dim3(p.dv >= 128 ? 128 : 64), 0, s, true, p);
     } else {
-        e = cudaFuncSetAttribute(attention_tiles_kernel<DP, DVP, FULL_P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = mg_raise_shared(attention_tiles_kernel<DP, DVP, FULL_P>, smem);
         if (e == cudaSuccess)
             e = mg_launch(attention_tiles_kernel<DP, DVP, FULL_P>, dim3(n_tiles, p.n_kv_head), dim3(128), smem, s, true, p);
     }

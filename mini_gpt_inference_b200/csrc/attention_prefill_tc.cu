@@ -557,8 +557,7 @@ int launch(const Prepared& a, cudaStream_t s) {
     using Z = Sizes<D>;
     // heads of 64: 113 KB, two CTAs per SM; of 128: 193 KB, one
     constexpr size_t smem = Z::Q_BYTES + 2 * Z::KV_STAGES * Z::KV_BYTES + 2 * Z::P_BYTES + sizeof(Sync) + ALIGN_SLACK;
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(attention_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t configured = mg_raise_shared(attention_prefill_tc_kernel<D>, smem);
     if (configured != cudaSuccess)
         return mg_set_error(MG_ERR_CUDA, "attention (prefill): cannot raise shared memory: %s", cudaGetErrorString(configured));
     const cudaError_t le =

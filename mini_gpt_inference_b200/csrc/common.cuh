@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 #define MG_OK 0
 #define MG_ERR_ARG -1
 #define MG_ERR_CUDA -2
@@ -212,6 +214,21 @@ static inline cudaError_t mg_launch(void (*kernel)(KArgs...), dim3 grid, dim3 bl
         cfg.numAttrs = 1;
     }
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device (more than 48 KB have to be asked for).
+inline PerDeviceLimits& mg_shared_limits() {
+    static PerDeviceLimits limits;
+    return limits;
+}
+template <typename... KArgs>
+static inline cudaError_t mg_raise_shared(void (*kernel)(KArgs...), size_t bytes) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)mg_shared_limits().raise((const void*)kernel, device, (int)bytes, [&] {
+        return (int)cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 // ---- index guards (guarded builds only) ------------------------------------------------------------

@@ -163,8 +163,7 @@ template <typename TIn, typename TOut, int EPI, int TM, int TN>
 cudaError_t launch_tiles(const TIn* a, const TIn* w, const float* bias, TOut* out, float* residual, int M, int N, int K, bool vec,
                          cudaStream_t s) {
     constexpr int smem = FMA_STAGES * 16 * (TM + TN) * PITCH * (int)sizeof(float);
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(gemm_fma_kernel<TIn, TOut, EPI, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t configured = mg_raise_shared(gemm_fma_kernel<TIn, TOut, EPI, TM, TN>, smem);
     if (configured != cudaSuccess) return configured;
     return mg_launch(gemm_fma_kernel<TIn, TOut, EPI, TM, TN>, dim3(ceil_div(N, 16 * TN), ceil_div(M, 16 * TM)), dim3(256), smem, s, true,
                      a, w, bias, out, residual, M, N, K, (int)vec);
@@ -273,8 +272,7 @@ cudaError_t launch_few(const float* a, const float* w, const float* bias, float*
     // ids at K = 512: 45 -> 33 us; 32 rows of w a CTA measured the same)
     const int stages = K <= FEW_WARPS * SLICE ? 1 : FEW_STAGES;
     auto bytes = [](int st) { return (int)((FEW_WARPS * st * (FEW_N + MT) * LINE + 2 * FEW_WARPS * MT * FEW_N) * sizeof(float)); };
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(gemm_few_kernel<EPI, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(FEW_STAGES));
+    const cudaError_t configured = mg_raise_shared(gemm_few_kernel<EPI, MT>, bytes(FEW_STAGES));
     if (configured != cudaSuccess) return configured;
     return mg_launch(gemm_few_kernel<EPI, MT>, dim3(ceil_div(N, FEW_N)), dim3(32 * FEW_WARPS), bytes(stages), s, true, a, w, bias,
                      out, residual, M, N, K, stages);

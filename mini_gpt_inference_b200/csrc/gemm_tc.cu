@@ -28,9 +28,6 @@
 // loads: each CTA loads its own tiles.
 #include <cuda.h>
 
-#include <mutex>
-#include <unordered_map>
-
 #include "blackwell.cuh"
 #include "moe_units.cuh"
 #include "tensor_map.cuh"
@@ -523,11 +520,7 @@ int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s, const Exten
     if (tiles <= SMS / CG && g.stages > num_kb) g.stages = num_kb;
     const size_t smem = (size_t)g.stages * stage_bytes + EPI_WARPS * BOXES * BOX_BYTES + sizeof(Control) + 1024;
     constexpr size_t most_dynamic = most - (MODE == EXPERTS ? 2 * 4 * (MAX_EXPERTS + 1) + 64 : 64);
-    static std::once_flag configured;
-    static cudaError_t e = cudaSuccess;
-    std::call_once(configured, [] {
-        e = cudaFuncSetAttribute(gemm_tc_kernel<CG, SUB, MODE, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most_dynamic);
-    });
+    const cudaError_t e = mg_raise_shared(gemm_tc_kernel<CG, SUB, MODE, EXACT>, most_dynamic);
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear: cannot raise shared memory: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CG * (tiles < SMS / CG ? tiles : SMS / CG)));

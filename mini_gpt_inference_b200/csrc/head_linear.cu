@@ -285,12 +285,8 @@ MG_API int mg_head_linear(const void* x, int x_ld, int x_off, int x_head, const 
                          out_off % 2 == 0 && out_head % 2 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0 &&
                          (uintptr_t)out % 4 == 0 && (head_gate || (gate_ld % 2 == 0 && (uintptr_t)gate % 4 == 0));
     if (is_bf16 && vectors && n_tokens <= FEW && few_smem(I, rows_are_inputs) <= 96 * 1024) {
-        static bool configured = false;
-        if (!configured) {
-            const cudaError_t ec = cudaFuncSetAttribute(head_linear_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-            if (ec != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "head_linear (shared memory): %s", cudaGetErrorString(ec));
-            configured = true;
-        }
+        const cudaError_t ec = mg_raise_shared(head_linear_few_kernel, 96 * 1024);
+        if (ec != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "head_linear (shared memory): %s", cudaGetErrorString(ec));
         MG_REQUIRE(ceil_div(J, FEW_OUT) <= 65535, "head_linear: too many outputs");
         const cudaError_t ef = mg_launch(head_linear_few_kernel, dim3(n_head, ceil_div(J, FEW_OUT)), dim3(128),
                                          few_smem(I, rows_are_inputs), s, true, (const bf16*)x, x_ld, x_off, x_head, (const bf16*)w,

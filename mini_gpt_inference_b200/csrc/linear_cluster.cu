@@ -235,8 +235,7 @@ MG_API int mg_linear_cluster(const void* x, const void* w, const float* bias, vo
     if (ntw == 2) kernel = mg == 2 ? linear_cluster_kernel<2, 2> : linear_cluster_kernel<4, 2>;
     else kernel = mg == 2 ? linear_cluster_kernel<2, 1> : linear_cluster_kernel<4, 1>;
     {
-        // (once per variant: the attribute is cheap to set again)
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t e = mg_raise_shared(kernel, 200 * 1024);
         if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear (cluster): cannot raise shared memory: %s", cudaGetErrorString(e));
     }
     const int clusters = (tiles + WARPS * ntw - 1) / (WARPS * ntw);

@@ -370,22 +370,13 @@ MG_API int mg_linear_skinny(const void* x, const float* x32, const int* row_inde
                "linear: the greedy choice goes with 32-bit stored outputs");
     a.amax_v = amax_v; a.amax_i = amax_i; a.amax_limit = (amax_limit <= 0 || amax_limit > N) ? N : amax_limit;
     const int grid = skinny_split(N, K, &a.k_splits, &a.tiles_per_cta);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear (skinny): cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
     cudaStream_t s = (cudaStream_t)stream;
     const bool amax = amax_v != nullptr;
-    const cudaError_t le =
-        mt == 8 ? (amax ? mg_launch(linear_skinny_kernel<8, true>, dim3(grid), dim3(THREADS), smem, s, true, a)
-                        : mg_launch(linear_skinny_kernel<8, false>, dim3(grid), dim3(THREADS), smem, s, true, a))
-                : (amax ? mg_launch(linear_skinny_kernel<16, true>, dim3(grid), dim3(THREADS), smem, s, true, a)
-                        : mg_launch(linear_skinny_kernel<16, false>, dim3(grid), dim3(THREADS), smem, s, true, a));
+    const auto kernel = mt == 8 ? (amax ? linear_skinny_kernel<8, true> : linear_skinny_kernel<8, false>)
+                                : (amax ? linear_skinny_kernel<16, true> : linear_skinny_kernel<16, false>);
+    const cudaError_t e = mg_raise_shared(kernel, 200 * 1024);
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear (skinny): cannot raise shared memory: %s", cudaGetErrorString(e));
+    const cudaError_t le = mg_launch(kernel, dim3(grid), dim3(THREADS), smem, s, true, a);
     if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear_skinny: %s", cudaGetErrorString(le));
     MG_CHECK_LAUNCH("linear_skinny");
     return MG_OK;

@@ -378,20 +378,13 @@ MG_API int mg_linear_stream(const void* x, const float* x32, const int* row_inde
     a.nchunks = nchunks;
     const int grid = stream_split(N, sms, &a.tiles_per_cta);
     const size_t smem = fixed + (size_t)WARPS * stages * TILE_N * ((size_t)kc * 2 + XPAD);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(linear_stream_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_stream_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_stream_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_stream_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear (stream): cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
-    cudaStream_t s = (cudaStream_t)stream;
-    const cudaError_t le = mt == 8    ? mg_launch(linear_stream_kernel<8>, dim3(grid), dim3(THREADS), smem, s, true, a)
-                           : mt == 16 ? mg_launch(linear_stream_kernel<16>, dim3(grid), dim3(THREADS), smem, s, true, a)
-                           : mt == 32 ? mg_launch(linear_stream_kernel<32>, dim3(grid), dim3(THREADS), smem, s, true, a)
-                                      : mg_launch(linear_stream_kernel<64>, dim3(grid), dim3(THREADS), smem, s, true, a);
+    const auto kernel = mt == 8    ? linear_stream_kernel<8>
+                        : mt == 16 ? linear_stream_kernel<16>
+                        : mt == 32 ? linear_stream_kernel<32>
+                                   : linear_stream_kernel<64>;
+    const cudaError_t e = mg_raise_shared(kernel, budget);
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear (stream): cannot raise shared memory: %s", cudaGetErrorString(e));
+    const cudaError_t le = mg_launch(kernel, dim3(grid), dim3(THREADS), smem, (cudaStream_t)stream, true, a);
     if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "linear_stream: %s", cudaGetErrorString(le));
     MG_CHECK_LAUNCH("linear_stream");
     return MG_OK;

@@ -695,15 +695,11 @@ WidePlan wide_plan(int M, int N, int K, bool can_slice, bool prologue) {
     return best;
 }
 
-// Launches the kernel for boxes of 8 * NTW rows (the first launch of a shape raises its shared memory).
+// Launches the kernel for boxes of 8 * NTW rows.
 template <int MT, int NTW, bool SOLO>
 cudaError_t launch_wide_as(int grid, size_t smem, cudaStream_t s, const CUtensorMap& map_w, const WideArgs& a) {
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(linear_wide_kernel<MT, NTW, SOLO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    const cudaError_t e = mg_raise_shared(linear_wide_kernel<MT, NTW, SOLO>, 227 * 1024);
+    if (e != cudaSuccess) return e;
     return mg_launch(linear_wide_kernel<MT, NTW, SOLO>, dim3(grid), dim3(THREADS), smem, s, true, map_w, a);
 }
 

@@ -409,9 +409,9 @@ template <typename T, bool MLSTM>
 int run_chunked(const ChunkParams& p, cudaStream_t s) {
     const int DvE = p.dv + (MLSTM ? 1 : 0);
     const size_t s1 = local_smem(p.L, p.d, DvE, MLSTM), s3 = output_smem(p.L, p.d, p.dv, MLSTM);
-    cudaError_t e = cudaFuncSetAttribute(chunk_local_kernel<T, MLSTM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
+    cudaError_t e = mg_raise_shared(chunk_local_kernel<T, MLSTM>, SMEM_LIMIT);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(chunk_output_kernel<T, MLSTM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
+        e = mg_raise_shared(chunk_output_kernel<T, MLSTM>, SMEM_LIMIT);
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "matrix memory (chunks): %s", cudaGetErrorString(e));
     e = mg_launch(chunk_local_kernel<T, MLSTM>, dim3(p.n_chunks, p.n_head), dim3(THREADS), s1, s, true, p);
     if (e == cudaSuccess)

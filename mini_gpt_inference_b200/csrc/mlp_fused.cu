@@ -380,17 +380,12 @@ MG_API int mg_mlp_fused(const float* x, float* out, float* spare, const float* g
     MlpArgs a;
     a.x = x; a.out = out; a.spare = spare; a.gain = gain; a.shift = shift; a.eps = eps;
     a.w1 = (const bf16*)w1; a.b1 = b1; a.w2p = (const bf16*)w2_packed; a.b2 = b2; a.M = M; a.C = C; a.F = F; a.activation = activation;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaSuccess;
-        for (auto fn : {mlp_fused_kernel<8>, mlp_fused_kernel<16>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "feed-forward (fused): cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    const auto kernel = mt == 8 ? mlp_fused_kernel<8> : mlp_fused_kernel<16>;
+    const cudaError_t e = mg_raise_shared(kernel, 200 * 1024);
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "feed-forward (fused): cannot raise shared memory: %s", cudaGetErrorString(e));
     const int grid = (F + FS - 1) / FS;
     cudaStream_t s = (cudaStream_t)stream;
-    const cudaError_t le = mg_launch(mt == 8 ? mlp_fused_kernel<8> : mlp_fused_kernel<16>, dim3(grid), dim3(THREADS), smem, s, true, a);
+    const cudaError_t le = mg_launch(kernel, dim3(grid), dim3(THREADS), smem, s, true, a);
     if (le != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "mlp_fused: %s", cudaGetErrorString(le));
     MG_CHECK_LAUNCH("mlp_fused");
     return MG_OK;

@@ -749,18 +749,12 @@ MG_API int mg_moe_gemm(const void* x, int ldx, const void* w, const int* offsets
                                 int, int, float);
         static const Kernel wide[3] = {moe_gemm_mma_kernel<0, 128, 2>, moe_gemm_mma_kernel<1, 128, 2>, moe_gemm_mma_kernel<2, 128, 2>};
         static const Kernel narrow[3] = {moe_gemm_mma_kernel<0, 64, 4>, moe_gemm_mma_kernel<1, 64, 4>, moe_gemm_mma_kernel<2, 64, 4>};
-        static bool configured = false;
-        if (!configured) {
-            for (int f = 0; f < 3; ++f) {
-                e = cudaFuncSetAttribute((const void*)wide[f], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_mma_smem(128, 2));
-                if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute((const void*)narrow[f], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_mma_smem(64, 4));
-                MG_LAUNCHED(e, "moe gemm (shared memory)");
-            }
-            configured = true;
-        }
-        e = mg_launch(few ? narrow[form] : wide[form], tgrid, dim3(128), few ? moe_mma_smem(64, 4) : moe_mma_smem(128, 2), s, true,
-                      (const bf16*)x, ldx, (const bf16*)w, stride, offsets, slot_entry, top, scale, out, N, K, x_rows, act, limit);
+        const Kernel kernel = few ? narrow[form] : wide[form];
+        const size_t smem = few ? moe_mma_smem(64, 4) : moe_mma_smem(128, 2);
+        e = mg_raise_shared(kernel, smem);
+        MG_LAUNCHED(e, "moe gemm (shared memory)");
+        e = mg_launch(kernel, tgrid, dim3(128), smem, s, true, (const bf16*)x, ldx, (const bf16*)w, stride, offsets, slot_entry, top,
+                      scale, out, N, K, x_rows, act, limit);
     } else if (is_bf16) {
         auto kernel = form == 1 ? moe_gemm_kernel<bf16, 1> : form == 2 ? moe_gemm_kernel<bf16, 2> : moe_gemm_kernel<bf16, 0>;
         e = mg_launch(kernel, grid, block, 0, s, true, (const bf16*)x, ldx, (const bf16*)w, stride, offsets, slot_entry, top, scale,

@@ -272,13 +272,13 @@ MG_API int mg_qk_norm_rotary(void* proj, int ld, int n_tokens, int n_head, int n
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
     if (is_bf16) {
-        e = smem > 48 * 1024 ? cudaFuncSetAttribute(qk_norm_rotary_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) : cudaSuccess;
+        e = smem > 48 * 1024 ? mg_raise_shared(qk_norm_rotary_kernel<bf16>, 160 * 1024) : cudaSuccess;
         if (e == cudaSuccess)
             e = mg_launch(qk_norm_rotary_kernel<bf16>, dim3(n_tokens), dim3(THREADS), smem, s, true, (bf16*)proj, ld, n_head,
                           n_kv_head, head_dim, v_dim, q_off, k_off, v_off, norm, eps, q_gain, k_gain, rot, freq, positions,
                           slots, (bf16*)k_pages, (bf16*)v_pages, page_tokens, num_pages, v_norm, v_eps, v_freq);
     } else {
-        e = smem > 48 * 1024 ? cudaFuncSetAttribute(qk_norm_rotary_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) : cudaSuccess;
+        e = smem > 48 * 1024 ? mg_raise_shared(qk_norm_rotary_kernel<float>, 160 * 1024) : cudaSuccess;
         if (e == cudaSuccess)
             e = mg_launch(qk_norm_rotary_kernel<float>, dim3(n_tokens), dim3(THREADS), smem, s, true, (float*)proj, ld, n_head,
                           n_kv_head, head_dim, v_dim, q_off, k_off, v_off, norm, eps, q_gain, k_gain, rot, freq, positions,
@@ -325,13 +325,13 @@ MG_API int mg_latent_prepare(const void* proj, int ld, int n_tokens, int n_head,
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
     if (is_bf16) {
-        e = smem > 48 * 1024 ? cudaFuncSetAttribute(latent_prepare_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) : cudaSuccess;
+        e = smem > 48 * 1024 ? mg_raise_shared(latent_prepare_kernel<bf16>, 160 * 1024) : cudaSuccess;
         if (e == cudaSuccess)
             e = mg_launch(latent_prepare_kernel<bf16>, dim3(n_tokens), dim3(THREADS), smem, s, true, (const bf16*)proj, ld,
                           n_head, q_off, q_dim, rot, low_off, rank, gain, eps, freq, (bf16*)q_out, positions, slots,
                           (bf16*)k_pages, (bf16*)v_pages, page_tokens, num_pages, neighbours, magnitude);
     } else {
-        e = smem > 48 * 1024 ? cudaFuncSetAttribute(latent_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) : cudaSuccess;
+        e = smem > 48 * 1024 ? mg_raise_shared(latent_prepare_kernel<float>, 160 * 1024) : cudaSuccess;
         if (e == cudaSuccess)
             e = mg_launch(latent_prepare_kernel<float>, dim3(n_tokens), dim3(THREADS), smem, s, true, (const float*)proj, ld,
                           n_head, q_off, q_dim, rot, low_off, rank, gain, eps, freq, (float*)q_out, positions, slots,

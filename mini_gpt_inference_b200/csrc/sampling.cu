@@ -704,12 +704,8 @@ MG_API int mg_sample(const float* logits, const float* temperature, const int* t
     }
     const size_t row_bytes = (size_t)limit * sizeof(float);
     const int cached = row_bytes <= 220 * 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "sample: cannot raise shared memory: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    const cudaError_t e = mg_raise_shared(sample_kernel, 220 * 1024);
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "sample: cannot raise shared memory: %s", cudaGetErrorString(e));
     sample_kernel<<<rows, SAMPLE_THREADS, cached ? row_bytes : 0, (cudaStream_t)stream>>>(
         logits, temperature, top_k, top_p, seed_lo, seed_hi, counter, out, vocab, limit, cached);
     MG_CHECK_LAUNCH("sample");
