@@ -23,9 +23,9 @@
 // Edges need no special case on the load side: TMA fills what lies outside the matrices with zeros (also a K that is no
 // multiple of 64), and its stores leave out what lies outside.
 //
-// Every wait on an mbarrier is bounded.  If one runs out, the kernel records a code in `status`, skips the rest of its
-// work, waits a moment for copies in flight, frees its TMEM and returns; the host reads `status` later.  No multicast
-// loads: each CTA loads its own tiles.
+// Every wait on an mbarrier is bounded.  If one runs out, the kernel records a code in `status`, stores no tile whose products are
+// not complete (a pair's CTAs learn of it by their own waits running out), waits a moment for copies in flight, frees its TMEM and
+// returns; the host reads `status` later.  No multicast loads: each CTA loads its own tiles.
 #include <cuda.h>
 
 #include "blackwell.cuh"
@@ -284,8 +284,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     umma_commit_group<CG>(smem_u32(&ctl->empty[s]));
                     if (++s == stages) { s = 0; parity ^= 1; }
                 }
-                umma_commit_group<CG>(smem_u32(&ctl->acc_full[a]));
+                if (ok) umma_commit_group<CG>(smem_u32(&ctl->acc_full[a]));
             }
+            // (an accumulator that is not whole is not handed on: the epilogues' own waits, in both CTAs of a pair, run out then)
             if (!ok) {
                 atomicExch(g.status, 2);
                 ctl->failed = 1;
@@ -314,7 +315,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             }
             bool good = mbar_wait(smem_u32(&ctl->acc_full[a]), twice ? (round >> 1) & 1 : 0);
-            if (!good) atomicExch(g.status, 3);
+            if (!good) {
+                atomicExch(g.status, 3);
+                ctl->failed = 1;
+            }
             good = good && (*(volatile uint32_t*)&ctl->failed == 0);
             if (!__all_sync(0xffffffffu, good)) break;       // tcgen05.ld needs the whole warp
             tc_fence_after();
