@@ -554,6 +554,12 @@ int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s, const Exten
 
 }  // namespace
 
+// How mg_linear_tc cuts a product: CTAs a tile (1 or 2), columns a tile, k blocks a stage (1 or 2).
+MG_API void mg_linear_tc_cut(int M, int N, int K, int out_bf16, int* cg, int* bn, int* sub) {
+    const Cut cut = choose_cut(M, N, K, out_bf16 != 0);
+    *cg = cut.cg; *bn = cut.bn; *sub = cut.sub;
+}
+
 // x: [M, K] bf16, w: [N, K] bf16 (both row-major).  Epilogues as mg_linear_simt.  `status` is a
 // device int that receives a non-zero code if a wait inside the kernel ran out.
 // Returns MG_ERR_UNSUPPORTED (and launches nothing) for sizes or alignments TMA cannot take:
@@ -586,7 +592,7 @@ MG_API int mg_linear_tc(const void* x, const void* w, const float* bias, void* o
     const Cut cut = choose_cut(M, N, K, g.out_bf16 != 0);
     MG_REQUIRE((long long)ceil_div(M, cut.cg * TILE_M) * ceil_div(N, cut.bn) < (1ll << 30), "linear: too many tiles");
     g.bn = cut.bn;
-        cudaStream_t s = (cudaStream_t)stream;
+    cudaStream_t s = (cudaStream_t)stream;
     if (cut.cg == 2) return cut.sub == 2 ? launch<2, 2, PLAIN>(x, w, g, s) : launch<2, 1, PLAIN>(x, w, g, s);
     if (M <= TILE_M) return cut.sub == 2 ? launch<1, 2, PLAIN, true>(x, w, g, s) : launch<1, 1, PLAIN, true>(x, w, g, s);
     return cut.sub == 2 ? launch<1, 2, PLAIN>(x, w, g, s) : launch<1, 1, PLAIN>(x, w, g, s);

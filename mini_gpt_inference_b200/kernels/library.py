@@ -88,6 +88,7 @@ _SIGNATURES = {
     "mg_linear_wide_parts": [_I, _I, _I, _I],
     "mg_argmax_merge": [_P, _P, _P, _I, _I, _P],
     "mg_linear_cluster": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "mg_linear_tc_cut": [_I, _I, _I, _I, _P, _P, _P],
     "mg_linear_tc": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "mg_paged_attention_generic": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P],
     "mg_attention_fp32": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I,
