@@ -125,15 +125,20 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 // Each CTA of the pair holds its half of the rows of A, of the rows of B and of the accumulator's rows; the CTA of rank 0
 // issues the products, and both CTAs' loads count on its barriers.  CG is 1 (one CTA by itself) or 2.
 
-// A shared-memory address with the bit that tells the pair's CTAs apart cleared: the same place in the CTA of rank 0.
-constexpr uint32_t PAIR_LEADER_MASK = 0xFEFFFFFFu;
+// The same place in the shared memory of the cluster's CTA of rank 0.
+__device__ __forceinline__ uint32_t leader_address(uint32_t a) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+    return r;
+}
 
+// bar: in a pair the barrier of the CTA of rank 0 (leader_address).
 template <int CG>
 __device__ __forceinline__ void tma_load_2d_group(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     if (CG == 1) { tma_load_2d(dst, map, bar, x, y); return; }
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"((uint64_t)map), "r"(bar & PAIR_LEADER_MASK), "r"(x), "r"(y)
+        ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y)
         : "memory");
 }
 
@@ -171,11 +176,7 @@ __device__ __forceinline__ void umma_commit_group(uint32_t bar) {
 
 // Arrive on the barrier at the same place in the CTA of rank 0 of the cluster.
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\t"
-        "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
-        ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
 }
 
 __device__ __forceinline__ uint32_t cluster_rank() {

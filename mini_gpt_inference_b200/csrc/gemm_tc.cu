@@ -180,6 +180,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (CG == 2) cluster_barrier();                          // the pair's barriers and both halves of TMEM are there
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
+    const uint32_t full0 = smem_u32(&ctl->full[0]), loads_on = CG == 2 ? leader_address(full0) : full0;   // a pair's loads count on rank 0's
     // Barriers and tensor memory are set up while the kernel in front drains; its results (the activations, the residual
     // stream) are touched only behind the wait.  The weights do not come from the kernel in front: their tiles of the
     // first round of stages are asked for before it.
@@ -191,8 +192,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (MODE != EXPERTS && loads && elect_one()) {
         const int n0 = place_of(first_tile).b_row;
         for (int kb = 0; kb < early; ++kb) {
-            const uint32_t full = smem_u32(&ctl->full[kb]), tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
-            if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
+            const uint32_t full = loads_on + kb * 8, tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
+            if (rank == 0) mbar_expect_tx(full0 + kb * 8, CG * stage_bytes);
 #pragma unroll
             for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
         }
@@ -226,7 +227,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const Place p = place_of(tile);
                 const int m0 = p.row, n0 = p.b_row, k0 = p.a_col;
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    const uint32_t full = smem_u32(&ctl->full[s]), stage = smem_u32(smem) + s * stage_bytes;
+                    const uint32_t full = loads_on + s * 8, stage = smem_u32(smem) + s * stage_bytes;
                     if (ahead > 0) {
                         --ahead;
 #pragma unroll
@@ -238,7 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             ok = false;
                             break;
                         }
-                        if (rank == 0) mbar_expect_tx(full, CG * stage_bytes);
+                        if (rank == 0) mbar_expect_tx(full0 + s * 8, CG * stage_bytes);
 #pragma unroll
                         for (int i = 0; i < SUB; ++i) {
                             tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
