@@ -77,6 +77,7 @@ struct KvSink {
 constexpr int PLAIN = 0;             // one matrix
 constexpr int HEADS = 1;             // a small matrix per head: columns a_off + h * a_head .. of A give columns o_off + h * o_head .. of D
 constexpr int EXPERTS = 2;           // a matrix per expert: rows offsets[e] .. offsets[e + 1] of A (and D) belong to expert e
+constexpr int HEADS_IN = 3;          // HEADS with matrices whose rows are inputs (their columns the results)
 constexpr int MAX_EXPERTS = 256;
 
 struct GemmArgs {
@@ -88,7 +89,7 @@ struct GemmArgs {
     KvSink sink;
     int* status;
     int ld_out;                      // elements between rows of D
-    int heads, a_off, a_head, o_off, o_head;               // HEADS; N and K are a head's
+    int heads, a_off, a_head, o_off, o_head;               // HEADS, HEADS_IN; N and K are a head's
     // EXPERTS: form 0 (32-bit results), 1 (gated: a matrix has N gate rows, then N up rows), 2 (activation), as in moe.cu;
     // scale: factor on the sums of row r's entry, slot_entry[r] (null: none)
     const int* offsets;
@@ -123,11 +124,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (the same register value in all lanes)
     const int rank = CG == 2 ? (int)cluster_rank() : 0;
+    constexpr bool BY_HEAD = MODE == HEADS || MODE == HEADS_IN;
     const bool glu = MODE == EXPERTS && g.form == 1;         // bn / 2 gate columns, then the up columns of the same results
     const int bn_out = glu ? bn / 2 : bn;                    // results a tile has
     int m_tiles = (g.M + CG * TILE_M - 1) / (CG * TILE_M);
     const int n_tiles = (g.N + bn_out - 1) / bn_out;
-    int tiles = m_tiles * n_tiles * (MODE == HEADS ? g.heads : 1);
+    int tiles = m_tiles * n_tiles * (BY_HEAD ? g.heads : 1);
     const int first_tile = (int)blockIdx.x / CG, tile_step = (int)gridDim.x / CG;
     __shared__ int expert_row[MODE == EXPERTS ? MAX_EXPERTS + 1 : 1], expert_tile[MODE == EXPERTS ? MAX_EXPERTS + 1 : 1];
     const int num_kb = (g.K + SUB * BLOCK_K - 1) / (SUB * BLOCK_K);     // stages' worth of K
@@ -150,15 +152,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             return p;
         }
         int nt = tile / m_tiles;
-        const int h = MODE == HEADS ? nt / n_tiles : 0;
+        const int h = BY_HEAD ? nt / n_tiles : 0;
         nt -= h * n_tiles;
         p.row = (tile % m_tiles) * CG * TILE_M + rank * TILE_M;
         p.rows_end = g.M;
         p.n0 = nt * bn;
-        p.a_col = MODE == HEADS ? g.a_off + h * g.a_head : 0;
-        p.b_row = (MODE == HEADS ? h * g.N : 0) + p.n0 + rank * b_rows;
-        p.out_col = (MODE == HEADS ? g.o_off + h * g.o_head : 0) + p.n0;
+        p.a_col = BY_HEAD ? g.a_off + h * g.a_head : 0;
+        p.b_row = MODE == HEADS_IN ? h * g.K : (MODE == HEADS ? h * g.N : 0) + p.n0 + rank * b_rows;
+        p.out_col = (BY_HEAD ? g.o_off + h * g.o_head : 0) + p.n0;
         return p;
+    };
+
+    // k block kb of B for a tile
+    auto load_b = [&](uint32_t tile_b, uint32_t full, int kb, const Place& p) {
+        if constexpr (MODE == HEADS_IN) {                    // 64 inputs by 64 results at a time
+            for (int n = 0; n < bn; n += 64)
+                tma_load_2d_group<CG>(tile_b + n * BLOCK_K * 2, &map_b, full, p.n0 + n, p.b_row + kb * BLOCK_K);
+        } else {
+#pragma unroll
+            for (int i = 0; i < SUB; ++i) {
+                tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, p.b_row);
+                if (glu)                                     // (the map's boxes are bn / 2 rows high)
+                    tma_load_2d_group<CG>(tile_b + i * b_tile_bytes + b_tile_bytes / 2, &map_b, full, (kb * SUB + i) * BLOCK_K, p.b_row + g.N);
+            }
+        }
     };
 
     MG_STAMP(gemm, 0);
@@ -190,12 +207,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int early = MODE == EXPERTS ? 0 : num_kb < stages ? num_kb : stages;
     const bool loads = warp == EPI_WARPS, issues = warp == EPI_WARPS + 1;
     if (MODE != EXPERTS && loads && elect_one()) {
-        const int n0 = place_of(first_tile).b_row;
+        const Place p = place_of(first_tile);
         for (int kb = 0; kb < early; ++kb) {
-            const uint32_t full = loads_on + kb * 8, tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
             if (rank == 0) mbar_expect_tx(full0 + kb * 8, CG * stage_bytes);
-#pragma unroll
-            for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
+            load_b(smem_u32(smem) + kb * stage_bytes + B_OFFSET, loads_on + kb * 8, kb, p);
         }
     }
     pdl_wait();
@@ -225,7 +240,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
                 const Place p = place_of(tile);
-                const int m0 = p.row, n0 = p.b_row, k0 = p.a_col;
+                const int m0 = p.row, k0 = p.a_col;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     const uint32_t full = loads_on + s * 8, stage = smem_u32(smem) + s * stage_bytes;
                     if (ahead > 0) {
@@ -241,13 +256,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         }
                         if (rank == 0) mbar_expect_tx(full0 + s * 8, CG * stage_bytes);
 #pragma unroll
-                        for (int i = 0; i < SUB; ++i) {
-                            tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
-                            tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
-                            if (glu)                         // (the map's boxes are bn / 2 rows high)
-                                tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes + b_tile_bytes / 2, &map_b, full,
-                                                      (kb * SUB + i) * BLOCK_K, n0 + g.N);
-                        }
+                        for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
+                        load_b(stage + B_OFFSET, full, kb, p);
                     }
                     if (++s == stages) { s = 0; parity ^= 1; }
                 }
@@ -256,7 +266,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (issues) {
         // ---- products of the stages as they arrive ----
         if (rank == 0 && elect_one()) {
-            const uint32_t idesc = instr_desc_bf16(CG * TILE_M, bn);
+            const uint32_t idesc = MODE == HEADS_IN ? instr_desc_bf16(TILE_M, 64, true) : instr_desc_bf16(CG * TILE_M, bn);
             const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
             int s = 0, round = 0;
             uint32_t parity = 0;
@@ -272,16 +282,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tc_fence_after();
                     // (shared memory ends below 2^18 bytes: the 14 bits of the address field hold address / 16 without a carry)
                     const uint64_t desc_a = desc0 + (uint64_t)((s * stage_bytes) >> 4), desc_b = desc_a + (B_OFFSET >> 4);
+                    if constexpr (MODE == HEADS_IN) {        // 64 results a product; rows of B are k, 16 of them 2 KB further
+                        for (int n = 0; n < bn; n += 64)
 #pragma unroll
-                    for (int i = 0; i < SUB; ++i)
+                            for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+                                umma_bf16_group<CG>(acc + n, desc_a + (uint64_t)((k * UMMA_K * 2) >> 4),
+                                                    desc_b + (uint64_t)((n * BLOCK_K * 2 + k * UMMA_K * 128) >> 4), idesc, (k | kb) != 0 ? 1u : 0u);
+                    } else {
 #pragma unroll
-                        for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                            // 16 elements further along K: 32 bytes inside the swizzled row
-                            const uint64_t step = (uint64_t)((k * UMMA_K * 2) >> 4);
-                            umma_bf16_group<CG>(acc, desc_a + (uint64_t)(i * (A_TILE_BYTES >> 4)) + step,
-                                                desc_b + (uint64_t)(i * (b_tile_bytes >> 4)) + step, idesc,
-                                                (i | k) != 0 || kb != 0 ? 1u : 0u);
-                        }
+                        for (int i = 0; i < SUB; ++i)
+#pragma unroll
+                            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                                // 16 elements further along K: 32 bytes inside the swizzled row
+                                const uint64_t step = (uint64_t)((k * UMMA_K * 2) >> 4);
+                                umma_bf16_group<CG>(acc, desc_a + (uint64_t)(i * (A_TILE_BYTES >> 4)) + step,
+                                                    desc_b + (uint64_t)(i * (b_tile_bytes >> 4)) + step, idesc,
+                                                    (i | k) != 0 || kb != 0 ? 1u : 0u);
+                            }
+                    }
                     umma_commit_group<CG>(smem_u32(&ctl->empty[s]));
                     if (++s == stages) { s = 0; parity ^= 1; }
                 }
@@ -512,7 +530,8 @@ int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s, const Exten
     CUtensorMap map_a, map_b, map_out = {};
     int rc = tensor_map(a, MODE == PLAIN ? g.M : extent->a_rows, MODE == PLAIN ? g.K : extent->a_cols, TILE_M, &map_a);
     if (rc != MG_OK) return rc;
-    rc = tensor_map(b, MODE == PLAIN ? g.N : extent->b_rows, g.K, glu ? g.bn / 2 : g.bn / CG, &map_b);
+    if (MODE == HEADS_IN) rc = tensor_map(b, extent->b_rows, g.N, BLOCK_K, &map_b);
+    else rc = tensor_map(b, MODE == PLAIN ? g.N : extent->b_rows, g.K, glu ? g.bn / 2 : g.bn / CG, &map_b);
     if (rc != MG_OK) return rc;
     if (g.boxes && (rc = tensor_map_store(g.out, g.M, g.ld_out, 32, !g.out_bf16, &map_out)) != MG_OK) return rc;
     const int stage_bytes = SUB * (A_TILE_BYTES + g.bn / CG * BLOCK_K * 2);
@@ -600,9 +619,10 @@ MG_API int mg_linear_tc(const void* x, const void* w, const float* bias, void* o
 }
 
 // One small product per head, bfloat16: out[m, o_off + h * o_head + n] = sum_k x[m, x_off + h * x_head + k] * w[h * N + n, k] for
-// n < N, k < K.  x: rows of x_ld elements, out: rows of out_ld.  Returns MG_ERR_UNSUPPORTED (and launches nothing) unless K and N
+// n < N, k < K, or, with rows_are_inputs, w[h * K + k, n] (read as it lies: tcgen05 takes either order of B from shared memory).
+// x: rows of x_ld elements, out: rows of out_ld.  Returns MG_ERR_UNSUPPORTED (and launches nothing) unless K and N
 // are multiples of 64 and the rows' parts lie on 16-byte boundaries (TMA).
-MG_API int mg_head_linear_tc(const void* x, int x_ld, int x_off, int x_head, const void* w, void* out, int out_ld, int out_off,
+MG_API int mg_head_linear_tc(const void* x, int x_ld, int x_off, int x_head, const void* w, int rows_are_inputs, void* out, int out_ld, int out_off,
                              int out_head, int M, int heads, int K, int N, int* status, void* stream) {
     if (M == 0) return MG_OK;
     MG_REQUIRE(M > 0 && heads > 0 && K > 0 && N > 0 && status != nullptr, "head_linear: bad sizes");
@@ -610,16 +630,17 @@ MG_API int mg_head_linear_tc(const void* x, int x_ld, int x_off, int x_head, con
                    out_off + (long long)(heads - 1) * out_head + N <= out_ld,
                "head_linear: heads outside the rows");
     if (K % 64 != 0 || N % 64 != 0 || x_ld % 8 != 0 || x_off % 8 != 0 || x_head % 8 != 0 || out_ld % 8 != 0 || out_off % 8 != 0 ||
-        out_head % 8 != 0 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) || (long long)heads * N > (1 << 30))
+        out_head % 8 != 0 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) || (long long)heads * (N > K ? N : K) > (1 << 30))
         return mg_set_error(MG_ERR_UNSUPPORTED, "head_linear: no tensor-core tiles for %d x %d", K, N);
     GemmArgs g = {};
     g.out = out; g.out_bf16 = 1; g.boxes = 1; g.epilogue = EPI_STORE;
     g.M = M; g.N = N; g.K = K; g.ld_out = out_ld; g.status = status;
     g.heads = heads; g.a_off = x_off; g.a_head = x_head; g.o_off = out_off; g.o_head = out_head;
     g.bn = N % 128 == 0 ? 128 : 64;
-    const Extent extent = {M, x_ld, heads * N, (long long)ceil_div(M, TILE_M) * heads * (N / g.bn)};
+    const Extent extent = {M, x_ld, heads * (rows_are_inputs ? K : N), (long long)ceil_div(M, TILE_M) * heads * (N / g.bn)};
     MG_REQUIRE(extent.tiles < (1ll << 30), "head_linear: too many tiles");
-    return launch<1, 1, HEADS>(x, w, g, (cudaStream_t)stream, &extent);
+    return rows_are_inputs ? launch<1, 1, HEADS_IN>(x, w, g, (cudaStream_t)stream, &extent)
+                           : launch<1, 1, HEADS>(x, w, g, (cudaStream_t)stream, &extent);
 }
 
 // The products of mg_moe_gemm on the tensor cores, rows by slot: x [n_entries, K] bfloat16 (a token's row for each of its

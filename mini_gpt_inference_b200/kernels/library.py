@@ -69,7 +69,7 @@ _SIGNATURES = {
     "mg_moe_few": [_P, _I, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "mg_moe_gather": [_P, _P, _I, _P, _I, _P, _I, _I, _I, _P],
     "mg_moe_gemm_tc": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P, _P],
-    "mg_head_linear_tc": [_P, _I, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "mg_head_linear_tc": [_P, _I, _I, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "mg_moe_combine": [_P, _P, _I, _P, _I, _I, _I, _P],
     "mg_glu": [_P, _P, _P, _I, _I, _I, _I, _F, _P],
     "mg_layernorm": [_P, _P, _P, _P, _I, _I, _F, _I, _P],

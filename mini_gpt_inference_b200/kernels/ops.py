@@ -1441,16 +1441,6 @@ class CudaOps:
             self._is_bf16(proj), self._stream()), "latent_pair_prepare")
         return out
 
-    def _head_rows(self, weight, n_head, n_in, n_out):
-        """The heads' matrices ``[n_head * n_in, n_out]``, whose rows are inputs, copied once with a row per output: a layout
-        change made when a matrix is first seen, not a computation of the step."""
-        key = ("head rows", weight.data_ptr())
-        hit = self._packed.get(key)
-        if hit is None or hit[0] is not weight:
-            hit = (weight, weight.view(n_head, n_in, n_out).transpose(1, 2).contiguous())
-            self._packed[key] = hit
-        return hit[1]
-
     def head_linear(self, x, x_off, x_head, weight, rows_are_inputs, n_head, n_in, n_out, gate=None, out=None, out_off=0,
                     out_head=None):
         """One small matrix per head: ``out[n, h, j] = sum_i x[n, h, i] * W_h[j, i]`` with ``weight``
@@ -1478,8 +1468,8 @@ class CudaOps:
         if (self.use_tensor_cores and gate is None and x.dtype == torch.bfloat16 and n > HEAD_TC_TOKENS and n_in % 64 == 0
                 and n_out % 64 == 0):
             code = self.lib.mg_head_linear_tc(
-                _ptr(x), x.shape[1], x_off, x_head, _ptr(self._head_rows(weight, n_head, n_in, n_out) if rows_are_inputs else weight),
-                _ptr(out), out.shape[1], out_off, out_head, n, n_head, n_in, n_out, _ptr(self.status), self._stream())
+                _ptr(x), x.shape[1], x_off, x_head, _ptr(weight), 1 if rows_are_inputs else 0, _ptr(out), out.shape[1],
+                out_off, out_head, n, n_head, n_in, n_out, _ptr(self.status), self._stream())
             if code != library.UNSUPPORTED:
                 self._run(code, "head_linear (tensor cores)")
                 return out

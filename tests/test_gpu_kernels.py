@@ -698,6 +698,10 @@ def test_heads_small_products_of_many_tokens(ops, n, heads, n_in, n_out, gap, ro
     assert ((got[..., :n_out].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
     rest = kept[:, 8:].reshape(n, heads, n_out + gap)[..., n_out:]
     assert torch.equal(got[..., n_out:], rest) and torch.equal(out[:, :8], kept[:, :8])
+    # the matrices are read as they are at the call: nothing of them is kept from one call for the next
+    w.mul_(-2.0)
+    again = ops.head_linear(x, 8, n_in + gap, w, rows_are_inputs, heads, n_in, n_out).view(n, heads, n_out)
+    assert torch.equal(again, -2.0 * got[..., :n_out])
     ops.check_status()
 
 
