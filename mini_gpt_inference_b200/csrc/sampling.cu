@@ -286,8 +286,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const uint32_t* __restrict__ seed_lo, const uint32_t* __restrict__ seed_hi,
-              const uint32_t* __restrict__ counter, int* __restrict__ out, int vocab, int limit, int cached) {
-    extern __shared__ float row_cache[];      // the scaled row, if the launch gave room for it
+              const uint32_t* __restrict__ counter, int* __restrict__ out, int vocab, int limit) {
     __shared__ float scratch[SAMPLE_THREADS / 32];
     __shared__ unsigned long long hist[256];
     __shared__ uint32_t sh_prefix;
@@ -303,16 +302,9 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     }
 
     const float safe_t = fmaxf(temp, 1e-6f);
-    // One pass over global memory: the scaled row goes to shared memory (a 50304-wide row is
-    // 197 KB and fits), every later pass reads it from there.
     float mx = -INFINITY;
-    for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-        const float x = lr[i] / safe_t;
-        if (cached) row_cache[i] = x;
-        mx = fmaxf(mx, x);
-    }
-    mx = block_reduce_max(mx, scratch);     // (its barriers also publish row_cache)
-#define ROW(i) (cached ? row_cache[i] : lr[i] / safe_t)
+    for (int i = tid; i < limit; i += SAMPLE_THREADS) mx = fmaxf(mx, lr[i] / safe_t);
+    mx = block_reduce_max(mx, scratch);
 
     // top-k: key of the k-th largest scaled logit
     uint32_t thr_key = 0u;
@@ -325,7 +317,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
             if (tid < 256) hist[tid] = 0ull;
             __syncthreads();
             for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-                const uint32_t key = order_key(ROW(i));
+                const uint32_t key = order_key(lr[i] / safe_t);
                 if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1ull);
             }
             __syncthreads();
@@ -353,7 +345,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     if (p < 1.f) {
         float part = 0.f;
         for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-            const float x = ROW(i);
+            const float x = lr[i] / safe_t;
             if (order_key(x) >= thr_key) part += expf(x - mx);
         }
         const float z_k = block_reduce_sum(part, scratch);
@@ -365,7 +357,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
             if (tid < 256) hist[tid] = 0ull;
             __syncthreads();
             for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-                const float x = ROW(i);
+                const float x = lr[i] / safe_t;
                 const uint32_t key = order_key(x);
                 if (key >= thr_key && (key & mask) == prefix) {
                     // + 1 so that a token whose probability underflows still marks its bin
@@ -398,7 +390,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     // normaliser of what is kept, then the inverse-CDF walk in index order
     float part = 0.f;
     for (int i = tid; i < limit; i += SAMPLE_THREADS) {
-        const float x = ROW(i);
+        const float x = lr[i] / safe_t;
         if (order_key(x) >= thr_key) part += expf(x - mx);
     }
     const float z = block_reduce_sum(part, scratch);
@@ -415,7 +407,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         const int i = t0 + tid;
         float e = 0.f;
         if (i < limit) {
-            const float x = ROW(i);
+            const float x = lr[i] / safe_t;
             if (order_key(x) >= thr_key) { e = expf(x - mx); if (e > 0.f) last_kept = i; }
         }
         float incl = e;                                            // inclusive scan in the warp
@@ -447,13 +439,12 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         __syncthreads();
     }
     if (tid == 0) out[row] = sh_found < 0 ? 0 : sh_found;
-#undef ROW
 }
 
-// ---- the same with a cluster of CTAs per row ------------------------------------------------------
-// What bounds a row is a chain of passes over it: eight counting passes and three sums.  One CTA holds a row in shared
-// memory and reads it anew in every pass (98 values a thread at 50,304 ids), one thread looks through a pass's 256 bins,
-// and its 64-bit sums of probability mass meet in a few bins, lane after lane.  Here a row's values stay in the registers
+// ---- the same with a cluster of CTAs per row, for up to 131,072 ids ---------------------------------
+// What bounds a row is a chain of passes over it: eight counting passes and three sums.  One CTA reads a row anew in every
+// pass (it used to hold rows of up to 56,320 ids in shared memory, 98 values a thread at 50,304), one thread looks through a
+// pass's 256 bins, and its 64-bit sums of probability mass meet in a few bins, lane after lane.  Here a row's values stay in the registers
 // of a cluster's CTAs (16 a thread), lanes that meet in one bin of mass add up among themselves first, a warp picks the
 // digit, and a pass ends in one cluster barrier behind which every CTA sums all histograms itself.
 // 50,304 ids, before and now: 24 rows with top-k 50 and top-p 0.8, 572 -> 45 us; with top-p 0.9 alone, 526 -> 69; plain
@@ -702,12 +693,8 @@ MG_API int mg_sample(const float* logits, const float* temperature, const int* t
         MG_CHECK_LAUNCH("sample (cluster)");
         return MG_OK;
     }
-    const size_t row_bytes = (size_t)limit * sizeof(float);
-    const int cached = row_bytes <= 220 * 1024;
-    const cudaError_t e = mg_raise_shared(sample_kernel, 220 * 1024);
-    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "sample: cannot raise shared memory: %s", cudaGetErrorString(e));
-    sample_kernel<<<rows, SAMPLE_THREADS, cached ? row_bytes : 0, (cudaStream_t)stream>>>(
-        logits, temperature, top_k, top_p, seed_lo, seed_hi, counter, out, vocab, limit, cached);
+    sample_kernel<<<rows, SAMPLE_THREADS, 0, (cudaStream_t)stream>>>(logits, temperature, top_k, top_p, seed_lo, seed_hi, counter,
+                                                                     out, vocab, limit);
     MG_CHECK_LAUNCH("sample");
     return MG_OK;
 }

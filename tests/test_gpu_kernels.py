@@ -332,12 +332,10 @@ def test_whole_feed_forward_in_one_kernel(ops, m, c, f, bias):
 @pytest.mark.parametrize("m", [17, 24, 32, 33, 50, 64, 65, 96, 100, 128])
 @pytest.mark.parametrize("n,k", [(1536, 512), (512, 2048), (509, 96), (200, 200), (77, 40), (2048, 4096),
                                  (6400, 1600), (4800, 1600), (5003, 520)])
-def test_mid_batch_projection_over_a_cluster(ops, m, n, k):
-    """17 to 128 tokens: K cut over the CTAs of a cluster, partial sums met through distributed
-    shared memory; every epilogue, against the formula and against the tensor-core kernel.  The
-    matrices of 4800 rows and more make a warp take two tiles (up to 64 tokens); beyond 64 tokens
-    the kernel holds six or eight groups of 16 tokens and serves matrices of up to 3 MB (the larger
-    ones here then go to the tensor-core kernel, and the comparison holds all the same)."""
+def test_mid_batch_projection_over_a_cluster(ops, monkeypatch, m, n, k):
+    """17 to 128 tokens: every epilogue of whichever kernel the rule gives the size to, against the formula; and up to 64
+    tokens the kernel that cuts K over the CTAs of a cluster (partial sums met through distributed shared memory) beside
+    the tensor-core GEMM."""
     x = randn(m, k, dtype=torch.bfloat16, seed=31)
     w = randn(n, k, dtype=torch.bfloat16, seed=32, scale=1 / math.sqrt(k))
     b = randn(n, seed=33)
@@ -346,12 +344,16 @@ def test_mid_batch_projection_over_a_cluster(ops, m, n, k):
     got = ops.linear(x, w, b, "none", torch.float32)
     assert ops.launches == before + 1
     assert (got.double() - want).abs().max() <= 2e-4
-    ops.use_cluster = False
-    try:
-        other = ops.linear(x, w, b, "none", torch.float32)
-    finally:
-        ops.use_cluster = True
-    assert (got - other).abs().max() <= 1e-4                  # same bf16 inputs, 32-bit sums
+    if m <= 64:
+        rule, sums = type(ops)._cluster_pays, []
+        for pays in (True, False):
+            monkeypatch.setattr(type(ops), "_cluster_pays", staticmethod(lambda m, n, k, pays=pays: pays))
+            sums.append(ops.linear(x, w, b, "none", torch.float32))
+        monkeypatch.setattr(type(ops), "_cluster_pays", staticmethod(rule))
+        assert torch.equal(got, sums[0 if rule(m, n, k) else 1])
+        assert (sums[0] - sums[1]).abs().max() <= 1e-4        # same bf16 inputs, 32-bit sums
+        if n > 200 and k > 200:                               # (two kernels: where sums are long, some differ in their last bit)
+            assert not torch.equal(sums[0], sums[1])
     res = randn(m, n, seed=34)
     keep = res.clone()
     ops.linear_residual(x, w, b, res)
