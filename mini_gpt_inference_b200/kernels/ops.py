@@ -525,13 +525,15 @@ class CudaOps:
     @staticmethod
     def _cluster_pays(m, n, k) -> bool:
         """Whether a bfloat16 product of 17 to 64 tokens is left to the kernel that cuts K over a cluster: its time grows with
-        the tokens and the matrix, that of the tensor-core GEMM with K alone.  Microseconds, cluster / GEMM, at 32 tokens:
-        512 x 128 4.2 / 3.2, 512 x 256 3.3 / 3.4, 2,048 x 512 3.8 / 4.3, 512 x 2,048 3.6 / 6.1, 1,600 x 6,400 11.3 / 16.2, but
-        2,304 x 768 6.4 / 4.9; at 64: 512 x 512 4.3 / 3.7, 2,048 x 512 5.7 / 4.2, 256 x 1,024 4.4 / 4.4, 512 x 2,048 5.6 / 6.1,
-        1,600 x 6,400 26 / 16.  Matrices of one tile (128 rows) stay here, 2.7 / 3.4 and 3.8 / 3.5 at K = 512."""
-        if n <= 128:
-            return True
-        return (n <= 2048 and k >= 256) if m <= 32 else (n <= 512 and k >= 1024)
+        the tokens and the matrix, that of the tensor-core GEMM with K alone, and it has its first weights under way before
+        the kernel in front ends.  So the line is drawn by whole decode steps (us, cluster / GEMM for the matrices at hand).  At
+        up to 32 tokens all but the head: width 768 at 17 and 32 tokens 428 / 447 and 446 / 473, 1,600 344 / 351 and 368 / 376,
+        2,048 246 / 273 at 17.  Beyond, by matrix: all of them at 64 tokens 355 / 348 at width 512, 652 / 577 at 768, 538 / 420
+        at 1,600, but a short and long one stays (1,024 x 2,048 twice a layer in four layers 573 / 598; 512 x 2,048 alone, cold,
+        6.1 / 10.0 a product), and one tile of 128 rows (4.4 / 5.1)."""
+        if m <= 32:
+            return n <= 8192
+        return n <= 128 or (n <= 512 and k >= 1024) or (n <= 1024 and k >= 2048)
 
     @staticmethod
     def _sink_args(kv_sink):
