@@ -548,10 +548,12 @@ attention_split_kernel(const AttnParams p) {
 
 // out[token, head] = (sum over ranges of 2^(m_s - M) O_s) / (sum of 2^(m_s - M) l_s), times the gate.
 // The ranges' maxima and sums come to shared memory, and the first ranges' results to registers, in one trip; the weights
-// are worked out once, and every thread sums its column over the ranges.
-constexpr int MERGE_AHEAD = 32;   // ranges whose results are asked for before the weights are known
+// are worked out once, and every thread sums its column over the ranges.  AHEAD: ranges whose results are asked for before the
+// weights are known (each costs instructions whether the token has it or not: 64 tokens, 16 heads of 512, 2 ranges, 8.7 us with
+// none ahead, 16.7 with 32).
 constexpr int MERGE_MAX = 1024;   // most ranges (mg_attention_mma_split_keys keeps to it)
 
+template <int AHEAD>
 __global__ void attention_merge_kernel(const AttnParams p) {
     __shared__ float weight[MERGE_MAX], sums[MERGE_MAX];
     __shared__ float norm;
@@ -567,10 +569,10 @@ __global__ void attention_merge_kernel(const AttnParams p) {
     }
     const int live = min(min(p.splits, MERGE_MAX),
                          KeyWalk(p, first_visible(p, position)).last(position) / p.split_keys + 1);   // ranges that hold keys
-    // everything is asked for at once: the ranges' maxima, and this thread's first column of the first MERGE_AHEAD ranges
-    float ahead[MERGE_AHEAD];
+    // everything is asked for at once: the ranges' maxima, and this thread's first column of the first AHEAD ranges
+    float ahead[AHEAD];
 #pragma unroll
-    for (int s = 0; s < MERGE_AHEAD; ++s)
+    for (int s = 0; s < AHEAD; ++s)
         ahead[s] = s < live && threadIdx.x < p.dv ? p.part_o[(base + s) * p.dv + threadIdx.x] : 0.f;
     for (int s = threadIdx.x; s < live; s += blockDim.x) {
         const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + (base + s) * 2);
@@ -598,11 +600,11 @@ __global__ void attention_merge_kernel(const AttnParams p) {
         float acc = 0.f;
         if (c == threadIdx.x) {
 #pragma unroll
-            for (int s = 0; s < MERGE_AHEAD; ++s)
+            for (int s = 0; s < AHEAD; ++s)
                 if (s < live) acc = fmaf(weight[s], ahead[s], acc);
         }
 #pragma unroll 8
-        for (int s = c == threadIdx.x ? MERGE_AHEAD : 0; s < live; ++s) acc = fmaf(weight[s], p.part_o[(base + s) * p.dv + c], acc);
+        for (int s = c == threadIdx.x ? AHEAD : 0; s < live; ++s) acc = fmaf(weight[s], p.part_o[(base + s) * p.dv + c], acc);
         acc *= norm;
         if (grow) acc *= logistic(__bfloat162float(grow[c]));
         orow[c] = __float2bfloat16_rn(acc);
@@ -893,6 +895,14 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
         }
 }
 
+cudaError_t launch_merge(const AttnParams& p, int threads, cudaStream_t s) {
+    const dim3 grid(p.n_tokens, p.n_head);
+    const bool few = (long long)p.n_tokens * p.n_head * threads <= 148ll * 2048;      // all on the GPU at once
+    if (p.splits <= 4) return mg_launch(attention_merge_kernel<4>, grid, dim3(threads), 0, s, true, p);
+    if (p.splits <= 8 || !few) return mg_launch(attention_merge_kernel<8>, grid, dim3(threads), 0, s, true, p);
+    return mg_launch(attention_merge_kernel<32>, grid, dim3(threads), 0, s, true, p);
+}
+
 // Bytes of shared memory of a CTA of `rows` rows of dpad features.
 constexpr size_t wide_smem(int rows, int dpad) { return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) + (size_t)4 * rows * sizeof(float); }
 constexpr size_t WIDE_MOST = 227 * 1024;
@@ -907,7 +917,7 @@ int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, cudaStre
         e = mg_launch(attention_wide_kernel<CW, RT>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
     }
     if (e == cudaSuccess && single)
-        e = mg_launch(attention_merge_kernel, dim3(p.n_tokens, p.n_head), dim3(p.dv > 256 ? 512 : p.dv > 128 ? 256 : 128), 0, s, true, p);
+        e = launch_merge(p, p.dv > 256 ? 512 : p.dv > 128 ? 256 : 128, s);
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "attention (wide rows): %s", cudaGetErrorString(e));
     return MG_OK;
 }
@@ -931,7 +941,7 @@ int launch(const AttnParams& p, int single_tokens, int n_tiles, cudaStream_t s) 
         if (e == cudaSuccess)
             e = mg_launch(attention_split_kernel<DP, DVP, FULL_P>, dim3(p.n_tokens, p.n_kv_head, p.splits), dim3(128), smem, s, true, p);
         if (e == cudaSuccess && p.counters == nullptr)
-            e = mg_launch(attention_merge_kernel, dim3(p.n_tokens, p.n_head), dim3(p.dv >= 128 ? 128 : 64), 0, s, true, p);
+            e = launch_merge(p, p.dv >= 128 ? 128 : 64, s);
     } else {
         e = mg_raise_shared(attention_tiles_kernel<DP, DVP, FULL_P>, smem);
         if (e == cudaSuccess)
