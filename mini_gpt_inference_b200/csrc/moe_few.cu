@@ -40,6 +40,32 @@ __device__ __forceinline__ void finish(float v, float u, int entry, int n, int N
     else reinterpret_cast<float*>(out)[to] = v * s;
 }
 
+// The entries of an expert behind its first 16: tokens named it several times (a router does so for a row whose scores are not
+// numbers).  One after the other, a warp to an output.  Rare, and a function of its own, so that the kernel keeps its registers.
+template <int FORM>
+__device__ __noinline__ void the_rest(const bf16* x, int ldx, const bf16* we, const int* ids, int n_entries, int top, const float* scale,
+                                      void* out, int e, int n0, int N, int K, int x_rows, int act, float limit) {
+    constexpr int MI = FORM == 1 ? 2 : 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i0 = 0, before = 0; i0 < n_entries; i0 += 32) {
+        unsigned mine = __ballot_sync(0xffffffffu, i0 + lane < n_entries && ids[i0 + lane] == e);
+        for (; mine != 0; mine &= mine - 1, ++before) {
+            if (before < MAX_TOKENS) continue;
+            const int entry = i0 + __ffs(mine) - 1, row = FORM != 0 ? entry / top : entry;
+            const bool there = MG_GUARDED(moe_few, MG_GUARD_ROW, row, x_rows);
+            for (int n = n0 + warp; n < min(n0 + ROWS, N); n += WARPS) {
+                float v[2] = {0.f, 0.f};
+                for (int k = lane; there && k < K; k += 32)
+#pragma unroll
+                    for (int i = 0; i < MI; ++i) v[i] = fmaf(to_float(x[(size_t)row * ldx + k]), to_float(we[(size_t)(i * N + n) * K + k]), v[i]);
+#pragma unroll
+                for (int i = 0; i < MI; ++i) v[i] = warp_sum(v[i]);
+                if (lane == 0) finish<FORM>(v[0], v[MI - 1], entry, n, N, scale, act, limit, out);
+            }
+        }
+    }
+}
+
 // Forms as mg_moe_gemm: 1 gated, 2 plain, 0 out.
 template <int FORM>
 __global__ void __launch_bounds__(32 * WARPS, FORM == 1 ? 0 : 5)
@@ -141,26 +167,7 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
         }
         finish<FORM>(v[0], v[MI - 1], lists[warp][c], n, N, scale, act, limit, out);
     }
-    if (entries <= MAX_TOKENS) return;
-    // More than 16 entries: tokens named the expert several times (a router does so for a row whose scores are not numbers).
-    // The rest one after the other, a warp to an output: rare, and the columns above keep their registers.
-    for (int i0 = 0, before = 0; i0 < n_entries; i0 += 32) {
-        unsigned mine = __ballot_sync(0xffffffffu, i0 + lane < n_entries && ids[i0 + lane] == e);
-        for (; mine != 0; mine &= mine - 1, ++before) {
-            if (before < MAX_TOKENS) continue;
-            const int entry = i0 + __ffs(mine) - 1, row = FORM != 0 ? entry / top : entry;
-            const bool there = MG_GUARDED(moe_few, MG_GUARD_ROW, row, x_rows);
-            for (int n = n0 + warp; n < min(n0 + ROWS, N); n += WARPS) {
-                float v[2] = {0.f, 0.f};
-                for (int k = lane; there && k < K; k += 32)
-#pragma unroll
-                    for (int i = 0; i < MI; ++i) v[i] = fmaf(to_float(x[(size_t)row * ldx + k]), to_float(we[(size_t)(i * N + n) * K + k]), v[i]);
-#pragma unroll
-                for (int i = 0; i < MI; ++i) v[i] = warp_sum(v[i]);
-                if (lane == 0) finish<FORM>(v[0], v[MI - 1], entry, n, N, scale, act, limit, out);
-            }
-        }
-    }
+    if (entries > MAX_TOKENS) the_rest<FORM>(x, ldx, we, ids, n_entries, top, scale, out, e, n0, N, K, x_rows, act, limit);
 }
 
 }  // namespace
