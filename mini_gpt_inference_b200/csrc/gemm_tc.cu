@@ -84,6 +84,7 @@ struct GemmArgs {
     const float* bias;
     void* out;                       // [M, N] bf16 or 32-bit; the residual stream for EPI_RESIDUAL
     int M, N, K, bn, stages;
+    int a_rows;                      // rows of A that a load brings: TILE_M, or fewer where A has no more
     int epilogue, out_bf16;
     int boxes;                       // rows of the output are multiples of 16 bytes: stored by TMA
     KvSink sink;
@@ -118,6 +119,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int b_rows = bn / CG;
     constexpr uint32_t B_OFFSET = SUB * A_TILE_BYTES;        // a stage: SUB tiles of A, then as many of B
     const uint32_t b_tile_bytes = b_rows * BLOCK_K * 2, stage_bytes = B_OFFSET + SUB * b_tile_bytes;
+    const uint32_t loaded = CG * SUB * (g.a_rows * BLOCK_K * 2 + b_tile_bytes);      // bytes that a stage's loads bring
     uint8_t* boxes = smem + (size_t)stages * stage_bytes;
     Control* ctl = (Control*)(boxes + EPI_WARPS * BOXES * BOX_BYTES);
 
@@ -209,7 +211,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (MODE != EXPERTS && loads && elect_one()) {
         const Place p = place_of(first_tile);
         for (int kb = 0; kb < early; ++kb) {
-            if (rank == 0) mbar_expect_tx(full0 + kb * 8, CG * stage_bytes);
+            if (rank == 0) mbar_expect_tx(full0 + kb * 8, loaded);
             load_b(smem_u32(smem) + kb * stage_bytes + B_OFFSET, loads_on + kb * 8, kb, p);
         }
     }
@@ -254,7 +256,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             ok = false;
                             break;
                         }
-                        if (rank == 0) mbar_expect_tx(full0 + s * 8, CG * stage_bytes);
+                        if (rank == 0) mbar_expect_tx(full0 + s * 8, loaded);
 #pragma unroll
                         for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
                         load_b(stage + B_OFFSET, full, kb, p);
@@ -487,11 +489,17 @@ struct Cut {
     int cg, bn, sub;
 };
 
+// Rows of A in a load.  (What a tile's other rows hold in shared memory goes into results that nobody stores.  Filling them with
+// zeros cost heads of 17 rows: 50,257 x 1,600 44.4 -> 38.9 us, 6,144 x 2,048 17.7 -> 13.6.)
+inline int box_rows(int M) { return M >= TILE_M ? TILE_M : (M + 31) / 32 * 32; }
+
 // The cut with the least time by a count of what bounds a tile, in microseconds (each figure from products of 64 to 2,048
 // rows by 512 to 50,304 columns at K of 512 to 8,192):
 //   a k block takes 0.175 of issue (0.125 where a stage holds two), or 0.0017 (in a pair, which reads half of B per CTA,
 //   0.0014) for each column of products, or its bytes at the 18.5 MB/us that all SMs together read from L2, whichever is most;
-//   a tile's epilogue takes 0.005 a column, beside the next tile's products if there is one, and a next tile 0.5 besides;
+//   a tile's epilogue takes 0.005 a column, beside the next tile's products if there is one, and a next tile 0.5 besides (0.2 where
+//   all tiles have the same rows of A; heads of 17 to 128 rows, 50,257 x 768 in tiles of 192 columns 25.2 to 31.4 us, of 128
+//   23.5 to 28.7; 32,000 x 1,024 in tiles of 256 21.2, of 128 19.5);
 //   a launch takes 2.8, that of pairs 4.5 (they wait for each other at both ends).
 // So pairs win where rounds of large tiles bound the time (2,048 x 6,144 x 2,048: 37.0 us, single CTAs 42.8), and single CTAs
 // below (2,048 x 1,536 x 512: 6.9 us, pairs 8.0).
@@ -504,13 +512,14 @@ inline Cut choose_cut(int M, int N, int K, bool out_bf16) {
             if (bn > grain && bn >= 2 * N) break;
             const long long tiles = (long long)ceil_div(M, cg * TILE_M) * ceil_div(N, bn);
             const long long places = SMS / cg, rounds = (tiles + places - 1) / places;
-            const int block_bytes = A_TILE_BYTES + bn / cg * BLOCK_K * 2, sub = block_bytes <= 24 * 1024 && num_kb > 1 ? 2 : 1;
+            const int b_bytes = bn / cg * BLOCK_K * 2, block_bytes = box_rows(M) * BLOCK_K * 2 + b_bytes;
+            const int sub = A_TILE_BYTES + b_bytes <= 24 * 1024 && num_kb > 1 ? 2 : 1;
             double block = sub == 2 ? 0.125 : 0.175;
             const double products = (cg == 2 ? 0.0014 : 0.0017) * bn, reads = (double)(tiles < places ? tiles : places) * cg * block_bytes / 18.5e6;
             if (products > block) block = products;
             if (reads > block) block = reads;
             const double tile = num_kb * block, epilogue = 0.005 * bn;
-            const double t = (cg == 2 ? 4.5 : 2.8) + (double)(rounds - 1) * (0.5 + (tile > epilogue ? tile : epilogue)) + tile + epilogue;
+            const double t = (cg == 2 ? 4.5 : 2.8) + (double)(rounds - 1) * ((M <= TILE_M ? 0.2 : 0.5) + (tile > epilogue ? tile : epilogue)) + tile + epilogue;
             if (t < least) { least = t; best = Cut{cg, bn, sub}; }
         }
     }
@@ -527,8 +536,9 @@ template <int CG, int SUB, int MODE, bool EXACT = false>
 int launch(const void* a, const void* b, GemmArgs g, cudaStream_t s, const Extent* extent = nullptr) {
     const bool glu = MODE == EXPERTS && g.form == 1;
     if (MODE == PLAIN) g.ld_out = g.N;
+    g.a_rows = MODE == EXPERTS ? TILE_M : box_rows(g.M);
     CUtensorMap map_a, map_b, map_out = {};
-    int rc = tensor_map(a, MODE == PLAIN ? g.M : extent->a_rows, MODE == PLAIN ? g.K : extent->a_cols, TILE_M, &map_a);
+    int rc = tensor_map(a, MODE == PLAIN ? g.M : extent->a_rows, MODE == PLAIN ? g.K : extent->a_cols, g.a_rows, &map_a);
     if (rc != MG_OK) return rc;
     if (MODE == HEADS_IN) rc = tensor_map(b, extent->b_rows, g.N, BLOCK_K, &map_b);
     else rc = tensor_map(b, MODE == PLAIN ? g.N : extent->b_rows, g.K, glu ? g.bn / 2 : g.bn / CG, &map_b);

@@ -1033,6 +1033,28 @@ def test_prompt_portions_of_heads_of_128_on_the_tensor_cores(ops, n_head, n_kv_h
     assert (got - want).norm() <= 1.03 * (general - want).norm()
 
 
+@pytest.mark.parametrize("n,context", [(3, 200), (3, 500), (3, 1990), (700, 500), (700, 1990)])
+def test_ranges_of_single_tokens_are_merged(ops, n, context):
+    """Few ranges and many, of few tokens and of more than the GPU holds at once (other numbers of ranges asked for ahead):
+    the same results as the general kernel, for tokens at all places of the context."""
+    n_head, n_kv_head, head_dim, page_tokens, g = 16, 4, 48, 16, torch.Generator().manual_seed(n + context)
+    pages = -(-context // page_tokens)
+    kv = [torch.randn(pages, n_kv_head, page_tokens, head_dim, generator=g).to(torch.bfloat16).cuda() for _ in range(2)]
+    qkv = torch.randn(n, (n_head + 2 * n_kv_head) * head_dim, generator=g).to(torch.bfloat16).cuda()
+    cache = SimpleNamespace(k_pages=kv[0], v_pages=kv[1], group=0, page_tokens=page_tokens, window=None, writes=False)
+    positions = torch.linspace(0, context - 1, n).to(torch.int32)
+    ctx = SimpleNamespace(block_tables=[torch.arange(pages, dtype=torch.int32).repeat(n, 1).cuda()], positions=positions.cuda(),
+                          token_request=torch.arange(n, dtype=torch.int32).cuda(), decode_only=True, max_ctx_after=context, extra={})
+    got = ops.paged_attention(qkv, n_head, n_kv_head, head_dim, head_dim ** -0.5, cache, ctx).float()
+    ops.use_mma_attention = False
+    try:
+        general = ops.paged_attention(qkv, n_head, n_kv_head, head_dim, head_dim ** -0.5, cache, ctx).float()
+    finally:
+        ops.use_mma_attention = True
+    assert (got - general).abs().max() <= 2.0 ** -7 * general.abs().max()      # the last place of the largest
+    assert not torch.equal(got, torch.zeros_like(got))
+
+
 @pytest.mark.parametrize("gain", [4.0, 9.0, 24.0])
 def test_prompt_attention_with_a_key_far_above_the_others(ops, gain):
     """One key, hundreds of positions into the prompt, scores 8 * gain above the rest (head 0; other
