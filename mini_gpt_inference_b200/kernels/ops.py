@@ -653,7 +653,8 @@ class CudaOps:
         if deferred is not None:
             x = deferred.materialize()
         self._want(x, weight.dtype, "linear input", 2)
-        if x.dtype == torch.bfloat16 and self.use_cluster and 0 < m <= CLUSTER_ROWS and k % 8 == 0 and self._cluster_pays(m, n, k):
+        if (x.dtype == torch.bfloat16 and self.use_cluster and 0 < m <= CLUSTER_ROWS and k % 8 == 0
+                and (self._cluster_pays(m, n, k) or not self.use_tensor_cores)):
             sink = self._sink_args(kv_sink)
             code = self.lib.mg_linear_cluster(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(residual),
                                               m, n, k, epilogue, out_bf16, *sink, self._stream())

@@ -363,6 +363,20 @@ def test_mid_batch_projection_over_a_cluster(ops, monkeypatch, m, n, k):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m,n,k", [(64, 2048, 512), (40, 6400, 1600), (33, 8192, 256)])
+def test_mid_batch_projection_without_the_tensor_core_gemm(ops, monkeypatch, m, n, k):
+    """With the tensor-core GEMM switched off, sizes that the rule gives to it go to the cluster kernel, not to the plain one."""
+    x, w = randn(m, k, dtype=torch.bfloat16, seed=35), randn(n, k, dtype=torch.bfloat16, seed=36, scale=1 / math.sqrt(k))
+    assert not ops._cluster_pays(m, n, k)
+    monkeypatch.setattr(ops, "use_tensor_cores", False)
+    got = ops.linear(x, w, None, "none", torch.float32)
+    out = torch.empty(m, n, device="cuda")
+    code = ops.lib.mg_linear_cluster(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), None, m, n, k, 0, 0, None, None, None, 0, 0, 0,
+                                     0, 0, torch.cuda.current_stream().cuda_stream)
+    assert code == 0 and torch.equal(got, out)
+    assert (got.double() - x.double() @ w.double().T).abs().max() <= 2e-4
+
+
 @pytest.mark.parametrize("m", [1, 5, 8, 16, 24, 33, 64])
 @pytest.mark.parametrize("vocab,k,limit", [(50304, 512, None), (50304, 512, 50257), (509, 96, 300), (77, 40, None),
                                            (9001, 200, 9000)])
