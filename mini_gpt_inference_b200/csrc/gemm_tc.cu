@@ -165,19 +165,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         return p;
     };
 
-    // k block kb of B for a tile
-    auto load_b = [&](uint32_t tile_b, uint32_t full, int kb, const Place& p) {
-        if constexpr (MODE == HEADS_IN) {                    // 64 inputs by 64 results at a time
-            for (int n = 0; n < bn; n += 64)
-                tma_load_2d_group<CG>(tile_b + n * BLOCK_K * 2, &map_b, full, p.n0 + n, p.b_row + kb * BLOCK_K);
-        } else {
-#pragma unroll
-            for (int i = 0; i < SUB; ++i) {
-                tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, p.b_row);
-                if (glu)                                     // (the map's boxes are bn / 2 rows high)
-                    tma_load_2d_group<CG>(tile_b + i * b_tile_bytes + b_tile_bytes / 2, &map_b, full, (kb * SUB + i) * BLOCK_K, p.b_row + g.N);
-            }
-        }
+    // HEADS_IN: k block kb of B, 64 inputs by 64 results at a time
+    auto load_inputs = [&](uint32_t tile_b, uint32_t full, int kb, int b_row, int n0) {
+        for (int n = 0; n < bn; n += 64) tma_load_2d_group<CG>(tile_b + n * BLOCK_K * 2, &map_b, full, n0 + n, b_row + kb * BLOCK_K);
     };
 
     MG_STAMP(gemm, 0);
@@ -210,9 +200,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const bool loads = warp == EPI_WARPS, issues = warp == EPI_WARPS + 1;
     if (MODE != EXPERTS && loads && elect_one()) {
         const Place p = place_of(first_tile);
+        const int n0 = p.b_row;
         for (int kb = 0; kb < early; ++kb) {
+            const uint32_t full = loads_on + kb * 8, tile_b = smem_u32(smem) + kb * stage_bytes + B_OFFSET;
             if (rank == 0) mbar_expect_tx(full0 + kb * 8, loaded);
-            load_b(smem_u32(smem) + kb * stage_bytes + B_OFFSET, loads_on + kb * 8, kb, p);
+            if constexpr (MODE == HEADS_IN) load_inputs(tile_b, full, kb, n0, p.n0);
+            else
+#pragma unroll
+                for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(tile_b + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
         }
     }
     pdl_wait();
@@ -242,7 +237,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
                 const Place p = place_of(tile);
-                const int m0 = p.row, k0 = p.a_col;
+                const int m0 = p.row, n0 = p.b_row, k0 = p.a_col;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     const uint32_t full = loads_on + s * 8, stage = smem_u32(smem) + s * stage_bytes;
                     if (ahead > 0) {
@@ -258,8 +253,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         }
                         if (rank == 0) mbar_expect_tx(full0 + s * 8, loaded);
 #pragma unroll
-                        for (int i = 0; i < SUB; ++i) tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
-                        load_b(stage + B_OFFSET, full, kb, p);
+                        for (int i = 0; i < SUB; ++i) {
+                            tma_load_2d_group<CG>(stage + i * A_TILE_BYTES, &map_a, full, k0 + (kb * SUB + i) * BLOCK_K, m0);
+                            if constexpr (MODE == HEADS_IN) {
+                                load_inputs(stage + B_OFFSET, full, kb, n0, p.n0);
+                                continue;
+                            }
+                            tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes, &map_b, full, (kb * SUB + i) * BLOCK_K, n0);
+                            if (glu)                         // (the map's boxes are bn / 2 rows high)
+                                tma_load_2d_group<CG>(stage + B_OFFSET + i * b_tile_bytes + b_tile_bytes / 2, &map_b, full,
+                                                      (kb * SUB + i) * BLOCK_K, n0 + g.N);
+                        }
                     }
                     if (++s == stages) { s = 0; parity ^= 1; }
                 }
