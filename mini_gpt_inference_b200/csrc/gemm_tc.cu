@@ -215,10 +215,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (MODE == EXPERTS) {
         for (int e = tid; e <= g.n_experts; e += THREADS) expert_row[e] = g.offsets[e];
         __syncthreads();
-        for (int e = tid; e <= g.n_experts; e += THREADS) {
+        if (warp == 0) {                                     // each expert's first tile: sums over 32 experts at a time
             int before = 0;
-            for (int i = 0; i < e; ++i) before += (expert_row[i + 1] - expert_row[i] + TILE_M - 1) / TILE_M;
-            expert_tile[e] = before;
+            for (int e0 = 0; e0 < g.n_experts; e0 += 32) {
+                const int e = e0 + lane;
+                int sum = e < g.n_experts ? (expert_row[e + 1] - expert_row[e] + TILE_M - 1) / TILE_M : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int n = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += n;
+                }
+                if (e < g.n_experts) expert_tile[e + 1] = before + sum;
+                before += __shfl_sync(0xffffffffu, sum, 31);
+            }
+            if (lane == 0) expert_tile[0] = 0;
         }
         __syncthreads();
         m_tiles = expert_tile[g.n_experts];

@@ -20,10 +20,12 @@ from .library import KernelLibraryError, check
 EPILOGUES = {"none": 0, "gelu_tanh": 1, "residual": 2, "relu_sq": 3}
 PLAIN_ACTIVATIONS = {"relu_sq": 0, "gelu_tanh": 1, "silu": 2}           # ... and the activation of a unit without a gate
 GATED_ACTIVATIONS = {"silu": 0, "clamped_swish": 1, "gelu_tanh": 2}     # the gated product of a unit's two halves
-MOE_TC_TOKENS = 64       # more tokens than this take the experts' tensor-core tiles ...
-MOE_TC_EXPERTS = 256     # ... for up to this many experts
-HEAD_TC_TOKENS = 64      # more tokens than this take the heads' small products on the tensor-core GEMM
+MOE_TC_EXPERTS = 256     # most experts the tensor-core tiles take
 MOE_FEW_TOKENS = 16      # most tokens the experts' kernels for few tokens take
+# More tokens than this take the heads' small products on the tensor-core GEMM.  (us, mma.sync / tcgen05: 16 heads of 128 -> 512
+# 12.0 / 4.9 at 65 tokens, 44.0 / 14.6 at 2,048; 512 -> 128 32.5 / 5.9 and 34.6 / 9.2; 8 of 64 -> 64 7.9 / 3.8 and 8.7 / 4.3.
+# It is the faster one from 17 tokens on, 8.2 / 4.9; steps of single tokens were left as they were.)
+HEAD_TC_TOKENS = 64
 SKINNY_ROWS = 16         # most tokens the small-batch projection kernel takes
 CLUSTER_ROWS = 64        # most tokens the mid-batch (K split over a cluster) projection kernel takes
 PREFETCH_MAX_BYTES = 32 << 20   # most of a following matrix that a streaming projection asks into L2
@@ -1588,6 +1590,32 @@ class CudaOps:
                                                self._is_bf16(y), self._stream()), "moe route (scored)")
         return ids, weights, gate
 
+    @staticmethod
+    def _moe_few_pays(entries, experts, width, inner) -> bool:
+        """Whether steps of up to 16 tokens take the experts' kernels that read the matrices with all loads in flight.  These start
+        a CTA for 16 outputs of every expert, chosen or not: with many experts of little work the tiles over grouped entries are
+        faster.  Microseconds, these / tiles, cold: 9 experts of 1,024 x 1,024 15.9 / 24.1 (1 token, 2 experts each) and 29.2 /
+        39.4 (16 tokens, 8 each); 32 of 512 x 128 12.8 / 13.3 and 18.4 / 18.4; 64 of 512 x 128 12.8 / 13.3 and 25.1 / 21.5; 64 of
+        1,024 x 256 20.5 / 24.5 and 44.0 / 38.9, of 1,024 x 1,024 19.4 / 31.7 and 92 / 108; 128 of 512 x 512 19.4 / 20.4 and 61 /
+        56, of 1,024 x 1,024 26.6 / 27.6 and 118 / 136; 256 of 512 x 128 22.5 / 17.4, of 1,024 x 1,024 43.0 / 33.8."""
+        work = width * inner
+        if experts <= 32:
+            return True
+        if experts <= 64:
+            return entries <= 64 or work >= 1 << 19
+        return experts <= 128 and width <= 1024 and work >= 1 << 20
+
+    @staticmethod
+    def _moe_tc_pays(entries, experts, width, inner) -> bool:
+        """Whether the experts' products of larger steps take the tensor-core GEMM's tiles (128 rows of one expert by 128 results;
+        their rows are gathered first) or those of the warp-level tensor cores (64 rows).  Whole feed-forwards, us, warp level /
+        tcgen05, cold, gated, by rows an expert: 9 experts of 1,024 x 1,024 57 / 59 (16), 69 / 63 (64), 100 / 82 (256), 120 / 94
+        (384); 32 of them 80 / 93 (16), 86 / 95 (32), 112 / 100 (64), 163 / 126 (128); 64 of 1,024 x 2,048 214 / 247 (32), 318 / 258
+        (64); 4 of 1,024 x 1,024 50 / 57 (128: 0.5 G multiply-adds), 73 / 60 (192: 0.8 G).  Smaller matrices win late or never: 9 of
+        512 x 256 49 / 57 (384), 16 of 1,024 x 512 90 / 100 (256), 64 of 1,024 x 512 125 / 129 (64)."""
+        work = width * inner
+        return work >= 1 << 20 and entries >= 64 * experts and entries * work >= 800_000_000
+
     def moe_experts(self, y, ids, weights, w_in, w_out, activation="silu", limit=0.0, gated=True, weigh_input=False):
         """``sum_k weights[t, k] * expert(ids[t, k])(y[t])`` as an ``EntrySum`` (every entry's product apart), with expert
         e as ``w_out[e] @ (silu(w_in[e][:F] @ y) * (w_in[e][F:] @ y))``, ``w_in`` [E, 2F, C], ``w_out`` [E, C, F], or, not
@@ -1606,6 +1634,7 @@ class CudaOps:
         is_bf16 = self._is_bf16(y)
         act = (GATED_ACTIVATIONS if gated else PLAIN_ACTIVATIONS)[activation]
         if (self.use_moe_few and is_bf16 and 0 < n <= MOE_FEW_TOKENS and width % 8 == 0 and inner % 8 == 0
+                and self._moe_few_pays(entries, experts, width, inner)
                 and experts <= 65535 and not (_ptr(y) | _ptr(w_in) | _ptr(w_out)) % 16):
             # few tokens: two kernels that find their entries themselves and read the matrices with all loads in flight
             entry_slot = torch.empty((n, top), dtype=torch.int32, device=self.device)
@@ -1624,8 +1653,8 @@ class CudaOps:
         self._run(self.lib.mg_moe_group(_ptr(ids), entries, experts, _ptr(offsets), _ptr(slot_entry), _ptr(entry_slot),
                                         self._stream()), "moe group")
         hidden = torch.empty((entries, inner), dtype=y.dtype, device=self.device)
-        if (self.use_tensor_cores and is_bf16 and n > MOE_TC_TOKENS and width % 8 == 0 and inner % 8 == 0
-                and experts <= MOE_TC_EXPERTS and not (_ptr(y) | _ptr(w_in) | _ptr(w_out)) % 16):
+        if (self.use_tensor_cores and is_bf16 and self._moe_tc_pays(entries, experts, width, inner) and width % 8 == 0
+                and inner % 8 == 0 and experts <= MOE_TC_EXPERTS and not (_ptr(y) | _ptr(w_in) | _ptr(w_out)) % 16):
             # many tokens: their rows gathered by slot, then the GEMM's tiles over each expert's rows
             rows = torch.empty((entries, width), dtype=y.dtype, device=self.device)
             self._run(self.lib.mg_moe_gather(_ptr(y), _ptr(offsets), experts, _ptr(slot_entry), top, _ptr(rows), entries, width, n,

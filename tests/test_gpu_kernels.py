@@ -723,7 +723,7 @@ def test_heads_small_products_of_many_tokens(ops, n, heads, n_in, n_out, gap, ro
 
 @pytest.mark.parametrize("gated,activation,weigh_input", [(True, "silu", False), (False, "relu_sq", True)])
 @pytest.mark.parametrize("n,width,inner,experts,top", [(65, 136, 200, 5, 2), (300, 264, 68 * 4, 3, 3), (700, 512, 384, 17, 2), (130, 72, 520, 200, 1)])
-def test_experts_of_many_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input):
+def test_experts_of_many_tokens(ops, monkeypatch, n, width, inner, experts, top, gated, activation, weigh_input):
     """Tiles over each expert's rows: experts without rows, rows that end inside a tile and inside a box of 32, widths that end
     inside a tile; against the products in 64 bits, hidden features rounded to bfloat16."""
     g = torch.Generator().manual_seed(n)
@@ -743,6 +743,7 @@ def test_experts_of_many_tokens(ops, n, width, inner, experts, top, gated, activ
             z = w_in[e].double() @ y[t].double() * (w if weigh_input else 1.0)
             h = z[:inner] * torch.sigmoid(z[:inner]) * z[inner:] if gated else z.clamp_min(0) ** 2
             want[t] += w_out[e].double() @ h.to(torch.bfloat16).double() * (1.0 if weigh_input else w)
+    monkeypatch.setattr(type(ops), "_moe_tc_pays", staticmethod(lambda *sizes: True))
     before = ops.launches
     ops.moe_experts_residual(y, ids.cuda(), weights, w_in, w_out, residual, activation, 0.0, gated, weigh_input)
     assert ops.launches == before + 5
@@ -757,7 +758,7 @@ def test_experts_of_many_tokens(ops, n, width, inner, experts, top, gated, activ
 @pytest.mark.parametrize("n,width,inner,experts,top", [(1, 1024, 1024, 9, 3), (8, 136, 200, 5, 2), (9, 264, 72, 3, 3), (16, 1160, 24, 4, 4),
                                                        (16, 8, 8, 70, 5)])
 @pytest.mark.parametrize("repeats", [False, True])
-def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activation, weigh_input, repeats):
+def test_experts_of_few_tokens(ops, monkeypatch, n, width, inner, experts, top, gated, activation, weigh_input, repeats):
     """Steps of up to 16 tokens: no further from the 64-bit result than the kernels of larger steps, at widths that end inside
     a warp's share of K and inside a CTA's rows, with up to 16 tokens an expert and padding rows; with tokens that name one
     expert several times (as a router's choice for a row of scores that are not numbers), up to 64 entries an expert."""
@@ -796,6 +797,7 @@ def test_experts_of_few_tokens(ops, n, width, inner, experts, top, gated, activa
             else:
                 h = a.clamp_min(0) ** 2 if activation == "relu_sq" else plain_gpt.gelu_tanh(a)
             want[t] += w_out[e].double() @ h.to(torch.bfloat16).double() * (1.0 if weigh_input else w)
+    monkeypatch.setattr(type(ops), "_moe_few_pays", staticmethod(lambda *sizes: True))
     before = ops.launches
     few = run()
     assert ops.launches == before + 3
