@@ -1049,6 +1049,44 @@ def test_prompt_portions_of_heads_of_128_on_the_tensor_cores(ops, n_head, n_kv_h
     assert (got - want).norm() <= 1.03 * (general - want).norm()
 
 
+@pytest.mark.parametrize("window", [0, 90])
+@pytest.mark.parametrize("n_head,n_kv_head,head_dim", [(4, 2, 48), (3, 3, 80), (8, 1, 128), (2, 2, 128)])
+def test_a_value_that_is_no_number_leaves_the_tokens_in_front_of_it_alone(ops, n_head, n_kv_head, head_dim, window):
+    """Portions of prompts of heads other than 64: results are finite exactly where the general kernel's are."""
+    n, page_tokens, g = 300, 16, torch.Generator().manual_seed(head_dim)
+    pages = -(-n // page_tokens)
+    kv = [torch.randn(pages, n_kv_head, page_tokens, head_dim, generator=g) for _ in range(2)]
+    for t, f, value in ((100, 5, "nan"), (101, 5, "inf"), (130, 6, "inf"), (131, 7, "-inf"), (256, 40, "nan"), (299, 0, "nan")):
+        kv[1][t // page_tokens, 0, t % page_tokens, f] = float(value)
+    qkv = torch.randn(n, (n_head + 2 * n_kv_head) * head_dim, generator=g).to(torch.bfloat16).cuda()
+    i32 = lambda v: torch.as_tensor(v, dtype=torch.int32).cuda()
+    from mini_gpt_inference_b200.parts.context import HostBatch, StepPlan
+
+    def run(begin):
+        plan = StepPlan()
+        ops.plan_prompt_attention(HostBatch([n - begin], [begin], [0], torch.bfloat16), plan, n_head, n_kv_head, head_dim)
+        ctx = SimpleNamespace(block_tables=[torch.arange(pages, dtype=torch.int32)[None].cuda()], positions=i32(range(begin, n)),
+                              token_request=i32([0] * (n - begin)), decode_only=False, max_ctx_after=n, host_q_len=[n - begin],
+                              req_q_len=i32([n - begin]), req_q_start=i32([0]),
+                              extra={k: torch.from_numpy(v).cuda() for k, v in plan.arrays.items()})
+        cache = SimpleNamespace(k_pages=kv[0].to(torch.bfloat16).cuda(), v_pages=kv[1].to(torch.bfloat16).cuda(), group=0,
+                                page_tokens=page_tokens, window=window or None, writes=False)
+        return ops.paged_attention(qkv[begin:], n_head, n_kv_head, head_dim, head_dim ** -0.5, cache, ctx).float()
+
+    for begin in (0, 37):
+        got = run(begin)
+        ops.use_mma_attention = ops.use_prefill_tc = False
+        try:
+            general = run(begin)
+        finally:
+            ops.use_mma_attention = ops.use_prefill_tc = True
+        finite = torch.isfinite(general)
+        assert finite.any() and not finite.all()
+        assert torch.equal(torch.isfinite(got), finite)
+        assert (got - general)[finite].abs().max() <= 1.6e-2
+    ops.check_status()
+
+
 @pytest.mark.parametrize("n,context", [(3, 200), (3, 500), (3, 1990), (700, 500), (700, 1990)])
 def test_ranges_of_single_tokens_are_merged(ops, n, context):
     """Few ranges and many, of few tokens and of more than the GPU holds at once (other numbers of ranges asked for ahead):
