@@ -16,8 +16,8 @@
 //   tiles  (portions of prompts): a tile is 64 / group consecutive tokens of one request with all the
 //          group's heads, 16 rows per warp; every warp walks every key block.  The CTA finds its
 //          request and tile from the requests' token counts on the device.
-//   split  (single tokens): a CTA is one token, one key/value head and one range of keys; the
-//          (128 keys unless the longest possible context would need more than 1,024 ranges); the
+//   split  (single tokens): a CTA is one token, one key/value head and one range of keys (128, or 64 where
+//          there are few rows, unless the longest possible context would need more than 1,024 ranges); the
 //          group's heads are the rows of one m16 tile, each warp takes 16 of a block's 64 keys, the
 //          warps' partial results meet in shared memory and go to scratch; the CTA that finishes a
 //          (token, key/value head) last merges the ranges, applies the gate and stores (or a second
@@ -693,9 +693,9 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 
 // ---- wide rows that hold their own values ------------------------------------------------------------
 // Key rows of several hundred features whose first dv features are also the values (cached latents): too wide for
-// query fragments and a whole row of results in one warp's registers.  A CTA of eight warps takes 32 rows, (token,
+// query fragments and a whole row of results in one warp's registers.  A CTA of eight warps takes 32 or 64 rows, (token,
 // head of the group) pairs in token order, and walks blocks of 64 keys (two buffers in turn).  The queries wait in
-// shared memory.  Warp (rg, cg) takes rows 16 rg .. 16 rg + 15: it multiplies them with keys 16 cg .. 16 cg + 15 of the
+// shared memory.  Warp (rg, cg) takes the rg-th 16 (or 32) of the rows: it multiplies them with keys 16 cg .. 16 cg + 15 of the
 // block, the four warps of a row group exchange their maxima through shared memory, each keeps the sum of its own
 // keys' weights (the sums meet after the last block), the weights go to shared memory as bfloat16, and the warp
 // then adds the block's 64 keys into columns CW cg .. CW cg + CW - 1 of its rows' results.  `single`: the rows are one

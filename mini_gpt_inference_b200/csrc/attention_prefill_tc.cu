@@ -8,17 +8,18 @@
 // mbarriers only (no __syncthreads in the loop, every wait bounded):
 //
 //   load warp        TMA tile loads of keys and values straight from the cache pages (one load
-//                    per page and tensor, 128-byte swizzle) into a ring of four stages; the keys of
-//                    this very step were written to the pages before the launch, so a portion of
-//                    a prompt and a whole prompt read the same numbers;
+//                    per page, tensor and 64 features, 128-byte swizzle) into a ring of four stages (heads
+//                    of 128: three); the keys of this very step were written to the pages before the
+//                    launch, so a portion of a prompt and a whole prompt read the same numbers;
 //   issue warp       S = Q K^T by tcgen05.mma (128 x 64, accumulator in one of two TMEM buffers,
-//                    issued one block ahead of the softmax), then O += P V (128 x 64, V taken as
-//                    it lies in the page as an MN-major operand, accumulated in TMEM over all
-//                    blocks of the chunk);
+//                    issued one block ahead of the softmax), then O += P V (128 x 64, twice for heads
+//                    of 128, V taken as it lies in the page as an MN-major operand, accumulated in
+//                    TMEM over all blocks of the chunk);
 //   softmax warps    four warps, a thread per query row: the row of S comes from TMEM into
 //                    registers in one trip, keys after the row's own position (and before its
 //                    window) are masked, P = 2^(s - ref) goes as bfloat16 into one of two swizzled
-//                    shared-memory tiles; the sum of P stays in 32-bit.
+//                    shared-memory tiles (heads of 128: as two bfloat16 numbers, the second what rounding
+//                    took off the first); the sum of P stays in 32-bit.
 //
 // `ref`, the exponent P is taken relative to, is the maximum of the row's first block.  It moves
 // only if a later block's weights would leave the range 2^60 relative to it (REF_LIMIT); then the
@@ -26,7 +27,7 @@
 // That almost never happens, so a block costs one pass over S and none over O.  The result,
 // O / sum, does not depend on ref beyond rounding.  A tile whose keys were cut into chunks leaves
 // (O, ref, sum) per chunk in scratch; the chunk that finishes last (a counter per tile and head
-// that resets itself) merges them.  Two CTAs share an SM.
+// that resets itself) merges them.  Two CTAs share an SM; of heads of 128, one has it alone.
 //
 // Rows of the tile that belong to no query of this work item are computed and dropped; value
 // rows past the item's last key are cleared in shared memory before they are multiplied.  Heads of

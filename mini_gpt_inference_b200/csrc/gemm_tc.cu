@@ -4,16 +4,17 @@
 //   D[m, n] = sum_k A[m, k] * B[n, k]        A: [M, K] activations, B: [N, K] weights, both K-major bf16
 //
 // A CTA, or a pair of CTAs (CG = 2, a cluster of two on neighbouring SMs whose tensor cores work on one product), computes
-// tiles of 128 * CG x BN of D, one after the other.  Six warps: four for the epilogue, one whose first thread loads (64
-// columns of K at a time into a ring of stages, 128-byte swizzle), one whose first thread issues the products.  In a pair
+// tiles of 128 * CG x BN of D, one after the other.  Ten warps: eight for the epilogue, one with a thread that loads (64 or 128
+// columns of K at a time into a ring of stages, 128-byte swizzle), one with a thread that issues the products.  In a pair
 // each CTA loads its own 128 rows of A and its half of the BN rows of B; the CTA of rank 0 issues for both.  The accumulator
 // lies in TMEM, twice if a CTA has more than one tile: the epilogue of a tile then runs beside the products of the next.
 //
-// Epilogue: a warp reads its 32 TMEM lanes (rows) 32 columns at a time, applies bias and activation, and lays the values
-// into its own 4 KB of shared memory in the swizzled order that the copy engine wants; one thread stores the box, or adds it
-// to the 32-bit residual stream (every element has one summand, so the sum is that of a load, an add and a store).  Keys and
-// values of the QKV projection are copied from the same 4 KB to their cache rows, eight lanes to 128 bytes.  Rows of D that
-// are no multiple of 16 bytes are written from there with plain stores, 32 neighbouring columns at a time.
+// Epilogue: two warps to each 32 TMEM lanes (rows), which take boxes of 128 bytes a row in turn.  A warp reads its lanes 32
+// columns at a time, applies bias and activation, and lays the values into one of its two boxes of 4 KB in shared memory, in the
+// swizzled order that the copy engine wants; one thread stores the box, or adds it to the 32-bit residual stream (every
+// element has one summand, so the sum is that of a load, an add and a store).  Keys and values of the QKV projection are
+// copied from the same box to their cache rows, eight lanes to 128 bytes.  Rows of D that are no multiple of 16 bytes are
+// written from there with plain stores, 32 neighbouring columns at a time.
 //
 // What bounds it: reading the tiles from L2.  A tile of 128 x 128 asks 32 KB for every 64 columns of K, 256 clocks of
 // tensor-core work; an SM takes in some 50 to 60 bytes a clock, so such a tile cannot run above half the tensor cores'
@@ -328,7 +329,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp < EPI_WARPS) {
-        // ---- epilogue: four warps, each on its own 32 lanes of TMEM ----
+        // ---- epilogue: eight warps, two to each 32 lanes of TMEM ----
         const int per_box = g.out_bf16 ? 64 : 32;            // columns of a 128-byte row
         const int quarter = warp & 3, first_box = (warp >> 2) * per_box;       // this warp's lanes, and its first columns
         const bool bias_wide = ((uintptr_t)g.bias & 15) == 0;
