@@ -298,6 +298,9 @@ __device__ __forceinline__ void attend(const uint32_t (&qf)[DP / 16][4], const b
 
 __device__ __forceinline__ float logistic(float x) { return 1.0f / (1.0f + expf(-x)); }
 
+// Bit 15 or 31 is set if the lower or upper of two bfloat16 numbers is an infinity or no number (its exponent all ones).
+__device__ __forceinline__ uint32_t odd_pair(uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; }
+
 // Two bfloat16 numbers, zero in the place of one that is an infinity or no number.
 __device__ __forceinline__ uint32_t finite_pair(uint32_t v) {
     if ((v & 0x7f80u) == 0x7f80u) v &= 0xffff0000u;
@@ -305,10 +308,38 @@ __device__ __forceinline__ uint32_t finite_pair(uint32_t v) {
     return v;
 }
 
-// (16 heads, 2,048 tokens of one prompt: heads of 48 127 -> 128 us a layer, of 80 277 -> 284; 8 prompts of 256 32 -> 33, 59 -> 62.)
-// Keys of a tile's blocks that some row does not see whole, at most: those of its own tokens and those where windows begin, two
-// blocks each; a key is noted by either of two threads.
-constexpr int MAX_ODD = 2 * 4 * KB;
+// Blocks of a tile that some row does not see whole, at most: two that hold its own tokens, two where windows begin.
+constexpr int MAX_MASKED = 4;
+
+// What a tile notes of such blocks: their first keys, and which keys have values that are infinities or no numbers.
+struct OddValues {
+    int any, j0[MAX_MASKED];
+    uint32_t keys[MAX_MASKED][KB / 32];
+};
+
+// The values that were taken out, added to the tile's finished rows where they see their keys; a thread has the same features of
+// all rows.  Rare, and a function of its own: in the kernel's body it costs a CTA a microsecond of instructions.
+__device__ __noinline__ void add_odd_values(const AttnParams& p, const OddValues* odd, const int* table, int kv_head, int first, int count) {
+    const int group = p.n_head / p.n_kv_head;
+    for (int i = 0; i < MAX_MASKED; ++i)
+        for (int k = 0; k < KB; ++k) {
+            if (((odd->keys[i][k >> 5] >> (k & 31)) & 1u) == 0u) continue;
+            const int j = odd->j0[i] + k, index = j / p.page_tokens;
+            const bf16* value = p.v_pages + (((size_t)table[index] * p.n_kv_head + kv_head) * p.page_tokens + j - index * p.page_tokens) * p.v_stride;
+            for (int c = threadIdx.x; c < p.dv; c += blockDim.x) {
+                const float v = __bfloat162float(value[c]);
+                if (isfinite(v)) continue;
+                for (int t = 0; t < count; ++t) {
+                    const int pos = p.positions[first + t];
+                    if (j > pos || (j < first_visible(p, pos) && j >= p.keep_first)) continue;
+                    for (int h = 0; h < group; ++h) {
+                        bf16* o = p.out + ((size_t)(first + t) * p.n_head + kv_head * group + h) * p.dv + c;
+                        *o = __float2bfloat16_rn(__bfloat162float(*o) + v);
+                    }
+                }
+            }
+        }
+}
 
 // ---- portions of prompts ---------------------------------------------------------------------------
 template <int DP, int DVP, bool FULL_P>
@@ -318,9 +349,12 @@ attention_tiles_kernel(const AttnParams p) {
     constexpr int STAGE = KB * (DP + PAD + DVP + PAD);     // elements of one buffer: keys, then values
     bf16* ks = reinterpret_cast<bf16*>(smem_raw);
     bf16* vs = ks + KB * (DP + PAD);
-    __shared__ int odd[FULL_P ? MAX_ODD : 1], n_odd;       // keys with values that are no finite numbers
+    __shared__ OddValues odd;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (FULL_P && tid == 0) n_odd = 0;
+    if (FULL_P && tid < MAX_MASKED * KB / 32) {
+        odd.keys[tid / (KB / 32)][tid % (KB / 32)] = 0u;
+        odd.any = 0;
+    }
     zero_padding<DP, DVP>(p, ks, vs, tid, 128);
     zero_padding<DP, DVP>(p, ks + STAGE, vs + STAGE, tid, 128);
     pdl_trigger();
@@ -372,6 +406,7 @@ attention_tiles_kernel(const AttnParams p) {
     const int warp_max_lo = warp_hi >= 0 ? first_visible(p, warp_hi) : 0;
     // ... and the same for all rows of the tile
     const int first_pos = p.positions[first], tile_max_lo = first_visible(p, hi);
+    int n_masked = 0;
 
     // two buffers take turns: the next block's copies are in flight while this one is multiplied
     const KeyWalk walk(p, lo_tile);
@@ -393,19 +428,21 @@ attention_tiles_kernel(const AttnParams p) {
         __syncthreads();
         if (FULL_P && (j0 + KB - 1 > first_pos || (j0 < tile_max_lo && j0 + KB > p.keep_first))) {
             // half a value row a thread
-            bool found = false;
-            bf16* const half_row = vs + buf * STAGE + (tid >> 1) * (DVP + PAD) + (tid & 1) * (DVP / 2);
+            uint32_t* const half_row = reinterpret_cast<uint32_t*>(vs + buf * STAGE + (tid >> 1) * (DVP + PAD) + (tid & 1) * (DVP / 2));
+            uint32_t any = 0;
 #pragma unroll
-            for (int c = 0; c < DVP / 16; ++c) {
-                uint4* const at = reinterpret_cast<uint4*>(half_row) + c;
-                const uint4 value = *at;
-                const uint4 kept = make_uint4(finite_pair(value.x), finite_pair(value.y), finite_pair(value.z), finite_pair(value.w));
-                if (kept.x != value.x || kept.y != value.y || kept.z != value.z || kept.w != value.w) {
-                    found = true;
-                    *at = kept;
-                }
+            for (int c = 0; c < DVP / 4; c += 4) {
+                const uint4 v = *reinterpret_cast<const uint4*>(half_row + c);
+                any |= odd_pair(v.x) | odd_pair(v.y) | odd_pair(v.z) | odd_pair(v.w);
             }
-            if (found) odd[min(atomicAdd(&n_odd, 1), MAX_ODD - 1)] = j0 + (tid >> 1);
+            if (any & 0x80008000u) {
+#pragma unroll 1
+                for (int c = 0; c < DVP / 4; ++c) half_row[c] = finite_pair(half_row[c]);
+                atomicOr(&odd.keys[min(n_masked, MAX_MASKED - 1)][tid >> 6], 1u << ((tid >> 1) & 31));
+                odd.j0[min(n_masked, MAX_MASKED - 1)] = j0;
+                odd.any = 1;
+            }
+            ++n_masked;
             __syncthreads();
         }
         if (j0 <= warp_hi)
@@ -413,24 +450,6 @@ attention_tiles_kernel(const AttnParams p) {
                                j0 + KB - 1 <= warp_first_pos && (j0 >= warp_max_lo || j0 + KB <= p.keep_first), p.scale_log2, m, l,
                                o, lane, slope_log2, biased, p.cap_log2, p.keep_first);
         __syncthreads();                                    // the buffer is free for the block after the next
-    }
-    if (FULL_P) {
-        for (int i = 0; i < min(n_odd, MAX_ODD); ++i) {
-            const int j = odd[i], index = j / p.page_tokens;
-            const bf16* value = p.v_pages + (((size_t)table[index] * p.n_kv_head + kv_head) * p.page_tokens + j - index * p.page_tokens) * p.v_stride;
-#pragma unroll
-            for (int n = 0; n < DVP / 8; ++n) {
-                const int c = n * 8 + 2 * (lane & 3);
-                if (c >= p.dv) continue;
-                const uint32_t v = *reinterpret_cast<const uint32_t*>(value + c);
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    if (j > pos[r] || (j < lo[r] && j >= p.keep_first)) continue;
-                    if ((v & 0x7f80u) == 0x7f80u) o[n][2 * r] += __uint_as_float(v << 16);
-                    if ((v & 0x7f800000u) == 0x7f800000u) o[n][2 * r + 1] += __uint_as_float(v & 0xffff0000u);
-                }
-            }
-        }
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -451,6 +470,10 @@ attention_tiles_kernel(const AttnParams p) {
             }
             *reinterpret_cast<uint32_t*>(orow + c) = pack_bf16(a, b);
         }
+    }
+    if (FULL_P && odd.any != 0) {
+        __syncthreads();                                    // the rows are stored
+        add_odd_values(p, &odd, table, kv_head, first, count);
     }
 }
 

@@ -74,24 +74,46 @@ struct Sizes {
     static constexpr int P_BYTES = P_PARTS * P_TILE;       // 16 or 32 KB, two of them
 };
 
-// (Heads of 128, 16 of them: one prompt of 2,048 tokens 63.9 -> 68.1 us a layer, 8 of 256 20.3 -> 23.8.)
-// Keys of an item's blocks that some row does not see whole, at most: those of its own 128 tokens and those where windows begin,
-// three blocks each; a key is noted by either of two threads.
-constexpr int MAX_ODD = 2 * 6 * BK;
+// Blocks of an item that some row does not see whole, at most: three that hold its own 128 tokens, three where windows begin.
+constexpr int MAX_MASKED = 6;
 
 struct __align__(8) Sync {
     uint64_t q_full, kv_full[MAX_KV_STAGES], kv_free[MAX_KV_STAGES], s_done[2], pv_done[2], block_done[2];
     uint32_t tmem_base;
     uint32_t failed;
     uint32_t last;            // this work item is the last of its tile to finish
-    int n_odd;                // keys noted in `odd` (heads of 128)
+    int any_odd;              // heads of 128: some value of a block that some row does not see whole is no finite number
+    int masked_key0[MAX_MASKED];            // ... those blocks' first keys
+    uint32_t odd[MAX_MASKED][BK / 32];      // ... and which of their keys
 };
+
+// Bit 15 or 31 is set if the lower or upper of two bfloat16 numbers is an infinity or no number (its exponent all ones).
+__device__ __forceinline__ uint32_t odd_pair(uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; }
 
 // Two bfloat16 numbers, zero in the place of one that is an infinity or no number.
 __device__ __forceinline__ uint32_t finite_pair(uint32_t v) {
     if ((v & 0x7f80u) == 0x7f80u) v &= 0xffff0000u;
     if ((v & 0x7f800000u) == 0x7f800000u) v &= 0xffffu;
     return v;
+}
+
+// The values that were taken out, added to a finished row (bfloat16 `out`, or an item's 32-bit `part`, BQ words between features)
+// where it sees their keys.  Rare, and a function of its own: in the kernel's body it costs a CTA a microsecond of instructions.
+__device__ __noinline__ void add_odd_values(const Sync* sync, const int* table, const bf16* v_pages, int n_kv_head, int kv_head,
+                                            int page_tokens, int d_head, int pos, int last_key, int window, bf16* out, float* part) {
+    for (int i = 0; i < MAX_MASKED; ++i)
+        for (int k = 0; k < BK; ++k) {
+            if (((sync->odd[i][k >> 5] >> (k & 31)) & 1u) == 0u) continue;
+            const int key = sync->masked_key0[i] + k, page = key <= last_key ? table[key / page_tokens] : -1;
+            if (page < 0 || key > pos || (window > 0 && key <= pos - window)) continue;
+            const bf16* const value = v_pages + (((size_t)page * n_kv_head + kv_head) * page_tokens + key % page_tokens) * d_head;
+            for (int d = 0; d < d_head; ++d) {
+                const float v = __bfloat162float(value[d]);
+                if (isfinite(v)) continue;
+                if (out) out[d] = __float2bfloat16_rn(__bfloat162float(out[d]) + v);
+                else part[(size_t)d * BQ] += v;
+            }
+        }
 }
 
 template <int D>
@@ -117,7 +139,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     uint8_t* v_tiles = k_tiles + KV_STAGES * KV_BYTES;
     uint8_t* p_tiles = v_tiles + KV_STAGES * KV_BYTES;   // two
     Sync* sync = (Sync*)(p_tiles + 2 * P_BYTES);
-    int* odd = (int*)(sync + 1);                       // keys with values that are no finite numbers (MAX_ODD, heads of 128)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int item = blockIdx.x, head = blockIdx.y;
@@ -155,7 +176,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_init(smem_u32(&sync->block_done[s]), SOFTMAX_THREADS);
         }
         sync->failed = 0;
-        sync->n_odd = 0;
+        sync->any_odd = 0;
+        for (int i = 0; i < MAX_MASKED; ++i) sync->odd[i][0] = sync->odd[i][1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -188,6 +210,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     pdl_wait();
 
     float ref = -INFINITY, run_sum = 0.f;               // softmax threads: see below
+    int n_masked = 0;                                   // blocks so far that some row does not see whole (heads of 128)
     bool good = true;
 
     if (warp == LOAD_WARP) {
@@ -295,7 +318,28 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int my_pos = pos0 + tid;                     // query position of this thread's row
         uint8_t* const p_row0 = p_tiles + (tid >> 3) * 1024 + (tid & 7) * 128;
         for (int it = 0; it < n_blocks; ++it) {
-            const int blk = first_blk + it;
+            const int blk = first_blk + it, key0 = blk * BK;
+            // Blocks that lie wholly before the first query of the tile (and inside every window)
+            // need no mask: the common case takes the short path.
+            const bool unmasked = (key0 + BK - 1 <= pos0) && (window <= 0 || key0 >= pos0 + BQ - window);
+            if (Z::P_PARTS == 2 && !unmasked) {
+                // while the scores are worked out: half a value row a thread, eight neighbouring threads' pieces in other banks
+                if (!warp_wait(smem_u32(&sync->kv_full[it % KV_STAGES]), (it / KV_STAGES) & 1)) { good = false; atomicExch(status, 25); break; }
+                uint8_t* const half_row = v_tiles + (it % KV_STAGES) * KV_BYTES + (tid & 1) * Z::KV_ATOM + (tid >> 1) * 128;
+                uint32_t any = 0;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(half_row + ((c + tid) & 7) * 16);
+                    any |= odd_pair(v.x) | odd_pair(v.y) | odd_pair(v.z) | odd_pair(v.w);
+                }
+                if (any & 0x80008000u) {
+                    for (int c = 0; c < 32; ++c) reinterpret_cast<uint32_t*>(half_row)[c] = finite_pair(reinterpret_cast<uint32_t*>(half_row)[c]);
+                    atomicOr(&sync->odd[min(n_masked, MAX_MASKED - 1)][tid >> 6], 1u << ((tid >> 1) & 31));
+                    sync->masked_key0[min(n_masked, MAX_MASKED - 1)] = key0;
+                    sync->any_odd = 1;
+                }
+                ++n_masked;
+            }
             if (!warp_wait(smem_u32(&sync->s_done[it & 1]), (it >> 1) & 1)) { good = false; atomicExch(status, 22); break; }
             tc_fence_after();
             // the thread's row of S(it) into registers: two loads in flight, one wait
@@ -305,13 +349,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 tmem_load_32(lane_addr + (uint32_t)((it & 1) * BK + c * 32), *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
             tmem_wait_ld();
 
-            const int key0 = blk * BK;
             // columns <= hi are not in the future (rows of the tile that are no query of this item see nothing)
             const int hi = tid < n_rows ? my_pos - key0 : -1;
             const int lo_col = (window > 0) ? (my_pos - window + 1 - key0) : -1;   // columns >= lo_col are in the window
-            // Blocks that lie wholly before the first query of the tile (and inside every window)
-            // need no mask: the common case takes the short path.
-            const bool unmasked = (key0 + BK - 1 <= pos0) && (window <= 0 || key0 >= pos0 + BQ - window);
             if (!unmasked) {
                 // keys this row may not see get the score -inf: they count for no maximum, their P is 2^-inf = 0
 #pragma unroll
@@ -407,23 +447,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     }
                 }
             }
-            if (Z::P_PARTS == 2 && !unmasked) {
-                // half a value row a thread; eight neighbouring rows' 16-byte pieces meet no bank twice
-                if (!warp_wait(smem_u32(&sync->kv_full[it % KV_STAGES]), (it / KV_STAGES) & 1)) { good = false; atomicExch(status, 25); break; }
-                uint8_t* const half_row = v_tiles + (it % KV_STAGES) * KV_BYTES + (tid & 1) * Z::KV_ATOM + (tid >> 1) * 128;
-                bool found = false;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint4* const at = reinterpret_cast<uint4*>(half_row + ((c + (tid >> 1)) & 7) * 16);
-                    const uint4 v = *at;
-                    const uint4 kept = make_uint4(finite_pair(v.x), finite_pair(v.y), finite_pair(v.z), finite_pair(v.w));
-                    if (kept.x != v.x || kept.y != v.y || kept.z != v.z || kept.w != v.w) {
-                        found = true;
-                        *at = kept;
-                    }
-                }
-                if (found) odd[min(atomicAdd(&sync->n_odd, 1), MAX_ODD - 1)] = key0 + (tid >> 1);
-            }
             // S(it) is in registers no more, P(it) is written (and the accumulator rescaled where it had
             // to be): visible to the tensor core, which may go on
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -439,19 +462,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
     }
     good = __syncthreads_and(good) && (*(volatile uint32_t*)&sync->failed == 0);
-    if (Z::P_PARTS == 2 && good && tid < n_rows) {
-        for (int i = 0; i < min(sync->n_odd, MAX_ODD); ++i) {
-            const int key = odd[i], page = key <= last_key ? table[key / page_tokens] : -1;
-            if (page < 0 || key > pos0 + tid || (window > 0 && key <= pos0 + tid - window)) continue;
-            const uint32_t* const value = reinterpret_cast<const uint32_t*>(v_pages + (((size_t)page * n_kv_head + kv_head) * page_tokens + key % page_tokens) * D);
-#pragma unroll
-            for (int d = 0; d < D; d += 2) {
-                const uint32_t v = value[d / 2];
-                if ((v & 0x7f80u) == 0x7f80u) o[d] = __float_as_uint(__uint_as_float(o[d]) + __uint_as_float(v << 16));
-                if ((v & 0x7f800000u) == 0x7f800000u) o[d + 1] = __float_as_uint(__uint_as_float(o[d + 1]) + __uint_as_float(v & 0xffff0000u));
-            }
-        }
-    }
+    const bool odd_values = Z::P_PARTS == 2 && good && sync->any_odd != 0 && tid < n_rows;
     if (good && n_chunks == 1) {
         if (tid < n_rows) {
             const float inv = run_sum > 0.f ? 1.0f / run_sum : 0.f;
@@ -477,6 +488,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
                 dst[c] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             }
+            if (odd_values)
+                add_odd_values(sync, table, v_pages, n_kv_head, kv_head, page_tokens, D, pos0 + tid, last_key, window,
+                               out + ((size_t)(row0 + tid) * n_head + head) * D, nullptr);
         }
     } else if (n_chunks > 1 && (partial == nullptr || counters == nullptr)) {
         if (tid == 0) atomicExch(status, 31);              // a tile cut along the keys, but nowhere to leave its parts
@@ -491,6 +505,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             for (int d = 0; d < D; ++d) dst[(size_t)d * BQ] = __uint_as_float(o[d]);
             dst[(size_t)D * BQ] = ref;
             dst[(size_t)(D + 1) * BQ] = run_sum;
+            if (odd_values)
+                add_odd_values(sync, table, v_pages, n_kv_head, kv_head, page_tokens, D, pos0 + tid, last_key, window, nullptr, dst);
         }
         __threadfence();
         __syncthreads();
@@ -604,8 +620,8 @@ struct Prepared {
 template <int D>
 int launch(const Prepared& a, cudaStream_t s) {
     using Z = Sizes<D>;
-    // heads of 64: 113 KB, two CTAs per SM; of 128: 197 KB, one
-    constexpr size_t smem = Z::Q_BYTES + 2 * Z::KV_STAGES * Z::KV_BYTES + 2 * Z::P_BYTES + sizeof(Sync) + (D == 128 ? MAX_ODD * sizeof(int) : 0) + ALIGN_SLACK;
+    // heads of 64: 113 KB, two CTAs per SM; of 128: 193 KB, one
+    constexpr size_t smem = Z::Q_BYTES + 2 * Z::KV_STAGES * Z::KV_BYTES + 2 * Z::P_BYTES + sizeof(Sync) + ALIGN_SLACK;
     const cudaError_t configured = mg_raise_shared(attention_prefill_tc_kernel<D>, smem);
     if (configured != cudaSuccess)
         return mg_set_error(MG_ERR_CUDA, "attention (prefill): cannot raise shared memory: %s", cudaGetErrorString(configured));
