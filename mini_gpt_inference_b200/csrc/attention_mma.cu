@@ -308,6 +308,8 @@ __device__ __forceinline__ uint32_t finite_pair(uint32_t v) {
     return v;
 }
 
+// (Looking for them: 16 heads, 50 prompts of 37 tokens, heads of 48 28.3 -> 30.3 us a layer, of 96 48.2 -> 49.7; a prompt of 2,048
+// tokens 127 -> 128, 274 -> 269.)
 // Blocks of a tile that some row does not see whole, at most: two that hold its own tokens, two where windows begin.
 constexpr int MAX_MASKED = 4;
 

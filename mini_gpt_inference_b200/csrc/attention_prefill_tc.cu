@@ -74,6 +74,7 @@ struct Sizes {
     static constexpr int P_BYTES = P_PARTS * P_TILE;       // 16 or 32 KB, two of them
 };
 
+// (Looking for odd values: 16 heads of 128, one prompt of 2,048 tokens 64.4 -> 64.9 us a layer, 8 of 256 20.7 -> 21.6.)
 // Blocks of an item that some row does not see whole, at most: three that hold its own 128 tokens, three where windows begin.
 constexpr int MAX_MASKED = 6;
 
