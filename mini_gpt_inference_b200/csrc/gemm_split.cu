@@ -1,0 +1,541 @@
+// out[m, n] = sum_k a[m, k] * w[n, k] (+ bias[n]) with an epilogue, in 32 bits, on the tensor cores.
+//
+// A 32-bit number is the sum of three bfloat16 numbers, exactly: its 24 bits are rounded to 8 three times, x = h + m + l with
+// |m| <= 2^-9 |h| and |l| <= 2^-18 |h|.  Products of bfloat16 numbers are exact in the tensor cores, so a product of two such sums is
+// six of theirs, h l', l h', m m', h m', m h' and h h'; the three that are left out are below 2^-27 of it.  What rounds is the
+// accumulator: it drops what lies below its last place at every addition of 16 products.  So K is cut into slices of 64; within
+// a slice the five small products of all its terms are summed first, then the four additions of h h', and a slice's sum is added to
+// those before it by an ordinary rounded addition.  Measured against 64 bits (64 terms, normal numbers): 7.8e-8 of the result's size,
+// a chain of fused multiply-adds 14.5e-8; 512 terms 9.9e-8 and 15.7e-8, 2,048 terms 13.4e-8 and 18.1e-8.
+//
+// Every element is summed in that one order whatever the number of rows and the kernel or tile that it falls in, so a token's
+// result does not depend on what else is in the batch (mma.sync and tcgen05.mma give the same bits; so do the two orders of the operands).
+//
+// Rows (of a or w) that hold an infinity, no number, a number of 2^126 or more, or none but zeros and numbers below 2^-90, do not
+// split so: results that meet such a row are summed by fused multiply-adds instead (fma_sum), again whatever is beside them.
+//
+// Two kernels:
+//   gemm_split_kernel   tiles of 128 rows x BN columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
+//                       (a slice ahead, in registers), split them, and lay the pieces into shared memory in the 128-byte swizzle;
+//                       one thread of theirs issues the 24 products of a slice; the warps then take the slice's sums out of
+//                       TMEM and add them to the totals in their registers, beside the next slice's products.
+//   gemm_split_few_kernel   up to 16 rows: a CTA takes 16 rows of w, each of its eight warps every eighth slice, operands by cp.async in
+//                       a ring of the warp's own (the first round of w before the wait for the kernel in front); the fragments
+//                       of mma.sync are split as they are read.  Bound by reading w and by the latency of a launch and a slice.
+// 2,048 rows, FMA tiles and these: 1,536 x 512 101 and 52 us, 2,048 x 512 123 and 53, 512 x 2,048 142 and 66; 8 rows (FMA and mma.sync):
+// 1,536 x 512 3.3 and 3.7, 512 x 2,048 7.5 and 7.3, 50,304 x 512 32.5 and 31.6; 16 rows 49.7 and 46.0.
+#include "blackwell.cuh"
+
+#define EPI_STORE 0      // out = acc + bias
+#define EPI_GELU 1       // out = gelu_tanh(acc + bias)
+#define EPI_RESIDUAL 2   // residual += acc + bias (in place)
+#define EPI_RELU_SQ 3    // out = max(acc + bias, 0)^2
+
+namespace {
+
+constexpr int SLICE = 64;            // terms summed by the tensor cores in one go: a 128-byte row of bfloat16
+constexpr int PIECES = 3;
+constexpr int SMALL = 5;             // products of pieces in front of h h'
+__host__ __device__ constexpr int piece_of_a(int t) { return t == 1 ? 2 : (t == 2 || t == 4) ? 1 : 0; }
+__host__ __device__ constexpr int piece_of_w(int t) { return t == 0 ? 2 : (t == 2 || t == 3) ? 1 : 0; }
+
+// The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third is exact, so its upper half is all of it.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECES]) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    p[0] = *reinterpret_cast<const uint32_t*>(&h);
+    x -= __uint_as_float(p[0] << 16);
+    y -= __uint_as_float(p[0] & 0xffff0000u);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
+    p[1] = *reinterpret_cast<const uint32_t*>(&m);
+    x -= __uint_as_float(p[1] << 16);
+    y -= __uint_as_float(p[1] & 0xffff0000u);
+    p[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+
+// The bits of |x| order as the numbers do, with infinities and no numbers on top.
+__device__ __forceinline__ uint32_t larger(uint32_t most, float x) { return max(most, __float_as_uint(x) & 0x7fffffffu); }
+__device__ __forceinline__ bool splits_badly(uint32_t most) {
+    return most >= 0x7e800000u || (most != 0 && most < 0x12800000u);         // 2^126, 2^-90
+}
+
+// Slices by fused multiply-adds from 0, their sums one after the other.
+__device__ __noinline__ float fma_sum(const float* a, const float* w, int K) {
+    float total = 0.f;
+    for (int k0 = 0; k0 < K; k0 += SLICE) {
+        float sum = 0.f;
+        for (int k = k0; k < min(k0 + SLICE, K); ++k) sum = fmaf(a[k], w[k], sum);
+        total += sum;
+    }
+    return total;
+}
+
+__device__ __forceinline__ float activate(float v, int epilogue) {
+    return epilogue == EPI_GELU ? gelu_tanh(v) : epilogue == EPI_RELU_SQ ? relu_sq(v) : v;
+}
+
+struct SplitArgs {
+    const float* a;
+    const float* w;
+    const float* bias;
+    float* out;                      // the residual stream for EPI_RESIDUAL
+    int M, N, K, epilogue;
+    int wide;                        // rows of the output lie on 16-byte boundaries
+    int* status;
+};
+
+// ---- tiles -----------------------------------------------------------------------------------------------
+constexpr int TILE_M = 128;
+constexpr int WORKERS = 512;         // threads that split and add up
+constexpr int ROW_BYTES = SLICE * 2;
+constexpr int SMS = 148;
+constexpr int OUT_BYTES = 32 * 64;   // a warp's place for 32 rows of 16 results on their way to memory
+constexpr int FLAGS = 3;             // sets of rows' marks: a set is written again two tiles' barriers after it was read
+
+template <int BN> __host__ __device__ constexpr int stage_bytes_of() { return PIECES * (TILE_M + BN) * ROW_BYTES; }
+template <int BN> __host__ __device__ constexpr int dynamic_bytes() { return 1024 + 2 * stage_bytes_of<BN>() + (WORKERS / 32) * OUT_BYTES; }
+
+template <int C>
+__device__ __forceinline__ void tmem_load_columns(uint32_t taddr, uint32_t (&r)[C]) {
+    if constexpr (C == 32) tmem_load_32(taddr, r);
+    else if constexpr (C == 16)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                       "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr) : "memory");
+}
+
+struct __align__(16) SplitControl {
+    uint64_t full[2], done[2];       // the pieces of a step are there; its products are done
+    uint32_t tmem_base;
+    uint32_t failed;
+};
+
+template <int BN>
+__global__ void __launch_bounds__(WORKERS, 1) gemm_split_kernel(const SplitArgs g) {
+    constexpr int STAGE = stage_bytes_of<BN>();
+    constexpr int A_PLANE = TILE_M * ROW_BYTES, W_PLANE = BN * ROW_BYTES;
+    constexpr int AC = TILE_M * 8 / WORKERS, WC = (BN * 8 + WORKERS - 1) / WORKERS;      // 8-number pieces of rows a thread splits
+    constexpr int CW = BN / 4;                                                           // totals a thread keeps
+    extern __shared__ uint8_t split_smem[];
+    __shared__ SplitControl ctl;
+    __shared__ __align__(16) uint8_t bad_a[FLAGS][TILE_M], bad_w[FLAGS][BN];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)split_smem + 1023) & ~(uintptr_t)1023);       // (the swizzle wants 1,024-byte boundaries)
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int m_tiles = (g.M + TILE_M - 1) / TILE_M, n_tiles = (g.N + BN - 1) / BN, tiles = m_tiles * n_tiles;
+    const int slices = (g.K + SLICE - 1) / SLICE;
+    const int my_tiles = ((int)blockIdx.x < tiles) ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    const long long steps = (long long)my_tiles * slices;
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&ctl.full[i]), WORKERS / 32);
+            mbar_init(smem_u32(&ctl.done[i]), 1);
+        }
+        ctl.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&ctl.tmem_base), 2 * BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = ctl.tmem_base;
+    pdl_trigger();
+
+    // The products of step i, once all warps have laid their pieces (which each does behind its last look at the accumulator
+    // and the stage of step i - 2: neither needs a barrier of its own).
+    auto multiply = [&](long long i) {
+        const int half = (int)(i & 1);
+        if (!warp_wait(smem_u32(&ctl.full[half]), (uint32_t)(i >> 1) & 1u)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+            constexpr uint32_t idesc = instr_desc_bf16(TILE_M, BN);
+            const uint64_t desc_a = smem_desc_sw128(smem_u32(smem) + half * STAGE), desc_w = desc_a + (uint64_t)((PIECES * A_PLANE) >> 4);
+            const uint32_t d = tmem_base + half * BN;
+#pragma unroll
+            for (int k = 0; k < SLICE / 16; ++k)
+#pragma unroll
+                for (int t = 0; t < SMALL; ++t)
+                    umma_bf16(d, desc_a + (uint64_t)((piece_of_a(t) * A_PLANE + k * 32) >> 4),
+                              desc_w + (uint64_t)((piece_of_w(t) * W_PLANE + k * 32) >> 4), idesc, (k | t) != 0 ? 1u : 0u);
+#pragma unroll
+            for (int k = 0; k < SLICE / 16; ++k) umma_bf16(d, desc_a + (uint64_t)((k * 32) >> 4), desc_w + (uint64_t)((k * 32) >> 4), idesc, 1u);
+            umma_commit(smem_u32(&ctl.done[half]));
+        }
+        __syncwarp();
+        return true;
+    };
+
+    // ---- loads, splitting, and the slices' sums ----
+    const int col8 = (tid & 7) * 8, row8 = tid >> 3;         // this thread's columns of a slice, and its rows row8 + 64 i
+    const bool has_w = BN * 8 >= WORKERS || tid < BN * 8;
+    float4 av[AC][2], wv[WC][2];
+    uint32_t most_a[AC], most_w[WC];
+    auto fetch = [&](float4 (&v)[2], const float* p, int row, int rows, int k) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* at = p + (size_t)row * g.K + k;
+        v[0] = row < rows && k < g.K ? *reinterpret_cast<const float4*>(at) : zero;
+        v[1] = row < rows && k + 4 < g.K ? *reinterpret_cast<const float4*>(at + 4) : zero;
+    };
+    auto fetch_a = [&](float4 (&v)[AC][2], int tile, int slice) {
+#pragma unroll
+        for (int i = 0; i < AC; ++i) fetch(v[i], g.a, (tile % m_tiles) * TILE_M + row8 + 64 * i, g.M, slice * SLICE + col8);
+    };
+    auto fetch_w = [&](float4 (&v)[WC][2], int tile, int slice) {
+        if (has_w)
+#pragma unroll
+            for (int i = 0; i < WC; ++i) fetch(v[i], g.w, (tile / m_tiles) * BN + row8 + 64 * i, g.N, slice * SLICE + col8);
+    };
+    auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most) {
+        uint32_t p[4][PIECES];
+        split_pair(v[0].x, v[0].y, p[0]);
+        split_pair(v[0].z, v[0].w, p[1]);
+        split_pair(v[1].x, v[1].y, p[2]);
+        split_pair(v[1].z, v[1].w, p[3]);
+        most = larger(larger(larger(larger(most, v[0].x), v[0].y), v[0].z), v[0].w);
+        most = larger(larger(larger(larger(most, v[1].x), v[1].y), v[1].z), v[1].w);
+        uint8_t* at = base + row * ROW_BYTES + (((tid & 7) ^ (row & 7)) << 4);
+#pragma unroll
+        for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(at + q * plane) = make_uint4(p[0][q], p[1][q], p[2][q], p[3][q]);
+    };
+    const int quarter = warp & 3, group = warp >> 2;         // this thread's row of TMEM is 32 quarter + lane, its columns CW group + 0 .. CW
+    const uint32_t sums_at = tmem_base + ((uint32_t)(quarter * 32) << 16) + group * CW;
+    float total[CW];
+#pragma unroll
+    for (int j = 0; j < CW; ++j) total[j] = 0.f;
+    bool ok = true;
+
+    // Takes step i's sums; behind a tile's last slice the tile's results go to memory.
+    auto add_up = [&](long long i, int slice, int tile, int flags) {
+        const int half = (int)(i & 1);
+        if (!warp_wait(smem_u32(&ctl.done[half]), (uint32_t)(i >> 1) & 1u)) return false;
+        tc_fence_after();
+        uint32_t r[CW];
+        tmem_load_columns<CW>(sums_at + half * BN, r);
+        tmem_wait_ld();
+        tc_fence_before();
+#pragma unroll
+        for (int j = 0; j < CW; ++j) total[j] += __uint_as_float(r[j]);
+        if (slice + 1 < slices) return true;
+        asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");            // all rows of the tile are marked
+        const int row0 = (tile % m_tiles) * TILE_M + quarter * 32, col0 = (tile / m_tiles) * BN + group * CW;
+        uint8_t* place = smem + 2 * STAGE + warp * OUT_BYTES;
+        constexpr int HALF = CW < 16 ? CW : 16, CHUNKS = HALF / 4, ROWS = 32 / CHUNKS;   // columns at a time, 16-byte chunks of them, rows an access
+#pragma unroll
+        for (int h = 0; h < CW; h += HALF) {
+            __syncwarp();
+            if (row0 < g.M) {
+#pragma unroll
+                for (int c = 0; c < CHUNKS; ++c)
+                    *reinterpret_cast<float4*>(place + lane * 64 + ((c ^ ((lane >> 1) & (CHUNKS - 1))) << 4)) =
+                        make_float4(total[h + 4 * c], total[h + 4 * c + 1], total[h + 4 * c + 2], total[h + 4 * c + 3]);
+            }
+            __syncwarp();
+            const int c = lane % CHUNKS, n = col0 + h + 4 * c;
+            for (int r = lane / CHUNKS; r < 32; r += ROWS) {
+                const int m = row0 + r;
+                if (m >= g.M || n >= g.N) break;
+                const float4 sums = *reinterpret_cast<const float4*>(place + r * 64 + ((c ^ ((r >> 1) & (CHUNKS - 1))) << 4));
+                float v[4] = {sums.x, sums.y, sums.z, sums.w};
+                const uint32_t marks = *reinterpret_cast<const uint32_t*>(&bad_w[flags][group * CW + h + 4 * c]);
+                if (marks != 0 || bad_a[flags][quarter * 32 + r] != 0) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < g.N && (bad_a[flags][quarter * 32 + r] != 0 || ((marks >> (8 * j)) & 255u) != 0))
+                            v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
+                }
+                float* dst = g.out + (size_t)m * g.N + n;
+                if (g.wide) {                                // (N is a multiple of 4: all four are there)
+                    if (g.bias != nullptr) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] += g.bias[n + j];
+                    }
+                    float4 y = make_float4(activate(v[0], g.epilogue), activate(v[1], g.epilogue), activate(v[2], g.epilogue), activate(v[3], g.epilogue));
+                    if (g.epilogue == EPI_RESIDUAL) {
+                        const float4 old = *reinterpret_cast<const float4*>(dst);
+                        y = make_float4(old.x + y.x, old.y + y.y, old.z + y.z, old.w + y.w);
+                    }
+                    *reinterpret_cast<float4*>(dst) = y;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < g.N) {
+                            const float y = activate(v[j] + (g.bias != nullptr ? g.bias[n + j] : 0.f), g.epilogue);
+                            if (g.epilogue == EPI_RESIDUAL) dst[j] += y;
+                            else dst[j] = y;
+                        }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < CW; ++j) total[j] = 0.f;
+        return true;
+    };
+
+    int tile = blockIdx.x, slice = 0, flags = 0;             // of the step that is split
+    int was_tile = 0, was_slice = 0, was_flags = 0;          // of the step in front of it
+    if (steps > 0) fetch_w(wv, tile, 0);                     // the weights do not come from the kernel in front
+    pdl_wait();
+    if (steps > 0) fetch_a(av, tile, 0);
+#pragma unroll
+    for (int i = 0; i < AC; ++i) most_a[i] = 0;
+#pragma unroll
+    for (int i = 0; i < WC; ++i) most_w[i] = 0;
+    for (long long i = 0; i < steps; ++i) {
+        uint8_t* stage = smem + (int)(i & 1) * STAGE;
+        const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
+        // (a row behind the last keeps what the place held: it gives results that nobody takes)
+#pragma unroll
+        for (int j = 0; j < AC; ++j)
+            if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
+        if (has_w)
+#pragma unroll
+            for (int j = 0; j < WC; ++j)
+                if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j]);
+        async_proxy_fence();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
+        const int this_tile = tile, this_slice = slice, this_flags = flags;
+        if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
+#pragma unroll
+            for (int j = 0; j < AC; ++j) {
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) most_a[j] = max(most_a[j], __shfl_xor_sync(0xffffffffu, most_a[j], o));
+                if ((tid & 7) == 0) bad_a[flags][row8 + 64 * j] = splits_badly(most_a[j]);
+                most_a[j] = 0;
+            }
+#pragma unroll
+            for (int j = 0; j < WC; ++j) {
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) most_w[j] = max(most_w[j], __shfl_xor_sync(0xffffffffu, most_w[j], o));
+                if (has_w && (tid & 7) == 0) bad_w[flags][row8 + 64 * j] = splits_badly(most_w[j]);
+                most_w[j] = 0;
+            }
+            slice = 0;
+            tile += gridDim.x;
+            if (++flags == FLAGS) flags = 0;
+        }
+        if (i + 1 < steps) {
+            fetch_a(av, tile, slice);
+            fetch_w(wv, tile, slice);
+        }
+        ok = warp != 0 || multiply(i);
+        if (ok && i > 0) ok = add_up(i - 1, was_slice, was_tile, was_flags);
+        if (!ok) break;
+        was_tile = this_tile; was_slice = this_slice; was_flags = this_flags;
+    }
+    if (ok && steps > 0) ok = add_up(steps - 1, was_slice, was_tile, was_flags);
+    if (!ok && lane == 0) {
+        atomicExch(g.status, 81);
+        ctl.failed = 1;
+    }
+    __syncwarp();
+    // a wait ran out: products that may still be under way get a moment to end
+    if (*(volatile uint32_t*)&ctl.failed != 0 && lane == 0)
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) tmem_dealloc(tmem_base, 2 * BN);
+}
+
+template <int BN>
+cudaError_t launch_tiles(const SplitArgs& g, cudaStream_t s) {
+    const cudaError_t configured = mg_raise_shared(gemm_split_kernel<BN>, dynamic_bytes<BN>());
+    if (configured != cudaSuccess) return configured;
+    const long long tiles = (long long)ceil_div(g.M, TILE_M) * ceil_div(g.N, BN);
+    return mg_launch(gemm_split_kernel<BN>, dim3((unsigned)(tiles < SMS ? tiles : SMS)), dim3(WORKERS), dynamic_bytes<BN>(), s, true, g);
+}
+
+// ---- a few rows ---------------------------------------------------------------------------------------------
+constexpr int FEW_WARPS = 8, FEW_STAGES = 2, FEW_N = 16;    // rows of w per CTA: the m of m16n8k16
+constexpr int LINE = SLICE + 8;                              // words between rows in shared memory: 8-byte reads of 4 rows meet no bank twice
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool there) {
+    const uint32_t bytes = there ? 16u : 0u;                 // (0: sixteen zero bytes are written)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// MT rows of a: 8 or 16.
+template <int MT>
+__global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const SplitArgs g, int stages) {
+    constexpr int NR = FEW_N, STAGE = (NR + MT) * LINE;      // words of a warp's stage: w's slice, then a's
+    constexpr int TB = MT / 8;
+    extern __shared__ __align__(16) float few_smem[];
+    __shared__ uint32_t most_w[NR], most_a[MT];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* ring = few_smem + warp * stages * STAGE;
+    float* parts = few_smem + FEW_WARPS * stages * STAGE;    // [2][warp][MT][NR]
+    const int n0 = blockIdx.x * NR, M = g.M, N = g.N, K = g.K;
+    const int slices = (K + SLICE - 1) / SLICE, rounds = (slices + FEW_WARPS - 1) / FEW_WARPS;
+
+    auto ask_w = [&](int r) {
+        float* dst = ring + (r & (stages - 1)) * STAGE;
+        const int k0 = (r * FEW_WARPS + warp) * SLICE;
+#pragma unroll
+        for (int i = 0; i < NR / 2; ++i) {
+            const int row = 2 * i + (lane >> 4), c = (lane & 15) * 4;
+            const bool there = n0 + row < N && k0 + c < K;
+            cp_async16(dst + row * LINE + c, there ? g.w + (size_t)(n0 + row) * K + k0 + c : g.w, there);
+        }
+    };
+    auto ask_a = [&](int r) {
+        float* dst = ring + (r & (stages - 1)) * STAGE + NR * LINE;
+        const int k0 = (r * FEW_WARPS + warp) * SLICE;
+#pragma unroll
+        for (int i = 0; i < MT / 2; ++i) {
+            const int row = 2 * i + (lane >> 4), c = (lane & 15) * 4;
+            const bool there = row < M && k0 + c < K;
+            cp_async16(dst + row * LINE + c, there ? g.a + (size_t)row * K + k0 + c : g.a, there);
+        }
+    };
+    pdl_trigger();
+    for (int r = 0; r < stages && r < rounds; ++r) ask_w(r);                // the weights depend on no kernel before
+    if (tid < NR) most_w[tid] = 0;
+    if (tid >= 32 && tid < 32 + MT) most_a[tid - 32] = 0;
+    __syncthreads();
+    pdl_wait();
+    for (int r = 0; r < FEW_STAGES; ++r) {
+        if (r < stages && r < rounds) ask_a(r);
+        cp_async_commit();
+    }
+    const int gr = lane >> 2, t2 = (lane & 3) * 2;
+    uint32_t mine_w[2] = {0, 0}, mine_a[TB];
+#pragma unroll
+    for (int b = 0; b < TB; ++b) mine_a[b] = 0;
+    float total = 0.f;                                                      // of row tid / NR, column n0 + tid % NR
+    for (int r = 0; r < rounds; ++r) {
+        cp_async_wait<FEW_STAGES - 1>();
+        __syncwarp();
+        const float* ws = ring + (r & (stages - 1)) * STAGE + gr * LINE + t2;
+        const float* as = ws + NR * LINE;
+        float c[TB][4];
+        uint32_t wh[SLICE / 16][4], ah[SLICE / 16][TB][2];                  // first pieces, whose products come last
+#pragma unroll
+        for (int b = 0; b < TB; ++b)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[b][e] = 0.f;
+#pragma unroll
+        for (int k = 0; k < SLICE / 16; ++k) {
+            uint32_t wp[PIECES][4], ap[PIECES][TB][2];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                                   // rows gr, gr + 8; columns 2 t, then 2 t + 8
+                const float2 x = *reinterpret_cast<const float2*>(ws + (e & 1) * 8 * LINE + 16 * k + (e >> 1) * 8);
+                uint32_t p[PIECES];
+                split_pair(x.x, x.y, p);
+                mine_w[e & 1] = larger(larger(mine_w[e & 1], x.x), x.y);
+#pragma unroll
+                for (int q = 0; q < PIECES; ++q) wp[q][e] = p[q];
+                wh[k][e] = p[0];
+            }
+#pragma unroll
+            for (int b = 0; b < TB; ++b)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float2 x = *reinterpret_cast<const float2*>(as + b * 8 * LINE + 16 * k + e * 8);
+                    uint32_t p[PIECES];
+                    split_pair(x.x, x.y, p);
+                    mine_a[b] = larger(larger(mine_a[b], x.x), x.y);
+#pragma unroll
+                    for (int q = 0; q < PIECES; ++q) ap[q][b][e] = p[q];
+                    ah[k][b][e] = p[0];
+                }
+#pragma unroll
+            for (int t = 0; t < SMALL; ++t)
+#pragma unroll
+                for (int b = 0; b < TB; ++b) mma_bf16(c[b], wp[piece_of_w(t)], ap[piece_of_a(t)][b][0], ap[piece_of_a(t)][b][1]);
+        }
+#pragma unroll
+        for (int k = 0; k < SLICE / 16; ++k)
+#pragma unroll
+            for (int b = 0; b < TB; ++b) mma_bf16(c[b], wh[k], ah[k][b][0], ah[k][b][1]);
+        __syncwarp();
+        if (r + stages < rounds) {
+            ask_w(r + stages);
+            ask_a(r + stages);
+        }
+        cp_async_commit();
+        float* part = parts + (r & 1) * FEW_WARPS * MT * NR + warp * MT * NR;
+#pragma unroll
+        for (int b = 0; b < TB; ++b)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][e];
+        if (r + 1 == rounds) {                                              // what each row's largest number is, over all warps
+#pragma unroll
+            for (int e = 0; e < 2; ++e) atomicMax(&most_w[gr + 8 * e], mine_w[e]);
+#pragma unroll
+            for (int b = 0; b < TB; ++b) atomicMax(&most_a[gr + 8 * b], mine_a[b]);
+        }
+        // (one barrier a round: the half written two rounds later was read before the barrier in between)
+        __syncthreads();
+        const int here = min(FEW_WARPS, slices - r * FEW_WARPS);
+        if (tid < MT * NR)
+            for (int s = 0; s < here; ++s) total += parts[(r & 1) * FEW_WARPS * MT * NR + s * MT * NR + tid];
+    }
+    cp_async_wait<0>();
+    const int m = tid / NR, n = n0 + tid % NR;
+    if (tid >= MT * NR || m >= M || n >= N) return;
+    if (splits_badly(most_a[m]) || splits_badly(most_w[tid % NR])) total = fma_sum(g.a + (size_t)m * K, g.w + (size_t)n * K, K);
+    const float y = activate(total + (g.bias != nullptr ? g.bias[n] : 0.f), g.epilogue);
+    float* dst = g.out + (size_t)m * N + n;
+    if (g.epilogue == EPI_RESIDUAL) *dst += y;
+    else *dst = y;
+}
+
+template <int MT>
+cudaError_t launch_few(const SplitArgs& g, cudaStream_t s) {
+    static_assert(MT * FEW_N <= 32 * FEW_WARPS, "a thread per result");
+    // one round of slices needs one stage: more CTAs fit an SM, and one's copies run beside another's sums
+    const int stages = g.K <= FEW_WARPS * SLICE ? 1 : FEW_STAGES;
+    auto bytes = [](int st) { return (int)((FEW_WARPS * st * (FEW_N + MT) * LINE + 2 * FEW_WARPS * MT * FEW_N) * sizeof(float)); };
+    const cudaError_t configured = mg_raise_shared(gemm_split_few_kernel<MT>, bytes(FEW_STAGES));
+    if (configured != cudaSuccess) return configured;
+    return mg_launch(gemm_split_few_kernel<MT>, dim3(ceil_div(g.N, FEW_N)), dim3(32 * FEW_WARPS), bytes(stages), s, true, g, stages);
+}
+
+}  // namespace
+
+// a: [M, K], w: [N, K], out: [M, N], all 32-bit and row-major; epilogues as mg_linear_simt.  `status` is a device int that receives
+// a non-zero code if a wait inside the kernel ran out.  Returns MG_ERR_UNSUPPORTED (and launches nothing) unless K is a
+// multiple of 4 and a and w lie on 16-byte boundaries: which kernel computes a matrix does not hang on the number of rows.
+MG_API int mg_linear_split(const float* a, const float* w, const float* bias, float* out, float* residual, int M, int N, int K,
+                           int epilogue, int* status, void* stream) {
+    if (M == 0) return MG_OK;
+    MG_REQUIRE(M > 0 && N > 0 && K > 0, "linear: bad sizes M=%d N=%d K=%d", M, N, K);
+    MG_REQUIRE(epilogue >= EPI_STORE && epilogue <= EPI_RELU_SQ, "linear: unknown epilogue %d", epilogue);
+    MG_REQUIRE(epilogue == EPI_RESIDUAL ? residual != nullptr : out != nullptr, "linear: missing output");
+    MG_REQUIRE(status != nullptr, "linear: missing status word");
+    if (K % 4 != 0 || (((uintptr_t)a | (uintptr_t)w) & 15))
+        return mg_set_error(MG_ERR_UNSUPPORTED, "linear: 32-bit tensor-core path needs K %% 4 == 0 and 16-byte aligned operands");
+    SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, status};
+    g.wide = N % 4 == 0 && ((uintptr_t)g.out & 15) == 0;
+    MG_REQUIRE((long long)ceil_div(M, TILE_M) * ceil_div(N, 32) < (1ll << 30), "linear: too many tiles");
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaError_t e;
+    if (M <= 16) {
+        e = M <= 8 ? launch_few<8>(g, s) : launch_few<16>(g, s);
+    } else {
+        // A slice takes 1.8 us in tiles of 32 columns, 2.05 in tiles of 64 and 2.8 in tiles of 128 (512 x 2,048, 128 rows: 58, 65
+        // and 89 us), so the rounds of tiles decide: 2,048 x 2,048 x 512 104, 71 and 53 us, 1,024 x 512 x 2,048 59, 66 and 90.
+        auto rounds = [&](int bn) { return (double)((ceil_div(M, TILE_M) * (long long)ceil_div(N, bn) + SMS - 1) / SMS); };
+        const double t128 = rounds(128) * 2.8, t64 = rounds(64) * 2.05, t32 = rounds(32) * 1.8;
+        if (t128 <= t64 && t128 <= t32) e = launch_tiles<128>(g, s);
+        else if (t64 <= t32) e = launch_tiles<64>(g, s);
+        else e = launch_tiles<32>(g, s);
+    }
+    if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "gemm_split: %s", cudaGetErrorString(e));
+    MG_CHECK_LAUNCH("gemm_split");
+    return MG_OK;
+}

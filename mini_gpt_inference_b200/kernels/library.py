@@ -77,6 +77,7 @@ _SIGNATURES = {
     "mg_gather_tokens": [_P, _P, _P, _I, _I, _P],
     "mg_kv_store": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "mg_linear_simt": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "mg_linear_split": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P],
     "mg_linear_skinny": [_P, _P, _P, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P,
                          _I, _I, _I, _I, _I, _P, _P, _I, _P],
     "mg_linear_skinny_ctas": [_I, _I],

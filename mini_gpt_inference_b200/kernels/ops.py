@@ -130,6 +130,7 @@ class CudaOps:
         self.use_prefill_tc = True
         self.use_mma_attention = True
         self.use_fp32_attention = True
+        self.use_split = True              # 32-bit products by bfloat16 pieces
         self.use_moe_few = True
         self.use_chunked_memory = True     # prompt portions of the matrix-memory mixers chunk by chunk (bfloat16)
         self.use_recurrence_ranges = True  # long prompt portions of the gated recurrence with the warps sharing the tokens
@@ -673,6 +674,13 @@ class CudaOps:
             if code != library.UNSUPPORTED:
                 self._run(code, "linear (tensor cores)")
                 return fused
+        if x.dtype == torch.float32 and self.use_split and not out_bf16:
+            # products of bfloat16 pieces on the tensor cores, whatever the number of rows (a row's bits do not hang on it)
+            code = self.lib.mg_linear_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(residual), m, n, k, epilogue,
+                                            _ptr(self.status), self._stream())
+            if code != library.UNSUPPORTED:
+                self._run(code, "linear (32-bit, tensor cores)")
+                return False
         self._run(self.lib.mg_linear_simt(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(residual),
                                       m, n, k, epilogue, self._is_bf16(x), out_bf16, self._stream()),
               "linear")

@@ -1002,6 +1002,35 @@ def test_32_bit_products_do_not_hang_on_the_rows_beside_them(ops, n, k):
     assert torch.equal(few, whole[:5])
 
 
+@pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 130])
+@pytest.mark.parametrize("n,k", [(130, 260), (33, 64), (64, 68), (1540, 1032), (5, 4)])
+def test_32_bit_products_by_bfloat16_pieces(ops, m, n, k):
+    """Tiles of 32 to 128 columns and the kernel of a few rows at their edges: no further from the 64-bit result than what a
+    32-bit sum of k terms may be off, as far as the FMA tiles with what is no number, infinite, huge or tiny, and by the
+    same sums as those where a row holds such numbers."""
+    x, w, b = randn(m, k, seed=41), randn(n, k, seed=42), randn(n, seed=43)
+    ref, size = x.double() @ w.double().T + b.double(), x.double().abs() @ w.double().abs().T + b.double().abs()
+    # three pieces hold all 24 bits; a slice of 64 terms is rounded (or cut) ten times at its full size, slices and bias once each
+    bound = (10 + -(-k // 64) + 2) * 2.0 ** -23 * size
+    assert ((ops.linear(x, w, b, "none", torch.float32).double() - ref).abs() <= bound).all()
+    x[0, k - 1], w[n - 1, 0] = float("inf"), float("nan")
+    if m > 7:
+        x[3], x[4], x[5, 1], x[6, k // 2] = 1e-36, 1e36, 2e38, float("nan")
+    w[1], w[2] = 0.0, 1e-38
+    w[3, k // 2] = -float("inf")
+    got = ops.linear(x, w, b, "none", torch.float32)
+    ops.use_split = False
+    try:
+        want = ops.linear(x, w, b, "none", torch.float32)
+    finally:
+        ops.use_split = True
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[0].nan_to_num(), want[0].nan_to_num()) and torch.equal(got[:, 2].nan_to_num(), want[:, 2].nan_to_num())
+    finite = torch.isfinite(want)
+    size = x.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((got.double() - want.double()).abs() <= 2 * (k + 2) * 2.0 ** -24 * size)[finite].all()
+
+
 @pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
 @pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window", [
     (4, 4, 128, 64, 0), (6, 2, 104, 16, 0), (5, 1, 48, 4, 0), (4, 4, 80, 24, 70), (2, 2, 96, 16, 0), (64, 1, 8, 8, 0),
