@@ -236,6 +236,11 @@ __device__ uint32_t philox_first(uint32_t k0, uint32_t k1, uint32_t c0, uint32_t
     return c[0];
 }
 
+// A row's draw from [0, 1).
+__device__ __forceinline__ float uniform(uint32_t seed_lo, uint32_t seed_hi, uint32_t counter) {
+    return (float)(philox_first(seed_lo, seed_hi, counter, 0u) >> 8) * (1.0f / 16777216.0f);
+}
+
 __device__ float block_reduce_max(float v, float* scratch) {
     v = warp_max(v);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -447,14 +452,14 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 // pass's 256 bins, and its 64-bit sums of probability mass meet in a few bins, lane after lane.  Here a row's values stay in the registers
 // of a cluster's CTAs (16 a thread), lanes that meet in one bin of mass add up among themselves first, a warp picks the
 // digit, and a pass ends in one cluster barrier behind which every CTA sums all histograms itself.
-// 50,304 ids, before and now: 24 rows with top-k 50 and top-p 0.8, 572 -> 45 us; with top-p 0.9 alone, 526 -> 69; plain
-// draws, 70 -> 17; 256 rows with both, 1,133 -> 336, plain draws, 123 -> 96.  1,000 ids, 24 rows with both: 60 -> 25.
+// 50,304 ids, one CTA and a cluster: 24 rows with top-k 50 and top-p 0.8, 572 -> 45 us (20 where few are left, see below); with
+// top-p 0.9 alone, 526 -> 69; plain draws, 70 -> 17; 256 rows, plain draws, 123 -> 96.
 
 // Descending over 256 bins: the digit and the sum in front of it.  `by_count`: the first bin whose inclusive sum reaches
 // `goal`; otherwise the last non-empty bin in front of which at most `goal` lies (the first non-empty one if none is).
 // One warp, 8 bins a lane.
 __device__ __forceinline__ void pick_digit(const unsigned long long* total, unsigned long long start, unsigned long long goal,
-                                           bool by_count, uint32_t* digit, unsigned long long* before) {
+                                           bool by_count, uint32_t* digit, unsigned long long* before, int* reached) {
     const int lane = threadIdx.x & 31;
     unsigned long long bin[8], sum = 0ull;
 #pragma unroll
@@ -482,7 +487,63 @@ __device__ __forceinline__ void pick_digit(const unsigned long long* total, unsi
         const int j = hits ? hit : first;
         *digit = j < 0 ? 0u : (uint32_t)(255 - 8 * lane - j);
         *before = hits ? hit_run : first_run;
+        *reached = hits != 0u;                                  // there is such a bin
     }
+}
+
+// ---- a row of which top-k leaves few ----
+// The k-th largest of the threads' largest values bounds the row's k-th largest from below, so one counting pass over one value
+// a thread tells which values can be kept at all: some 60 for k = 50.  They go to the first CTA, which compares each with each
+// and draws: four cluster barriers instead of a dozen.  24 rows with top-k 50 and top-p 0.8, passes over all values and
+// this: 50,304 ids 40.5 -> 20.3 us, 1,000 ids 22.2 -> 10.6, 131,072 ids 91 -> 41; 256 rows of 50,304 ids 335 -> 135.
+constexpr int KEPT = SAMPLE_THREADS;                            // most of them: one a thread
+
+// Bins of the distance to the row's largest value, eight to each power of two from 2^-12 on; rising with the distance.
+__device__ __forceinline__ int gap_bin(float gap) { return max(0, (int)(__float_as_uint(gap) >> 20) - ((127 - 12) << 3)); }
+
+// One CTA draws among `n` values, in index order, that hold all that top-k keeps.  scaled, key, mass: KEPT places each.
+__device__ __forceinline__ void draw_among(int n, const float* scaled, const int* index, uint32_t* key, unsigned long long* mass,
+                                           float mx, int k, float p, float u, float* scratch, int* found, int* last, int* out) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool in = tid < n;
+    const float x = in ? scaled[tid] : 0.f;
+    const uint32_t mine = in ? order_key(x) : 0u;
+    if (in) key[tid] = mine;
+    __syncthreads();
+    int larger = 0;
+    for (int j = 0; j < n; ++j) larger += key[j] > mine ? 1 : 0;
+    bool keep = in && larger < k;
+    const float weight = keep ? expf(x - mx) : 0.f;
+    if (p < 1.f) {
+        const float kept = block_reduce_sum(weight, scratch);
+        const unsigned long long target = (unsigned long long)((double)p * (double)kept * (double)FIXED_ONE);
+        if (in) mass[tid] = keep ? (unsigned long long)(weight * FIXED_ONE) + 1ull : 0ull;
+        __syncthreads();
+        unsigned long long before = 0ull;
+        for (int j = 0; j < n; ++j) before += key[j] > mine ? mass[j] : 0ull;
+        keep = keep && before <= target;
+    }
+    const float w = keep ? weight : 0.f;
+    float incl = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) scratch[warp] = incl;
+    __syncthreads();
+    float before = 0.f, z = 0.f;
+    for (int i = 0; i < SAMPLE_THREADS / 32; ++i) {
+        if (i == warp) before = z;
+        z += scratch[i];
+    }
+    if (w > 0.f) {
+        atomicMax(last, index[tid]);
+        if (before + incl > u * z) atomicMin(found, index[tid]);
+    }
+    __syncthreads();
+    if (tid == 0) *out = *found != 0x7fffffff ? *found : max(0, *last);
 }
 
 template <int ROW_CTAS, int NV>
@@ -500,13 +561,43 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
     __shared__ int sh_index, sh_last;
     __shared__ uint32_t sh_digit;
     __shared__ unsigned long long sh_before;
+    __shared__ int sh_odd, sh_reached, sh_few;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = blockIdx.x / ROW_CTAS, rank = (int)cluster.block_rank();
     const float* lr = logits + (size_t)row * vocab;
     const int begin = rank * chunk, end = min(limit, begin + chunk);      // this CTA's ids; thread t has begin + t, + 512, ...
     const float temp = temperature[row];
-    if (temp <= 0.f) {   // greedy row: one CTA, lowest index among the largest
-        if (rank == 0) greedy_row(lr, limit, out + row, scratch, &sh_index);
+    if (temp <= 0.f) {   // greedy row: the lowest index among the largest
+        // Where all CTAs are on the GPU at once, those of the row share it (24 rows of 50,304 ids 8.9 -> 6.1 us); where they are
+        // not, the others leave it to the first (256 rows 23 us, shared 42; 24 rows of 131,072 ids 13.8 and 18.7).
+        if (ROW_CTAS == 1 || gridDim.x > 148 * (NV > 16 ? 1 : 2)) {
+            if (rank == 0) greedy_row(lr, limit, out + row, scratch, &sh_index);
+            return;
+        }
+        float best = -INFINITY;
+        int at = 0x7fffffff;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = begin + v * SAMPLE_THREADS + tid;
+            const float y = i < end ? lr[i] : NAN;              // (what is no number never wins)
+            if (y > best || (y == best && i < at)) { best = y; at = i; }
+        }
+        const float most = block_reduce_max(best, scratch);
+        if (tid == 0) { sh_max = most; sh_index = 0x7fffffff; }
+        __syncthreads();
+        if (best == most && at != 0x7fffffff) atomicMin(&sh_index, at);
+        cluster.sync();
+        if (rank == 0 && tid == 0) {
+            best = -INFINITY;
+            at = 0x7fffffff;
+            for (int r = 0; r < ROW_CTAS; ++r) {                // (in index order: the first of equals is the lowest)
+                const float y = *cluster.map_shared_rank(&sh_max, r);
+                const int i = *cluster.map_shared_rank(&sh_index, r);
+                if (i != 0x7fffffff && (y > best || at == 0x7fffffff)) { best = y; at = i; }
+            }
+            out[row] = at == 0x7fffffff ? 0 : at;
+        }
+        cluster.sync();                                         // rank 0 has read the others' shared memory
         return;
     }
     const float safe_t = fmaxf(temp, 1e-6f);
@@ -521,11 +612,20 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
 #pragma unroll
     for (int v = 0; v < NV; ++v) mx = fmaxf(mx, x[v]);
     const float block_max = block_reduce_max(mx, scratch);
-    if (tid == 0) { sh_max = block_max; sh_index = 0x7fffffff; sh_last = -1; }
+    bool nan = false;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) nan = nan || x[v] != x[v];
+    const bool any_nan = __syncthreads_or(nan);
+    if (tid == 0) { sh_max = block_max; sh_index = 0x7fffffff; sh_last = -1; sh_odd = any_nan; }
     if (tid < 256) hist[0][tid] = 0ull;
     cluster.sync();
     mx = -INFINITY;
-    for (int r = 0; r < ROW_CTAS; ++r) mx = fmaxf(mx, *cluster.map_shared_rank(&sh_max, r));
+    bool odd = false;                                           // a value that is no number, or a largest that is infinite
+    for (int r = 0; r < ROW_CTAS; ++r) {
+        mx = fmaxf(mx, *cluster.map_shared_rank(&sh_max, r));
+        odd = odd || *cluster.map_shared_rank(&sh_odd, r) != 0;
+    }
+    odd = odd || !(fabsf(mx) < INFINITY);
 
     uint32_t thr_key = 0u;
     int turn = 0;
@@ -540,13 +640,90 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
             hist[turn ^ 1][tid] = 0ull;                         // read by the others before this barrier, written after it
         }
         __syncthreads();
-        if (warp == 0) pick_digit(total, start, goal, by_count, &sh_digit, &sh_before);
+        if (warp == 0) pick_digit(total, start, goal, by_count, &sh_digit, &sh_before, &sh_reached);
         __syncthreads();
         turn ^= 1;
     };
 
-    // top-k: key of the k-th largest scaled logit
     const int k = top_k ? top_k[row] : 0;
+    const float p = top_p ? top_p[row] : 1.f;
+    if (k > 0 && k < limit && k <= KEPT && !odd) {
+        __shared__ float few_x[2][KEPT];                            // this CTA's; those of all, in the first CTA
+        __shared__ int few_i[2][KEPT], few_at[NV * (SAMPLE_THREADS / 32)];
+        float mine = -INFINITY;                                     // this thread's largest
+#pragma unroll
+        for (int v = 0; v < NV; ++v) mine = fmaxf(mine, x[v]);
+        const int own_bin = gap_bin(mx - mine);
+        if (own_bin < 256) atomicAdd(reinterpret_cast<uint32_t*>(hist[turn]) + 2 * (255 - own_bin), 1u);
+        next_digit(0ull, (unsigned long long)k, true);
+        if (sh_reached) {
+            const int bin = 255 - (int)sh_digit;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const bool in = begin + v * SAMPLE_THREADS + tid < end && gap_bin(mx - x[v]) <= bin;
+                const uint32_t who = __ballot_sync(0xffffffffu, in);
+                if (lane == 0) few_at[v * (SAMPLE_THREADS / 32) + warp] = __popc(who);
+            }
+            __syncthreads();
+            if (warp == 0) {                                        // the counts, in index order, become first places
+                constexpr int PER = NV * (SAMPLE_THREADS / 32) / 32;
+                int count[PER], sum = 0;
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    count[j] = few_at[lane * PER + j];
+                    sum += count[j];
+                }
+                int incl = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                int at = incl - sum;
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    few_at[lane * PER + j] = at;
+                    at += count[j];
+                }
+                if (lane == 31) sh_few = incl;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int i = begin + v * SAMPLE_THREADS + tid;
+                const bool in = i < end && gap_bin(mx - x[v]) <= bin;
+                const uint32_t who = __ballot_sync(0xffffffffu, in);
+                const int at = few_at[v * (SAMPLE_THREADS / 32) + warp] + __popc(who & ((1u << lane) - 1u));
+                if (in && at < KEPT) {
+                    few_x[0][at] = x[v];
+                    few_i[0][at] = i;
+                }
+            }
+            cluster.sync();
+            int n = 0;
+            for (int r = 0; r < ROW_CTAS; ++r) n += *cluster.map_shared_rank(&sh_few, r);
+            if (n <= KEPT) {
+                if (rank == 0) {
+                    int at = 0;
+                    for (int r = 0; r < ROW_CTAS; ++r) {
+                        const int count = *cluster.map_shared_rank(&sh_few, r);
+                        if (tid < count) {
+                            few_x[1][at + tid] = *cluster.map_shared_rank(&few_x[0][tid], r);
+                            few_i[1][at + tid] = *cluster.map_shared_rank(&few_i[0][tid], r);
+                        }
+                        at += count;
+                    }
+                }
+                cluster.sync();                                     // the others' shared memory is not read from here on
+                if (rank == 0)
+                    draw_among(n, few_x[1], few_i[1], reinterpret_cast<uint32_t*>(few_x[0]), &hist[0][0], mx, k, p,
+                               uniform(seed_lo[row], seed_hi[row], counter[row]), scratch, &sh_index, &sh_last, out + row);
+                return;
+            }
+        }
+    }
+
+    // top-k: key of the k-th largest scaled logit
     if (k > 0 && k < limit) {
         uint32_t prefix = 0u, mask = 0u;
         unsigned long long remaining = (unsigned long long)k;
@@ -566,7 +743,6 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
     }
 
     // top-p: lowest key whose mass of strictly larger keys is <= p * (mass kept by top-k)
-    const float p = top_p ? top_p[row] : 1.f;
     if (p < 1.f) {
         float part = 0.f;
 #pragma unroll
@@ -629,9 +805,7 @@ sample_cluster_kernel(const float* __restrict__ logits, const float* __restrict_
         last = max(last, *cluster.map_shared_rank(&sh_last, r));
     }
     cluster.sync();                                             // the others' shared memory is not read from here on
-    const uint32_t rnd = philox_first(seed_lo[row], seed_hi[row], counter[row], 0u);
-    const float u = (float)(rnd >> 8) * (1.0f / 16777216.0f);      // [0, 1)
-    const float target = u * z;
+    const float target = uniform(seed_lo[row], seed_hi[row], counter[row]) * z;
     float base = 0.f;
     int owner = -1;                                             // the CTA in whose ids the sum passes the target
     for (int r = 0; r < ROW_CTAS; ++r) {

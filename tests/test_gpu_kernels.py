@@ -1368,6 +1368,33 @@ def test_sampler_at_the_edges_of_its_cuts(ops, vocab):
             assert 0 <= got[r] < limit and want[got[r]] > 0, (r, got[r])
 
 
+@pytest.mark.parametrize("vocab", [700, 8193, 40001, 70000])
+def test_sampler_with_few_left_by_top_k(ops, vocab):
+    """Up to 512 values that top-k can keep go to one CTA; more (ties, a large k), infinite values
+    take the passes over the whole row.  Every drawn id is in the oracle's support, and greedy rows have the lowest index among equals."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(10, vocab, generator=g) * 2.0
+    logits[1] = logits[1].round()                                          # thousands of ties
+    logits[2, 5:] = -float("inf")                                          # fewer numbers than k
+    logits[3] = 0.0
+    logits[4] = logits[4] * 1e-4
+    logits[5, vocab // 2] = float("inf")
+    logits[6, 3] = logits[6, vocab - 1] = 30.0
+    logits[7, 11], logits[7, 12], logits[7, vocab - 2] = 25.0, float("nan"), 25.0
+    logits[8] = -float("inf")
+    logits[9] -= 1e4
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32).cuda()              # noqa: E731
+    f32 = lambda v: torch.tensor(v, dtype=torch.float32).cuda()            # noqa: E731
+    k, p = [512, 3, 50, 40, 513, 7, 1, 9, 4, 64], [0.95, 1.0, 0.7, 1.0, 0.9, 1.0, 0.3, 1.0, 1.0, 0.6]
+    temperature = [1.3, 1.0, 0.8, 1.0, 1.0, 0.9, 1.0, 0.0, 0.0, 1.0]
+    for n in range(4):
+        got = ops.sample(logits.cuda(), f32(temperature), i32(k), f32(p), i32([n] * 10), i32(list(range(10))), i32([n] * 10)).tolist()
+        assert 0 <= got[5] < vocab and got[6] in (3, vocab - 1) and got[7] == 11 and got[8] == 0
+        for r in (0, 1, 2, 3, 4, 9):
+            want = plain_gpt.sampling_distribution(logits[r], temperature[r], k[r], min(1.0, p[r] + 1e-5) if p[r] < 1 else None)
+            assert want[got[r]] > 0, (r, got[r])
+
+
 def test_sampler_is_greedy_at_zero_and_repeatable_by_seed(ops):
     g = torch.Generator().manual_seed(4)
     logits = torch.randn(6, 1000, generator=g).cuda()
