@@ -3,10 +3,11 @@
 // A 32-bit number is the sum of three bfloat16 numbers, exactly: its 24 bits are rounded to 8 three times, x = h + m + l with
 // |m| <= 2^-9 |h| and |l| <= 2^-18 |h|.  Products of bfloat16 numbers are exact in the tensor cores, so a product of two such sums is
 // six of theirs, h l', l h', m m', h m', m h' and h h'; the three that are left out are below 2^-27 of it.  What rounds is the
-// accumulator: it drops what lies below its last place at every addition of 16 products.  So K is cut into slices of 64; within
-// a slice the five small products of all its terms are summed first, then the four additions of h h', and a slice's sum is added to
-// those before it by an ordinary rounded addition.  Measured against 64 bits (64 terms, normal numbers): 7.8e-8 of the result's size,
-// a chain of fused multiply-adds 14.5e-8; 512 terms 9.9e-8 and 15.7e-8, 2,048 terms 13.4e-8 and 18.1e-8.
+// accumulator: it drops what lies below its last place at every addition of 16 products.  So K is cut into slices of 64, and a
+// slice's products go into three accumulators: those of h h', those of h m' and m h', and the other three, each some 2^8 below the
+// one before.  A slice's sum, h h' + (the second + the third), is added to those before it; these are ordinary rounded additions.
+// Errors against 64 bits, of the result's size, chains of fused multiply-adds and this: 512 terms 15.7e-8 and 9.3e-8, 2,048 terms
+// 18.1e-8 and 12.9e-8 (in one accumulator, the small products first: 9.9e-8 and 13.4e-8).
 //
 // Every element is summed in that one order whatever the number of rows and the kernel or tile that it falls in, so a token's
 // result does not depend on what else is in the batch (mma.sync and tcgen05.mma give the same bits; so do the two orders of the operands).
@@ -15,15 +16,16 @@
 // split so: results that meet such a row are summed by fused multiply-adds instead (fma_sum), again whatever is beside them.
 //
 // Two kernels:
-//   gemm_split_kernel   tiles of 128 rows x BN columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
-//                       (a slice ahead, in registers), split them, and lay the pieces into shared memory in the 128-byte swizzle;
-//                       one thread of theirs issues the 24 products of a slice; the warps then take the slice's sums out of
-//                       TMEM and add them to the totals in their registers, beside the next slice's products.
+//   gemm_split_kernel   tiles of 128 rows x 64 columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
+//                       (a slice ahead, in registers), split them, and lay the pieces into shared memory in the 128-byte swizzle,
+//                       the three of w's rows one behind the other, so that h, m and l of a's meet 3, 2 and 1 of them in one
+//                       instruction each.  A thread of the 17th warp issues the 12 products of a slice; the sixteen then take
+//                       the sums out of TMEM and add them to the totals in their registers, beside the next slice's products.
 //   gemm_split_few_kernel   up to 16 rows: a CTA takes 16 rows of w, each of its eight warps every eighth slice, operands by cp.async in
 //                       a ring of the warp's own (the first round of w before the wait for the kernel in front); the fragments
 //                       of mma.sync are split as they are read.  Bound by reading w and by the latency of a launch and a slice.
-// 2,048 rows, FMA tiles and these: 1,536 x 512 101 and 52 us, 2,048 x 512 123 and 53, 512 x 2,048 142 and 66; 8 rows (FMA and mma.sync):
-// 1,536 x 512 3.3 and 3.7, 512 x 2,048 7.5 and 7.3, 50,304 x 512 32.5 and 31.6; 16 rows 49.7 and 46.0.
+// 2,048 rows, FMA tiles and these: 1,536 x 512 101 and 42 us, 2,048 x 512 123 and 54, 512 x 2,048 142 and 48; 8 rows (FMA and mma.sync):
+// 1,536 x 512 3.3 and 3.6, 512 x 2,048 7.5 and 6.9, 50,304 x 512 32.5 and 31.5; 16 rows 49.7 and 47.1.
 #include "blackwell.cuh"
 
 #define EPI_STORE 0      // out = acc + bias
@@ -35,9 +37,6 @@ namespace {
 
 constexpr int SLICE = 64;            // terms summed by the tensor cores in one go: a 128-byte row of bfloat16
 constexpr int PIECES = 3;
-constexpr int SMALL = 5;             // products of pieces in front of h h'
-__host__ __device__ constexpr int piece_of_a(int t) { return t == 1 ? 2 : (t == 2 || t == 4) ? 1 : 0; }
-__host__ __device__ constexpr int piece_of_w(int t) { return t == 0 ? 2 : (t == 2 || t == 3) ? 1 : 0; }
 
 // The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third is exact, so its upper half is all of it.
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECES]) {
@@ -84,28 +83,24 @@ struct SplitArgs {
 };
 
 // ---- tiles -----------------------------------------------------------------------------------------------
-constexpr int TILE_M = 128;
+// A slice takes 1.45 us, 1.1 with few rows: the operands of the next one come from L2 (48 KB) while a slice is split, and the splitting
+// itself is 24 numbers a thread.  Tiles of 32 columns take the same time a slice (512 x 2,048, 128 rows: 48 and 46 us).  In the form
+// with one accumulator, six instructions for the six products and a worker that issued them as well, a slice took 2.05 us.
+constexpr int TILE_M = 128, BN = 64;
 constexpr int WORKERS = 512;         // threads that split and add up
+constexpr int THREADS = WORKERS + 32;
 constexpr int ROW_BYTES = SLICE * 2;
 constexpr int SMS = 148;
 constexpr int OUT_BYTES = 32 * 64;   // a warp's place for 32 rows of 16 results on their way to memory
 constexpr int FLAGS = 3;             // sets of rows' marks: a set is written again two tiles' barriers after it was read
 
-template <int BN> __host__ __device__ constexpr int stage_bytes_of() { return PIECES * (TILE_M + BN) * ROW_BYTES; }
-template <int BN> __host__ __device__ constexpr int dynamic_bytes() { return 1024 + 2 * stage_bytes_of<BN>() + (WORKERS / 32) * OUT_BYTES; }
+constexpr int STAGE = PIECES * (TILE_M + BN) * ROW_BYTES;    // the pieces of a slice: a's three planes, then w's
+constexpr int DYNAMIC_BYTES = 1024 + 2 * STAGE + (WORKERS / 32) * OUT_BYTES;
 
-template <int C>
-__device__ __forceinline__ void tmem_load_columns(uint32_t taddr, uint32_t (&r)[C]) {
-    if constexpr (C == 32) tmem_load_32(taddr, r);
-    else if constexpr (C == 16)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                       "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                     : "r"(taddr) : "memory");
-    else
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                     : "r"(taddr) : "memory");
+__device__ __forceinline__ void tmem_load_8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
 }
 
 struct __align__(16) SplitControl {
@@ -114,11 +109,10 @@ struct __align__(16) SplitControl {
     uint32_t failed;
 };
 
-template <int BN>
-__global__ void __launch_bounds__(WORKERS, 1) gemm_split_kernel(const SplitArgs g) {
-    constexpr int STAGE = stage_bytes_of<BN>();
+__global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs g) {
     constexpr int A_PLANE = TILE_M * ROW_BYTES, W_PLANE = BN * ROW_BYTES;
-    constexpr int AC = TILE_M * 8 / WORKERS, WC = (BN * 8 + WORKERS - 1) / WORKERS;      // 8-number pieces of rows a thread splits
+    constexpr int AC = TILE_M * 8 / WORKERS, WC = BN * 8 / WORKERS;      // 8-number pieces of rows a thread splits
+    constexpr int SUMS = 256;               // columns of TMEM for a slice's sums, of which 3 BN are used
     constexpr int CW = BN / 4;                                                           // totals a thread keeps
     extern __shared__ uint8_t split_smem[];
     __shared__ SplitControl ctl;
@@ -139,199 +133,203 @@ __global__ void __launch_bounds__(WORKERS, 1) gemm_split_kernel(const SplitArgs 
         ctl.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(smem_u32(&ctl.tmem_base), 2 * BN);
+    if (warp == WORKERS / 32) tmem_alloc(smem_u32(&ctl.tmem_base), 2 * SUMS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl.tmem_base;
     pdl_trigger();
 
-    // The products of step i, once all warps have laid their pieces (which each does behind its last look at the accumulator
-    // and the stage of step i - 2: neither needs a barrier of its own).
-    auto multiply = [&](long long i) {
-        const int half = (int)(i & 1);
-        if (!warp_wait(smem_u32(&ctl.full[half]), (uint32_t)(i >> 1) & 1u)) return false;
-        tc_fence_after();
+    if (warp == WORKERS / 32) {
+        // ---- the products of a step, once all warps have laid its pieces (which each does behind its last look at the sums
+        // and the stage of the step before the last: neither needs a barrier of its own) ----
         if (elect_one()) {
-            constexpr uint32_t idesc = instr_desc_bf16(TILE_M, BN);
-            const uint64_t desc_a = smem_desc_sw128(smem_u32(smem) + half * STAGE), desc_w = desc_a + (uint64_t)((PIECES * A_PLANE) >> 4);
-            const uint32_t d = tmem_base + half * BN;
+            const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+            bool there = true;
+            for (long long i = 0; i < steps && there; ++i) {
+                const int half = (int)(i & 1);
+                there = mbar_wait(smem_u32(&ctl.full[half]), (uint32_t)(i >> 1) & 1u);
+                if (!there) break;
+                tc_fence_after();
+                const uint64_t desc_a = desc0 + (uint64_t)(half * (STAGE >> 4)), desc_w = desc_a + (uint64_t)((PIECES * A_PLANE) >> 4);
+                const uint32_t d = tmem_base + half * SUMS;
 #pragma unroll
-            for (int k = 0; k < SLICE / 16; ++k)
+                for (int k = 0; k < SLICE / 16; ++k)
 #pragma unroll
-                for (int t = 0; t < SMALL; ++t)
-                    umma_bf16(d, desc_a + (uint64_t)((piece_of_a(t) * A_PLANE + k * 32) >> 4),
-                              desc_w + (uint64_t)((piece_of_w(t) * W_PLANE + k * 32) >> 4), idesc, (k | t) != 0 ? 1u : 0u);
-#pragma unroll
-            for (int k = 0; k < SLICE / 16; ++k) umma_bf16(d, desc_a + (uint64_t)((k * 32) >> 4), desc_w + (uint64_t)((k * 32) >> 4), idesc, 1u);
-            umma_commit(smem_u32(&ctl.done[half]));
+                    for (int q = 0; q < PIECES; ++q)         // piece q of a meets pieces 0 .. 2 - q of w: sums q ..
+                        umma_bf16(d + q * BN, desc_a + (uint64_t)((q * A_PLANE + k * 32) >> 4), desc_w + (uint64_t)((k * 32) >> 4),
+                                  instr_desc_bf16(TILE_M, (PIECES - q) * BN), (k | q) != 0 ? 1u : 0u);
+                umma_commit(smem_u32(&ctl.done[half]));
+            }
+            if (!there) {
+                atomicExch(g.status, 82);
+                ctl.failed = 1;
+            }
         }
-        __syncwarp();
-        return true;
-    };
-
-    // ---- loads, splitting, and the slices' sums ----
-    const int col8 = (tid & 7) * 8, row8 = tid >> 3;         // this thread's columns of a slice, and its rows row8 + 64 i
-    const bool has_w = BN * 8 >= WORKERS || tid < BN * 8;
-    float4 av[AC][2], wv[WC][2];
-    uint32_t most_a[AC], most_w[WC];
-    auto fetch = [&](float4 (&v)[2], const float* p, int row, int rows, int k) {
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* at = p + (size_t)row * g.K + k;
-        v[0] = row < rows && k < g.K ? *reinterpret_cast<const float4*>(at) : zero;
-        v[1] = row < rows && k + 4 < g.K ? *reinterpret_cast<const float4*>(at + 4) : zero;
-    };
-    auto fetch_a = [&](float4 (&v)[AC][2], int tile, int slice) {
+    } else {
+        // ---- loads, splitting, and the slices' sums ----
+        const int col8 = (tid & 7) * 8, row8 = tid >> 3;         // this thread's columns of a slice, and its rows row8 + 64 i
+        float4 av[AC][2], wv[WC][2];
+        uint32_t most_a[AC], most_w[WC];
+        auto fetch = [&](float4 (&v)[2], const float* p, int row, int rows, int k) {
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* at = p + (size_t)row * g.K + k;
+            v[0] = row < rows && k < g.K ? *reinterpret_cast<const float4*>(at) : zero;
+            v[1] = row < rows && k + 4 < g.K ? *reinterpret_cast<const float4*>(at + 4) : zero;
+        };
+        auto fetch_a = [&](float4 (&v)[AC][2], int tile, int slice) {
 #pragma unroll
-        for (int i = 0; i < AC; ++i) fetch(v[i], g.a, (tile % m_tiles) * TILE_M + row8 + 64 * i, g.M, slice * SLICE + col8);
-    };
-    auto fetch_w = [&](float4 (&v)[WC][2], int tile, int slice) {
-        if (has_w)
+            for (int i = 0; i < AC; ++i) fetch(v[i], g.a, (tile % m_tiles) * TILE_M + row8 + 64 * i, g.M, slice * SLICE + col8);
+        };
+        auto fetch_w = [&](float4 (&v)[WC][2], int tile, int slice) {
 #pragma unroll
             for (int i = 0; i < WC; ++i) fetch(v[i], g.w, (tile / m_tiles) * BN + row8 + 64 * i, g.N, slice * SLICE + col8);
-    };
-    auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most) {
-        uint32_t p[4][PIECES];
-        split_pair(v[0].x, v[0].y, p[0]);
-        split_pair(v[0].z, v[0].w, p[1]);
-        split_pair(v[1].x, v[1].y, p[2]);
-        split_pair(v[1].z, v[1].w, p[3]);
-        most = larger(larger(larger(larger(most, v[0].x), v[0].y), v[0].z), v[0].w);
-        most = larger(larger(larger(larger(most, v[1].x), v[1].y), v[1].z), v[1].w);
-        uint8_t* at = base + row * ROW_BYTES + (((tid & 7) ^ (row & 7)) << 4);
+        };
+        auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most) {
+            uint32_t p[4][PIECES];
+            split_pair(v[0].x, v[0].y, p[0]);
+            split_pair(v[0].z, v[0].w, p[1]);
+            split_pair(v[1].x, v[1].y, p[2]);
+            split_pair(v[1].z, v[1].w, p[3]);
+            most = larger(larger(larger(larger(most, v[0].x), v[0].y), v[0].z), v[0].w);
+            most = larger(larger(larger(larger(most, v[1].x), v[1].y), v[1].z), v[1].w);
+            uint8_t* at = base + row * ROW_BYTES + (((tid & 7) ^ (row & 7)) << 4);
 #pragma unroll
-        for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(at + q * plane) = make_uint4(p[0][q], p[1][q], p[2][q], p[3][q]);
-    };
-    const int quarter = warp & 3, group = warp >> 2;         // this thread's row of TMEM is 32 quarter + lane, its columns CW group + 0 .. CW
-    const uint32_t sums_at = tmem_base + ((uint32_t)(quarter * 32) << 16) + group * CW;
-    float total[CW];
-#pragma unroll
-    for (int j = 0; j < CW; ++j) total[j] = 0.f;
-    bool ok = true;
-
-    // Takes step i's sums; behind a tile's last slice the tile's results go to memory.
-    auto add_up = [&](long long i, int slice, int tile, int flags) {
-        const int half = (int)(i & 1);
-        if (!warp_wait(smem_u32(&ctl.done[half]), (uint32_t)(i >> 1) & 1u)) return false;
-        tc_fence_after();
-        uint32_t r[CW];
-        tmem_load_columns<CW>(sums_at + half * BN, r);
-        tmem_wait_ld();
-        tc_fence_before();
-#pragma unroll
-        for (int j = 0; j < CW; ++j) total[j] += __uint_as_float(r[j]);
-        if (slice + 1 < slices) return true;
-        asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");            // all rows of the tile are marked
-        const int row0 = (tile % m_tiles) * TILE_M + quarter * 32, col0 = (tile / m_tiles) * BN + group * CW;
-        uint8_t* place = smem + 2 * STAGE + warp * OUT_BYTES;
-        constexpr int HALF = CW < 16 ? CW : 16, CHUNKS = HALF / 4, ROWS = 32 / CHUNKS;   // columns at a time, 16-byte chunks of them, rows an access
-#pragma unroll
-        for (int h = 0; h < CW; h += HALF) {
-            __syncwarp();
-            if (row0 < g.M) {
-#pragma unroll
-                for (int c = 0; c < CHUNKS; ++c)
-                    *reinterpret_cast<float4*>(place + lane * 64 + ((c ^ ((lane >> 1) & (CHUNKS - 1))) << 4)) =
-                        make_float4(total[h + 4 * c], total[h + 4 * c + 1], total[h + 4 * c + 2], total[h + 4 * c + 3]);
-            }
-            __syncwarp();
-            const int c = lane % CHUNKS, n = col0 + h + 4 * c;
-            for (int r = lane / CHUNKS; r < 32; r += ROWS) {
-                const int m = row0 + r;
-                if (m >= g.M || n >= g.N) break;
-                const float4 sums = *reinterpret_cast<const float4*>(place + r * 64 + ((c ^ ((r >> 1) & (CHUNKS - 1))) << 4));
-                float v[4] = {sums.x, sums.y, sums.z, sums.w};
-                const uint32_t marks = *reinterpret_cast<const uint32_t*>(&bad_w[flags][group * CW + h + 4 * c]);
-                if (marks != 0 || bad_a[flags][quarter * 32 + r] != 0) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n + j < g.N && (bad_a[flags][quarter * 32 + r] != 0 || ((marks >> (8 * j)) & 255u) != 0))
-                            v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
-                }
-                float* dst = g.out + (size_t)m * g.N + n;
-                if (g.wide) {                                // (N is a multiple of 4: all four are there)
-                    if (g.bias != nullptr) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) v[j] += g.bias[n + j];
-                    }
-                    float4 y = make_float4(activate(v[0], g.epilogue), activate(v[1], g.epilogue), activate(v[2], g.epilogue), activate(v[3], g.epilogue));
-                    if (g.epilogue == EPI_RESIDUAL) {
-                        const float4 old = *reinterpret_cast<const float4*>(dst);
-                        y = make_float4(old.x + y.x, old.y + y.y, old.z + y.z, old.w + y.w);
-                    }
-                    *reinterpret_cast<float4*>(dst) = y;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n + j < g.N) {
-                            const float y = activate(v[j] + (g.bias != nullptr ? g.bias[n + j] : 0.f), g.epilogue);
-                            if (g.epilogue == EPI_RESIDUAL) dst[j] += y;
-                            else dst[j] = y;
-                        }
-                }
-            }
-        }
+            for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(at + q * plane) = make_uint4(p[0][q], p[1][q], p[2][q], p[3][q]);
+        };
+        const int quarter = warp & 3, group = warp >> 2;         // this thread's row of TMEM is 32 quarter + lane, its columns CW group + 0 .. CW
+        const uint32_t sums_at = tmem_base + ((uint32_t)(quarter * 32) << 16) + group * CW;
+        float total[CW];
 #pragma unroll
         for (int j = 0; j < CW; ++j) total[j] = 0.f;
-        return true;
-    };
+        bool ok = true;
 
-    int tile = blockIdx.x, slice = 0, flags = 0;             // of the step that is split
-    int was_tile = 0, was_slice = 0, was_flags = 0;          // of the step in front of it
-    if (steps > 0) fetch_w(wv, tile, 0);                     // the weights do not come from the kernel in front
-    pdl_wait();
-    if (steps > 0) fetch_a(av, tile, 0);
+        // Takes step i's sums; behind a tile's last slice the tile's results go to memory.
+        auto add_up = [&](long long i, int slice, int tile, int flags) {
+            const int half = (int)(i & 1);
+            if (!warp_wait(smem_u32(&ctl.done[half]), (uint32_t)(i >> 1) & 1u)) return false;
+            tc_fence_after();
 #pragma unroll
-    for (int i = 0; i < AC; ++i) most_a[i] = 0;
+            for (int c = 0; c < CW; c += 8) {
+                uint32_t r[PIECES][8];
 #pragma unroll
-    for (int i = 0; i < WC; ++i) most_w[i] = 0;
-    for (long long i = 0; i < steps; ++i) {
-        uint8_t* stage = smem + (int)(i & 1) * STAGE;
-        const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
-        // (a row behind the last keeps what the place held: it gives results that nobody takes)
+                for (int q = 0; q < PIECES; ++q) tmem_load_8(sums_at + half * SUMS + q * BN + c, r[q]);
+                tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < AC; ++j)
-            if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
-        if (has_w)
+                for (int j = 0; j < 8; ++j) total[c + j] += __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+            }
+            tc_fence_before();
+            if (slice + 1 < slices) return true;
+            asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");            // all rows of the tile are marked
+            const int row0 = (tile % m_tiles) * TILE_M + quarter * 32, col0 = (tile / m_tiles) * BN + group * CW;
+            uint8_t* place = smem + 2 * STAGE + warp * OUT_BYTES;
+            constexpr int HALF = 16, CHUNKS = HALF / 4, ROWS = 32 / CHUNKS;   // columns at a time, 16-byte chunks of them, rows an access
+#pragma unroll
+            for (int h = 0; h < CW; h += HALF) {
+                __syncwarp();
+                if (row0 < g.M) {
+#pragma unroll
+                    for (int c = 0; c < CHUNKS; ++c)
+                        *reinterpret_cast<float4*>(place + lane * 64 + ((c ^ ((lane >> 1) & (CHUNKS - 1))) << 4)) =
+                            make_float4(total[h + 4 * c], total[h + 4 * c + 1], total[h + 4 * c + 2], total[h + 4 * c + 3]);
+                }
+                __syncwarp();
+                const int c = lane % CHUNKS, n = col0 + h + 4 * c;
+                for (int r = lane / CHUNKS; r < 32; r += ROWS) {
+                    const int m = row0 + r;
+                    if (m >= g.M || n >= g.N) break;
+                    const float4 sums = *reinterpret_cast<const float4*>(place + r * 64 + ((c ^ ((r >> 1) & (CHUNKS - 1))) << 4));
+                    float v[4] = {sums.x, sums.y, sums.z, sums.w};
+                    const uint32_t marks = *reinterpret_cast<const uint32_t*>(&bad_w[flags][group * CW + h + 4 * c]);
+                    if (marks != 0 || bad_a[flags][quarter * 32 + r] != 0) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (n + j < g.N && (bad_a[flags][quarter * 32 + r] != 0 || ((marks >> (8 * j)) & 255u) != 0))
+                                v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
+                    }
+                    float* dst = g.out + (size_t)m * g.N + n;
+                    if (g.wide) {                                // (N is a multiple of 4: all four are there)
+                        if (g.bias != nullptr) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[j] += g.bias[n + j];
+                        }
+                        float4 y = make_float4(activate(v[0], g.epilogue), activate(v[1], g.epilogue), activate(v[2], g.epilogue), activate(v[3], g.epilogue));
+                        if (g.epilogue == EPI_RESIDUAL) {
+                            const float4 old = *reinterpret_cast<const float4*>(dst);
+                            y = make_float4(old.x + y.x, old.y + y.y, old.z + y.z, old.w + y.w);
+                        }
+                        *reinterpret_cast<float4*>(dst) = y;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (n + j < g.N) {
+                                const float y = activate(v[j] + (g.bias != nullptr ? g.bias[n + j] : 0.f), g.epilogue);
+                                if (g.epilogue == EPI_RESIDUAL) dst[j] += y;
+                                else dst[j] = y;
+                            }
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < CW; ++j) total[j] = 0.f;
+            return true;
+        };
+
+        int tile = blockIdx.x, slice = 0, flags = 0;             // of the step that is split
+        int was_tile = 0, was_slice = 0, was_flags = 0;          // of the step in front of it
+        if (steps > 0) fetch_w(wv, tile, 0);                     // the weights do not come from the kernel in front
+        pdl_wait();
+        if (steps > 0) fetch_a(av, tile, 0);
+#pragma unroll
+        for (int i = 0; i < AC; ++i) most_a[i] = 0;
+#pragma unroll
+        for (int i = 0; i < WC; ++i) most_w[i] = 0;
+        for (long long i = 0; i < steps; ++i) {
+            uint8_t* stage = smem + (int)(i & 1) * STAGE;
+            const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
+            // (a row behind the last keeps what the place held: it gives results that nobody takes)
+#pragma unroll
+            for (int j = 0; j < AC; ++j)
+                if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
 #pragma unroll
             for (int j = 0; j < WC; ++j)
                 if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j]);
-        async_proxy_fence();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
-        const int this_tile = tile, this_slice = slice, this_flags = flags;
-        if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
+            async_proxy_fence();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
+            const int this_tile = tile, this_slice = slice, this_flags = flags;
+            if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
 #pragma unroll
-            for (int j = 0; j < AC; ++j) {
+                for (int j = 0; j < AC; ++j) {
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1) most_a[j] = max(most_a[j], __shfl_xor_sync(0xffffffffu, most_a[j], o));
-                if ((tid & 7) == 0) bad_a[flags][row8 + 64 * j] = splits_badly(most_a[j]);
-                most_a[j] = 0;
+                    for (int o = 1; o < 8; o <<= 1) most_a[j] = max(most_a[j], __shfl_xor_sync(0xffffffffu, most_a[j], o));
+                    if ((tid & 7) == 0) bad_a[flags][row8 + 64 * j] = splits_badly(most_a[j]);
+                    most_a[j] = 0;
+                }
+#pragma unroll
+                for (int j = 0; j < WC; ++j) {
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) most_w[j] = max(most_w[j], __shfl_xor_sync(0xffffffffu, most_w[j], o));
+                    if ((tid & 7) == 0) bad_w[flags][row8 + 64 * j] = splits_badly(most_w[j]);
+                    most_w[j] = 0;
+                }
+                slice = 0;
+                tile += gridDim.x;
+                if (++flags == FLAGS) flags = 0;
             }
-#pragma unroll
-            for (int j = 0; j < WC; ++j) {
-#pragma unroll
-                for (int o = 1; o < 8; o <<= 1) most_w[j] = max(most_w[j], __shfl_xor_sync(0xffffffffu, most_w[j], o));
-                if (has_w && (tid & 7) == 0) bad_w[flags][row8 + 64 * j] = splits_badly(most_w[j]);
-                most_w[j] = 0;
+            if (i + 1 < steps) {
+                fetch_a(av, tile, slice);
+                fetch_w(wv, tile, slice);
             }
-            slice = 0;
-            tile += gridDim.x;
-            if (++flags == FLAGS) flags = 0;
+            if (i > 0) ok = add_up(i - 1, was_slice, was_tile, was_flags);
+            if (!ok) break;
+            was_tile = this_tile; was_slice = this_slice; was_flags = this_flags;
         }
-        if (i + 1 < steps) {
-            fetch_a(av, tile, slice);
-            fetch_w(wv, tile, slice);
+        if (ok && steps > 0) ok = add_up(steps - 1, was_slice, was_tile, was_flags);
+        if (!ok && lane == 0) {
+            atomicExch(g.status, 81);
+            ctl.failed = 1;
         }
-        ok = warp != 0 || multiply(i);
-        if (ok && i > 0) ok = add_up(i - 1, was_slice, was_tile, was_flags);
-        if (!ok) break;
-        was_tile = this_tile; was_slice = this_slice; was_flags = this_flags;
-    }
-    if (ok && steps > 0) ok = add_up(steps - 1, was_slice, was_tile, was_flags);
-    if (!ok && lane == 0) {
-        atomicExch(g.status, 81);
-        ctl.failed = 1;
     }
     __syncwarp();
     // a wait ran out: products that may still be under way get a moment to end
@@ -340,15 +338,14 @@ __global__ void __launch_bounds__(WORKERS, 1) gemm_split_kernel(const SplitArgs 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == WORKERS / 32) tmem_dealloc(tmem_base, 2 * SUMS);
 }
 
-template <int BN>
 cudaError_t launch_tiles(const SplitArgs& g, cudaStream_t s) {
-    const cudaError_t configured = mg_raise_shared(gemm_split_kernel<BN>, dynamic_bytes<BN>());
+    const cudaError_t configured = mg_raise_shared(gemm_split_kernel, DYNAMIC_BYTES);
     if (configured != cudaSuccess) return configured;
     const long long tiles = (long long)ceil_div(g.M, TILE_M) * ceil_div(g.N, BN);
-    return mg_launch(gemm_split_kernel<BN>, dim3((unsigned)(tiles < SMS ? tiles : SMS)), dim3(WORKERS), dynamic_bytes<BN>(), s, true, g);
+    return mg_launch(gemm_split_kernel, dim3((unsigned)(tiles < SMS ? tiles : SMS)), dim3(THREADS), DYNAMIC_BYTES, s, true, g);
 }
 
 // ---- a few rows ---------------------------------------------------------------------------------------------
@@ -421,12 +418,13 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
         __syncwarp();
         const float* ws = ring + (r & (stages - 1)) * STAGE + gr * LINE + t2;
         const float* as = ws + NR * LINE;
-        float c[TB][4];
-        uint32_t wh[SLICE / 16][4], ah[SLICE / 16][TB][2];                  // first pieces, whose products come last
+        float c[TB][PIECES][4];                                             // the three accumulators
 #pragma unroll
         for (int b = 0; b < TB; ++b)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) c[b][e] = 0.f;
+            for (int q = 0; q < PIECES; ++q)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[b][q][e] = 0.f;
 #pragma unroll
         for (int k = 0; k < SLICE / 16; ++k) {
             uint32_t wp[PIECES][4], ap[PIECES][TB][2];
@@ -438,7 +436,6 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
                 mine_w[e & 1] = larger(larger(mine_w[e & 1], x.x), x.y);
 #pragma unroll
                 for (int q = 0; q < PIECES; ++q) wp[q][e] = p[q];
-                wh[k][e] = p[0];
             }
 #pragma unroll
             for (int b = 0; b < TB; ++b)
@@ -450,17 +447,14 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
                     mine_a[b] = larger(larger(mine_a[b], x.x), x.y);
 #pragma unroll
                     for (int q = 0; q < PIECES; ++q) ap[q][b][e] = p[q];
-                    ah[k][b][e] = p[0];
                 }
 #pragma unroll
-            for (int t = 0; t < SMALL; ++t)
+            for (int q = 0; q < PIECES; ++q)                                // (a's piece, w's piece: in the order of the tiles)
 #pragma unroll
-                for (int b = 0; b < TB; ++b) mma_bf16(c[b], wp[piece_of_w(t)], ap[piece_of_a(t)][b][0], ap[piece_of_a(t)][b][1]);
+                for (int v = 0; v + q < PIECES; ++v)
+#pragma unroll
+                    for (int b = 0; b < TB; ++b) mma_bf16(c[b][q + v], wp[v], ap[q][b][0], ap[q][b][1]);
         }
-#pragma unroll
-        for (int k = 0; k < SLICE / 16; ++k)
-#pragma unroll
-            for (int b = 0; b < TB; ++b) mma_bf16(c[b], wh[k], ah[k][b][0], ah[k][b][1]);
         __syncwarp();
         if (r + stages < rounds) {
             ask_w(r + stages);
@@ -471,7 +465,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
 #pragma unroll
         for (int b = 0; b < TB; ++b)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][e];
+            for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][0][e] + (c[b][1][e] + c[b][2][e]);
         if (r + 1 == rounds) {                                              // what each row's largest number is, over all warps
 #pragma unroll
             for (int e = 0; e < 2; ++e) atomicMax(&most_w[gr + 8 * e], mine_w[e]);
@@ -521,19 +515,13 @@ MG_API int mg_linear_split(const float* a, const float* w, const float* bias, fl
         return mg_set_error(MG_ERR_UNSUPPORTED, "linear: 32-bit tensor-core path needs K %% 4 == 0 and 16-byte aligned operands");
     SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, status};
     g.wide = N % 4 == 0 && ((uintptr_t)g.out & 15) == 0;
-    MG_REQUIRE((long long)ceil_div(M, TILE_M) * ceil_div(N, 32) < (1ll << 30), "linear: too many tiles");
+    MG_REQUIRE((long long)ceil_div(M, TILE_M) * ceil_div(N, BN) < (1ll << 30), "linear: too many tiles");
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
     if (M <= 16) {
         e = M <= 8 ? launch_few<8>(g, s) : launch_few<16>(g, s);
     } else {
-        // A slice takes 1.8 us in tiles of 32 columns, 2.05 in tiles of 64 and 2.8 in tiles of 128 (512 x 2,048, 128 rows: 58, 65
-        // and 89 us), so the rounds of tiles decide: 2,048 x 2,048 x 512 104, 71 and 53 us, 1,024 x 512 x 2,048 59, 66 and 90.
-        auto rounds = [&](int bn) { return (double)((ceil_div(M, TILE_M) * (long long)ceil_div(N, bn) + SMS - 1) / SMS); };
-        const double t128 = rounds(128) * 2.8, t64 = rounds(64) * 2.05, t32 = rounds(32) * 1.8;
-        if (t128 <= t64 && t128 <= t32) e = launch_tiles<128>(g, s);
-        else if (t64 <= t32) e = launch_tiles<64>(g, s);
-        else e = launch_tiles<32>(g, s);
+        e = launch_tiles(g, s);
     }
     if (e != cudaSuccess) return mg_set_error(MG_ERR_CUDA, "gemm_split: %s", cudaGetErrorString(e));
     MG_CHECK_LAUNCH("gemm_split");
