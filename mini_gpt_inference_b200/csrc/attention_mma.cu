@@ -695,10 +695,10 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 
 // ---- wide rows that hold their own values ------------------------------------------------------------
 // Key rows of several hundred features whose first dv features are also the values (cached latents): too wide for
-// query fragments and a whole row of results in one warp's registers.  A CTA of eight warps takes 32 or 64 rows, (token,
+// query fragments and a whole row of results in one warp's registers.  A CTA of eight warps takes 16, 32 or 64 rows, (token,
 // head of the group) pairs in token order, and walks blocks of 64 keys (two buffers in turn).  The queries wait in
 // shared memory.  Warp (rg, cg) takes the rg-th 16 (or 32) of the rows: it multiplies them with keys 16 cg .. 16 cg + 15 of the
-// block, the four warps of a row group exchange their maxima through shared memory, each keeps the sum of its own
+// block, the warps of a row group exchange their maxima through shared memory, each keeps the sum of its own
 // keys' weights (the sums meet after the last block), the weights go to shared memory as bfloat16, and the warp
 // then adds the block's 64 keys into columns CW cg .. CW cg + CW - 1 of its rows' results.  `single`: the rows are one
 // token's heads and the CTA takes one range of its keys; results go to scratch as the merge kernel reads them.
@@ -707,19 +707,23 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 // serves twice the products and a block of keys twice the rows.  Rows in shared memory are multiples of 128 bytes, their 16-byte
 // chunks in the order (chunk ^ row % 8), so that eight rows' chunks meet no bank twice without padding: 64 rows and two blocks
 // of 576 features just fit.  Prompts of 4 requests of 1,021 tokens, 16 heads, 576 / 512 features, a window of 512, in three layers:
-// six launches of 279 us with one, 57 us less each with two.
+// six launches of 279 us with one, 57 us less each with two, 19 less again with a block's row addresses looked up at once.
+//
+// RG: groups of rows.  One token's heads are often 16 rows: then all eight warps are column groups of that one tile, of 8 keys and an eighth
+// of the values each, instead of four of them working on rows of zeros, and the queries come by cp.async behind the keys instead
+// of through registers in front of them.  4 tokens at contexts of a thousand, the same sizes: 12.0 -> 8.6 us.
 __device__ __forceinline__ int swizzled(int row, int chunk, int row_elements) { return row * row_elements + ((chunk ^ (row & 7)) << 3); }
 
-template <int CW, int RT>
+template <int CW, int RT, int RG>
 __global__ void __launch_bounds__(256, 1)
 attention_wide_kernel(const AttnParams p, const int single, const int dpad, const int row_tiles) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    constexpr int WIDE_ROWS = 32 * RT;
-    bf16* qs = reinterpret_cast<bf16*>(smem_raw);                     // [32 RT][dpad]
+    constexpr int WIDE_ROWS = 16 * RT * RG, CG = 8 / RG, NT = KB / CG / 8;     // rows a CTA, column groups, a warp's tiles of 8 keys
+    bf16* qs = reinterpret_cast<bf16*>(smem_raw);                     // [WIDE_ROWS][dpad]
     bf16* kbuf = qs + WIDE_ROWS * dpad;                                // [2][KB][dpad]
-    bf16* ps = kbuf + 2 * KB * dpad;                                   // [32 RT][KB]
-    float* mx = reinterpret_cast<float*>(ps + WIDE_ROWS * KB);         // [4][32 RT]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp & 1, cg = warp >> 1;
+    bf16* ps = kbuf + 2 * KB * dpad;                                   // [WIDE_ROWS][KB]
+    float* mx = reinterpret_cast<float*>(ps + WIDE_ROWS * KB);         // [CG][WIDE_ROWS]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp % RG, cg = warp / RG;
     // columns d .. dpad of the key rows are never loaded: zeros, once
     if (p.d < dpad) {
         const int extra = (dpad - p.d) >> 3;
@@ -766,19 +770,6 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
     }
     const int* table = p.block_table + (size_t)request * p.max_pages;
 
-    // the queries of the tile's rows; rows without a token and columns beyond d as zeros
-    {
-        const int chunks = dpad >> 3;
-        for (int i = tid; i < WIDE_ROWS * chunks; i += 256) {
-            const int r = i / chunks, c = (i - r * chunks) * 8, row = row_base + r;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (row < rows_total && c < p.d) {
-                const int t = single ? 0 : row / group, h = single ? row : row - t * group;
-                v = *reinterpret_cast<const uint4*>(p.q + (size_t)(first_token + t) * p.q_stride + (size_t)(kv_head * group + h) * p.d + c);
-            }
-            *reinterpret_cast<uint4*>(qs + swizzled(r, c >> 3, dpad)) = v;
-        }
-    }
     // this lane's two rows of each tile
     int pos[RT][2], lo[RT][2];
     float m[RT][2], l[RT][2], o[RT][CW / 8][4];
@@ -800,23 +791,36 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
 
     const int page_shift = (p.page_tokens & (p.page_tokens - 1)) == 0 ? __ffs(p.page_tokens) - 1 : -1;
     const int chunks = p.d >> 3;
-    // a warp copies eight of a block's keys, a row's 16-byte chunks across its lanes
+    // a warp copies eight of a block's keys, a row's 16-byte chunks across its lanes; where the rows lie is looked up for all
+    // eight at once
     auto load_keys = [&](int j0, bf16* dst) {
-        for (int key = warp * 8; key < warp * 8 + 8; ++key) {
-            const int j = j0 + key;
-            const bool real = j >= lo_all && j <= j_last;
-            size_t row = 0;
-            if (real) {
-                const int index = page_shift >= 0 ? j >> page_shift : j / p.page_tokens;
-                const int within = page_shift >= 0 ? j & (p.page_tokens - 1) : j - index * p.page_tokens;
-                int page = table[index];
-                if (!MG_GUARDED(attention_mma, MG_GUARD_PAGE, page, p.num_pages)) page = 0;
-                row = ((size_t)page * p.n_kv_head + kv_head) * p.page_tokens + within;
-            }
-            for (int c = lane; c < chunks; c += 32) cp_async16(dst + swizzled(key, c, dpad), p.k_pages + row * p.d + c * 8, real);
+        const int own = j0 + warp * 8 + (lane & 7);
+        int at = -1;                                        // (a cache of 2^31 rows as wide as these fits no GPU)
+        if (own >= lo_all && own <= j_last) {
+            const int index = page_shift >= 0 ? own >> page_shift : own / p.page_tokens;
+            const int within = page_shift >= 0 ? own & (p.page_tokens - 1) : own - index * p.page_tokens;
+            int page = table[index];
+            if (!MG_GUARDED(attention_mma, MG_GUARD_PAGE, page, p.num_pages)) page = 0;
+            at = (page * p.n_kv_head + kv_head) * p.page_tokens + within;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = __shfl_sync(0xffffffffu, at, i);
+            const bf16* from = p.k_pages + (size_t)max(row, 0) * p.d;
+            for (int c = lane; c < chunks; c += 32) cp_async16(dst + swizzled(warp * 8 + i, c, dpad), from + c * 8, row >= 0);
         }
     };
     load_keys(j_first, kbuf);
+    // the queries of the tile's rows; rows without a token and columns beyond d as zeros
+    for (int r = warp; r < WIDE_ROWS; r += 8) {
+        const int row = row_base + r, t = single ? 0 : row / group, h = single ? row : row - t * group;
+        const bool live = row < rows_total;
+        const bf16* from = p.q + (live ? (size_t)(first_token + t) * p.q_stride + (size_t)(kv_head * group + h) * p.d : 0);
+        for (int c = lane; c < (dpad >> 3); c += 32) {
+            const bool real = live && c < chunks;
+            cp_async16(qs + swizzled(r, c, dpad), from + (real ? c * 8 : 0), real);
+        }
+    }
     cp_async_commit();
     if (j_first + KB <= j_last) load_keys(j_first + KB, kbuf + KB * dpad);
     cp_async_commit();
@@ -825,32 +829,50 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
         cp_async_wait<1>();                                // (one group a block, empty ones behind the last)
         __syncthreads();                                   // the block is here, for everyone
         const bf16* kb = kbuf + buf * KB * dpad;
-        float s[RT][2][4];
+        float s[RT][NT][4];
 #pragma unroll
         for (int i = 0; i < RT; ++i)
 #pragma unroll
-            for (int n = 0; n < 2; ++n) s[i][n][0] = s[i][n][1] = s[i][n][2] = s[i][n][3] = 0.f;
-        const int a_row = rg * RT * 16 + (lane & 15), b_row = cg * 16 + (lane >> 4) * 8 + (lane & 7);
+            for (int n = 0; n < NT; ++n) s[i][n][0] = s[i][n][1] = s[i][n][2] = s[i][n][3] = 0.f;
+        const int a_row = rg * RT * 16 + (lane & 15);
+        if constexpr (NT == 2) {
+            const int b_row = cg * 16 + (lane >> 4) * 8 + (lane & 7);
 #pragma unroll 4
-        for (int kk = 0; kk < dpad; kk += 16) {
-            uint32_t b[4];
-            ldsm4(b, kb + swizzled(b_row, (kk >> 3) + ((lane >> 3) & 1), dpad));
+            for (int kk = 0; kk < dpad; kk += 16) {
+                uint32_t b[4];
+                ldsm4(b, kb + swizzled(b_row, (kk >> 3) + ((lane >> 3) & 1), dpad));
 #pragma unroll
-            for (int i = 0; i < RT; ++i) {
-                uint32_t a[4];
-                ldsm4(a, qs + swizzled(a_row + 16 * i, (kk >> 3) + (lane >> 4), dpad));
-                mma16816(s[i][0], a, b[0], b[1]);
-                mma16816(s[i][1], a, b[2], b[3]);
+                for (int i = 0; i < RT; ++i) {
+                    uint32_t a[4];
+                    ldsm4(a, qs + swizzled(a_row + 16 * i, (kk >> 3) + (lane >> 4), dpad));
+                    mma16816(s[i][0], a, b[0], b[1]);
+                    mma16816(s[i][1], a, b[2], b[3]);
+                }
+            }
+        } else {                                           // eight keys: a load brings 32 of their columns
+            const int b_row = cg * 8 + (lane & 7);
+#pragma unroll 3
+            for (int kk = 0; kk < dpad; kk += 32) {
+                uint32_t b[4];
+                ldsm4(b, kb + swizzled(b_row, (kk >> 3) + (lane >> 3), dpad));
+#pragma unroll
+                for (int i = 0; i < RT; ++i)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        uint32_t a[4];
+                        ldsm4(a, qs + swizzled(a_row + 16 * i, (kk >> 3) + 2 * u + (lane >> 4), dpad));
+                        mma16816(s[i][0], a, b[2 * u], b[2 * u + 1]);
+                    }
             }
         }
 #pragma unroll
         for (int i = 0; i < RT; ++i) {
             float bm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int j = j0 + cg * 16 + n * 8 + 2 * (lane & 3) + (e & 1), r = e >> 1;
+                    const int j = j0 + (cg * NT + n) * 8 + 2 * (lane & 3) + (e & 1), r = e >> 1;
                     float sc = s[i][n][e] * p.scale_log2;
                     if (p.cap_log2 > 0.f) sc = p.cap_log2 * tanhf(sc / p.cap_log2);
                     const float v = (j <= pos[i][r] && j >= lo[i][r]) ? sc : -INFINITY;
@@ -871,7 +893,9 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r;
-                const float all = fmaxf(fmaxf(mx[row], mx[WIDE_ROWS + row]), fmaxf(mx[2 * WIDE_ROWS + row], mx[3 * WIDE_ROWS + row]));
+                float all = mx[row];
+#pragma unroll
+                for (int w = 1; w < CG; ++w) all = fmaxf(all, mx[w * WIDE_ROWS + row]);
                 const float nm = fmaxf(m[i][r], all);
                 corr[r] = (m[i][r] == -INFINITY) ? 0.f : exp2_approx(m[i][r] - nm);
                 base[r] = (nm == -INFINITY) ? 0.f : nm;
@@ -879,7 +903,7 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
             }
             float bs[2] = {0.f, 0.f};
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
+            for (int n = 0; n < NT; ++n) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float pr = exp2_approx(s[i][n][e] - base[e >> 1]);
@@ -888,7 +912,7 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
                 }
 #pragma unroll
                 for (int r = 0; r < 2; ++r)
-                    *reinterpret_cast<uint32_t*>(ps + swizzled((rg * RT + i) * 16 + (lane >> 2) + 8 * r, cg * 2 + n, KB) + 2 * (lane & 3)) =
+                    *reinterpret_cast<uint32_t*>(ps + swizzled((rg * RT + i) * 16 + (lane >> 2) + 8 * r, cg * NT + n, KB) + 2 * (lane & 3)) =
                         pack_bf16(s[i][n][2 * r], s[i][n][2 * r + 1]);
             }
 #pragma unroll
@@ -942,7 +966,9 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
             if (pos[i][r] < 0) continue;
             const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r, t = single ? 0 : (row_base + row) / group;
             const int token = first_token + t, head = kv_head * group + row_base + row - t * group;
-            float sum = mx[row] + mx[WIDE_ROWS + row] + mx[2 * WIDE_ROWS + row] + mx[3 * WIDE_ROWS + row];
+            float sum = mx[row];
+#pragma unroll
+            for (int w = 1; w < CG; ++w) sum += mx[w * WIDE_ROWS + row];
             if (single) {
                 const size_t slot = ((size_t)token * p.n_head + head) * p.splits + blockIdx.z;
                 if (cg == 0 && (lane & 3) == 0) {
@@ -984,18 +1010,19 @@ cudaError_t launch_merge(const AttnParams& p, int threads, cudaStream_t s) {
     return mg_launch(attention_merge_kernel<32>, grid, dim3(threads), 0, s, true, p);
 }
 
-// Bytes of shared memory of a CTA of `rows` rows of dpad features.
-constexpr size_t wide_smem(int rows, int dpad) { return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) + (size_t)4 * rows * sizeof(float); }
+// Bytes of shared memory of a CTA of `rows` rows of dpad features (a maximum for each row and column group).
+constexpr size_t wide_smem(int rows, int dpad) { return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) + (size_t)(rows <= 16 ? 8 : 4) * rows * sizeof(float); }
 constexpr size_t WIDE_MOST = 227 * 1024;
 
-template <int CW, int RT>
+template <int CW, int RT, int RG>
 int launch_wide(const AttnParams& p, int single, int n_tiles, int dpad, cudaStream_t s) {
-    const int group = p.n_head / p.n_kv_head, row_tiles = (group + 32 * RT - 1) / (32 * RT);
-    const size_t smem = wide_smem(32 * RT, dpad);
-    cudaError_t e = mg_raise_shared(attention_wide_kernel<CW, RT>, smem);
+    constexpr int rows = 16 * RT * RG;
+    const int group = p.n_head / p.n_kv_head, row_tiles = (group + rows - 1) / rows;
+    const size_t smem = wide_smem(rows, dpad);
+    cudaError_t e = mg_raise_shared(attention_wide_kernel<CW, RT, RG>, smem);
     if (e == cudaSuccess) {
         const dim3 grid = single ? dim3(p.n_tokens * row_tiles, p.n_kv_head, p.splits) : dim3(n_tiles, p.n_kv_head);
-        e = mg_launch(attention_wide_kernel<CW, RT>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
+        e = mg_launch(attention_wide_kernel<CW, RT, RG>, grid, dim3(256), smem, s, true, p, single, dpad, row_tiles);
     }
     if (e == cudaSuccess && single)
         e = launch_merge(p, p.dv > 256 ? 512 : p.dv > 128 ? 256 : 128, s);
@@ -1154,10 +1181,19 @@ MG_API int mg_attention_wide(const void* q, int q_stride, const void* k_pages, c
         MG_REQUIRE(req_q_start && req_q_len && n_tiles > 0, "attention (wide rows): no tiles");
     }
     cudaStream_t s = (cudaStream_t)stream;
-#define MG_LAUNCH_WIDE(CW) return rows == 64 ? launch_wide<CW, 2>(p, single_tokens, n_tiles, dpad, s) : launch_wide<CW, 1>(p, single_tokens, n_tiles, dpad, s)
+    // one token's heads in one tile of 16 rows: the eight warps are column groups of it
+    const bool narrow = single_tokens && n_head / n_kv_head <= 16 && dv_pad >= 128;
+#define MG_LAUNCH_WIDE(CW) return rows == 64 ? launch_wide<CW, 2, 2>(p, single_tokens, n_tiles, dpad, s) : launch_wide<CW, 1, 2>(p, single_tokens, n_tiles, dpad, s)
     if (dv_pad == 64) MG_LAUNCH_WIDE(16);
-    if (dv_pad == 128) MG_LAUNCH_WIDE(32);
-    if (dv_pad == 256) MG_LAUNCH_WIDE(64);
+    if (dv_pad == 128) {
+        if (narrow) return launch_wide<16, 1, 1>(p, 1, 0, dpad, s);
+        MG_LAUNCH_WIDE(32);
+    }
+    if (dv_pad == 256) {
+        if (narrow) return launch_wide<32, 1, 1>(p, 1, 0, dpad, s);
+        MG_LAUNCH_WIDE(64);
+    }
+    if (narrow) return launch_wide<64, 1, 1>(p, 1, 0, dpad, s);
     MG_LAUNCH_WIDE(128);
 #undef MG_LAUNCH_WIDE
 }
