@@ -11,8 +11,13 @@
 // The entries (token, k) of an expert are found by each warp from the ids themselves, so no grouping kernel runs in front:
 // results lie by entry, and entry_slot is the identity (-1 for padding rows).
 //
+// The second product (form 0) reads the same ids as the first, which runs right in front of it, and its matrices come from no
+// kernel: so its CTAs, as far as they find room beside the first product's, look up their entries and have their rows under way
+// before the first product is done.  (Registers for a CTA's first 1,024 columns across that wait: four CTAs an SM, not five.)
+//
 // 4 tokens, 8 experts of 1,024 x 1,024 and one that every token uses (19 MB a product): 12.7 and 14.0 us, and 3.4 for the
-// grouping, with the tiles of moe.cu.
+// grouping, with the tiles of moe.cu; 8.3 and 7.9 here, 3 less for the two since the second starts early (16 decode steps of four
+// such layers 7,041 -> 6,845 us).
 #include "common.cuh"
 #include "moe_units.cuh"
 
@@ -68,7 +73,7 @@ __device__ __noinline__ void the_rest(const bf16* x, int ldx, const bf16* we, co
 
 // Forms as mg_moe_gemm: 1 gated, 2 plain, 0 out.
 template <int FORM>
-__global__ void __launch_bounds__(32 * WARPS, FORM == 1 ? 0 : 5)
+__global__ void __launch_bounds__(32 * WARPS, FORM == 1 ? 0 : FORM == 0 ? 4 : 5)
 moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, long long w_expert_stride,
                const int* __restrict__ ids, int n_entries, int top, const float* __restrict__ scale, void* __restrict__ out,
                int* __restrict__ entry_slot, int n_experts, int N, int K, int x_rows, int act, float limit) {
@@ -77,19 +82,31 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
     __shared__ float sums[WARPS][MI * ROWS][MAX_TOKENS + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int e = blockIdx.y, n0 = blockIdx.x * ROWS;
-    pdl_trigger();
-    pdl_wait();
+    // The second product's kernel (form 0) may start once all of the first's are behind their wait: the ids are there then, written
+    // by a kernel that has ended, and its rows of the matrices can be under way while the first product is worked out.
+    if (FORM == 0) {
+        pdl_trigger();
+    } else {
+        pdl_wait();
+        pdl_trigger();
+    }
     // the expert's entries, in order; every warp finds them for itself
     int count = 0;
     for (int i0 = 0; i0 < n_entries; i0 += 32) {
-        const int i = i0 + lane, id = i < n_entries ? ids[i] : -1;
+        const int i = i0 + lane, id = i < n_entries ? __ldcg(ids + i) : -1;
         const unsigned mine = __ballot_sync(0xffffffffu, id == e);
         const int rank = count + __popc(mine & ((1u << lane) - 1u));
         if (id == e && rank < MAX_TOKENS) lists[warp][rank] = i;
         count += __popc(mine);
-        if (FORM == 0 && e == 0 && blockIdx.x == 0 && warp == 0 && i < n_entries) entry_slot[i] = id >= 0 && id < n_experts ? i : -1;
     }
-    if (count == 0) return;
+    if (FORM == 0 && e == 0 && blockIdx.x == 0 && warp == 0) {
+        pdl_wait();                                        // (nothing is written before it)
+        for (int i = lane; i < n_entries; i += 32) entry_slot[i] = ids[i] >= 0 && ids[i] < n_experts ? i : -1;
+    }
+    if (count == 0) {
+        if (FORM == 0) pdl_wait();                         // the kernel ends behind the one in front
+        return;
+    }
     const int entries = count;
     count = min(count, MAX_TOKENS);
     __syncwarp();
@@ -102,6 +119,23 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
             const int n = n0 + g + 8 * h;
             w_row[i][h] = n < N ? we + (size_t)(i * N + n) * K + 8 * t : nullptr;
         }
+    uint4 a[MI][2][4];
+    auto load_w = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {                      // 32 columns each: four lanes' 64 bytes of a row
+            const int k = k0 + 32 * q;
+            const bool in = k + 8 * t < K;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    a[i][h][q] = w_row[i][h] != nullptr && in ? __ldcs(reinterpret_cast<const uint4*>(w_row[i][h] + k)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    if (FORM == 0) {
+        load_w(warp * 128);
+        pdl_wait();
+    }
     const bf16* x_row[2] = {nullptr, nullptr};             // its tokens (columns g and g + 8)
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -117,17 +151,8 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const bool second = count > 8;                         // the same in all lanes
     for (int k0 = warp * 128; k0 < K; k0 += WARPS * 128) {
-        uint4 a[MI][2][4], b[2][4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {                      // 32 columns each: four lanes' 64 bytes of a row
-            const int k = k0 + 32 * q;
-            const bool in = k + 8 * t < K;
-#pragma unroll
-            for (int i = 0; i < MI; ++i)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    a[i][h][q] = w_row[i][h] != nullptr && in ? __ldcs(reinterpret_cast<const uint4*>(w_row[i][h] + k)) : zero;
-        }
+        uint4 b[2][4];
+        if (FORM != 0 || k0 != warp * 128) load_w(k0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int k = k0 + 32 * q;
@@ -174,7 +199,8 @@ moe_few_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w, 
 
 // One of the two products for every entry of a step of up to 16 tokens.  ids: [n_tokens * top] chosen experts (-1: none; a token
 // may name an expert several times); scale: [entries] or null; x: [x_rows, ldx], rows by token (forms 1 and 2) or by entry (form 0);
-// out: [entries, N], bfloat16 (forms 1 and 2) or 32-bit; entry_slot: [entries], written by form 0: the entry itself, or -1.
+// out: [entries, N], bfloat16 (forms 1 and 2) or 32-bit; entry_slot: [entries], written by form 0: the entry itself, or -1.  Form 0 is
+// launched right behind form 1 or 2 on the same ids: it reads them before that kernel has ended.
 // Returns MG_ERR_UNSUPPORTED (and launches nothing) for sizes and alignments it does not take.
 MG_API int mg_moe_few(const void* x, int ldx, const void* w, const int* ids, int n_tokens, int top, const float* scale, void* out,
                       int* entry_slot, int n_experts, int N, int K, int x_rows, int form, int act, float limit, void* stream) {
