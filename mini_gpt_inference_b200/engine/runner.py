@@ -97,11 +97,16 @@ class _ShapeGraph:
     graph: object
     logits: torch.Tensor | None
     kernels: int
+    head: tuple | None = None      # (context, the head's input rows) where the head runs behind the graph
 
 
 class ModelRunner:
     GRAPH_ROWS = (1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256)
     SHAPE_GRAPHS = 16              # most captured prompt-step shapes kept at a time
+    # Logits of a prompt step that are at least this many bytes, of at least this many rows, are not part of its graph: the head runs
+    # behind it into a tensor of the caller's own, where a graph's logits would have to be copied (511 rows of 50,304 ids, 103 MB:
+    # 38 us of 401; a launch of its own costs some 2).
+    HEAD_APART_BYTES, HEAD_APART_ROWS = 16 << 20, 65
 
     def __init__(self, model: DecoderModel, manager: CacheManager, storage: CacheStorage,
                  ops, act_dtype: torch.dtype, device, max_context: int | None = None,
@@ -570,6 +575,8 @@ class ModelRunner:
         self.shape_graph_replays += 1
         if hasattr(self.ops, "launches"):
             self.ops.launches += state.kernels
+        if state.head is not None:
+            return self.model.head.forward(*state.head)
         if state.logits is None:
             return None
         return state.logits.clone() if copy else state.logits
@@ -577,10 +584,13 @@ class ModelRunner:
     def _forward(self, ctx):
         """The model's forward pass over one batch; the kernel set is told that a pass begins (what
         it remembers from launch to launch, such as which matrix followed which, starts anew)."""
+        self._begin()
+        return self.model.forward(ctx)
+
+    def _begin(self) -> None:
         begin = getattr(self.ops, "begin_forward", None)
         if begin is not None:
             begin()
-        return self.model.forward(ctx)
 
     def _stage(self, state: _ShapeGraph, packed: _Packed) -> None:
         if self._copy_done is not None:
@@ -610,8 +620,15 @@ class ModelRunner:
         if dependent is not None:
             dependent(True)
         try:
+            apart = (packed.wanted >= self.HEAD_APART_ROWS
+                     and 4 * packed.wanted * self.vocab_size >= self.HEAD_APART_BYTES)
             with _no_collection(), torch.cuda.graph(graph, pool=self._graph_pool):
-                state.logits = self._forward(ctx)
+                if apart:
+                    self._begin()
+                    rows = self.model.head_input(ctx)
+                    state.head = (ctx, rows.materialize() if hasattr(rows, "materialize") else rows)
+                else:
+                    state.logits = self._forward(ctx)
         finally:
             if dependent is not None:
                 dependent(False)

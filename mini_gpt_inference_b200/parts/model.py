@@ -87,6 +87,12 @@ class DecoderModel:
     # ---- one step ------------------------------------------------------------------------
     def forward(self, ctx):
         """Run ``ctx``'s tokens; return 32-bit logits ``[len(ctx.logit_rows), vocab]``."""
+        y = self.head_input(ctx)
+        return None if y is None else self.head.forward(ctx, y)
+
+    def head_input(self, ctx):
+        """Run ``ctx``'s tokens up to the head: the wanted rows behind the final norm (or that norm still to be applied, for a
+        head that takes one so); None if nothing is wanted."""
         if getattr(ctx, "shared", None) is not None:
             ctx.shared.clear()
         if self.embedding_cache is not None:
@@ -109,6 +115,6 @@ class DecoderModel:
         if self.spec.streams is not None:
             x = ctx.ops.streams_sum(x)
         if getattr(self.head, "accepts_deferred_norm", False):
-            return self.head.forward(ctx, self.final_norm.defer(ctx, x, ctx.logit_rows))
+            return self.final_norm.defer(ctx, x, ctx.logit_rows)
         rows = ctx.ops.gather_rows(x, ctx.logit_rows)
-        return self.head.forward(ctx, self.final_norm.forward(ctx, rows))
+        return self.final_norm.forward(ctx, rows)

@@ -168,6 +168,23 @@ def test_prompt_steps_of_a_repeated_shape_are_replayed(which, dtype):
     runner.manager.check()
 
 
+@pytest.mark.parametrize("which,dtype", list(itertools.product("AB", ["float32", "bfloat16"])))
+def test_head_behind_a_replayed_step(which, dtype):
+    """Logits too large to be copied out of a graph are computed behind it: the plain ones, in a tensor that later steps
+    leave alone."""
+    cfg, tensors, runner, tol = _setup(which, dtype, False)
+    runner.HEAD_APART_BYTES, runner.HEAD_APART_ROWS = 0, 2
+    n = cfg.n_positions - 1
+    outs = []
+    for rep in range(5):
+        tokens = tokens_for(cfg, n, 90 + rep)
+        outs.append((tokens, runner.step([StepEntry("r", tokens, list(range(n)))])))
+        runner.finish("r")
+    assert runner.shape_graph_replays == 3
+    for tokens, got in outs:
+        assert_close(got, plain_logits(cfg, tensors, tokens), tol, "the head behind a replayed step")
+
+
 def test_captured_shapes_are_bounded():
     cfg, tensors, runner, tol = _setup("A", "bfloat16", False)
     runner.SHAPE_GRAPHS = 3
