@@ -978,7 +978,7 @@ def run_ours(args) -> dict:
                            "frac": round(flops / (pre_ms * 1e-3) / (peak * 1e12), 4) if peak else None,
                            "of": peak_source}
         if args.dtype == "bfloat16":
-            # the true 32-bit path of the same model (FMA kernels, 32-bit weights and cache)
+            # the true 32-bit path of the same model (32-bit weights, cache and results)
             args32 = argparse.Namespace(**{**vars(args), "dtype": "float32"})
             _, t, _, ctx32, _ = device_decode(args32, args.batch, min(args.steps, 16), 3, min_seconds=0.0,
                                               max_windows=2)
