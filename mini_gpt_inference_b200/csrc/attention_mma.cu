@@ -697,8 +697,8 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 // Key rows of several hundred features whose first dv features are also the values (cached latents): too wide for
 // query fragments and a whole row of results in one warp's registers.  A CTA of eight warps takes 16, 32 or 64 rows, (token,
 // head of the group) pairs in token order, and walks blocks of 64 keys (two buffers in turn).  The queries wait in
-// shared memory.  Warp (rg, cg) takes the rg-th 16 (or 32) of the rows: it multiplies them with keys 16 cg .. 16 cg + 15 of the
-// block, the warps of a row group exchange their maxima through shared memory, each keeps the sum of its own
+// shared memory.  Warp (rg, cg) takes the rg-th 16 (or 32) of the rows: it multiplies them with the cg-th 16 (or 8, see RG) of the
+// block's keys, the warps of a row group exchange their maxima through shared memory, each keeps the sum of its own
 // keys' weights (the sums meet after the last block), the weights go to shared memory as bfloat16, and the warp
 // then adds the block's 64 keys into columns CW cg .. CW cg + CW - 1 of its rows' results.  `single`: the rows are one
 // token's heads and the CTA takes one range of its keys; results go to scratch as the merge kernel reads them.
@@ -711,7 +711,9 @@ __global__ void attention_merge_kernel(const AttnParams p) {
 //
 // RG: groups of rows.  One token's heads are often 16 rows: then all eight warps are column groups of that one tile, of 8 keys and an eighth
 // of the values each, instead of four of them working on rows of zeros, and the queries come by cp.async behind the keys instead
-// of through registers in front of them.  4 tokens at contexts of a thousand, the same sizes: 12.0 -> 8.6 us.
+// of through registers in front of them.  4 tokens at contexts of a thousand, the same sizes: 12.0 -> 8.6 us.  The weights are
+// summed in the order of the other form all the same: two warps' 8 keys make one sum, which the second takes over from the first
+// behind the barrier that the weights wait for anyway, so a head has the same bits in a tile of 16 rows and in one of 32.
 __device__ __forceinline__ int swizzled(int row, int chunk, int row_elements) { return row * row_elements + ((chunk ^ (row & 7)) << 3); }
 
 template <int CW, int RT, int RG>
@@ -723,6 +725,8 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
     bf16* kbuf = qs + WIDE_ROWS * dpad;                                // [2][KB][dpad]
     bf16* ps = kbuf + 2 * KB * dpad;                                   // [WIDE_ROWS][KB]
     float* mx = reinterpret_cast<float*>(ps + WIDE_ROWS * KB);         // [CG][WIDE_ROWS]
+    float2* first_sums = reinterpret_cast<float2*>(mx + CG * WIDE_ROWS);      // (one row group) [CG / 2][32]
+    constexpr int SUM_STEP = NT == 2 ? 1 : 2;                          // column groups that make one sum of weights: the last of them keeps it
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = warp % RG, cg = warp / RG;
     // columns d .. dpad of the key rows are never loaded: zeros, once
     if (p.d < dpad) {
@@ -887,9 +891,10 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
             }
         }
         __syncthreads();
+        float corr[RT][2];
 #pragma unroll
         for (int i = 0; i < RT; ++i) {
-            float corr[2], base[2];
+            float base[2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r;
@@ -897,18 +902,16 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
 #pragma unroll
                 for (int w = 1; w < CG; ++w) all = fmaxf(all, mx[w * WIDE_ROWS + row]);
                 const float nm = fmaxf(m[i][r], all);
-                corr[r] = (m[i][r] == -INFINITY) ? 0.f : exp2_approx(m[i][r] - nm);
+                corr[i][r] = (m[i][r] == -INFINITY) ? 0.f : exp2_approx(m[i][r] - nm);
                 base[r] = (nm == -INFINITY) ? 0.f : nm;
                 m[i][r] = nm;
             }
-            float bs[2] = {0.f, 0.f};
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float pr = exp2_approx(s[i][n][e] - base[e >> 1]);
                     s[i][n][e] = pr;
-                    bs[e >> 1] += pr;
                 }
 #pragma unroll
                 for (int r = 0; r < 2; ++r)
@@ -916,20 +919,37 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
                         pack_bf16(s[i][n][2 * r], s[i][n][2 * r + 1]);
             }
 #pragma unroll
+            for (int n = 0; n < CW / 8; ++n) {
+                o[i][n][0] *= corr[i][0];
+                o[i][n][1] *= corr[i][0];
+                o[i][n][2] *= corr[i][1];
+                o[i][n][3] *= corr[i][1];
+            }
+        }
+        // the block's weights onto the sums: 16 keys' at a time, one after the other in a lane, then over the four lanes
+        auto add_weights = [&](int i, float2 start) {
+            float bs[2] = {start.x, start.y};
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) bs[e >> 1] += s[i][n][e];
+#pragma unroll
             for (int r = 0; r < 2; ++r) {
                 bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 1);
                 bs[r] += __shfl_xor_sync(0xffffffffu, bs[r], 2);
-                l[i][r] = l[i][r] * corr[r] + bs[r];
+                l[i][r] = l[i][r] * corr[i][r] + bs[r];
             }
+        };
+        if constexpr (NT == 2) {
 #pragma unroll
-            for (int n = 0; n < CW / 8; ++n) {
-                o[i][n][0] *= corr[0];
-                o[i][n][1] *= corr[0];
-                o[i][n][2] *= corr[1];
-                o[i][n][3] *= corr[1];
-            }
+            for (int i = 0; i < RT; ++i) add_weights(i, make_float2(0.f, 0.f));
+        } else if ((cg & 1) == 0) {
+            first_sums[(cg >> 1) * 32 + lane] = make_float2(s[0][0][0] + s[0][0][1], s[0][0][2] + s[0][0][3]);
         }
         __syncthreads();                                   // all 64 keys' weights of the warp's rows are there
+        if constexpr (NT == 1) {
+            if ((cg & 1) != 0) add_weights(0, first_sums[(cg >> 1) * 32 + lane]);
+        }
 #pragma unroll
         for (int kk = 0; kk < KB / 16; ++kk) {
             uint32_t a[RT][4];
@@ -951,7 +971,7 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
         if (j0 + 2 * KB <= j_last) load_keys(j0 + 2 * KB, kbuf + buf * KB * dpad);
         cp_async_commit();
     }
-    // the four warps of a row group kept the sums of their own keys: they meet here
+    // the warps of a row group kept the sums of their own 16 keys of each block: they meet here
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RT; ++i)
@@ -966,9 +986,9 @@ attention_wide_kernel(const AttnParams p, const int single, const int dpad, cons
             if (pos[i][r] < 0) continue;
             const int row = (rg * RT + i) * 16 + (lane >> 2) + 8 * r, t = single ? 0 : (row_base + row) / group;
             const int token = first_token + t, head = kv_head * group + row_base + row - t * group;
-            float sum = mx[row];
+            float sum = mx[(SUM_STEP - 1) * WIDE_ROWS + row];
 #pragma unroll
-            for (int w = 1; w < CG; ++w) sum += mx[w * WIDE_ROWS + row];
+            for (int w = 2 * SUM_STEP - 1; w < CG; w += SUM_STEP) sum += mx[w * WIDE_ROWS + row];
             if (single) {
                 const size_t slot = ((size_t)token * p.n_head + head) * p.splits + blockIdx.z;
                 if (cg == 0 && (lane & 3) == 0) {
@@ -1010,8 +1030,12 @@ cudaError_t launch_merge(const AttnParams& p, int threads, cudaStream_t s) {
     return mg_launch(attention_merge_kernel<32>, grid, dim3(threads), 0, s, true, p);
 }
 
-// Bytes of shared memory of a CTA of `rows` rows of dpad features (a maximum for each row and column group).
-constexpr size_t wide_smem(int rows, int dpad) { return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) + (size_t)(rows <= 16 ? 8 : 4) * rows * sizeof(float); }
+// Bytes of shared memory of a CTA of `rows` rows of dpad features (a maximum for each row and column group; 16 rows: first sums of weights).
+constexpr size_t wide_smem(int rows, int dpad) {
+    return ((size_t)(rows + 2 * KB) * dpad + (size_t)rows * KB) * sizeof(bf16) +
+           (rows <= 16 ? (size_t)8 * rows * sizeof(float) + 4 * 32 * sizeof(float2) : (size_t)4 * rows * sizeof(float));
+}
+static_assert(wide_smem(16, 64) <= wide_smem(32, 64), "what 32 rows fit in, 16 do");
 constexpr size_t WIDE_MOST = 227 * 1024;
 
 template <int CW, int RT, int RG>

@@ -365,6 +365,35 @@ def test_attention_over_wide_rows_that_hold_their_values(path, heads, d, dv, pt)
     assert torch.allclose(got.double().cpu(), want, atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("heads,d,dv,window,softcap", [(1, 160, 128, 0, 0.0), (5, 264, 200, 0, 0.0), (16, 576, 512, 0, 0.0),
+                                                       (16, 576, 512, 512, 0.0), (13, 520, 264, 130, 20.0)])
+def test_single_tokens_over_wide_rows_have_the_bits_of_larger_tiles(heads, d, dv, window, softcap):
+    """Up to 16 heads are one tile of 16 rows and all eight warps its column groups; more are tiles of 32 rows.  The weights'
+    sums are added up in the same order: the same heads among 17 have the same bits, whatever the window, cap and context.  (A
+    sum that differs in its last bit moves one bfloat16 result in some 2^15: hundreds of queries.)"""
+    from mini_gpt_inference_b200.cache.storage import PagedKVView
+    from mini_gpt_inference_b200.kernels.ops import default_ops
+
+    ops = default_ops("cuda:0")
+    gen = torch.Generator().manual_seed(heads * d + dv)
+    pt, pages = 32, 32
+    lengths = [1021, 5, 64, 700] + torch.randint(1, 1025, (1020 // heads,), generator=gen).tolist()
+    tables = [torch.randperm(pages, generator=gen).tolist() for _ in lengths]
+    k_dev = torch.randn(pages, 1, pt, d, generator=gen).to(device="cuda:0", dtype=torch.bfloat16)
+    q = torch.randn(len(lengths), 17, d, generator=gen).to(device="cuda:0", dtype=torch.bfloat16)
+    cache = PagedKVView(k_dev, k_dev, 0, pt, window or None, False, values_in_keys=True)
+    ctx = _AttentionContext(tables, list(range(len(lengths))), [n - 1 for n in lengths], [1] * len(lengths), True)
+
+    def run(n_head):
+        rows = q[:, :n_head].reshape(len(lengths), n_head * d).contiguous()
+        launches = ops.launches
+        out = ops.paged_attention_general(rows, n_head, 1, d, dv, 1.0 / d ** 0.5, cache, ctx, softcap=softcap or None)
+        assert ops.launches - launches == 2                               # the wide kernel and its merge
+        return out.view(len(lengths), n_head, dv)
+
+    assert torch.equal(run(heads), run(17)[:, :heads])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("tokens", [1, 5, 16, 150])
 @pytest.mark.parametrize("heads,n_in,n_out", [(3, 24, 40), (5, 72, 136), (2, 200, 16), (4, 20, 12)])
