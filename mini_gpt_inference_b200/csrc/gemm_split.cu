@@ -204,23 +204,27 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
         for (int j = 0; j < CW; ++j) total[j] = 0.f;
         bool ok = true;
 
-        // Takes step i's sums; behind a tile's last slice the tile's results go to memory.
+        // Takes step i's sums; behind a tile's last slice the tile's results go to memory.  A warp whose wait ran out (ok) takes and
+        // gives nothing any more, but goes on to every barrier: the others may have got their wait and stand there.
         auto add_up = [&](long long i, int slice, int tile, int flags) {
             const int half = (int)(i & 1);
-            if (!warp_wait(smem_u32(&ctl.done[half]), (uint32_t)(i >> 1) & 1u)) return false;
-            tc_fence_after();
+            if (ok) ok = warp_wait(smem_u32(&ctl.done[half]), (uint32_t)(i >> 1) & 1u);
+            if (ok) {
+                tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < CW; c += 8) {
-                uint32_t r[PIECES][8];
+                for (int c = 0; c < CW; c += 8) {
+                    uint32_t r[PIECES][8];
 #pragma unroll
-                for (int q = 0; q < PIECES; ++q) tmem_load_8(sums_at + half * SUMS + q * BN + c, r[q]);
-                tmem_wait_ld();
+                    for (int q = 0; q < PIECES; ++q) tmem_load_8(sums_at + half * SUMS + q * BN + c, r[q]);
+                    tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 8; ++j) total[c + j] += __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+                    for (int j = 0; j < 8; ++j) total[c + j] += __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+                }
+                tc_fence_before();
             }
-            tc_fence_before();
-            if (slice + 1 < slices) return true;
+            if (slice + 1 < slices) return;
             asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");            // all rows of the tile are marked
+            if (!ok) return;
             const int row0 = (tile % m_tiles) * TILE_M + quarter * 32, col0 = (tile / m_tiles) * BN + group * CW;
             uint8_t* place = smem + 2 * STAGE + warp * OUT_BYTES;
             constexpr int HALF = 16, CHUNKS = HALF / 4, ROWS = 32 / CHUNKS;   // columns at a time, 16-byte chunks of them, rows an access
@@ -272,7 +276,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
             }
 #pragma unroll
             for (int j = 0; j < CW; ++j) total[j] = 0.f;
-            return true;
         };
 
         int tile = blockIdx.x, slice = 0, flags = 0;             // of the step that is split
@@ -287,16 +290,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
         for (long long i = 0; i < steps; ++i) {
             uint8_t* stage = smem + (int)(i & 1) * STAGE;
             const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
-            // (a row behind the last keeps what the place held: it gives results that nobody takes)
+            if (ok) {
+                // (a row behind the last keeps what the place held: it gives results that nobody takes)
 #pragma unroll
-            for (int j = 0; j < AC; ++j)
-                if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
+                for (int j = 0; j < AC; ++j)
+                    if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
 #pragma unroll
-            for (int j = 0; j < WC; ++j)
-                if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j]);
-            async_proxy_fence();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
+                for (int j = 0; j < WC; ++j)
+                    if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j]);
+                async_proxy_fence();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
+            }
             const int this_tile = tile, this_slice = slice, this_flags = flags;
             if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
 #pragma unroll
@@ -317,15 +322,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
                 tile += gridDim.x;
                 if (++flags == FLAGS) flags = 0;
             }
-            if (i + 1 < steps) {
+            if (i + 1 < steps && ok) {
                 fetch_a(av, tile, slice);
                 fetch_w(wv, tile, slice);
             }
-            if (i > 0) ok = add_up(i - 1, was_slice, was_tile, was_flags);
-            if (!ok) break;
+            if (i > 0) add_up(i - 1, was_slice, was_tile, was_flags);
             was_tile = this_tile; was_slice = this_slice; was_flags = this_flags;
         }
-        if (ok && steps > 0) ok = add_up(steps - 1, was_slice, was_tile, was_flags);
+        if (steps > 0) add_up(steps - 1, was_slice, was_tile, was_flags);
         if (!ok && lane == 0) {
             atomicExch(g.status, 81);
             ctl.failed = 1;
