@@ -12,8 +12,10 @@
 // Every element is summed in that one order whatever the number of rows and the kernel or tile that it falls in, so a token's
 // result does not depend on what else is in the batch (mma.sync and tcgen05.mma give the same bits; so do the two orders of the operands).
 //
-// Rows (of a or w) that hold an infinity, no number, a number of 2^126 or more, or none but zeros and numbers below 2^-90, do not
-// split so: results that meet such a row are summed by fused multiply-adds instead (fma_sum), again whatever is beside them.
+// Rows (of a or w) that hold an infinity, no number, a number of 2^126 or more or one whose last piece falls below bfloat16's least number
+// (possible below 2^-109) do not split so.  And sums of pieces could pass the end of the range where the sum itself does not, or run into
+// infinities of both signs: a row of a and one of w whose largest numbers make that possible over K terms.  Results
+// that meet either are summed by fused multiply-adds instead (fma_sum), again whatever is beside them.
 //
 // Two kernels:
 //   gemm_split_kernel   tiles of 128 rows x 64 columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
@@ -38,8 +40,9 @@ namespace {
 constexpr int SLICE = 64;            // terms summed by the tensor cores in one go: a 128-byte row of bfloat16
 constexpr int PIECES = 3;
 
-// The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third is exact, so its upper half is all of it.
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECES]) {
+// The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third's upper half is all of it, as long
+// as it does not fall below bfloat16's least number: what is cut off then shows in the low half of `lost`.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECES], uint32_t& lost) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     p[0] = *reinterpret_cast<const uint32_t*>(&h);
     x -= __uint_as_float(p[0] << 16);
@@ -48,13 +51,22 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECE
     p[1] = *reinterpret_cast<const uint32_t*>(&m);
     x -= __uint_as_float(p[1] << 16);
     y -= __uint_as_float(p[1] & 0xffff0000u);
+    lost |= __float_as_uint(x) | __float_as_uint(y);
     p[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
 
 // The bits of |x| order as the numbers do, with infinities and no numbers on top.
 __device__ __forceinline__ uint32_t larger(uint32_t most, float x) { return max(most, __float_as_uint(x) & 0x7fffffffu); }
-__device__ __forceinline__ bool splits_badly(uint32_t most) {
-    return most >= 0x7e800000u || (most != 0 && most < 0x12800000u);         // 2^126, 2^-90
+// What a row counts for: the exponent e (as stored) of its largest number, which is below 2^(e - 126); UNSPLIT if it does not split.
+constexpr uint32_t UNSPLIT = 512;
+__device__ __forceinline__ uint32_t most_of(uint32_t most, uint32_t lost) { return (lost & 0xffffu) != 0 ? 0x7fffffffu : most; }
+__device__ __forceinline__ uint32_t reach(uint32_t most) { return most >= 0x7e800000u ? UNSPLIT : most >> 23; }      // 2^126
+// K products of a row with e and one with f stay below K 2^(e + f - 252), pieces' sums below 1.02 of that.  Up to this e + f
+// they stay below 2^127: no sum of theirs ends, or passes, beyond the range.
+inline int highest_reach(int K) {
+    int log2_k = 0;
+    while ((1ll << log2_k) < K) ++log2_k;
+    return 378 - log2_k;
 }
 
 // Slices by fused multiply-adds from 0, their sums one after the other.
@@ -79,6 +91,7 @@ struct SplitArgs {
     float* out;                      // the residual stream for EPI_RESIDUAL
     int M, N, K, epilogue;
     int wide;                        // rows of the output lie on 16-byte boundaries
+    uint32_t highest;                // reaches of two rows that add up to more: by fused multiply-adds
     int* status;
 };
 
@@ -116,7 +129,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
     constexpr int CW = BN / 4;                                                           // totals a thread keeps
     extern __shared__ uint8_t split_smem[];
     __shared__ SplitControl ctl;
-    __shared__ __align__(16) uint8_t bad_a[FLAGS][TILE_M], bad_w[FLAGS][BN];
+    __shared__ __align__(16) uint16_t reach_a[FLAGS][TILE_M], reach_w[FLAGS][BN];
     uint8_t* smem = (uint8_t*)(((uintptr_t)split_smem + 1023) & ~(uintptr_t)1023);       // (the swizzle wants 1,024-byte boundaries)
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -170,7 +183,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
         // ---- loads, splitting, and the slices' sums ----
         const int col8 = (tid & 7) * 8, row8 = tid >> 3;         // this thread's columns of a slice, and its rows row8 + 64 i
         float4 av[AC][2], wv[WC][2];
-        uint32_t most_a[AC], most_w[WC];
+        uint32_t most_a[AC], most_w[WC], lost_a[AC], lost_w[WC];
         auto fetch = [&](float4 (&v)[2], const float* p, int row, int rows, int k) {
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             const float* at = p + (size_t)row * g.K + k;
@@ -185,12 +198,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
 #pragma unroll
             for (int i = 0; i < WC; ++i) fetch(v[i], g.w, (tile / m_tiles) * BN + row8 + 64 * i, g.N, slice * SLICE + col8);
         };
-        auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most) {
+        auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most, uint32_t& lost) {
             uint32_t p[4][PIECES];
-            split_pair(v[0].x, v[0].y, p[0]);
-            split_pair(v[0].z, v[0].w, p[1]);
-            split_pair(v[1].x, v[1].y, p[2]);
-            split_pair(v[1].z, v[1].w, p[3]);
+            split_pair(v[0].x, v[0].y, p[0], lost);
+            split_pair(v[0].z, v[0].w, p[1], lost);
+            split_pair(v[1].x, v[1].y, p[2], lost);
+            split_pair(v[1].z, v[1].w, p[3], lost);
             most = larger(larger(larger(larger(most, v[0].x), v[0].y), v[0].z), v[0].w);
             most = larger(larger(larger(larger(most, v[1].x), v[1].y), v[1].z), v[1].w);
             uint8_t* at = base + row * ROW_BYTES + (((tid & 7) ^ (row & 7)) << 4);
@@ -244,13 +257,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
                     if (m >= g.M || n >= g.N) break;
                     const float4 sums = *reinterpret_cast<const float4*>(place + r * 64 + ((c ^ ((r >> 1) & (CHUNKS - 1))) << 4));
                     float v[4] = {sums.x, sums.y, sums.z, sums.w};
-                    const uint32_t marks = *reinterpret_cast<const uint32_t*>(&bad_w[flags][group * CW + h + 4 * c]);
-                    if (marks != 0 || bad_a[flags][quarter * 32 + r] != 0) {
+                    const ushort4 of_w = *reinterpret_cast<const ushort4*>(&reach_w[flags][group * CW + h + 4 * c]);
+                    const uint32_t of_a = reach_a[flags][quarter * 32 + r], reaches[4] = {of_w.x, of_w.y, of_w.z, of_w.w};
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (n + j < g.N && (bad_a[flags][quarter * 32 + r] != 0 || ((marks >> (8 * j)) & 255u) != 0))
-                                v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
-                    }
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < g.N && of_a + reaches[j] > g.highest)
+                            v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
                     float* dst = g.out + (size_t)m * g.N + n;
                     if (g.wide) {                                // (N is a multiple of 4: all four are there)
                         if (g.bias != nullptr) {
@@ -284,9 +296,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
         pdl_wait();
         if (steps > 0) fetch_a(av, tile, 0);
 #pragma unroll
-        for (int i = 0; i < AC; ++i) most_a[i] = 0;
+        for (int i = 0; i < AC; ++i) most_a[i] = lost_a[i] = 0;
 #pragma unroll
-        for (int i = 0; i < WC; ++i) most_w[i] = 0;
+        for (int i = 0; i < WC; ++i) most_w[i] = lost_w[i] = 0;
         for (long long i = 0; i < steps; ++i) {
             uint8_t* stage = smem + (int)(i & 1) * STAGE;
             const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
@@ -294,10 +306,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
                 // (a row behind the last keeps what the place held: it gives results that nobody takes)
 #pragma unroll
                 for (int j = 0; j < AC; ++j)
-                    if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j]);
+                    if (m0 + row8 + 64 * j < g.M) lay(av[j], stage, A_PLANE, row8 + 64 * j, most_a[j], lost_a[j]);
 #pragma unroll
                 for (int j = 0; j < WC; ++j)
-                    if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j]);
+                    if (n0 + row8 + 64 * j < g.N) lay(wv[j], stage + PIECES * A_PLANE, W_PLANE, row8 + 64 * j, most_w[j], lost_w[j]);
                 async_proxy_fence();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&ctl.full[(int)(i & 1)]));
@@ -306,17 +318,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
             if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
 #pragma unroll
                 for (int j = 0; j < AC; ++j) {
+                    most_a[j] = most_of(most_a[j], lost_a[j]);
 #pragma unroll
                     for (int o = 1; o < 8; o <<= 1) most_a[j] = max(most_a[j], __shfl_xor_sync(0xffffffffu, most_a[j], o));
-                    if ((tid & 7) == 0) bad_a[flags][row8 + 64 * j] = splits_badly(most_a[j]);
-                    most_a[j] = 0;
+                    if ((tid & 7) == 0) reach_a[flags][row8 + 64 * j] = (uint16_t)reach(most_a[j]);
+                    most_a[j] = lost_a[j] = 0;
                 }
 #pragma unroll
                 for (int j = 0; j < WC; ++j) {
+                    most_w[j] = most_of(most_w[j], lost_w[j]);
 #pragma unroll
                     for (int o = 1; o < 8; o <<= 1) most_w[j] = max(most_w[j], __shfl_xor_sync(0xffffffffu, most_w[j], o));
-                    if ((tid & 7) == 0) bad_w[flags][row8 + 64 * j] = splits_badly(most_w[j]);
-                    most_w[j] = 0;
+                    if ((tid & 7) == 0) reach_w[flags][row8 + 64 * j] = (uint16_t)reach(most_w[j]);
+                    most_w[j] = lost_w[j] = 0;
                 }
                 slice = 0;
                 tile += gridDim.x;
@@ -413,9 +427,9 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
         cp_async_commit();
     }
     const int gr = lane >> 2, t2 = (lane & 3) * 2;
-    uint32_t mine_w[2] = {0, 0}, mine_a[TB];
+    uint32_t mine_w[2] = {0, 0}, lost_w[2] = {0, 0}, mine_a[TB], lost_a[TB];
 #pragma unroll
-    for (int b = 0; b < TB; ++b) mine_a[b] = 0;
+    for (int b = 0; b < TB; ++b) mine_a[b] = lost_a[b] = 0;
     float total = 0.f;                                                      // of row tid / NR, column n0 + tid % NR
     for (int r = 0; r < rounds; ++r) {
         cp_async_wait<FEW_STAGES - 1>();
@@ -436,7 +450,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
             for (int e = 0; e < 4; ++e) {                                   // rows gr, gr + 8; columns 2 t, then 2 t + 8
                 const float2 x = *reinterpret_cast<const float2*>(ws + (e & 1) * 8 * LINE + 16 * k + (e >> 1) * 8);
                 uint32_t p[PIECES];
-                split_pair(x.x, x.y, p);
+                split_pair(x.x, x.y, p, lost_w[e & 1]);
                 mine_w[e & 1] = larger(larger(mine_w[e & 1], x.x), x.y);
 #pragma unroll
                 for (int q = 0; q < PIECES; ++q) wp[q][e] = p[q];
@@ -447,7 +461,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
                 for (int e = 0; e < 2; ++e) {
                     const float2 x = *reinterpret_cast<const float2*>(as + b * 8 * LINE + 16 * k + e * 8);
                     uint32_t p[PIECES];
-                    split_pair(x.x, x.y, p);
+                    split_pair(x.x, x.y, p, lost_a[b]);
                     mine_a[b] = larger(larger(mine_a[b], x.x), x.y);
 #pragma unroll
                     for (int q = 0; q < PIECES; ++q) ap[q][b][e] = p[q];
@@ -472,9 +486,9 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
             for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][0][e] + (c[b][1][e] + c[b][2][e]);
         if (r + 1 == rounds) {                                              // what each row's largest number is, over all warps
 #pragma unroll
-            for (int e = 0; e < 2; ++e) atomicMax(&most_w[gr + 8 * e], mine_w[e]);
+            for (int e = 0; e < 2; ++e) atomicMax(&most_w[gr + 8 * e], most_of(mine_w[e], lost_w[e]));
 #pragma unroll
-            for (int b = 0; b < TB; ++b) atomicMax(&most_a[gr + 8 * b], mine_a[b]);
+            for (int b = 0; b < TB; ++b) atomicMax(&most_a[gr + 8 * b], most_of(mine_a[b], lost_a[b]));
         }
         // (one barrier a round: the half written two rounds later was read before the barrier in between)
         __syncthreads();
@@ -485,7 +499,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
     cp_async_wait<0>();
     const int m = tid / NR, n = n0 + tid % NR;
     if (tid >= MT * NR || m >= M || n >= N) return;
-    if (splits_badly(most_a[m]) || splits_badly(most_w[tid % NR])) total = fma_sum(g.a + (size_t)m * K, g.w + (size_t)n * K, K);
+    if (reach(most_a[m]) + reach(most_w[tid % NR]) > g.highest) total = fma_sum(g.a + (size_t)m * K, g.w + (size_t)n * K, K);
     const float y = activate(total + (g.bias != nullptr ? g.bias[n] : 0.f), g.epilogue);
     float* dst = g.out + (size_t)m * N + n;
     if (g.epilogue == EPI_RESIDUAL) *dst += y;
@@ -517,7 +531,7 @@ MG_API int mg_linear_split(const float* a, const float* w, const float* bias, fl
     MG_REQUIRE(status != nullptr, "linear: missing status word");
     if (K % 4 != 0 || (((uintptr_t)a | (uintptr_t)w) & 15))
         return mg_set_error(MG_ERR_UNSUPPORTED, "linear: 32-bit tensor-core path needs K %% 4 == 0 and 16-byte aligned operands");
-    SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, status};
+    SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, (uint32_t)highest_reach(K), status};
     g.wide = N % 4 == 0 && ((uintptr_t)g.out & 15) == 0;
     MG_REQUIRE((long long)ceil_div(M, TILE_M) * ceil_div(N, BN) < (1ll << 30), "linear: too many tiles");
     cudaStream_t s = (cudaStream_t)stream;

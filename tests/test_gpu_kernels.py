@@ -1031,6 +1031,41 @@ def test_32_bit_products_by_bfloat16_pieces(ops, m, n, k):
     assert ((got.double() - want.double()).abs() <= 2 * (k + 2) * 2.0 ** -24 * size)[finite].all()
 
 
+@pytest.mark.parametrize("m", [8, 16, 130])
+@pytest.mark.parametrize("n,k", [(70, 260), (33, 64)])
+def test_32_bit_products_near_the_ends_of_the_range(ops, m, n, k):
+    """Rows whose products pass the end of the range (and those that end just inside it) give what the FMA tiles give, infinities of
+    the same sign and no numbers in the same places; numbers so small that bfloat16 pieces do not hold them keep their bits beside large ones."""
+    x, w = randn(m, k, seed=51), randn(n, k, seed=52)
+    x[0], w[0] = 3e25, 1e25
+    x[1], w[1] = x[1].abs() * 1e20, -w[1].abs() * 1e30
+    x[2], w[2] = 0.0, 0.0
+    x[2, :4], w[2, :4] = 1.9999 * 2.0 ** 63, 1.9999 * 2.0 ** 61              # four products that just stay inside
+    x[3], w[3] = x[3] * 2.0 ** 60, w[3] * 2.0 ** 62
+    x[4, k // 2:], w[4, : k // 2] = x[4, k // 2:] * 2.0 ** -114, 0.0            # large numbers meet zeros, and small ones large ones
+    w[4, k // 2:] = w[4, k // 2:] * 2.0 ** 40
+    x[5], w[5] = x[5] * 2.0 ** -70, w[5] * 2.0 ** -70                        # results below the least normal number
+    w[6] = w[6] * 2.0 ** -130
+    x[7] = x[7] * 2.0 ** 124
+    got = ops.linear(x, w, None, "none", torch.float32)
+    ops.use_split = False
+    try:
+        want = ops.linear(x, w, None, "none", torch.float32)
+    finally:
+        ops.use_split = True
+    ops.check_status()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)]) and torch.isfinite(got[2, 2])
+    assert torch.isinf(want).any() and torch.isfinite(want[4]).any()
+    ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    finite = torch.isfinite(want)
+    # the bound of the test above; below the normal numbers every addition is cut at 2^-149 instead
+    steps = 10 + -(-k // 64) + 2
+    bound = (steps * 2.0 ** -23 * size).clamp(min=steps * -(-k // 64) * 2.0 ** -149)
+    by_fma = ((k + 2) * 2.0 ** -24 * size).clamp(min=(k + 2) * 2.0 ** -149)
+    assert ((got.double() - ref).abs() <= torch.maximum(bound, by_fma))[finite].all()
+
+
 @pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
 @pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window", [
     (4, 4, 128, 64, 0), (6, 2, 104, 16, 0), (5, 1, 48, 4, 0), (4, 4, 80, 24, 70), (2, 2, 96, 16, 0), (64, 1, 8, 8, 0),
