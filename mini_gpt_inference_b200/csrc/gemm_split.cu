@@ -15,7 +15,8 @@
 // Rows (of a or w) that hold an infinity, no number, a number of 2^126 or more or one whose last piece falls below bfloat16's least number
 // (possible below 2^-109) do not split so.  And sums of pieces could pass the end of the range where the sum itself does not, or run into
 // infinities of both signs: a row of a and one of w whose largest numbers make that possible over K terms.  Results
-// that meet either are summed by fused multiply-adds instead (fma_sum), again whatever is beside them.
+// that meet either are summed by fused multiply-adds instead, slices of 64 from 0 and their sums one after the other, again whatever
+// is beside them: a CTA that has such results walks their operands a second time.
 //
 // Two kernels:
 //   gemm_split_kernel   tiles of 128 rows x 64 columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
@@ -55,12 +56,23 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[PIECE
     p[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
 
-// The bits of |x| order as the numbers do, with infinities and no numbers on top.
-__device__ __forceinline__ uint32_t larger(uint32_t most, float x) { return max(most, __float_as_uint(x) & 0x7fffffffu); }
-// What a row counts for: the exponent e (as stored) of its largest number, which is below 2^(e - 126); UNSPLIT if it does not split.
+// The bits of first pieces without their signs order as the numbers do, with infinities and no numbers on top: the largest of a
+// row's, for each half of the pairs.
+__device__ __forceinline__ uint32_t larger(uint32_t most, uint32_t h) { return __vmaxu2(most, h & 0x7fff7fffu); }
+__device__ __forceinline__ uint32_t larger(uint32_t most, uint32_t h, uint32_t i) { return __vimax3_u16x2(most, h & 0x7fff7fffu, i & 0x7fff7fffu); }
+__device__ __forceinline__ uint32_t most_of(uint32_t most, uint32_t lost) { return (lost & 0xffffu) != 0 ? 0x7fff7fffu : most; }
+// What a row counts for: the exponent e (as stored) of its largest number's first piece, so that all are below 2^(e - 126); UNSPLIT
+// if it does not split.
 constexpr uint32_t UNSPLIT = 512;
-__device__ __forceinline__ uint32_t most_of(uint32_t most, uint32_t lost) { return (lost & 0xffffu) != 0 ? 0x7fffffffu : most; }
-__device__ __forceinline__ uint32_t reach(uint32_t most) { return most >= 0x7e800000u ? UNSPLIT : most >> 23; }      // 2^126
+__device__ __forceinline__ uint32_t reach(uint32_t most) {
+    const uint32_t of_both = max(most & 0xffffu, most >> 16);
+    return of_both >= 0x7e80u ? UNSPLIT : of_both >> 7;         // 2^126
+}
+__device__ __forceinline__ uint32_t eight_lanes_max(uint32_t v) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
 // K products of a row with e and one with f stay below K 2^(e + f - 252), pieces' sums below 1.02 of that.  Up to this e + f
 // they stay below 2^127: no sum of theirs ends, or passes, beyond the range.
 inline int highest_reach(int K) {
@@ -69,16 +81,16 @@ inline int highest_reach(int K) {
     return 378 - log2_k;
 }
 
-// Slices by fused multiply-adds from 0, their sums one after the other.
-__device__ __noinline__ float fma_sum(const float* a, const float* w, int K) {
-    float total = 0.f;
-    for (int k0 = 0; k0 < K; k0 += SLICE) {
-        float sum = 0.f;
-        for (int k = k0; k < min(k0 + SLICE, K); ++k) sum = fmaf(a[k], w[k], sum);
-        total += sum;
-    }
-    return total;
+__device__ __forceinline__ float dot4(float4 x, float4 y, float sum) {
+    return fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, sum))));
 }
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool there) {
+    const uint32_t bytes = there ? 16u : 0u;                 // (0: sixteen zero bytes are written)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ float activate(float v, int epilogue) {
     return epilogue == EPI_GELU ? gelu_tanh(v) : epilogue == EPI_RELU_SQ ? relu_sq(v) : v;
@@ -91,9 +103,16 @@ struct SplitArgs {
     float* out;                      // the residual stream for EPI_RESIDUAL
     int M, N, K, epilogue;
     int wide;                        // rows of the output lie on 16-byte boundaries
-    uint32_t highest;                // reaches of two rows that add up to more: by fused multiply-adds
+    int highest;                     // reaches of two rows that add up to more: by fused multiply-adds
     int* status;
 };
+
+// What becomes of a finished sum of column n.
+__device__ __forceinline__ void finish(const SplitArgs& g, float sum, int n, float* dst) {
+    const float y = activate(sum + (g.bias != nullptr ? g.bias[n] : 0.f), g.epilogue);
+    if (g.epilogue == EPI_RESIDUAL) *dst += y;
+    else *dst = y;
+}
 
 // ---- tiles -----------------------------------------------------------------------------------------------
 // A slice takes 1.45 us, 1.1 with few rows: the operands of the next one come from L2 (48 KB) while a slice is split, and the splitting
@@ -110,25 +129,111 @@ constexpr int FLAGS = 3;             // sets of rows' marks: a set is written ag
 constexpr int STAGE = PIECES * (TILE_M + BN) * ROW_BYTES;    // the pieces of a slice: a's three planes, then w's
 constexpr int DYNAMIC_BYTES = 1024 + 2 * STAGE + (WORKERS / 32) * OUT_BYTES;
 
+constexpr int CW = BN / 4;           // results a worker has
+constexpr int ODD_WORDS = 64;        // marks of tiles with results for the multiply-adds: a CTA's tiles from the 2,048th on share the last one
+
 __device__ __forceinline__ void tmem_load_8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr) : "memory");
 }
 
+// The results that the pieces do not serve, of the tiles that are marked, by fused multiply-adds.  All threads of the CTA, behind its last tile.
+// The tile's rows, a's and then w's, pass through two buffers in turn, 32 columns of each and 4 words of space (16-byte reads of 8 rows
+// meet no bank twice), and are looked over again for what they count for.  512 x 2,048, 128 rows that hold what is no number: 246 us, else 46.
+constexpr int FMA_COLS = SLICE / 2, FMA_LINE = FMA_COLS + 4, FMA_ROWS = TILE_M + BN, FMA_BUFFER = FMA_ROWS * FMA_LINE;
+static_assert(2 * FMA_BUFFER * (int)sizeof(float) <= 2 * STAGE, "the buffers take the stages' place");
+
+__device__ __noinline__ void fma_tiles(const SplitArgs& g, float* buffers, uint16_t* reaches, const uint32_t* odd_tiles, int m_tiles, int my_tiles) {
+    const int tid = threadIdx.x, tr = (tid >> 4) & 31, tc = tid & 15, chunks = 2 * ((g.K + SLICE - 1) / SLICE);
+    for (int t = 0; t < my_tiles; ++t) {
+        const int mark = min(t, 32 * ODD_WORDS - 1);
+        if (((odd_tiles[mark >> 5] >> (mark & 31)) & 1u) == 0) continue;
+        const int tile = (int)blockIdx.x + t * (int)gridDim.x, m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
+        auto ask = [&](int c) {
+            if (c < chunks && tid < WORKERS)
+#pragma unroll
+                for (int u = 0; u < FMA_ROWS * (FMA_COLS / 4) / WORKERS; ++u) {
+                    const int at = tid + u * WORKERS, row = at / (FMA_COLS / 4), col = (at % (FMA_COLS / 4)) * 4, k = c * FMA_COLS + col;
+                    const bool of_a = row < TILE_M, there = k < g.K && (of_a ? m0 + row < g.M : n0 + row - TILE_M < g.N);
+                    const float* from = of_a ? g.a + (size_t)(m0 + row) * g.K + k : g.w + (size_t)(n0 + row - TILE_M) * g.K + k;
+                    cp_async16(buffers + (c & 1) * FMA_BUFFER + row * FMA_LINE + col, there ? from : g.a, there);
+                }
+            cp_async_commit();
+        };
+        float total[4][4], acc[4][4];                            // of rows tr + 32 i and columns tc + 16 j
+        uint32_t most = 0, lost = 0;                             // of row tid
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) total[i][j] = acc[i][j] = 0.f;
+        ask(0);
+        for (int c = 0; c < chunks; ++c) {
+            ask(c + 1);
+            cp_async_wait<1>();
+            __syncthreads();                                     // the chunk is there for all
+            const float* of = buffers + (c & 1) * FMA_BUFFER;
+            if (tid < FMA_ROWS)
+#pragma unroll 2
+                for (int k = 0; k < FMA_COLS; k += 2) {
+                    const float2 x = *reinterpret_cast<const float2*>(of + tid * FMA_LINE + k);
+                    uint32_t p[PIECES];
+                    split_pair(x.x, x.y, p, lost);
+                    most = larger(most, p[0]);
+                }
+            if (tid < WORKERS)
+#pragma unroll 2
+                for (int k = 0; k < FMA_COLS; k += 4) {
+                    float4 x[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(of + (tr + 32 * i) * FMA_LINE + k);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 y = *reinterpret_cast<const float4*>(of + (TILE_M + tc + 16 * j) * FMA_LINE + k);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[i][j] = dot4(x[i], y, acc[i][j]);
+                    }
+                }
+            if ((c & 1) != 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        total[i][j] += acc[i][j];
+                        acc[i][j] = 0.f;
+                    }
+            }
+            __syncthreads();                                     // its buffer takes the chunk after the next
+        }
+        if (tid < FMA_ROWS) reaches[tid] = (uint16_t)reach(most_of(most, lost));
+        __syncthreads();
+        if (tid < WORKERS)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = m0 + tr + 32 * i, room = g.highest - reaches[tr + 32 * i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int n = n0 + tc + 16 * j;
+                    if (m < g.M && n < g.N && reaches[TILE_M + tc + 16 * j] > room) finish(g, total[i][j], n, g.out + (size_t)m * g.N + n);
+                }
+            }
+        __syncthreads();                                         // (the next tile's rows)
+    }
+}
+
 struct __align__(16) SplitControl {
     uint64_t full[2], done[2];       // the pieces of a step are there; its products are done
     uint32_t tmem_base;
-    uint32_t failed;
+    uint32_t failed, odd;            // no more waiting; a tile is marked
 };
 
-__global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs g) {
+__global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ SplitArgs g) {
     constexpr int A_PLANE = TILE_M * ROW_BYTES, W_PLANE = BN * ROW_BYTES;
     constexpr int AC = TILE_M * 8 / WORKERS, WC = BN * 8 / WORKERS;      // 8-number pieces of rows a thread splits
     constexpr int SUMS = 256;               // columns of TMEM for a slice's sums, of which 3 BN are used
-    constexpr int CW = BN / 4;                                                           // totals a thread keeps
     extern __shared__ uint8_t split_smem[];
     __shared__ SplitControl ctl;
+    __shared__ uint32_t odd_tiles[ODD_WORDS];
     __shared__ __align__(16) uint16_t reach_a[FLAGS][TILE_M], reach_w[FLAGS][BN];
     uint8_t* smem = (uint8_t*)(((uintptr_t)split_smem + 1023) & ~(uintptr_t)1023);       // (the swizzle wants 1,024-byte boundaries)
     const int tid = threadIdx.x, lane = tid & 31;
@@ -138,12 +243,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
     const int my_tiles = ((int)blockIdx.x < tiles) ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     const long long steps = (long long)my_tiles * slices;
 
+    if (tid < ODD_WORDS) odd_tiles[tid] = 0;
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&ctl.full[i]), WORKERS / 32);
             mbar_init(smem_u32(&ctl.done[i]), 1);
         }
-        ctl.failed = 0;
+        ctl.failed = ctl.odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WORKERS / 32) tmem_alloc(smem_u32(&ctl.tmem_base), 2 * SUMS);
@@ -190,13 +296,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
             v[0] = row < rows && k < g.K ? *reinterpret_cast<const float4*>(at) : zero;
             v[1] = row < rows && k + 4 < g.K ? *reinterpret_cast<const float4*>(at + 4) : zero;
         };
-        auto fetch_a = [&](float4 (&v)[AC][2], int tile, int slice) {
+        auto fetch_a = [&](float4 (&v)[AC][2], int m0, int slice) {
 #pragma unroll
-            for (int i = 0; i < AC; ++i) fetch(v[i], g.a, (tile % m_tiles) * TILE_M + row8 + 64 * i, g.M, slice * SLICE + col8);
+            for (int i = 0; i < AC; ++i) fetch(v[i], g.a, m0 + row8 + 64 * i, g.M, slice * SLICE + col8);
         };
-        auto fetch_w = [&](float4 (&v)[WC][2], int tile, int slice) {
+        auto fetch_w = [&](float4 (&v)[WC][2], int n0, int slice) {
 #pragma unroll
-            for (int i = 0; i < WC; ++i) fetch(v[i], g.w, (tile / m_tiles) * BN + row8 + 64 * i, g.N, slice * SLICE + col8);
+            for (int i = 0; i < WC; ++i) fetch(v[i], g.w, n0 + row8 + 64 * i, g.N, slice * SLICE + col8);
         };
         auto lay = [&](const float4 (&v)[2], uint8_t* base, int plane, int row, uint32_t& most, uint32_t& lost) {
             uint32_t p[4][PIECES];
@@ -204,8 +310,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
             split_pair(v[0].z, v[0].w, p[1], lost);
             split_pair(v[1].x, v[1].y, p[2], lost);
             split_pair(v[1].z, v[1].w, p[3], lost);
-            most = larger(larger(larger(larger(most, v[0].x), v[0].y), v[0].z), v[0].w);
-            most = larger(larger(larger(larger(most, v[1].x), v[1].y), v[1].z), v[1].w);
+            most = larger(larger(most, p[0][0], p[1][0]), p[2][0], p[3][0]);
             uint8_t* at = base + row * ROW_BYTES + (((tid & 7) ^ (row & 7)) << 4);
 #pragma unroll
             for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(at + q * plane) = make_uint4(p[0][q], p[1][q], p[2][q], p[3][q]);
@@ -258,13 +363,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
                     const float4 sums = *reinterpret_cast<const float4*>(place + r * 64 + ((c ^ ((r >> 1) & (CHUNKS - 1))) << 4));
                     float v[4] = {sums.x, sums.y, sums.z, sums.w};
                     const ushort4 of_w = *reinterpret_cast<const ushort4*>(&reach_w[flags][group * CW + h + 4 * c]);
-                    const uint32_t of_a = reach_a[flags][quarter * 32 + r], reaches[4] = {of_w.x, of_w.y, of_w.z, of_w.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n + j < g.N && of_a + reaches[j] > g.highest)
-                            v[j] = fma_sum(g.a + (size_t)m * g.K, g.w + (size_t)(n + j) * g.K, g.K);
+                    const int room = g.highest - reach_a[flags][quarter * 32 + r];
+                    const bool odd[4] = {of_w.x > room, of_w.y > room, of_w.z > room, of_w.w > room};
+                    const bool any = odd[0] || odd[1] || odd[2] || odd[3];
+                    if (any) {                                   // left for fma_tiles
+                        const int at = min((tile - (int)blockIdx.x) / (int)gridDim.x, 32 * ODD_WORDS - 1);
+                        ctl.odd = 1;
+                        atomicOr(&odd_tiles[at >> 5], 1u << (at & 31));
+                    }
                     float* dst = g.out + (size_t)m * g.N + n;
-                    if (g.wide) {                                // (N is a multiple of 4: all four are there)
+                    if (g.wide && !any) {                        // (N is a multiple of 4: all four are there)
                         if (g.bias != nullptr) {
 #pragma unroll
                             for (int j = 0; j < 4; ++j) v[j] += g.bias[n + j];
@@ -278,11 +386,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
                     } else {
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            if (n + j < g.N) {
-                                const float y = activate(v[j] + (g.bias != nullptr ? g.bias[n + j] : 0.f), g.epilogue);
-                                if (g.epilogue == EPI_RESIDUAL) dst[j] += y;
-                                else dst[j] = y;
-                            }
+                            if (n + j < g.N && !odd[j]) finish(g, v[j], n + j, dst + j);
                     }
                 }
             }
@@ -291,17 +395,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
         };
 
         int tile = blockIdx.x, slice = 0, flags = 0;             // of the step that is split
+        int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
         int was_tile = 0, was_slice = 0, was_flags = 0;          // of the step in front of it
-        if (steps > 0) fetch_w(wv, tile, 0);                     // the weights do not come from the kernel in front
+        if (steps > 0) fetch_w(wv, n0, 0);                       // the weights do not come from the kernel in front
         pdl_wait();
-        if (steps > 0) fetch_a(av, tile, 0);
+        if (steps > 0) fetch_a(av, m0, 0);
 #pragma unroll
         for (int i = 0; i < AC; ++i) most_a[i] = lost_a[i] = 0;
 #pragma unroll
         for (int i = 0; i < WC; ++i) most_w[i] = lost_w[i] = 0;
         for (long long i = 0; i < steps; ++i) {
             uint8_t* stage = smem + (int)(i & 1) * STAGE;
-            const int m0 = (tile % m_tiles) * TILE_M, n0 = (tile / m_tiles) * BN;
             if (ok) {
                 // (a row behind the last keeps what the place held: it gives results that nobody takes)
 #pragma unroll
@@ -318,27 +422,25 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
             if (++slice == slices) {                             // the tile's rows are known: eight lanes have each row
 #pragma unroll
                 for (int j = 0; j < AC; ++j) {
-                    most_a[j] = most_of(most_a[j], lost_a[j]);
-#pragma unroll
-                    for (int o = 1; o < 8; o <<= 1) most_a[j] = max(most_a[j], __shfl_xor_sync(0xffffffffu, most_a[j], o));
-                    if ((tid & 7) == 0) reach_a[flags][row8 + 64 * j] = (uint16_t)reach(most_a[j]);
+                    const uint32_t all = eight_lanes_max(reach(most_of(most_a[j], lost_a[j])));
+                    if ((tid & 7) == 0) reach_a[flags][row8 + 64 * j] = (uint16_t)all;
                     most_a[j] = lost_a[j] = 0;
                 }
 #pragma unroll
                 for (int j = 0; j < WC; ++j) {
-                    most_w[j] = most_of(most_w[j], lost_w[j]);
-#pragma unroll
-                    for (int o = 1; o < 8; o <<= 1) most_w[j] = max(most_w[j], __shfl_xor_sync(0xffffffffu, most_w[j], o));
-                    if ((tid & 7) == 0) reach_w[flags][row8 + 64 * j] = (uint16_t)reach(most_w[j]);
+                    const uint32_t all = eight_lanes_max(reach(most_of(most_w[j], lost_w[j])));
+                    if ((tid & 7) == 0) reach_w[flags][row8 + 64 * j] = (uint16_t)all;
                     most_w[j] = lost_w[j] = 0;
                 }
                 slice = 0;
                 tile += gridDim.x;
+                m0 = (tile % m_tiles) * TILE_M;
+                n0 = (tile / m_tiles) * BN;
                 if (++flags == FLAGS) flags = 0;
             }
             if (i + 1 < steps && ok) {
-                fetch_a(av, tile, slice);
-                fetch_w(wv, tile, slice);
+                fetch_a(av, m0, slice);
+                fetch_w(wv, n0, slice);
             }
             if (i > 0) add_up(i - 1, was_slice, was_tile, was_flags);
             was_tile = this_tile; was_slice = this_slice; was_flags = this_flags;
@@ -357,6 +459,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const SplitArgs 
     __syncthreads();
     tc_fence_after();
     if (warp == WORKERS / 32) tmem_dealloc(tmem_base, 2 * SUMS);
+    if (ctl.failed == 0 && ctl.odd != 0) fma_tiles(g, reinterpret_cast<float*>(smem), &reach_a[0][0], odd_tiles, m_tiles, my_tiles);
 }
 
 cudaError_t launch_tiles(const SplitArgs& g, cudaStream_t s) {
@@ -370,13 +473,6 @@ cudaError_t launch_tiles(const SplitArgs& g, cudaStream_t s) {
 constexpr int FEW_WARPS = 8, FEW_STAGES = 2, FEW_N = 16;    // rows of w per CTA: the m of m16n8k16
 constexpr int LINE = SLICE + 8;                              // words between rows in shared memory: 8-byte reads of 4 rows meet no bank twice
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool there) {
-    const uint32_t bytes = there ? 16u : 0u;                 // (0: sixteen zero bytes are written)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -389,7 +485,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
     constexpr int NR = FEW_N, STAGE = (NR + MT) * LINE;      // words of a warp's stage: w's slice, then a's
     constexpr int TB = MT / 8;
     extern __shared__ __align__(16) float few_smem[];
-    __shared__ uint32_t most_w[NR], most_a[MT];
+    __shared__ uint32_t reach_w[NR], reach_a[MT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float* ring = few_smem + warp * stages * STAGE;
     float* parts = few_smem + FEW_WARPS * stages * STAGE;    // [2][warp][MT][NR]
@@ -418,8 +514,8 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
     };
     pdl_trigger();
     for (int r = 0; r < stages && r < rounds; ++r) ask_w(r);                // the weights depend on no kernel before
-    if (tid < NR) most_w[tid] = 0;
-    if (tid >= 32 && tid < 32 + MT) most_a[tid - 32] = 0;
+    if (tid < NR) reach_w[tid] = 0;
+    if (tid >= 32 && tid < 32 + MT) reach_a[tid - 32] = 0;
     __syncthreads();
     pdl_wait();
     for (int r = 0; r < FEW_STAGES; ++r) {
@@ -451,7 +547,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
                 const float2 x = *reinterpret_cast<const float2*>(ws + (e & 1) * 8 * LINE + 16 * k + (e >> 1) * 8);
                 uint32_t p[PIECES];
                 split_pair(x.x, x.y, p, lost_w[e & 1]);
-                mine_w[e & 1] = larger(larger(mine_w[e & 1], x.x), x.y);
+                mine_w[e & 1] = larger(mine_w[e & 1], p[0]);
 #pragma unroll
                 for (int q = 0; q < PIECES; ++q) wp[q][e] = p[q];
             }
@@ -462,7 +558,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
                     const float2 x = *reinterpret_cast<const float2*>(as + b * 8 * LINE + 16 * k + e * 8);
                     uint32_t p[PIECES];
                     split_pair(x.x, x.y, p, lost_a[b]);
-                    mine_a[b] = larger(larger(mine_a[b], x.x), x.y);
+                    mine_a[b] = larger(mine_a[b], p[0]);
 #pragma unroll
                     for (int q = 0; q < PIECES; ++q) ap[q][b][e] = p[q];
                 }
@@ -484,11 +580,11 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
         for (int b = 0; b < TB; ++b)
 #pragma unroll
             for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][0][e] + (c[b][1][e] + c[b][2][e]);
-        if (r + 1 == rounds) {                                              // what each row's largest number is, over all warps
+        if (r + 1 == rounds) {                                              // what each row counts for, over all warps
 #pragma unroll
-            for (int e = 0; e < 2; ++e) atomicMax(&most_w[gr + 8 * e], most_of(mine_w[e], lost_w[e]));
+            for (int e = 0; e < 2; ++e) atomicMax(&reach_w[gr + 8 * e], reach(most_of(mine_w[e], lost_w[e])));
 #pragma unroll
-            for (int b = 0; b < TB; ++b) atomicMax(&most_a[gr + 8 * b], most_of(mine_a[b], lost_a[b]));
+            for (int b = 0; b < TB; ++b) atomicMax(&reach_a[gr + 8 * b], reach(most_of(mine_a[b], lost_a[b])));
         }
         // (one barrier a round: the half written two rounds later was read before the barrier in between)
         __syncthreads();
@@ -496,14 +592,53 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
         if (tid < MT * NR)
             for (int s = 0; s < here; ++s) total += parts[(r & 1) * FEW_WARPS * MT * NR + s * MT * NR + tid];
     }
-    cp_async_wait<0>();
     const int m = tid / NR, n = n0 + tid % NR;
-    if (tid >= MT * NR || m >= M || n >= N) return;
-    if (reach(most_a[m]) + reach(most_w[tid % NR]) > g.highest) total = fma_sum(g.a + (size_t)m * K, g.w + (size_t)n * K, K);
-    const float y = activate(total + (g.bias != nullptr ? g.bias[n] : 0.f), g.epilogue);
-    float* dst = g.out + (size_t)m * N + n;
-    if (g.epilogue == EPI_RESIDUAL) *dst += y;
-    else *dst = y;
+    const bool mine = tid < MT * NR && m < M && n < N;
+    const bool odd = mine && (int)(reach_a[m] + reach_w[tid % NR]) > g.highest;
+    if (__syncthreads_or(odd)) {                                            // the rounds once more, by fused multiply-adds
+        constexpr int NB = NR / 8, MB = MT / 4;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int r = 0; r < rounds; ++r) {
+            ask_w(r);
+            ask_a(r);
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncwarp();
+            const float* ws = ring + (r & (stages - 1)) * STAGE + (lane & 7) * LINE;
+            const float* as = ring + (r & (stages - 1)) * STAGE + (NR + (lane >> 3)) * LINE;
+            float acc[MB][NB];
+#pragma unroll
+            for (int i = 0; i < MB; ++i)
+#pragma unroll
+                for (int j = 0; j < NB; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+            for (int k = 0; k < SLICE; k += 4) {
+                float4 wv[NB];
+#pragma unroll
+                for (int j = 0; j < NB; ++j) wv[j] = *reinterpret_cast<const float4*>(ws + 8 * j * LINE + k);
+#pragma unroll
+                for (int i = 0; i < MB; ++i) {
+                    const float4 av = *reinterpret_cast<const float4*>(as + 4 * i * LINE + k);
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) acc[i][j] = dot4(av, wv[j], acc[i][j]);
+                }
+            }
+            __syncwarp();
+            float* part = parts + (r & 1) * FEW_WARPS * MT * NR;            // (one barrier a round, as above)
+#pragma unroll
+            for (int i = 0; i < MB; ++i)
+#pragma unroll
+                for (int j = 0; j < NB; ++j) part[(warp * MT + (lane >> 3) + 4 * i) * NR + (lane & 7) + 8 * j] = acc[i][j];
+            __syncthreads();
+            const int here = min(FEW_WARPS, slices - r * FEW_WARPS);
+            if (tid < MT * NR)
+                for (int s = 0; s < here; ++s) sum += part[s * MT * NR + tid];
+        }
+        if (odd) total = sum;
+    }
+    if (!mine) return;
+    finish(g, total, n, g.out + (size_t)m * N + n);
 }
 
 template <int MT>
@@ -531,7 +666,7 @@ MG_API int mg_linear_split(const float* a, const float* w, const float* bias, fl
     MG_REQUIRE(status != nullptr, "linear: missing status word");
     if (K % 4 != 0 || (((uintptr_t)a | (uintptr_t)w) & 15))
         return mg_set_error(MG_ERR_UNSUPPORTED, "linear: 32-bit tensor-core path needs K %% 4 == 0 and 16-byte aligned operands");
-    SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, (uint32_t)highest_reach(K), status};
+    SplitArgs g = {a, w, bias, epilogue == EPI_RESIDUAL ? residual : out, M, N, K, epilogue, 0, highest_reach(K), status};
     g.wide = N % 4 == 0 && ((uintptr_t)g.out & 15) == 0;
     MG_REQUIRE((long long)ceil_div(M, TILE_M) * ceil_div(N, BN) < (1ll << 30), "linear: too many tiles");
     cudaStream_t s = (cudaStream_t)stream;

@@ -1066,6 +1066,59 @@ def test_32_bit_products_near_the_ends_of_the_range(ops, m, n, k):
     assert ((got.double() - ref).abs() <= torch.maximum(bound, by_fma))[finite].all()
 
 
+@pytest.mark.parametrize("n,k", [(4100, 68), (4101, 260)])
+def test_32_bit_products_of_many_tiles_with_rows_that_do_not_split(ops, n, k):
+    """Four tiles of 128 x 64 a CTA, so that the sets of marks are used again, with such rows in several of them: those results are the
+    FMA tiles' to the bit, added into a residual stream once, and all others what they are without such rows."""
+    m = 1030
+    x, w, b = randn(m, k, seed=61), randn(n, k, seed=62), randn(n, seed=63)
+    clean = ops.linear(x, w, b, "none", torch.float32)
+    xs, ws = [0, 127, 300, 640, 1029], [5, 1000, 2047, 4099]
+    for i, r in enumerate(xs):
+        x[r, (37 * i) % k] = (float("nan"), float("inf"), 1e-37, 3e38, -float("inf"))[i]
+    for i, r in enumerate(ws):
+        w[r, (11 * i) % k] = (float("nan"), 2e-38, 1.7e38, -float("inf"))[i]
+    res = randn(m, n, seed=64)
+    got, added = ops.linear(x, w, b, "none", torch.float32), res.clone()
+    ops.linear_residual(x, w, b, added)
+    ops.use_split = False
+    try:
+        want = ops.linear(x, w, b, "none", torch.float32)
+    finally:
+        ops.use_split = True
+    ops.check_status()
+    odd = torch.zeros(m, n, dtype=torch.bool, device="cuda")
+    odd[xs], odd[:, ws] = True, True
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.isnan(want).any()
+    assert torch.equal(got[odd].nan_to_num(7.0), want[odd].nan_to_num(7.0)) and torch.equal(got[~odd], clean[~odd])
+    assert torch.equal(added.nan_to_num(7.0), (res + got).nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("m", [8, 128])
+def test_32_bit_products_of_rows_that_do_not_split_take_no_age(ops, m):
+    """Inputs that hold what is no number take a second walk over the operands, not a chain of dependent loads for each result
+    (2 to 5 times the usual time; 14 and 69 times it so)."""
+    n, k = 512, 2048
+    x, w, out = randn(m, k, seed=71), randn(n, k, seed=72), torch.empty(m, n, device="cuda")
+
+    def microseconds():
+        best = float("inf")
+        for _ in range(8):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            start.record()
+            for _ in range(20):
+                ops.linear(x, w, None, "none", torch.float32, out=out)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end) * 1e3 / 20)
+        return best
+
+    usual = microseconds()
+    x[:, 3] = float("nan")
+    assert microseconds() < 10 * max(usual, 5.0) and torch.isnan(out).all()
+
+
 @pytest.mark.parametrize("single", [False, True], ids=["portions", "single"])
 @pytest.mark.parametrize("n_head,n_kv_head,head_dim,page_tokens,window", [
     (4, 4, 128, 64, 0), (6, 2, 104, 16, 0), (5, 1, 48, 4, 0), (4, 4, 80, 24, 70), (2, 2, 96, 16, 0), (64, 1, 8, 8, 0),
