@@ -1,13 +1,15 @@
 // out[m, n] = sum_k a[m, k] * w[n, k] (+ bias[n]) with an epilogue, in 32 bits, on the tensor cores.
 //
-// A 32-bit number is the sum of three bfloat16 numbers, exactly: its 24 bits are rounded to 8 three times, x = h + m + l with
-// |m| <= 2^-9 |h| and |l| <= 2^-18 |h|.  Products of bfloat16 numbers are exact in the tensor cores, so a product of two such sums is
-// six of theirs, h l', l h', m m', h m', m h' and h h'; the three that are left out are below 2^-27 of it.  What rounds is the
-// accumulator: it drops what lies below its last place at every addition of 16 products.  So K is cut into slices of 64, and a
-// slice's products go into three accumulators: those of h h', those of h m' and m h', and the other three, each some 2^8 below the
-// one before.  A slice's sum, h h' + (the second + the third), is added to those before it; these are ordinary rounded additions.
-// Errors against 64 bits, of the result's size, chains of fused multiply-adds and this: 512 terms 15.7e-8 and 9.3e-8, 2,048 terms
-// 18.1e-8 and 12.9e-8 (in one accumulator, the small products first: 9.9e-8 and 13.4e-8).
+// A 32-bit number down to 2^-109 is the sum of three bfloat16 numbers, exactly: its 24 bits are rounded to 8 three times, x = h + m + l
+// with |m| <= 2^-8 |h| and |l| <= 2^-17 |h|.  Products of bfloat16 numbers are exact in the tensor cores, so a product of two such
+// sums is nine of theirs; l l', below 2^-33 of it, is left out.  What rounds is the accumulator: it drops what lies below its last place
+// at every addition of 16 products, where an ordinary addition rounds, so sums of one sign come out too small.  So K is cut into
+// slices of 64, and of a slice's h h' only two such additions follow each other: its halves have an accumulator each.  The other
+// seven products, which are 2^8 and more below, have two of their own (see ACCUMULATORS).  The four meet, and a slice's sum is
+// added to those before it, in ordinary rounded additions; a single product is rounded once.
+// Errors against 64 bits, of the result's size and in 1e-8, chains of fused multiply-adds and this: numbers of both signs, 64 terms
+// 14.4 and 5.4, 512 terms 15.5 and 7.8, 2,048 terms 17.9 and 11.9, 6,400 terms 23.2 and 19.0; of one sign 12.2 and 5.9, 6.6 and 6.4,
+// 9.2 and 9.8, 13.4 and 13.8 (with all four additions of h h' in one accumulator 9.0, 9.3, 11.9 and 15.4).
 //
 // Every element is summed in that one order whatever the number of rows and the kernel or tile that it falls in, so a token's
 // result does not depend on what else is in the batch (mma.sync and tcgen05.mma give the same bits; so do the two orders of the operands).
@@ -21,14 +23,15 @@
 // Two kernels:
 //   gemm_split_kernel   tiles of 128 rows x 64 columns by tcgen05.  Sixteen warps read both operands of a slice from global memory
 //                       (a slice ahead, in registers), split them, and lay the pieces into shared memory in the 128-byte swizzle,
-//                       the three of w's rows one behind the other, so that h, m and l of a's meet 3, 2 and 1 of them in one
-//                       instruction each.  A thread of the 17th warp issues the 12 products of a slice; the sixteen then take
-//                       the sums out of TMEM and add them to the totals in their registers, beside the next slice's products.
+//                       the three of w's rows one behind the other.  A thread of the 17th warp issues the 18 products of a slice;
+//                       the sixteen then take the sums out of TMEM and add them to the totals in their registers, beside the
+//                       next slice's products.
 //   gemm_split_few_kernel   up to 16 rows: a CTA takes 16 rows of w, each of its eight warps every eighth slice, operands by cp.async in
 //                       a ring of the warp's own (the first round of w before the wait for the kernel in front); the fragments
 //                       of mma.sync are split as they are read.  Bound by reading w and by the latency of a launch and a slice.
-// 2,048 rows, FMA tiles and these: 1,536 x 512 101 and 42 us, 2,048 x 512 123 and 54, 512 x 2,048 142 and 48; 8 rows (FMA and mma.sync):
-// 1,536 x 512 3.3 and 3.6, 512 x 2,048 7.5 and 6.9, 50,304 x 512 32.5 and 31.5; 16 rows 49.7 and 47.1.
+// 2,048 rows, FMA tiles and these: 1,536 x 512 102 and 43 us, 2,048 x 512 124 and 56, 512 x 2,048 143 and 48; 17 rows (FMA tiles of 64 rows)
+// 25.5 and 13.9, 25.8 and 14.0, 93.9 and 40; 8 rows (FMA and mma.sync) 3.3 and 3.5, 4.0 and 3.9, 7.6 and 7.1, 50,304 x 512 32.6 and 32.6; 16 rows
+// 4.4 and 4.0, 4.9 and 4.4, 10.7 and 9.7, 50.0 and 49.6.  (1,536 x 512 at 8 rows is the price of the same bits in both kernels.)
 #include "blackwell.cuh"
 
 #define EPI_STORE 0      // out = acc + bias
@@ -40,6 +43,13 @@ namespace {
 
 constexpr int SLICE = 64;            // terms summed by the tensor cores in one go: a 128-byte row of bfloat16
 constexpr int PIECES = 3;
+static_assert(SLICE == 64, "four steps of 16");
+
+// The accumulators of a slice: h h' of its second half, those of its first, and for each of its four steps of 16 terms, in this order,
+// h m', m h', m m', l h' in the third and h l', m l', l m' in the fourth.
+constexpr int ACCUMULATORS = 4;
+__device__ __forceinline__ constexpr int accumulator(int q, int v) { return 1 + (q == 0 ? v : q == 1 ? (v == 2 ? 2 : 1) : v + 1); }
+__device__ __forceinline__ float slice_sum(float second, float first, float rest, float below) { return (first + second) + (rest + below); }
 
 // The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third's upper half is all of it, as long
 // as it does not fall below bfloat16's least number: what is cut off then shows in the low half of `lost`.
@@ -116,8 +126,11 @@ __device__ __forceinline__ void finish(const SplitArgs& g, float sum, int n, flo
 
 // ---- tiles -----------------------------------------------------------------------------------------------
 // A slice takes 1.45 us, 1.1 with few rows: the operands of the next one come from L2 (48 KB) while a slice is split, and the splitting
-// itself is 24 numbers a thread.  Tiles of 32 columns take the same time a slice (512 x 2,048, 128 rows: 48 and 46 us).  In the form
-// with one accumulator, six instructions for the six products and a worker that issued them as well, a slice took 2.05 us.
+// itself is 24 numbers a thread.  Tiles of 32 columns take the same time a slice (512 x 2,048, 128 rows: 48 and 46 us).  With a worker
+// that issued the products as well, a slice took 2.05 us.  Eight products and four accumulators, in the place of six and three, cost
+// 2 to 3 % (42 -> 43, 47 -> 48 us), and 4 to 5 % among a model's other kernels (43.2 -> 45.1, 60.9 -> 63.3, 49.9 -> 52.4 us): what a worker
+// does for a slice counts, and how long the products take (in 30 instructions of 64 columns 9 %).  The sums are taken out four columns
+// at a time: eight want more registers than there are (52 us for 48).
 constexpr int TILE_M = 128, BN = 64;
 constexpr int WORKERS = 512;         // threads that split and add up
 constexpr int THREADS = WORKERS + 32;
@@ -132,10 +145,9 @@ constexpr int DYNAMIC_BYTES = 1024 + 2 * STAGE + (WORKERS / 32) * OUT_BYTES;
 constexpr int CW = BN / 4;           // results a worker has
 constexpr int ODD_WORDS = 64;        // marks of tiles with results for the multiply-adds: a CTA's tiles from the 2,048th on share the last one
 
-__device__ __forceinline__ void tmem_load_8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr) : "memory");
+__device__ __forceinline__ void tmem_load_4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
 
 // The results that the pieces do not serve, of the tiles that are marked, by fused multiply-adds.  All threads of the CTA, behind its last tile.
@@ -230,7 +242,7 @@ struct __align__(16) SplitControl {
 __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ SplitArgs g) {
     constexpr int A_PLANE = TILE_M * ROW_BYTES, W_PLANE = BN * ROW_BYTES;
     constexpr int AC = TILE_M * 8 / WORKERS, WC = BN * 8 / WORKERS;      // 8-number pieces of rows a thread splits
-    constexpr int SUMS = 256;               // columns of TMEM for a slice's sums, of which 3 BN are used
+    constexpr int SUMS = ACCUMULATORS * BN;  // columns of TMEM for a slice's sums
     extern __shared__ uint8_t split_smem[];
     __shared__ SplitControl ctl;
     __shared__ uint32_t odd_tiles[ODD_WORDS];
@@ -272,12 +284,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 tc_fence_after();
                 const uint64_t desc_a = desc0 + (uint64_t)(half * (STAGE >> 4)), desc_w = desc_a + (uint64_t)((PIECES * A_PLANE) >> 4);
                 const uint32_t d = tmem_base + half * SUMS;
+                // columns 16 k .. of a's piece q, of w's piece v and the n - 1 behind it, for the accumulators from `sums` on
+                auto products = [&](int k, int q, int v, int n, int sums, bool add) {
+                    umma_bf16(d + sums * BN, desc_a + (uint64_t)((q * A_PLANE + k * 32) >> 4), desc_w + (uint64_t)((v * W_PLANE + k * 32) >> 4),
+                              instr_desc_bf16(TILE_M, n * BN), add ? 1u : 0u);
+                };
 #pragma unroll
-                for (int k = 0; k < SLICE / 16; ++k)
-#pragma unroll
-                    for (int q = 0; q < PIECES; ++q)         // piece q of a meets pieces 0 .. 2 - q of w: sums q ..
-                        umma_bf16(d + q * BN, desc_a + (uint64_t)((q * A_PLANE + k * 32) >> 4), desc_w + (uint64_t)((k * 32) >> 4),
-                                  instr_desc_bf16(TILE_M, (PIECES - q) * BN), (k | q) != 0 ? 1u : 0u);
+                for (int k = 0; k < SLICE / 16; ++k) {
+                    if (k < SLICE / 32) {
+                        products(k, 0, 0, 3, 1, k != 0);
+                    } else {
+                        products(k, 0, 0, 1, 0, k != SLICE / 32);
+                        products(k, 0, 1, 2, 2, true);
+                    }
+                    products(k, 1, 0, 1, 2, true);
+                    products(k, 1, 1, 2, 2, true);
+                    products(k, 2, 0, 2, 2, true);
+                }
                 umma_commit(smem_u32(&ctl.done[half]));
             }
             if (!there) {
@@ -330,13 +353,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             if (ok) {
                 tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < CW; c += 8) {
-                    uint32_t r[PIECES][8];
+                for (int c = 0; c < CW; c += 4) {
+                    uint32_t r[ACCUMULATORS][4];
 #pragma unroll
-                    for (int q = 0; q < PIECES; ++q) tmem_load_8(sums_at + half * SUMS + q * BN + c, r[q]);
+                    for (int q = 0; q < ACCUMULATORS; ++q) tmem_load_4(sums_at + half * SUMS + q * BN + c, r[q]);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) total[c + j] += __uint_as_float(r[0][j]) + (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j]));
+                    for (int j = 0; j < 4; ++j)
+                        total[c + j] += slice_sum(__uint_as_float(r[0][j]), __uint_as_float(r[1][j]), __uint_as_float(r[2][j]), __uint_as_float(r[3][j]));
                 }
                 tc_fence_before();
             }
@@ -481,7 +505,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 
 // MT rows of a: 8 or 16.
 template <int MT>
-__global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const SplitArgs g, int stages) {
+__global__ void __launch_bounds__(32 * FEW_WARPS, MT == 8 ? 3 : 2) gemm_split_few_kernel(const SplitArgs g, int stages) {
     constexpr int NR = FEW_N, STAGE = (NR + MT) * LINE;      // words of a warp's stage: w's slice, then a's
     constexpr int TB = MT / 8;
     extern __shared__ __align__(16) float few_smem[];
@@ -532,11 +556,11 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
         __syncwarp();
         const float* ws = ring + (r & (stages - 1)) * STAGE + gr * LINE + t2;
         const float* as = ws + NR * LINE;
-        float c[TB][PIECES][4];                                             // the three accumulators
+        float c[TB][ACCUMULATORS][4];
 #pragma unroll
         for (int b = 0; b < TB; ++b)
 #pragma unroll
-            for (int q = 0; q < PIECES; ++q)
+            for (int q = 0; q < ACCUMULATORS; ++q)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) c[b][q][e] = 0.f;
 #pragma unroll
@@ -565,9 +589,11 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
 #pragma unroll
             for (int q = 0; q < PIECES; ++q)                                // (a's piece, w's piece: in the order of the tiles)
 #pragma unroll
-                for (int v = 0; v + q < PIECES; ++v)
+                for (int v = 0; v < PIECES; ++v) {
+                    if (q + v > PIECES) continue;
 #pragma unroll
-                    for (int b = 0; b < TB; ++b) mma_bf16(c[b][q + v], wp[v], ap[q][b][0], ap[q][b][1]);
+                    for (int b = 0; b < TB; ++b) mma_bf16(c[b][q + v == 0 && k >= SLICE / 32 ? 0 : accumulator(q, v)], wp[v], ap[q][b][0], ap[q][b][1]);
+                }
         }
         __syncwarp();
         if (r + stages < rounds) {
@@ -579,7 +605,7 @@ __global__ void __launch_bounds__(32 * FEW_WARPS) gemm_split_few_kernel(const Sp
 #pragma unroll
         for (int b = 0; b < TB; ++b)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = c[b][0][e] + (c[b][1][e] + c[b][2][e]);
+            for (int e = 0; e < 4; ++e) part[(8 * b + t2 + (e & 1)) * NR + gr + 8 * (e >> 1)] = slice_sum(c[b][0][e], c[b][1][e], c[b][2][e], c[b][3][e]);
         if (r + 1 == rounds) {                                              // what each row counts for, over all warps
 #pragma unroll
             for (int e = 0; e < 2; ++e) atomicMax(&reach_w[gr + 8 * e], reach(most_of(mine_w[e], lost_w[e])));

@@ -1066,6 +1066,41 @@ def test_32_bit_products_near_the_ends_of_the_range(ops, m, n, k):
     assert ((got.double() - ref).abs() <= torch.maximum(bound, by_fma))[finite].all()
 
 
+@pytest.mark.parametrize("m", [16, 256])
+def test_32_bit_products_hold_all_bits_of_their_inputs(ops, m):
+    """A result of one product is that product, rounded once: h h' is exact in its accumulator, and what lies below (the cut of
+    the rest, 2^-31 of the product at most, and l l') moves the rounding by less than a thirtieth of its half place."""
+    n, k = 96, 132
+    g = torch.Generator(device="cuda").manual_seed(81)
+    w = 1.0 + 2.0 ** -8 + 2.0 ** -14 * torch.randn(n, k, generator=g, device="cuda")       # (where m m' and m l' are largest)
+    w[n // 2:] = randn(n - n // 2, k, seed=82)
+    x = torch.zeros(m, k, device="cuda")
+    at = torch.arange(m, device="cuda") % k
+    x[torch.arange(m, device="cuda"), at] = 1.0 + 2.0 ** -8 + 2.0 ** -14 * torch.randn(m, generator=g, device="cuda")
+    want = x.double() @ w.double().T
+    got = ops.linear(x, w, None, "none", torch.float32)
+    assert ((got.double() - want).abs() <= 2.0 ** -24 * (1 + 1 / 30) * want.abs()).all()
+
+
+@pytest.mark.parametrize("k", [64, 512])
+def test_32_bit_sums_of_one_sign_are_no_further_off_than_multiply_adds(ops, k):
+    """The tensor cores cut where an addition rounds, so sums of numbers of one sign come out too small, by as much in every slice: few
+    such additions may follow each other among a slice's largest products."""
+    x, w = randn(512, k, seed=91).abs(), randn(256, k, seed=92).abs()
+    want = x.double() @ w.double().T
+
+    def error():
+        return float((ops.linear(x, w, None, "none", torch.float32).double() - want).norm() / want.norm())
+
+    here = error()
+    ops.use_split = False
+    try:
+        by_fma = error()
+    finally:
+        ops.use_split = True
+    assert here <= 1.05 * by_fma
+
+
 @pytest.mark.parametrize("n,k", [(4100, 68), (4101, 260)])
 def test_32_bit_products_of_many_tiles_with_rows_that_do_not_split(ops, n, k):
     """Four tiles of 128 x 64 a CTA, so that the sets of marks are used again, with such rows in several of them: those results are the
