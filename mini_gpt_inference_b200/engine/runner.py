@@ -576,6 +576,7 @@ class ModelRunner:
         if hasattr(self.ops, "launches"):
             self.ops.launches += state.kernels
         if state.head is not None:
+            self._begin()                                 # (what ran last, a head or another model's pass, is not in front of it)
             return self.model.head.forward(*state.head)
         if state.logits is None:
             return None

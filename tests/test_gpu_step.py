@@ -185,6 +185,59 @@ def test_head_behind_a_replayed_step(which, dtype):
         assert_close(got, plain_logits(cfg, tensors, tokens), tol, "the head behind a replayed step")
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_no_matrix_is_said_to_follow_the_head_of_a_replayed_step(dtype):
+    """A head behind a replayed step follows nothing that the kernel set saw: a hint from whatever ran last, the head of the replay
+    before it or another model's matrix, would have later steps ask the wrong matrix into L2."""
+    cfg, tensors, runner, tol = _setup("A", dtype, False)
+    other = _setup("B", dtype, False)
+    runner.HEAD_APART_BYTES, runner.HEAD_APART_ROWS = 0, 2
+    ops, head, n = runner.ops, runner.model.head.embedding.weight, cfg.n_positions - 1
+    assert other[2].ops is ops                                            # (models of a device share it)
+    for rep in range(4):
+        if rep == 3:
+            other[2].step([StepEntry("o", tokens_for(other[0], 9, 1), [8])])      # another model's pass in between
+            last = ops._last_weight
+        ops._next_weight.clear()
+        tokens = tokens_for(cfg, n, 90 + rep)
+        got = runner.step([StepEntry("r", tokens, list(range(n)))])
+        if rep >= 2:
+            assert head.data_ptr() not in ops._next_weight and not ops._next_weight        # a replay and its head: no hint at all
+        if rep < 3:
+            runner.finish("r")
+    assert runner.shape_graph_replays == 2 and last is not None
+    # and a decode step behind it is right
+    more = runner.step([StepEntry("r", [5], [0])])
+    want = plain_logits(cfg, tensors, tokens + [5])
+    assert_close(torch.cat([got, more]), want, tol, "a decode step behind a replayed step's head")
+
+
+@pytest.mark.parametrize("family,which", [("fakilorn", "A"), ("nogatar", "A"), ("nogatar", "B")])
+def test_other_heads_behind_a_replayed_step(family, which):
+    """Heads with a scale and heads of their own matrix with a cap, behind replayed steps and with decode steps after them."""
+    import importlib
+
+    from mini_gpt_inference_b200 import FakilornConfig, NogatarConfig
+    from mini_gpt_inference_b200.engine.build import load_model, make_runner
+    from mini_gpt_inference_b200.kernels.ops import default_ops
+
+    cases = importlib.import_module(f"{family}_cases")
+    raw = cases.config(which)
+    tensors = cases.random_weights(raw, 5)
+    kind = {"fakilorn": FakilornConfig, "nogatar": NogatarConfig}[family]
+    loaded = load_model(config=kind.from_dict(raw), tensors=tensors, dtype="float32", device="cuda:0")
+    runner = make_runner(loaded, default_ops("cuda:0"), 8, 40, 2)
+    runner.HEAD_APART_BYTES, runner.HEAD_APART_ROWS = 0, 2
+    n = 67
+    for rep in range(4):
+        tokens = cases.tokens_for(raw, n + 2, 60 + rep)
+        got = [runner.step([StepEntry("r", tokens[:n], list(range(n)))])]
+        got += [runner.step([StepEntry("r", tokens[t: t + 1], [0])]) for t in (n, n + 1)]
+        runner.finish("r")
+        cases.assert_rows_close(torch.cat(got), cases.plain_logits(raw, tensors, tokens), 3e-4, f"{family} {which}, pass {rep}")
+    assert runner.shape_graph_replays == 2
+
+
 def test_captured_shapes_are_bounded():
     cfg, tensors, runner, tol = _setup("A", "bfloat16", False)
     runner.SHAPE_GRAPHS = 3
