@@ -811,6 +811,50 @@ def test_experts_of_few_tokens(ops, monkeypatch, n, width, inner, experts, top, 
     assert (few - want).abs().max() <= 2e-2
 
 
+@pytest.mark.parametrize("n,width,inner,experts,top", [(4, 1024, 1024, 9, 3), (16, 264, 72, 3, 3), (1, 2048, 136, 8, 2)])
+def test_experts_of_few_tokens_started_ahead(ops, monkeypatch, n, width, inner, experts, top):
+    """In a captured step the second product's kernel starts, and reads the ids, before the first has ended.  Layer after layer, with ids
+    that change from replay to replay (padding, experts without a token, all tokens at one expert): the bits of kernels that
+    run one after the other."""
+    g = torch.Generator().manual_seed(n + width)
+    layers = 3
+    y = randn(n, width, dtype=torch.bfloat16, seed=44)
+    w_in = [randn(experts, 2 * inner, width, dtype=torch.bfloat16, seed=45 + i, scale=1 / math.sqrt(width)) for i in range(layers)]
+    w_out = [randn(experts, width, inner, dtype=torch.bfloat16, seed=55 + i, scale=1 / math.sqrt(inner)) for i in range(layers)]
+    ids = [torch.zeros(n, top, dtype=torch.int32, device="cuda") for _ in range(layers)]
+    weights, residual = torch.rand(n, top, generator=g).cuda(), torch.zeros(n, width, device="cuda")
+    monkeypatch.setattr(type(ops), "_moe_few_pays", staticmethod(lambda *sizes: True))
+
+    def run():
+        ops.scale_(residual, 0.0)
+        for i in range(layers):
+            ops.moe_experts_residual(y, ids[i], weights, w_in[i], w_out[i], residual, "silu", 7.0, True, False)
+
+    run()
+    torch.cuda.synchronize()
+    graph, launches = torch.cuda.CUDAGraph(), ops.launches
+    ops.set_dependent_launch(True)
+    try:
+        with torch.cuda.graph(graph):
+            run()
+    finally:
+        ops.set_dependent_launch(False)
+    assert ops.launches == launches + 1 + 3 * layers
+    for turn in range(6):
+        for i in range(layers):
+            chosen = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(n)]).to(torch.int32)
+            if turn % 3 == 1:
+                chosen[-1] = -1
+            if turn % 3 == 2:
+                chosen[:] = (turn + i) % experts
+            ids[i].copy_(chosen)
+        run()
+        want = residual.clone()
+        for _ in range(3):
+            graph.replay()
+            assert torch.equal(residual, want), turn
+
+
 def _attention_case(ops, dtype, n_head, n_kv_head, head_dim, page_tokens, window, lengths, q_lens,
                     seed=0, spike=None, portions=False):
     """Requests with `lengths[i]` tokens in total, of which the last `q_lens[i]` are new.
@@ -1005,7 +1049,7 @@ def test_32_bit_products_do_not_hang_on_the_rows_beside_them(ops, n, k):
 @pytest.mark.parametrize("m", [1, 8, 9, 16, 17, 130])
 @pytest.mark.parametrize("n,k", [(130, 260), (33, 64), (64, 68), (1540, 1032), (5, 4)])
 def test_32_bit_products_by_bfloat16_pieces(ops, m, n, k):
-    """Tiles of 32 to 128 columns and the kernel of a few rows at their edges: no further from the 64-bit result than what a
+    """Tiles of 128 x 64 and the kernel of a few rows at their edges: no further from the 64-bit result than what a
     32-bit sum of k terms may be off, as far as the FMA tiles with what is no number, infinite, huge or tiny, and by the
     same sums as those where a row holds such numbers."""
     x, w, b = randn(m, k, seed=41), randn(n, k, seed=42), randn(n, seed=43)
