@@ -8,8 +8,8 @@
 // seven products, which are 2^8 and more below, have two of their own (see ACCUMULATORS).  The four meet, and a slice's sum is
 // added to those before it, in ordinary rounded additions; a single product is rounded once.
 // Errors against 64 bits, of the result's size and in 1e-8, chains of fused multiply-adds and this: numbers of both signs, 64 terms
-// 14.4 and 5.4, 512 terms 15.5 and 7.8, 2,048 terms 17.9 and 11.9, 6,400 terms 23.2 and 19.0; of one sign 12.2 and 5.9, 6.6 and 6.4,
-// 9.2 and 9.8, 13.4 and 13.8 (with all four additions of h h' in one accumulator 9.0, 9.3, 11.9 and 15.4).
+// 14.4 and 5.1, 512 terms 15.5 and 7.6, 2,048 terms 17.9 and 11.8, 6,400 terms 23.2 and 19.1; of one sign 12.2 and 5.5, 6.6 and 6.4,
+// 9.2 and 9.8, 13.4 and 13.9 (with all four additions of h h' in one accumulator 9.0, 9.3, 11.9 and 15.4).
 //
 // Every element is summed in that one order whatever the number of rows and the kernel or tile that it falls in, so a token's
 // result does not depend on what else is in the batch (mma.sync and tcgen05.mma give the same bits; so do the two orders of the operands).
@@ -49,7 +49,7 @@ static_assert(SLICE == 64, "four steps of 16");
 // h m', m h', m m', l h' in the third and h l', m l', l m' in the fourth.
 constexpr int ACCUMULATORS = 4;
 __device__ __forceinline__ constexpr int accumulator(int q, int v) { return 1 + (q == 0 ? v : q == 1 ? (v == 2 ? 2 : 1) : v + 1); }
-__device__ __forceinline__ float slice_sum(float second, float first, float rest, float below) { return (first + second) + (rest + below); }
+__device__ __forceinline__ float slice_sum(float second, float first, float rest, float below) { return first + (second + (rest + below)); }
 
 // The pieces of two neighbouring numbers, as pairs of bfloat16 (x in the low half).  The third's upper half is all of it, as long
 // as it does not fall below bfloat16's least number: what is cut off then shows in the low half of `lost`.
